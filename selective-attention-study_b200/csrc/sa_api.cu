@@ -80,6 +80,7 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   p->out_lowp = nullptr;
   p->out_lowp_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
   p->dv_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
+  p->dk_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
   p->external_selector = (sel != nullptr);
   if (sel != nullptr) {
     p->q0 = Strided{sel->q0, sel->q0_stride[0], 0, sel->q0_stride[1]};
@@ -91,23 +92,33 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   return SA_OK;
 }
 
+// Tensor-core engine: dq_acc (all heads), dk0 (the selecting head), the row statistics, dO in bf16.  CUDA-core engine:
+// dq_acc, dk_acc, dq0, dk0, dbar, dO in fp32.
 struct BackwardWorkspace {
-  size_t dq_acc, dk_acc, dq0, dk0, dbar, d_out_lowp, total;
+  size_t dq_acc, dk_acc, dq0, dk0, stats, d_out, total;
 };
 
 BackwardWorkspace carve(const sa_problem* in) {
-  const size_t rows = (size_t)in->batch * in->heads * in->seq;
+  const bool tensor_core = in->engine == SA_ENGINE_TCGEN05;
+  const size_t nrows = (size_t)in->batch * in->heads;
+  const size_t rows = nrows * in->seq, padded = nrows * ((size_t)(in->seq + 127) / 128 * 128);
   const size_t elems = rows * in->head_dim;
   const size_t elems0 = (size_t)in->batch * in->seq * in->head_dim;
   BackwardWorkspace w{};
   size_t off = 0;
-  w.dq_acc = off; off = align_up(off + elems * 4, 256);
-  w.dk_acc = off; off = align_up(off + elems * 4, 256);
-  w.dq0 = off; off = align_up(off + elems0 * 4, 256);
-  w.dk0 = off; off = align_up(off + elems0 * 4, 256);
-  w.dbar = off; off = align_up(off + rows * 4, 256);
-  w.d_out_lowp = off;   // d_out converted for the engine: bf16/fp16 (tensor-core) or fp32 (CUDA-core)
-  off = align_up(off + elems * (in->engine == SA_ENGINE_TCGEN05 ? 2 : 4), 256);
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off = align_up(off + bytes, 256);
+    return at;
+  };
+  w.dq_acc = take(elems * 4);
+  if (!tensor_core) {
+    w.dk_acc = take(elems * 4);
+    w.dq0 = take(elems0 * 4);
+  }
+  w.dk0 = take(elems0 * 4);
+  w.stats = take(tensor_core ? padded * 8 : rows * 4);
+  w.d_out = take(elems * (tensor_core ? 2 : 4));
   w.total = off;
   return w;
 }
@@ -398,53 +409,59 @@ int backward_common(const sa_problem* in, const void* q, const void* k, const vo
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* base = static_cast<char*>(workspace);
   float* dq_acc = reinterpret_cast<float*>(base + w.dq_acc);
-  float* dk_acc = reinterpret_cast<float*>(base + w.dk_acc);
-  float* dq0 = reinterpret_cast<float*>(base + w.dq0);
   float* dk0 = reinterpret_cast<float*>(base + w.dk0);
-  float* dbar = reinterpret_cast<float*>(base + w.dbar);
+  float* stats = reinterpret_cast<float*>(base + w.stats);
   const int64_t rows = (int64_t)p.batch * p.heads * p.seq;
-  const int64_t per_head = (int64_t)p.seq * p.head_dim;
-  const size_t elems = (size_t)rows * p.head_dim;
-  const size_t elems0 = (size_t)p.batch * per_head;
-
-  // dq_acc, dq0 and dk0 are accumulated with atomics and start at zero (the workspace's dq0/dk0 pair is contiguous).
-  SA_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, elems * 4, s));
-  if (sel != nullptr) {            // the selector's gradients go to the caller, unfolded
-    dq0 = dq0_out;
-    dk0 = dk0_out;
-    SA_CUDA_CHECK(cudaMemsetAsync(dq0, 0, elems0 * 4, s));
-    SA_CUDA_CHECK(cudaMemsetAsync(dk0, 0, elems0 * 4, s));
-  } else {
-    SA_CUDA_CHECK(cudaMemsetAsync(dq0, 0, (w.dk0 - w.dq0) + elems0 * 4, s));
-  }
-  const float* fold_q = sel ? nullptr : dq0;
-  const float* fold_k = sel ? nullptr : dk0;
+  const size_t elems0 = (size_t)p.batch * p.seq * p.head_dim;
 
   if (in->engine == SA_ENGINE_SIMT) {
-    const float* d_out_f32 = static_cast<const float*>(d_out);
-    void* copy = nullptr;
-    if (d_out_dtype != SA_F32) {
-      copy = base + w.d_out_lowp;
-      d_out_f32 = static_cast<const float*>(copy);
+    float* dk_acc = reinterpret_cast<float*>(base + w.dk_acc);
+    float* dq0 = reinterpret_cast<float*>(base + w.dq0);
+    // dq_acc, dq0 and dk0 are accumulated with atomics and start at zero (the workspace's dq0/dk0 pair is contiguous).
+    SA_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, (size_t)rows * p.head_dim * 4, s));
+    if (sel != nullptr) {            // the selector's gradients go to the caller, unfolded
+      dq0 = dq0_out;
+      dk0 = dk0_out;
+      SA_CUDA_CHECK(cudaMemsetAsync(dq0, 0, elems0 * 4, s));
+      SA_CUDA_CHECK(cudaMemsetAsync(dk0, 0, elems0 * 4, s));
+    } else {
+      SA_CUDA_CHECK(cudaMemsetAsync(dq0, 0, (w.dk0 - w.dq0) + elems0 * 4, s));
     }
-    st = launch_dbar(out, d_out, d_out_dtype, rows, p.head_dim, dbar, copy, SA_F32, nullptr, p.heads, p.seq, s);
+    const float* d_out_f32 = static_cast<const float*>(d_out);
+    float* copy = nullptr;
+    if (d_out_dtype != SA_F32) {
+      copy = reinterpret_cast<float*>(base + w.d_out);
+      d_out_f32 = copy;
+    }
+    st = launch_dbar(out, d_out, d_out_dtype, rows, p.head_dim, stats, copy, s);
     if (st != SA_OK) return st;
-    st = simt_backward(p, lse2, carry, dbar, d_out_f32, dq_acc, dk_acc, dq0, dk0, dv, s);
+    st = simt_backward(p, lse2, carry, stats, d_out_f32, dq_acc, dk_acc, dq0, dk0, dv, s);
     if (st != SA_OK) return st;
-    st = launch_fold_cast(dk_acc, fold_k, dk, p.dtype, p.batch, p.heads, per_head, nullptr, p.head_dim, s);
+    st = launch_fold_cast(dk_acc, sel ? nullptr : dk0, dk, p.dtype, p.batch, p.heads, p.seq, p.head_dim, nullptr, s);
     if (st != SA_OK) return st;
-    return launch_fold_cast(dq_acc, fold_q, dq, p.dtype, p.batch, p.heads, per_head, nullptr, p.head_dim, s);
+    return launch_fold_cast(dq_acc, sel ? nullptr : dq0, dq, p.dtype, p.batch, p.heads, p.seq, p.head_dim, nullptr, s);
   }
   st = tc_backward_supported(p);
   if (st != SA_OK) return st;
-  void* d_out_lowp = base + w.d_out_lowp;
-  st = launch_dbar(out, d_out, d_out_dtype, rows, p.head_dim, dbar, d_out_lowp, p.dtype, d_out_rows, p.heads, p.seq, s);
+  if (dk_rows != nullptr) p.dk_rows = *dk_rows;
+  RowLayout do_rows = d_out_rows ? *d_out_rows : contiguous_rows(p.heads, p.seq, p.head_dim);
+  // A bf16 cotangent with 16-byte aligned rows is read by the kernel where it is.
+  const bool in_place = d_out_dtype == SA_BF16 && (reinterpret_cast<uintptr_t>(d_out) & 15) == 0 && do_rows.sb % 8 == 0 &&
+                        do_rows.sh % 8 == 0 && do_rows.st % 8 == 0;
+  void* copy = in_place ? nullptr : base + w.d_out;
+  float* dq0 = sel ? dq0_out : nullptr;
+  if (sel) dk0 = dk0_out;
+  st = launch_row_stats(out, d_out, d_out_dtype, do_rows, lse2, stats, copy, dq_acc, dq0, self_selecting(p) ? nullptr : dk0,
+                        p.batch, p.heads, p.seq, p.head_dim, s);
   if (st != SA_OK) return st;
-  st = tc_backward(p, lse2, carry, dbar, d_out_lowp, dq_acc, dk_acc, dq0, dk0, dv, s);
+  if (!in_place) do_rows = contiguous_rows(p.heads, p.seq, p.head_dim);
+  st = tc_backward(p, stats, carry, in_place ? d_out : copy, do_rows, dq_acc, dq0, dk0, dk, dv, s);
   if (st != SA_OK) return st;
-  st = launch_fold_cast(dk_acc, fold_k, dk, p.dtype, p.batch, p.heads, per_head, dk_rows, p.head_dim, s);
-  if (st != SA_OK) return st;
-  return launch_fold_cast(dq_acc, fold_q, dq, p.dtype, p.batch, p.heads, per_head, dq_rows, p.head_dim, s);
+  if (sel == nullptr) {              // head 0's dk: its own and the selection's, summed in fp32
+    st = launch_fold_cast(dk0, nullptr, dk, p.dtype, p.batch, 1, p.seq, p.head_dim, &p.dk_rows, s);
+    if (st != SA_OK) return st;
+  }
+  return launch_fold_cast(dq_acc, nullptr, dq, p.dtype, p.batch, p.heads, p.seq, p.head_dim, dq_rows, s);
 }
 }  // namespace
 

@@ -60,6 +60,7 @@ struct Problem {
   void* out_lowp;        // null: not requested
   RowLayout out_lowp_rows;
   RowLayout dv_rows;     // where dv rows go (default: contiguous (batch, heads, seq, head_dim))
+  RowLayout dk_rows;     // the same for dk (tensor-core engine)
   // Tensor-core engine, optional: the table of live (query tile, key tile) pairs (sa_tc_skip.cu).  The forward
   // fills it after its selection pass and leaves out the dead tiles; the backward of the same call reads it.
   void* tile_table;      // null: every causal tile is computed
@@ -81,20 +82,27 @@ int tc_available();
 int tc_supported(const Problem& p);
 int tc_forward(const Problem& p, float* out, float* lse2, float* carry, float* total, cudaStream_t s);
 int tc_backward_supported(const Problem& p);
-int tc_backward(const Problem& p, const float* lse2, const float* carry, const float* dbar,
-                const void* d_out_lowp, float* dq_acc, float* dk_acc, float* dq0, float* dk0,
-                void* dv, cudaStream_t s);
+// `stats`: what launch_row_stats wrote; `d_out` bf16 rows at `d_out_rows`.  dq_acc (fp32, zeroed) receives dQ, and dQ0 in
+// its head 0, or in dq0 with an external selector.  dk0 (fp32, zeroed) receives dK0, and also head 0's own dK unless the
+// selector is external; the other heads' dK rows are written to dk in bf16.
+int tc_backward(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+                float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s);
+// Rows that hold their own selection (one head per selector): head 0 of every batch entry is the only head.
+inline bool self_selecting(const Problem& p) { return p.heads == 1 && !p.external_selector; }
 
 // ---- helper launches shared by both engines --------------------------------------------------------
-// dbar[row] = sum_d d_out[row, d] * out[row, d]; optionally also writes d_out rounded to `lowp_dtype`.
-// `d_out_rows` (may be null: contiguous) says where the rows of d_out start; `heads`, `seq` split a row index.
-int launch_dbar(const float* out, const void* d_out, int d_out_dtype, int64_t rows, int head_dim,
-                float* dbar, void* d_out_lowp, int lowp_dtype, const RowLayout* d_out_rows, int heads, int seq,
+// dbar[row] = sum_d d_out[row, d] * out[row, d]; optionally also writes d_out converted to fp32 (CUDA-core engine).
+int launch_dbar(const float* out, const void* d_out, int d_out_dtype, int64_t rows, int head_dim, float* dbar, float* d_out_f32,
                 cudaStream_t s);
-// dst[b, h] = cast(acc[b, h] + (h == 0 ? acc0[b] : 0)), rows of head_dim elements; `dst_rows` (may be null:
-// contiguous) says where the rows of dst start.
-int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, int batch, int heads,
-                     int64_t seq_times_dim, const RowLayout* dst_rows, int head_dim, cudaStream_t s);
+// The tensor-core engine's form: -lse2 and -dbar in blocks of 64 queries ([row][block][2][64], up to the end of the last
+// 128-query tile), optionally dO rounded to bf16, and zeros in dq_acc and (head 0's rows) in zero_a, zero_b if given.
+int launch_row_stats(const float* out, const void* d_out, int d_out_dtype, const RowLayout& in_rows, const float* lse2,
+                     float* stats, void* d_out_bf16, float* dq_acc, float* zero_a, float* zero_b, int batch, int heads, int seq,
+                     int head_dim, cudaStream_t s);
+// dst[b, h] = cast(acc[b, h] + (h == 0 ? acc0[b] : 0)), rows of head_dim elements; acc0 may be null; `dst_rows` (may be
+// null: contiguous) says where the rows of dst start.
+int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, int batch, int heads, int seq, int head_dim,
+                     const RowLayout* dst_rows, cudaStream_t s);
 
 size_t decode_workspace_floats(int batch, int heads, int groups, int length, int head_dim);
 int decode_step(int dtype, int batch, int heads, int groups, int length, int capacity, int head_dim, int exempt,

@@ -1,6 +1,6 @@
 // Bandwidth-bound helpers of the Selective Attention operator (sm_100a):
-//   dbar      dbar[row] = sum_d dO[row, d] * out[row, d], optionally also dO rounded to bf16 / fp16
-//             (reference: src/selective_attention/kernels.py:635-636)
+//   dbar      dbar[row] = sum_d dO[row, d] * out[row, d]   (reference: src/selective_attention/kernels.py:635-636)
+//   row stats the tensor-core engine's form of it: -lse2 and -dbar in blocks, dO in bf16, zeroed accumulators
 //   fold/cast dq = cast(dq_acc + [head 0] dq0)            (reference: kernels.py:662-666)
 //   decode    one cached decode step                       (reference: src/selective_attention/mixers.py:115-130)
 #include "sa_common.cuh"
@@ -10,13 +10,11 @@
 namespace sa {
 namespace {
 
-// ---- dbar -----------------------------------------------------------------------------------------
+// ---- dbar (CUDA-core engine) ------------------------------------------------------------------------
 // A group of D / 4 consecutive lanes owns one row; every lane handles 4 consecutive elements.
-template <typename TDO, typename TLOW, int D, bool kWriteLow>
+template <typename TDO, int D>
 __global__ void __launch_bounds__(256) dbar_kernel(const float* __restrict__ out, const TDO* __restrict__ d_out,
-                                                   int64_t rows, float* __restrict__ dbar,
-                                                   TLOW* __restrict__ d_out_low, bool strided, RowLayout in_rows, int heads,
-                                                   int seq) {
+                                                   int64_t rows, float* __restrict__ dbar, float* __restrict__ d_out_f32) {
   constexpr int kLanes = D / 4;
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t row = gid / kLanes;
@@ -24,84 +22,127 @@ __global__ void __launch_bounds__(256) dbar_kernel(const float* __restrict__ out
   float sum = 0.f;
   if (row < rows) {
     const int64_t off = row * D + lane * 4;
-    int64_t off_in = off;
-    if (strided) {                            // d_out rows sit in the caller's (batch, seq, heads, head_dim) activation gradient
-      const int64_t bh = row / seq;
-      const int64_t t = row - bh * seq;
-      const int b = (int)(bh / heads), h = (int)(bh - (int64_t)b * heads);
-      off_in = in_rows.at(b, h, t) + lane * 4;
-    }
     float4 o = *reinterpret_cast<const float4*>(out + off);
     float g[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) g[e] = to_float<TDO>(d_out[off_in + e]);
+    for (int e = 0; e < 4; ++e) g[e] = to_float<TDO>(d_out[off + e]);
     sum = g[0] * o.x + g[1] * o.y + g[2] * o.z + g[3] * o.w;
-    if (kWriteLow) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) d_out_low[off + e] = from_float<TLOW>(g[e]);
-    }
+    if (d_out_f32 != nullptr) *reinterpret_cast<float4*>(d_out_f32 + off) = make_float4(g[0], g[1], g[2], g[3]);
   }
 #pragma unroll
   for (int s = kLanes / 2; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
   if (row < rows && lane == 0) dbar[row] = sum;
 }
 
-template <typename TDO, typename TLOW, bool kWriteLow>
-int dbar_by_dim(const float* out, const void* d_out, int64_t rows, int head_dim, float* dbar, void* low,
-                const RowLayout* in_rows, int heads, int seq, cudaStream_t s) {
-  const bool strided = in_rows != nullptr;
-  const RowLayout rl = strided ? *in_rows : RowLayout{0, 0, 0};
-  const int64_t threads = rows * (head_dim / 4);
-  const unsigned blocks = (unsigned)((threads + 255) / 256);
+template <typename TDO>
+int dbar_by_dim(const float* out, const void* d_out, int64_t rows, int head_dim, float* dbar, float* d_out_f32, cudaStream_t s) {
+  const unsigned blocks = (unsigned)((rows * (head_dim / 4) + 255) / 256);
   const TDO* g = static_cast<const TDO*>(d_out);
-  TLOW* l = static_cast<TLOW*>(low);
   ProfileScope prof(SA_KERNEL_DBAR, s);
   switch (head_dim) {
-    case 16: count_launch(), dbar_kernel<TDO, TLOW, 16, kWriteLow><<<blocks, 256, 0, s>>>(out, g, rows, dbar, l, strided, rl, heads, seq); break;
-    case 32: count_launch(), dbar_kernel<TDO, TLOW, 32, kWriteLow><<<blocks, 256, 0, s>>>(out, g, rows, dbar, l, strided, rl, heads, seq); break;
-    case 64: count_launch(), dbar_kernel<TDO, TLOW, 64, kWriteLow><<<blocks, 256, 0, s>>>(out, g, rows, dbar, l, strided, rl, heads, seq); break;
-    case 128: count_launch(), dbar_kernel<TDO, TLOW, 128, kWriteLow><<<blocks, 256, 0, s>>>(out, g, rows, dbar, l, strided, rl, heads, seq); break;
+    case 16: count_launch(), dbar_kernel<TDO, 16><<<blocks, 256, 0, s>>>(out, g, rows, dbar, d_out_f32); break;
+    case 32: count_launch(), dbar_kernel<TDO, 32><<<blocks, 256, 0, s>>>(out, g, rows, dbar, d_out_f32); break;
+    case 64: count_launch(), dbar_kernel<TDO, 64><<<blocks, 256, 0, s>>>(out, g, rows, dbar, d_out_f32); break;
+    case 128: count_launch(), dbar_kernel<TDO, 128><<<blocks, 256, 0, s>>>(out, g, rows, dbar, d_out_f32); break;
     default: return SA_ERR_UNSUPPORTED;
   }
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;
 }
 
-template <typename TDO>
-int dbar_by_low(const float* out, const void* d_out, int64_t rows, int head_dim, float* dbar, void* low,
-                int low_dtype, const RowLayout* in_rows, int heads, int seq, cudaStream_t s) {
-  if (low == nullptr) return dbar_by_dim<TDO, float, false>(out, d_out, rows, head_dim, dbar, nullptr, in_rows, heads, seq, s);
-  if (low_dtype == SA_BF16) return dbar_by_dim<TDO, __nv_bfloat16, true>(out, d_out, rows, head_dim, dbar, low, in_rows, heads, seq, s);
-  if (low_dtype == SA_F16) return dbar_by_dim<TDO, __half, true>(out, d_out, rows, head_dim, dbar, low, in_rows, heads, seq, s);
-  if (low_dtype == SA_F32) return dbar_by_dim<TDO, float, true>(out, d_out, rows, head_dim, dbar, low, in_rows, heads, seq, s);
-  return SA_ERR_BAD_ARGUMENT;
+// ---- row statistics (tensor-core engine) -------------------------------------------------------------
+// One pass over out and dO: dbar = sum_d dO * out, the bf16 copy of dO where the caller's is not one the TMA can read,
+// and the zeros that the backward kernel's reductions start from (dq_acc, and dk0 / dq0 for the selecting head).  What the
+// backward kernel wants per query, -lse2 and -dbar, goes out as blocks of 64 queries, [row n][block][-lse2 x 64, -dbar x 64]
+// with blocks up to the end of the last 128-query tile (-inf and 0 there: such a query has P = 0), so that a 64-query half
+// takes its statistics in one 512-byte bulk copy whatever the sequence length.
+// Bound by memory: reads 4 + sizeof(dO) and writes 4 (+ 2) bytes an element; a separate memset of the same zeros cost a
+// launch and nothing less.
+template <typename TDO, int D>
+__global__ void __launch_bounds__(256) row_stats_kernel(const float* __restrict__ out, const TDO* __restrict__ d_out,
+                                                        RowLayout in_rows, bool vec, const float* __restrict__ lse2,
+                                                        float* __restrict__ stats, __nv_bfloat16* __restrict__ d_out_low,
+                                                        float* __restrict__ dq_acc, float* __restrict__ zero_a,
+                                                        float* __restrict__ zero_b, int heads, int seq, int padded,
+                                                        int64_t rows) {
+  constexpr int kLanes = D / 4;
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t row = gid / kLanes;               // (n, padded query index)
+  const int lane = (int)(gid % kLanes);
+  if (row >= rows) return;                         // whole groups of lanes leave together: rows * kLanes threads work
+  const int n = (int)(row / padded), t = (int)(row - (int64_t)n * padded);
+  const int b = n / heads, h = n - b * heads;
+  float sum = 0.f;
+  if (t < seq) {
+    const int64_t off = ((int64_t)n * seq + t) * D + lane * 4;
+    const TDO* src = d_out + in_rows.at(b, h, t) + lane * 4;
+    const float4 o = *reinterpret_cast<const float4*>(out + off);
+    TDO raw[4];
+    if (vec) {
+      if constexpr (sizeof(TDO) == 4) *reinterpret_cast<float4*>(raw) = *reinterpret_cast<const float4*>(src);
+      else *reinterpret_cast<uint2*>(raw) = *reinterpret_cast<const uint2*>(src);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) raw[e] = src[e];
+    }
+    float g[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) g[e] = to_float<TDO>(raw[e]);
+    sum = g[0] * o.x + g[1] * o.y + g[2] * o.z + g[3] * o.w;
+    if (d_out_low != nullptr)
+      *reinterpret_cast<uint2*>(d_out_low + off) = make_uint2(tc::pack_bf16(g[0], g[1]), tc::pack_bf16(g[2], g[3]));
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(dq_acc + off) = zero;
+    if (h == 0) {
+      const int64_t off0 = ((int64_t)b * seq + t) * D + lane * 4;
+      if (zero_a != nullptr) *reinterpret_cast<float4*>(zero_a + off0) = zero;
+      if (zero_b != nullptr) *reinterpret_cast<float4*>(zero_b + off0) = zero;
+    }
+  }
+#pragma unroll
+  for (int s = kLanes / 2; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+  if (lane == 0) {
+    float* block = stats + ((int64_t)n * (padded >> 6) + (t >> 6)) * 128 + (t & 63);
+    block[0] = (t < seq) ? -lse2[(int64_t)n * seq + t] : -INFINITY;
+    block[64] = (t < seq) ? -sum : 0.f;
+  }
 }
 
 // ---- fold + cast ------------------------------------------------------------------------------------
+// Eight elements a thread: two or four 16-byte loads in flight and one 16-byte store (bf16, fp16) where dst allows it.
 template <typename T>
 __global__ void __launch_bounds__(256) fold_cast_kernel(const float* __restrict__ acc, const float* __restrict__ acc0,
                                                         T* __restrict__ dst, int heads, int64_t per_head,
-                                                        int64_t total4, bool strided, RowLayout dst_rows, int head_dim) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total4) return;
-  int64_t e = idx * 4;
-  int64_t row = e / per_head;                 // (batch, head) row
-  int64_t within = e - row * per_head;
-  int b = (int)(row / heads), h = (int)(row - (int64_t)b * heads);
-  float4 a = *reinterpret_cast<const float4*>(acc + e);
+                                                        int64_t total8, bool vec, RowLayout dst_rows, int head_dim) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= total8) return;
+  const int64_t e = idx * 8;
+  const int64_t row = e / per_head;           // (batch, head) row
+  const int64_t within = e - row * per_head;
+  const int b = (int)(row / heads), h = (int)(row - (int64_t)b * heads);
+  float x[8];
+  *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(acc + e);
+  *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(acc + e + 4);
   if (h == 0 && acc0 != nullptr) {
-    float4 z = *reinterpret_cast<const float4*>(acc0 + (int64_t)b * per_head + within);
-    a.x += z.x; a.y += z.y; a.z += z.z; a.w += z.w;
+    const float* z = acc0 + (int64_t)b * per_head + within;
+    float y[8];
+    *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(z);
+    *reinterpret_cast<float4*>(y + 4) = *reinterpret_cast<const float4*>(z + 4);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] += y[u];
   }
-  int64_t o = e;
-  if (strided) {                              // rows go into the caller's (batch, seq, ..., heads, head_dim) gradient buffer
-    const int64_t t = within / head_dim;
-    o = dst_rows.at(b, h, t) + (within - t * head_dim);
+  const int64_t t = within / head_dim;
+  T* out = dst + dst_rows.at(b, h, t) + (within - t * head_dim);
+  T w[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) w[u] = from_float<T>(x[u]);
+  if (vec) {
+#pragma unroll
+    for (int u = 0; u < (int)sizeof(T) / 2; ++u) reinterpret_cast<uint4*>(out)[u] = reinterpret_cast<const uint4*>(w)[u];
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) out[u] = w[u];
   }
-  dst[o + 0] = from_float<T>(a.x);
-  dst[o + 1] = from_float<T>(a.y);
-  dst[o + 2] = from_float<T>(a.z);
-  dst[o + 3] = from_float<T>(a.w);
 }
 
 // ---- decode -----------------------------------------------------------------------------------------
@@ -162,15 +203,6 @@ __device__ __forceinline__ void load8(const T* p, float (&x)[8]) {
 template <typename T>
 __device__ __forceinline__ void load8_shared(const uint8_t* p, float (&x)[8]) {
   load8<T>(reinterpret_cast<const T*>(p), x);
-}
-
-// Untiled bulk copy global -> shared memory, completion counted in bytes on an mbarrier.  Both addresses and the
-// size are multiples of 16 bytes.
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   tc::smem_u32(smem_dst)),
-               "l"(gmem_src), "r"(bytes), "r"(tc::smem_u32(bar))
-               : "memory");
 }
 
 constexpr int kDecStages = 3;                   // stages of 8 KB of K + 8 KB of V
@@ -277,8 +309,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     uint8_t* dst = ring + (size_t)(st % kDecStages) * 2 * kDecStageBytes;
     uint64_t* bar = &full[st % kDecStages];
     tc::mbar_expect_tx(bar, 2 * bytes);
-    bulk_load(dst, kb + (int64_t)j0 * kRowBytes, bytes, bar);
-    bulk_load(dst + kDecStageBytes, vb + (int64_t)j0 * kRowBytes, bytes, bar);
+    tc::bulk_load(dst, kb + (int64_t)j0 * kRowBytes, bytes, bar);
+    tc::bulk_load(dst + kDecStageBytes, vb + (int64_t)j0 * kRowBytes, bytes, bar);
   };
   float qv[8];
   load8<T>(q1 + (int64_t)n * D + lane * 8, qv);
@@ -537,36 +569,77 @@ int decode_impl(int batch, int heads, int groups, int length, int capacity, int 
 
 }  // namespace
 
-int launch_dbar(const float* out, const void* d_out, int d_out_dtype, int64_t rows, int head_dim, float* dbar,
-                void* d_out_lowp, int lowp_dtype, const RowLayout* d_out_rows, int heads, int seq, cudaStream_t s) {
+int launch_dbar(const float* out, const void* d_out, int d_out_dtype, int64_t rows, int head_dim, float* dbar, float* d_out_f32,
+                cudaStream_t s) {
   switch (d_out_dtype) {
-    case SA_F32: return dbar_by_low<float>(out, d_out, rows, head_dim, dbar, d_out_lowp, lowp_dtype, d_out_rows, heads, seq, s);
-    case SA_BF16: return dbar_by_low<__nv_bfloat16>(out, d_out, rows, head_dim, dbar, d_out_lowp, lowp_dtype, d_out_rows, heads, seq, s);
-    case SA_F16: return dbar_by_low<__half>(out, d_out, rows, head_dim, dbar, d_out_lowp, lowp_dtype, d_out_rows, heads, seq, s);
+    case SA_F32: return dbar_by_dim<float>(out, d_out, rows, head_dim, dbar, d_out_f32, s);
+    case SA_BF16: return dbar_by_dim<__nv_bfloat16>(out, d_out, rows, head_dim, dbar, d_out_f32, s);
+    case SA_F16: return dbar_by_dim<__half>(out, d_out, rows, head_dim, dbar, d_out_f32, s);
   }
   return SA_ERR_BAD_ARGUMENT;
 }
 
-int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, int batch, int heads,
-                     int64_t seq_times_dim, const RowLayout* dst_rows, int head_dim, cudaStream_t s) {
-  const bool strided = dst_rows != nullptr;
-  const RowLayout rl = strided ? *dst_rows : RowLayout{0, 0, 0};
-  const int64_t total4 = (int64_t)batch * heads * seq_times_dim / 4;
-  const unsigned blocks = (unsigned)((total4 + 255) / 256);
+namespace {
+bool aligned_rows(const void* ptr, const RowLayout& r, int64_t elem_bytes, int64_t align) {
+  return (reinterpret_cast<uintptr_t>(ptr) & (align - 1)) == 0 && (r.sb * elem_bytes) % align == 0 &&
+         (r.sh * elem_bytes) % align == 0 && (r.st * elem_bytes) % align == 0;
+}
+template <typename TDO>
+int row_stats_by_dim(const float* out, const void* d_out, const RowLayout& in_rows, bool vec, const float* lse2, float* stats,
+                     void* d_out_bf16, float* dq_acc, float* zero_a, float* zero_b, int batch, int heads, int seq, int head_dim,
+                     cudaStream_t s) {
+  const int padded = (seq + 127) / 128 * 128;
+  const int64_t rows = (int64_t)batch * heads * padded;          // a multiple of 128: a warp's rows exist or not together
+  const unsigned blocks = (unsigned)((rows * (head_dim / 4) + 255) / 256);
+  const TDO* g = static_cast<const TDO*>(d_out);
+  __nv_bfloat16* low = static_cast<__nv_bfloat16*>(d_out_bf16);
+  ProfileScope prof(SA_KERNEL_DBAR, s);
+  count_launch();
+  if (head_dim == 64)
+    row_stats_kernel<TDO, 64><<<blocks, 256, 0, s>>>(out, g, in_rows, vec, lse2, stats, low, dq_acc, zero_a, zero_b, heads, seq, padded, rows);
+  else if (head_dim == 128)
+    row_stats_kernel<TDO, 128><<<blocks, 256, 0, s>>>(out, g, in_rows, vec, lse2, stats, low, dq_acc, zero_a, zero_b, heads, seq, padded, rows);
+  else
+    return SA_ERR_UNSUPPORTED;
+  SA_CUDA_CHECK(cudaGetLastError());
+  return SA_OK;
+}
+}  // namespace
+
+int launch_row_stats(const float* out, const void* d_out, int d_out_dtype, const RowLayout& in_rows, const float* lse2,
+                     float* stats, void* d_out_bf16, float* dq_acc, float* zero_a, float* zero_b, int batch, int heads, int seq,
+                     int head_dim, cudaStream_t s) {
+  const int64_t es = d_out_dtype == SA_F32 ? 4 : 2;
+  const bool vec = aligned_rows(d_out, in_rows, es, 4 * es);
+  switch (d_out_dtype) {
+    case SA_F32: return row_stats_by_dim<float>(out, d_out, in_rows, vec, lse2, stats, d_out_bf16, dq_acc, zero_a, zero_b, batch, heads, seq, head_dim, s);
+    case SA_BF16: return row_stats_by_dim<__nv_bfloat16>(out, d_out, in_rows, vec, lse2, stats, d_out_bf16, dq_acc, zero_a, zero_b, batch, heads, seq, head_dim, s);
+    case SA_F16: return row_stats_by_dim<__half>(out, d_out, in_rows, vec, lse2, stats, d_out_bf16, dq_acc, zero_a, zero_b, batch, heads, seq, head_dim, s);
+  }
+  return SA_ERR_BAD_ARGUMENT;
+}
+
+int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, int batch, int heads, int seq, int head_dim,
+                     const RowLayout* dst_rows, cudaStream_t s) {
+  const RowLayout rl = dst_rows ? *dst_rows : contiguous_rows(heads, seq, head_dim);
+  const int64_t per_head = (int64_t)seq * head_dim;
+  const int64_t total8 = (int64_t)batch * heads * per_head / 8;
+  const unsigned blocks = (unsigned)((total8 + 255) / 256);
+  const bool vec = aligned_rows(dst, rl, dtype == SA_F32 ? 4 : 2, 16);
   switch (dtype) {
     case SA_F32:
       count_launch();
-      fold_cast_kernel<float><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<float*>(dst), heads, seq_times_dim, total4, strided, rl, head_dim);
+      fold_cast_kernel<float><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<float*>(dst), heads, per_head, total8, vec, rl, head_dim);
       break;
     case SA_BF16:
       count_launch();
-      fold_cast_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<__nv_bfloat16*>(dst), heads,
-                                                             seq_times_dim, total4, strided, rl, head_dim);
+      fold_cast_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<__nv_bfloat16*>(dst), heads, per_head, total8,
+                                                             vec, rl, head_dim);
       break;
     case SA_F16:
       count_launch();
-      fold_cast_kernel<__half><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<__half*>(dst), heads, seq_times_dim,
-                                                      total4, strided, rl, head_dim);
+      fold_cast_kernel<__half><<<blocks, 256, 0, s>>>(acc, acc0, static_cast<__half*>(dst), heads, per_head, total8, vec, rl,
+                                                      head_dim);
       break;
     default: return SA_ERR_BAD_ARGUMENT;
   }

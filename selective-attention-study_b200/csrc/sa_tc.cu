@@ -5,10 +5,10 @@
 namespace sa {
 namespace tc {
 int forward(const Problem& p, float* out, float* lse2, float* carry, float* total, cudaStream_t s);
-int backward(const Problem& p, const float* lse2, const float* carry, const float* dbar, const void* d_out_bf16,
-             float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s);
-int backward_wide(const Problem& p, const float* lse2, const float* carry, const float* dbar, const void* d_out_bf16,
-                  float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s);
+int backward(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+             float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s);
+int backward_wide(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+                  float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s);
 }  // namespace tc
 
 int tc_available() { return 1; }
@@ -28,9 +28,9 @@ int tc_backward_supported(const Problem& p) {
   return tc_supported(p);
 }
 
-int tc_backward(const Problem& p, const float* lse2, const float* carry, const float* dbar, const void* d_out_lowp,
-                float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
-  if (p.head_dim == 128) return tc::backward_wide(p, lse2, carry, dbar, d_out_lowp, dq_acc, dk_acc, dq0, dk0, dv, s);
-  return tc::backward(p, lse2, carry, dbar, d_out_lowp, dq_acc, dk_acc, dq0, dk0, dv, s);
+int tc_backward(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+                float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s) {
+  auto run = p.head_dim == 128 ? tc::backward_wide : tc::backward;
+  return run(p, stats, carry, d_out, d_out_rows, dq_acc, dq0, dk0, dk, dv, s);
 }
 }  // namespace sa

@@ -1,43 +1,48 @@
-// Tensor-core engine, backward (sm_100a: TMA loads and reduce-adds, tcgen05 MMAs, fp32 accumulators in TMEM).
+// Tensor-core engine, backward at head_dim 64 (sm_100a: TMA loads and reduce-adds, tcgen05 MMAs, fp32 accumulators in TMEM).
 //
 // One CTA owns one 128-key tile of one head and walks the query tiles LAST TO FIRST in 64-query halves.  All
 // score-shaped tiles are computed transposed, KEYS on the TMEM lanes (S^T = K Q^T, dP^T = V dO^T, L0^T = K0 Q0^T), so
-// one thread owns one key and sees that key's queries along its registers.  The two running sums down the query
+// one thread owns one key and sees all 64 queries of a half along its registers.  The two running sums down the query
 // axis are then thread-local fp32 recurrences walked from the last query to the first:
-//     F[i]  = carry_after_tile - sum_{r >= i} sel[r]          (history term rebuilt per key)
+//     F[i]  = carry_after_half - sum_{r >= i} sel[r]          (history term rebuilt per key)
 //     U[i]  = suffix + sum_{i' > i} dz[i']                      (logit gradient of later queries)
 // with  P = exp2(z - lse),  dz = P (dP - dbar),  g = gate ? -U : 0.
 //
-// Roles.  Warps 0-15 (four warpgroups) do the arithmetic: within a half each warpgroup takes 16 query columns of
-// every key row; chunk totals are exchanged through shared memory so the recurrences chain across chunks, halves
-// and tiles.  Warp 16 is the control warp: one lane issues every TMA load and every MMA.
+// TWO CHAINS.  A half is a serial chain (scores -> selection -> probabilities -> dz -> g -> the products that consume
+// them) whose links are hand-overs between the arithmetic warps and the tensor pipe.  With all warps on one half at a time
+// the SM idles at each of them: 10.4 k cycles per 128 x 128 tile of which ~3.8 k were issue slots.  Here the upper halves
+// (chain 0) and the lower halves (chain 1) of the tiles belong to one warpgroup each, with their own two score tiles in TMEM,
+// so that one chain computes while the other waits.  What couples them is little: the history of a half starts from a
+// checkpoint of its own (the carry after the tile, or the carry before it plus the half's own sum), and the running sum
+// of dz is handed from half to half, per key, through one shared-memory word (`run_s`).
 //
-// Operand sources and issue points.  Measured on B200, a head-tile of a form with every operand in shared memory and
-// each product issued when its inputs appear costs ~10.5 k cycles of which the arithmetic is ~3 k and the MMAs ~4 k;
-// the rest is hand-over latency, because every product the arithmetic warps wait for is issued only after an arrival
-// of theirs has travelled to the control warp and the MMA's completion has travelled back.  Here each such product is
-// issued one arithmetic pass EARLIER than it is needed, into columns that are free by then:
-//     L0^T of half n + 1 -> Z   when the selection pass of half n has read Z
-//     S^T  of half n + 1 -> Y   when P^T and dz^T of half n (which live in Y) have been handed to dV and dK
-//     dP^T of half n + 1 -> X   when g^T of half n (which lives in X) has been handed to dK0
-// K and V sit in TMEM as bf16 pairs (A of S^T and dP^T); P^T, dz^T and g^T are written by each thread as bf16 pairs
-// over the score columns that SAME thread has just read (its 16 columns of Y hold P^T then dz^T, 8 packed columns
-// each; its 16 columns of X hold g^T), so no barrier is needed between reading a score tile and overwriting it, and
-// dV, dK, dK0 read their A operand from TMEM with a stride of 16 columns per 16-query step.  L0^T = K0 Q0^T and the
-// per-tile dQ = dz K, dQ0 = g K0 take both operands from shared memory.  TMEM, 512 columns: K, V (32 each) | dV, dK,
-// dK0 | Z | X | Y | one accumulator shared by dQ and dQ0 (64 each): dQ is read out at the tile's end, dQ0 in the
-// middle of the next tile's first half.  The query-side tiles (Q, Q0, dO) arrive per half through a ring of three
-// 24 KB slots; dQ / dQ0 leave through their own fp32 staging tile and TMA reduce-add.
+// Roles.  Warps 0-3 and 4-7: the two chains.  Warps 8-11: read dQ and dQ0 out of TMEM, scale, stage and TMA-reduce-add them
+// into fp32 global rows.  Warp 12 issues every MMA, in the order in which the events of two chains half a tile apart come.
+// Warp 13, one lane: TMA loads.
+//
+// TMEM, 512 columns: dV | dK | one accumulator shared by dQ and dQ0 | per chain W1 and W2 | dK0 (64 each).
+//     W1: L0^T of half n -> (read) -> dP^T of half n -> (read) -> g^T as bf16 pairs -> dK0 -> L0^T of half n + 2
+//     W2: S^T of half n -> (read) -> P^T and dz^T as bf16 pairs -> dV, dK -> S^T of half n + 2
+// so each product is issued as soon as the columns that it goes to are free, a pass or more before it is needed; only L0^T
+// is waited for, and the other chain covers that.  P^T, dz^T, g^T are A operands from TMEM; dz and g also go to shared
+// memory, from where dQ = dz K and dQ0 = g K0 are computed per 128-query tile.
+//
+// What bounds it.  Shared memory (128 B/clk) moves 528 KB per 128 x 128 tile: score operands 144, B operands of dV, dK, dK0
+// 48, dQ, dQ0 operands 96, dz and g written 64, dQ, dQ0 staged and reduced 128, loads 48 = 4.2 k cycles; the tensor pipe needs
+// 2.7 k, the issue slots ~3 k.  And the INSTRUCTION CACHE: everything that runs at one time has to fit 32 KB (measured: what
+// does not fit is fetched at 2.7 cycles an instruction, for each chain separately since they are half a tile apart).  The
+// first form of this kernel, with 45 KB of loops, ran at 15.5 k cycles a tile; hence the compact waits (Waiter), the rolled
+// MMA loop over halves (its order is the same for both chains), low words of descriptors, 32-bit shared addresses.
+// Measured at B = 4, H = 16, T = 16384: 16.6 ms with sixteen warps in lock step, 12.3 ms with two chains (SELF: 12.3, 9.3).
 //
 // SELF variant (one head per selector, i.e. the per-head form reshaped to (B H, 1, T, D)): the selection logits are the
-// head's own logits, so S^T serves as L0^T, and since Q0 = Q and K0 = K the two gradient paths add before the MMAs:
-// dK += (dz + g)^T Q and dQ = (dz + g) K, with (dz + g)^T in this thread's X columns.  40 MMAs per query tile instead
-// of 64, no Q0 / K0 tiles, no Z, one read-out per tile (deferred into the next tile's first half).
+// head's own logits, so S^T serves as L0^T (read twice), and since Q0 = Q and K0 = K the two gradient paths add before the
+// MMAs: dK += (dz + g)^T Q and dQ = (dz + g) K, with (dz + g)^T in W1.  40 MMAs per query tile instead of 64, no Q0 / K0
+// tiles, and the columns of dK0 hold K and V as bf16 pairs (A of the score products, 64 KB less shared-memory traffic).
 //
-// Code shape.  The diagonal tile, the only one that needs the causal mask inside the tile, is the LAST tile of a CTA's
-// walk: the loop holds the unmasked form of the per-half arithmetic only and the masked form runs once after it, and
-// the two halves of a tile are inlined (constant barrier parities and tile addresses).  That removes no work and 8 % of
-// the time.  LIVE: with a table of live tiles (sa_tc_skip.cu) the walk starts at the key tile's last live query tile.
+// The diagonal tile, the only one that needs the causal mask inside the tile, is the LAST tile of a CTA's walk: the loop
+// holds the unmasked form only and the masked form runs once after it.  LIVE: with a table of live tiles (sa_tc_skip.cu)
+// the walk starts at the key tile's last live query tile.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:196-268 (one head), :271-364 (the shared
 // selection-gradient products).
@@ -49,35 +54,61 @@ namespace sa {
 namespace tc {
 namespace {
 
-using namespace bwd;
+using bwd::ex2;
+using bwd::find_top_tile;
+using bwd::kHalfTile;
+using bwd::kRowTile;
+using bwd::kTile;
+using bwd::load_ahead;
+using bwd::store_key_grads;
+using bwd::tile_of_block;
 
-constexpr int kRing = 3;             // half-tile slots of Q, Q0, dO in flight
+constexpr int kPairThreads = 512;     // two chains, the read-out warpgroup, the MMA and load warps (two warps idle)
+// Registers: 512 x 128 at launch; the chains keep 64 values and their masks, the rest needs little: 256 x 168 + 256 x 88.
+constexpr int kChainRegs = 168, kOtherRegs = 88;
+constexpr int kMmaWarp = 12, kLoadWarp = 13;
+constexpr int kStatBytes = 512;       // -lse2 and -dbar of 64 queries
 
-struct Smem {
-  static constexpr int k = 0;                              // [128 keys][64], stationary
+template <bool SELF>
+struct PairSmem {
+  static constexpr int kRing = SELF ? 5 : 3;                                 // half tiles of Q, dO in flight
+  static constexpr int kRing0 = SELF ? 0 : 3;                                // half tiles of Q0
+  static constexpr int kSlot = 2 * kHalfTile;                                // Q, dO
+  static constexpr int k = 0;                                                // [128 keys][64], stationary
   static constexpr int v = k + kRowTile;
   static constexpr int k0 = v + kRowTile;
-  static constexpr int ring = k0 + kRowTile;               // kRing x (Q, Q0, dO) half tiles [64 queries][64]
-  static constexpr int dz = ring + kRing * 3 * kHalfTile;  // [128 keys][128 queries] bf16 as two query-half tiles
+  static constexpr int ring = SELF ? k0 : k0 + kRowTile;
+  static constexpr int ring0 = ring + kRing * kSlot;
+  static constexpr int dz = ring0 + kRing0 * kHalfTile;                      // [128 keys][128 queries] bf16 as two query-half tiles
   static constexpr int g = dz + 2 * kRowTile;
-  static constexpr int out = g + 2 * kRowTile;             // fp32 [128 queries][64] as two [128][32] boxes
-  static constexpr int total = out + 2 * kRowTile;         // 216 KB
+  static constexpr int out = SELF ? g : g + 2 * kRowTile;                    // fp32 [128 queries][64]: per warp two [32][32] boxes
+  static constexpr int stat = out + 2 * kRowTile;                            // kRing x (-lse2, -dbar)
+  static constexpr int total = stat + kRing * kStatBytes;
 };
 
-// TMEM columns (Z, X, Y: sa_tc_bwd_passes.cuh)
-constexpr uint32_t kColK = 0, kColV = 32, kColDV = 64, kColDK = 128, kColDK0 = 192, kColDQ = 448;
+// TMEM columns
+constexpr uint32_t kDV = 0, kDK = 64, kDQ = 128, kW = 192, kDK0 = 448, kKA = 448, kVA = 480;
+__device__ __forceinline__ constexpr uint32_t w1_of(uint32_t chain) { return kW + 128 * chain; }
+__device__ __forceinline__ constexpr uint32_t w2_of(uint32_t chain) { return kW + 128 * chain + 64; }
+
+// The signs of two floats as a pair of 16-bit masks (0xffff where the sign bit is set).
+__device__ __forceinline__ uint32_t sign_masks(float lo, float hi) {
+  uint32_t m;
+  asm("prmt.b32 %0, %1, %2, 0xffbb;" : "=r"(m) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+  return m;
+}
 
 template <bool SELF, bool LIVE>   // LIVE: a table of live tiles is given (sa_tc_skip.cu)
-__global__ void __launch_bounds__(kThreads, 1) backward_kernel(
+__global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dq0,
     const __grid_constant__ CUtensorMap map_q0, const __grid_constant__ CUtensorMap map_k0,
-    const float* __restrict__ lse2, const float* __restrict__ carry, const float* __restrict__ dbar,
-    float* __restrict__ dk_acc, float* __restrict__ dk0, __nv_bfloat16* __restrict__ dv, int heads, int seq,
-    int ntiles, int exempt, float scale, WaitCtx status, RowLayout dv_rows, const uint8_t* __restrict__ alive) {
-  using L = Smem;
-  constexpr int D = 64;
+    const float* __restrict__ stats, const float* __restrict__ carry, __nv_bfloat16* __restrict__ dk,
+    float* __restrict__ dk0, __nv_bfloat16* __restrict__ dv, int heads, int dq0_rows, int seq, int ntiles, int exempt, float scale,
+    const __grid_constant__ WaitCtx status, RowLayout dk_rows, RowLayout dv_rows, const uint8_t* __restrict__ alive) {
+  using L = PairSmem<SELF>;
+  constexpr int D = 64, R = L::kRing;
   // One (batch, head) row after the other, and within a row the key tiles with the most query tiles first: the CTAs
   // resident at one time belong to one or two rows and walk the same query tiles from the last one down, so every
   // Q, Q0, dO tile is fetched from DRAM once and then served from L2 to the row's other CTAs.
@@ -85,40 +116,22 @@ __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
   tile_of_block(blockIdx.x, ntiles, gridDim.x / ntiles, LIVE, n, nj);
   const int b = n / heads, h = n - b * heads;
 
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // Completion barriers (MMA commits and TMA loads) and arrival barriers (arithmetic warps).  bar_l0 .. bar_g complete
-  // one phase per half; each side reaches its next wait on one of them only after the other side has consumed the
-  // previous phase, so a poller can never see two phases complete between two polls.
-  __shared__ uint64_t bar_kv, bar_setup, bar_ld[kRing], bar_free[kRing], bar_l0, bar_s, bar_dp, bar_sel, bar_early, bar_g,
-      bar_dq, bar_dq0, bar_dqread, bar_dq0read, bar_fin;
+  // Barriers.  Completion: LD, LD0 TMA loads; L0, S, DP score products of a chain's half; FREE, FREE0 the last MMA that reads
+  // a slot; DQ, DQ0 a tile's query-side product.  Arrival, one arrival per warp: SEL L0^T read; DZ P^T and dz^T written, S^T
+  // and dP^T read; G g^T written; TOK the running sum of dz handed on; ACC the shared accumulator read.
+  enum : int { KV = 0, SETUP = 1, FIN = 2, DQ = 3, DQ0 = 4, ACC = 5, L0 = 6, S = 8, DP = 10, SEL = 12, DZ = 14, G = 16, TOK = 18,
+               LD = 20, FREE = 25, LD0 = 30, FREE0 = 33, kBars = 36 };
+  __shared__ uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(16) float lse_s[kTile];
-  __shared__ __align__(16) float dbar_s[kTile];
-  __shared__ float sel_tot[kGroups][kTile];
-  __shared__ float dz_tot[kGroups][kTile];
+  __shared__ float run_s[kTile];
+  __shared__ int top_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  __shared__ int top_s;
   if (LIVE && warp == 1) find_top_tile(alive, n, nj, ntiles, lane, &top_s);
   if (tid == 0) {
-    mbar_init(&bar_kv, 1);
-    for (int u = 0; u < kRing; ++u) {
-      mbar_init(&bar_ld[u], 1);
-      mbar_init(&bar_free[u], 1);
-    }
-    mbar_init(&bar_setup, kComputeThreads / 32);
-    mbar_init(&bar_l0, 1);
-    mbar_init(&bar_s, 1);
-    mbar_init(&bar_dp, 1);
-    mbar_init(&bar_sel, 1);
-    mbar_init(&bar_early, 1);
-    mbar_init(&bar_g, kComputeThreads / 32);
-    mbar_init(&bar_dq, 1);
-    mbar_init(&bar_dq0, 1);
-    mbar_init(&bar_dqread, 1);
-    mbar_init(&bar_dq0read, 1);
-    mbar_init(&bar_fin, 1);
+    for (int u = 0; u < kBars; ++u) mbar_init(&bars[u], u == SETUP ? 8 : (u == ACC || (u >= SEL && u < LD)) ? 4 : 1);
     mbar_init_fence();
   }
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
@@ -126,345 +139,494 @@ __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t sa = smem_u32(smem);
+  const uint32_t sa = smem_u32(smem), bar0 = smem_u32(bars);
+  auto bar = [&](int id) { return bar0 + 8u * (uint32_t)id; };
+  Waiter wait;
+  wait.begin(status);
   const int mi_top = LIVE ? top_s : ntiles - 1;   // the walk starts at the last query tile, or at the last live one
   const int n_iter = mi_top - nj + 1;
-  const int n_half = 2 * n_iter;
+  const int n_half = 2 * n_iter;                  // half hn: tile mi_top - hn / 2, chain hn & 1 (chain 0: the upper half)
 
-  if (warp == kComputeThreads / 32) {
-    // =============================== control warp: TMA loads and MMA issue ===============================
+  if (warp >= 8) {
+  regs_shrink<kOtherRegs>();
+  if (warp == kLoadWarp) {
+    // ========================================== TMA loads ==================================================
     if (lane == 0) {
-      const uint32_t idesc_t = instr_desc_bf16(128, 64, false, false);     // keys x 64 queries, K = D
-      const uint32_t idesc_acc = instr_desc_bf16(128, 64, false, true);    // A K-major (keys x queries), B MN-major
-      const uint32_t idesc_dq = instr_desc_bf16(128, 64, true, true);      // A MN-major (queries x keys), B MN-major
-      // Half index hn counts from the last query half: tile it = hn / 2 (query tile mi_top - it), upper half of
-      // the tile first.  Its operands sit in ring slot hn % kRing.
-      auto load_half = [&](int hn) {
-        const int it = hn >> 1, hf = 1 - (hn & 1), slot = hn % kRing;
-        const int row0 = (mi_top - it) * kTile + hf * 64;
-        uint8_t* st = smem + L::ring + slot * 3 * kHalfTile;
-        mbar_expect_tx(&bar_ld[slot], (SELF ? 2 : 3) * kHalfTile);
-        tma_load_4d(st, &map_q, &bar_ld[slot], 0, row0, h, b);
-        if (!SELF) tma_load_4d(st + kHalfTile, &map_q0, &bar_ld[slot], 0, row0, 0, b);
-        tma_load_4d(st + 2 * kHalfTile, &map_do, &bar_ld[slot], 0, row0, n, 0);
+      auto row_of = [&](int hn) { return (mi_top - (hn >> 1)) * kTile + (1 - (hn & 1)) * 64; };
+      auto load_qdo = [&](int hn, int slot) {
+        const int row0 = row_of(hn);
+        uint8_t* st = smem + L::ring + slot * L::kSlot;
+        mbar_expect_tx(&bars[LD + slot], 2 * kHalfTile + kStatBytes);
+        tma_load_4d(st, &map_q, &bars[LD + slot], 0, row0, h, b);
+        tma_load_4d(st + kHalfTile, &map_do, &bars[LD + slot], 0, row0, h, b);
+        bulk_load(smem + L::stat + slot * kStatBytes, stats + ((int64_t)n * 2 * ntiles + (row0 >> 6)) * (kStatBytes / 4), kStatBytes,
+                  &bars[LD + slot]);
       };
-      auto at = [](uint64_t desc, uint32_t byte_off) { return desc + (uint64_t)(byte_off >> 4); };
-      const uint64_t kK0 = smem_desc(sa + L::k0, 16, 1024);                   // K-major A of L0^T
-      const uint64_t mK = smem_desc(sa + L::k, kRowTile, 1024), mK0 = smem_desc(sa + L::k0, kRowTile, 1024);
-      const uint64_t mDZ = smem_desc(sa + L::dz, kRowTile, 1024), mG = smem_desc(sa + L::g, kRowTile, 1024);
-      const uint64_t kRingD = smem_desc(sa + L::ring, 16, 1024);             // Q, Q0, dO half tiles as K-major B
-      const uint64_t mRingD = smem_desc(sa + L::ring, kRowTile, 1024);       // the same tiles as "K rows" operands
-      auto ring_off = [](int hn) { return (uint32_t)((hn % kRing) * 3 * kHalfTile); };
-      auto issue_l0 = [&](int hn) {                                          // L0^T -> Z (both operands in shared memory)
-        const uint32_t st = ring_off(hn);
-        mbar_wait(&bar_ld[hn % kRing], (uint32_t)((hn / kRing) & 1), status, 401);
-        tc_fence_after_sync();
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ss(tmem + kColZ, at(kK0, ks * 32), at(kRingD, st + kHalfTile + ks * 32), idesc_t, ks > 0);
-        mma_commit(&bar_l0);
+      auto load_q0 = [&](int hn, int slot) {
+        mbar_expect_tx(&bars[LD0 + slot], kHalfTile);
+        tma_load_4d(smem + L::ring0 + slot * kHalfTile, &map_q0, &bars[LD0 + slot], 0, row_of(hn), 0, b);
       };
-      auto issue_s = [&](int hn) {                                           // S^T -> Y (A = K from TMEM)
-        const uint32_t st = ring_off(hn);
-        if (SELF) {                                                          // (otherwise issue_l0 has waited for the slot)
-          mbar_wait(&bar_ld[hn % kRing], (uint32_t)((hn / kRing) & 1), status, 401);
-          tc_fence_after_sync();
-        }
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ts(tmem + kColY, tmem + kColK + ks * 8, at(kRingD, st + ks * 32), idesc_t, ks > 0);
-        mma_commit(&bar_s);
-      };
-      auto issue_dp = [&](int hn) {                                          // dP^T -> X (A = V from TMEM)
-        const uint32_t st = ring_off(hn);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ts(tmem + kColX, tmem + kColV + ks * 8, at(kRingD, st + 2 * kHalfTile + ks * 32), idesc_t, ks > 0);
-        mma_commit(&bar_dp);
-      };
-      // dV += P^T dO; dK += dz^T Q: A from TMEM, 16 queries = 8 packed columns at a stride of 16 columns
-      auto issue_dv_dk = [&](int hn) {
-        const uint32_t st = ring_off(hn);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ts(tmem + kColDV, tmem + kColY + ks * 16, at(mRingD, st + 2 * kHalfTile + ks * 2048), idesc_acc,
-                 (hn == 0 && ks == 0) ? 0u : 1u);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ts(tmem + kColDK, tmem + kColY + ks * 16 + 8, at(mRingD, st + ks * 2048), idesc_acc,
-                 (hn == 0 && ks == 0) ? 0u : 1u);
-      };
-      auto issue_dk0 = [&](int hn) {                                         // dK0 += g^T Q0 (A from TMEM)
-        const uint32_t st = ring_off(hn);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ts(tmem + kColDK0, tmem + kColX + ks * 16, at(mRingD, st + kHalfTile + ks * 2048), idesc_acc,
-                 (hn == 0 && ks == 0) ? 0u : 1u);
-        mma_commit(&bar_free[hn % kRing]);                                   // every MMA reading this ring slot is issued
-      };
-      auto issue_dq0 = [&](int it) {                                         // dQ0 = g K0 into the shared accumulator
-        mbar_wait(&bar_dqread, (uint32_t)(it & 1), status, 407);             // dQ of that tile has been read out
-        tc_fence_after_sync();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          mma_ss(tmem + kColDQ, at(mG, ks * 2048), at(mK0, ks * 2048), idesc_dq, ks > 0);
-        mma_commit(&bar_dq0);
-      };
-
-      mbar_expect_tx(&bar_kv, (SELF ? 2 : 3) * kRowTile);
-      tma_load_4d(smem + L::k, &map_k, &bar_kv, 0, nj * kTile, h, b);
-      tma_load_4d(smem + L::v, &map_v, &bar_kv, 0, nj * kTile, h, b);
-      if (!SELF) tma_load_4d(smem + L::k0, &map_k0, &bar_kv, 0, nj * kTile, 0, b);
-      for (int hn = 0; hn < kRing && hn < n_half; ++hn) load_half(hn);
-      mbar_wait(&bar_setup, 0, status, 400);                   // K and V are in TMEM
-      tc_fence_after_sync();
-      if (!SELF) issue_l0(0);
-      issue_s(0);
-      issue_dp(0);
-
-#pragma unroll 2   // the half's parity becomes a constant in each copy (-1.2 %; by six, to fix the ring slot too: +8 %)
+      mbar_expect_tx(&bars[KV], (SELF ? 2 : 3) * kRowTile);
+      if (!SELF) tma_load_4d(smem + L::k0, &map_k0, &bars[KV], 0, nj * kTile, 0, b);
+      tma_load_4d(smem + L::k, &map_k, &bars[KV], 0, nj * kTile, h, b);
+      tma_load_4d(smem + L::v, &map_v, &bars[KV], 0, nj * kTile, h, b);
+      // The slots of a half come free in the order dz, g of one half, then of the next: (Q, dO) first, then Q0.
+      int slot = 0, slot0 = 0;
+      uint32_t par = 1, par0 = 1;                                  // of the freeing before this fill (the first fills wait for none)
+#pragma unroll 1
       for (int hn = 0; hn < n_half; ++hn) {
-        const int second = hn & 1, it = hn >> 1;               // second: the lower half, which completes a query tile
-        const uint32_t ph = (uint32_t)(hn & 1);
-        const bool more = hn + 1 < n_half;
-        if (hn >= 1 && hn - 1 + kRing < n_half) {             // the slot of half hn - 1 is free once its last MMA is done
-          mbar_wait(&bar_free[(hn - 1) % kRing], (uint32_t)(((hn - 1) / kRing) & 1), status, 403);
-          load_half(hn - 1 + kRing);
-        }
+        if (hn >= R) wait(bar(FREE + slot), par, 402);
+        load_qdo(hn, slot);
+        if (++slot == R) { slot = 0; par ^= 1u; }
         if (!SELF) {
-          mbar_wait(&bar_sel, ph, status, 402);                // L0^T read by every thread: Z takes the next half's
-          tc_fence_after_sync();
-          if (more) issue_l0(hn + 1);
-          if (!second && it > 0) issue_dq0(it - 1);            // dQ0 of the previous tile (its dQ was read out at that tile's end)
-        }
-        mbar_wait(&bar_early, ph, status, 404);                // P^T (and dz^T) in place, S^T and dP^T read
-        tc_fence_after_sync();
-        if (SELF) {
-          const uint32_t st = ring_off(hn);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)                       // dV += P^T dO; dK waits for dz + g
-            mma_ts(tmem + kColDV, tmem + kColY + ks * 16, at(mRingD, st + 2 * kHalfTile + ks * 2048), idesc_acc,
-                   (hn == 0 && ks == 0) ? 0u : 1u);
-        } else {
-          issue_dv_dk(hn);                                     // they read P^T and dz^T, which the next S^T overwrites
-        }
-        if (more) issue_s(hn + 1);
-        if (!SELF && second) {                                 // dQ = dz K over all 128 keys
-          if (it > 0) {
-            mbar_wait(&bar_dq0read, (uint32_t)((it - 1) & 1), status, 405);   // dQ0 of the previous tile has been read out
-            tc_fence_after_sync();
-          }
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            mma_ss(tmem + kColDQ, at(mDZ, ks * 2048), at(mK, ks * 2048), idesc_dq, ks > 0);
-          mma_commit(&bar_dq);
-        }
-        mbar_wait(&bar_g, ph, status, 406);                    // g^T and the g half written (one head per selector: dz + g)
-        tc_fence_after_sync();
-        if (SELF) {
-          const uint32_t st = ring_off(hn);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)                       // dK += (dz + g)^T Q, A from TMEM (this thread's X columns)
-            mma_ts(tmem + kColDK, tmem + kColX + ks * 16, at(mRingD, st + ks * 2048), idesc_acc,
-                   (hn == 0 && ks == 0) ? 0u : 1u);
-          mma_commit(&bar_free[hn % kRing]);
-        } else {
-          issue_dk0(hn);                                       // it reads g^T, which the next dP^T overwrites
-        }
-        if (more) issue_dp(hn + 1);
-        if (SELF && second) {                                  // dQ = (dz + g) K over all 128 keys
-          if (it > 0) {
-            mbar_wait(&bar_dqread, (uint32_t)((it - 1) & 1), status, 407);    // dQ of the previous tile has been read out
-            tc_fence_after_sync();
-          }
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            mma_ss(tmem + kColDQ, at(mDZ, ks * 2048), at(mK, ks * 2048), idesc_dq, ks > 0);
-          mma_commit(&bar_dq);
+          if (hn >= 3) wait(bar(FREE0 + slot0), par0, 403);
+          load_q0(hn, slot0);
+          if (++slot0 == 3) { slot0 = 0; par0 ^= 1u; }
         }
       }
-      if (!SELF) issue_dq0(n_iter - 1);
-      mma_commit(&bar_fin);
     }
     __syncwarp();
-  } else {
-    // ======================================= arithmetic warps ============================================
-    const int row = tid & 127, wg = tid >> 7;
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);   // a warp reaches lanes 32 (warp % 4) ..
-    const int j = nj * kTile + row;
-    float dz_state = 0.f;            // sum of dz over the queries already visited (later queries), this key
-
-    Ctx ctx;
-    ctx.dz_tile = smem + L::dz;
-    ctx.g_tile = smem + L::g;
-    ctx.tmem = tmem;
-    ctx.lane_base = lane_base;
-    ctx.row = row;
-    ctx.wg = wg;
-    ctx.selectable = (j >= exempt);
-    ctx.c1 = scale * kLog2e;
-    ctx.lse_s = lse_s;
-    ctx.dbar_s = dbar_s;
-    ctx.sel_tot = sel_tot;
-    ctx.dz_tot = dz_tot;
-    ctx.status = status;
-
-    auto fetch_lse = [&](int mi) {
-      const int i = mi * kTile + tid;
-      return (tid < kTile && i < seq) ? load_ahead(lse2 + (int64_t)n * seq + i) : INFINITY;   // +inf: P = 0 for padded queries
+  } else if (warp == kMmaWarp) {
+    // ========================================== MMA issue ==================================================
+    // The whole warp walks this code, so that addresses and descriptors stay in uniform registers; one elected lane issues.
+    const uint32_t idesc_t = instr_desc_bf16(128, 64, false, false);     // keys x 64 queries, K = D
+    const uint32_t idesc_acc = instr_desc_bf16(128, 64, false, true);    // A K-major (keys x queries), B MN-major
+    const uint32_t idesc_dq = instr_desc_bf16(128, 64, true, true);      // A MN-major (queries x keys), B MN-major
+    const uint32_t kBase = desc_low(sa, 16);                             // K-major views (rows = M or N index)
+    const uint32_t mBase = desc_low(sa, kRowTile);                       // MN-major views (rows = K index)
+    auto at = [](uint32_t low, uint32_t byte_off) { return low + (byte_off >> 4); };
+    const int tiles = LIVE ? __shfl_sync(0xffffffffu, n_iter, 0) : n_iter;
+    auto await = [&](int id, uint32_t parity, int site) {
+      wait.left = wait_call(bar(id), parity, site, wait.left);
     };
-    auto fetch_dbar = [&](int mi) {
-      const int i = mi * kTile + tid;
-      return (tid < kTile && i < seq) ? load_ahead(dbar + (int64_t)n * seq + i) : 0.f;
-    };
-    auto fetch_carry = [&](int mi) {
-      return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1) * seq + j) : 0.f;
-    };
-    float next_lse = fetch_lse(mi_top), next_dbar = fetch_dbar(mi_top), next_carry = fetch_carry(mi_top);
-
-    // K and V rows from their landing tiles into TMEM as bf16 pairs (A operands of the score products); warpgroup
-    // wg moves 16 of the 64 d columns = two 16-byte chunks = 8 packed columns of each matrix
-    mbar_wait(&bar_kv, 0, status, 409);
-    {
-      const int offs[2] = {L::k, L::v};
-      const uint32_t cols[2] = {kColK, kColV};
+    // TMEM addresses: the CTA owns all 512 columns, so they start at column 0.
+    // d (64 columns) = A x B over four K steps of 16: A from shared memory, or from TMEM (8 packed columns a step)
+    auto product_ss = [&](uint32_t d, uint32_t a_off, uint32_t b_off, int done) {
+      if (elect_one()) {
+        const uint32_t bl = at(kBase, b_off);
+        mma_ss_low<false>(d, at(kBase, a_off), bl, idesc_t);
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        uint32_t w8[8];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const uint4 v4 = *reinterpret_cast<const uint4*>(smem + offs[m] + swz_off(row, wg * 2 + c));
-          w8[4 * c] = v4.x; w8[4 * c + 1] = v4.y; w8[4 * c + 2] = v4.z; w8[4 * c + 3] = v4.w;
-        }
-        tmem_st8(lane_base + cols[m] + wg * 8, w8);
+        for (int ks = 1; ks < 4; ++ks) mma_ss_low<true>(d, at(kBase, a_off + ks * 32), at(bl, ks * 32), idesc_t);
+        mma_commit(bar(done));
       }
+      __syncwarp();
+    };
+    auto product_ts = [&](uint32_t d, uint32_t a_col, uint32_t b_off, int done) {
+      if (elect_one()) {
+        const uint32_t bl = at(kBase, b_off);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mma_ts_low(d, a_col + ks * 8, at(bl, ks * 32), idesc_t, ks > 0 ? 1u : 0u);
+        mma_commit(bar(done));
+      }
+      __syncwarp();
+    };
+    auto issue_l0 = [&](uint32_t c, uint32_t slot) {                     // L0^T -> W1
+      product_ss(w1_of(c), L::k0, L::ring0 + slot * kHalfTile, L0 + (int)c);
+    };
+    auto issue_s = [&](uint32_t c, uint32_t slot) {                      // S^T -> W2
+      if (SELF) product_ts(w2_of(c), kKA, L::ring + slot * L::kSlot, S + (int)c);
+      else product_ss(w2_of(c), L::k, L::ring + slot * L::kSlot, S + (int)c);
+    };
+    auto issue_dp = [&](uint32_t c, uint32_t slot) {                     // dP^T -> W1
+      if (SELF) product_ts(w1_of(c), kVA, L::ring + slot * L::kSlot + kHalfTile, DP + (int)c);
+      else product_ss(w1_of(c), L::v, L::ring + slot * L::kSlot + kHalfTile, DP + (int)c);
+    };
+    // acc (64 columns) += A (TMEM, 16 queries are 8 packed columns) x the half tile at `off`
+    auto accumulate = [&](uint32_t acc, uint32_t a_col, uint32_t off, uint32_t keep) {
+      const uint32_t rows = at(mBase, off);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) mma_ts_low(acc, a_col + ks * 8, at(rows, ks * 2048), idesc_acc, ks > 0 ? 1u : keep);
+    };
+    auto issue_dq = [&](uint32_t a_off, uint32_t b_off, int done) {  // dQ = dz K, dQ0 = g K0 over the tile's 128 keys
+      if (elect_one()) {
+        mma_ss_low<false>(kDQ, at(mBase, a_off), at(mBase, b_off), idesc_dq);
+#pragma unroll
+        for (int ks = 1; ks < 8; ++ks) mma_ss_low<true>(kDQ, at(mBase, a_off + ks * 2048), at(mBase, b_off + ks * 2048), idesc_dq);
+        mma_commit(bar(done));
+      }
+      __syncwarp();
+    };
+    // Half hn of chain hn & 1 uses slot hn mod ring; `Ring` walks the halves in order.
+    struct Ring { uint32_t slot, par; };
+    auto next = [](Ring& x, uint32_t ring) {
+      if (++x.slot == ring) { x.slot = 0; x.par ^= 1u; }
+    };
+    Ring s_ring{0, 0}, l_ring{0, 0};                                     // of the next S^T and L0^T to issue
+    Ring use{0, 0}, use0{0, 0}, sel{0, 0};                               // of the half whose products are served (dz, g; selection)
+    auto ask_s = [&](uint32_t c) {                                       // S^T (SELF: and dP^T) of the chain's next half
+      await(LD + (int)s_ring.slot, s_ring.par, 403);
+      issue_s(c, s_ring.slot);
+      if (SELF) issue_dp(c, s_ring.slot);
+      next(s_ring, R);
+    };
+    auto ask_l0 = [&](uint32_t c) {
+      await(LD0 + (int)l_ring.slot, l_ring.par, 404);
+      issue_l0(c, l_ring.slot);
+      next(l_ring, 3);
+    };
+    // Chain 1 runs half a tile behind chain 0: while half hn is in its selection, the half before it, of the other chain,
+    // comes to its dz and g.  The order below is the order in which their events come then.
+    await(SELF ? SETUP : KV, 0, 400);                          // K, V (and K0) in place
+    ask_s(0);
+    if (!SELF) ask_l0(0);
+    ask_s(1);
+    if (!SELF) ask_l0(1);
+    const int halves = 2 * tiles;
+#pragma unroll 1
+    for (int hn = 0; hn <= halves; ++hn) {
+      const uint32_t c = (uint32_t)(hn & 1), p = c ^ 1u;                 // chain of half hn, and of the half before it
+      if (!SELF && hn < halves) {                                        // L0^T read: dP^T takes its columns
+        await(SEL + (int)c, (uint32_t)((hn >> 1) & 1), 405);
+        issue_dp(c, sel.slot);
+        next(sel, R);
+      }
+      if (hn == 0) continue;
+      const uint32_t ph = (uint32_t)(((hn - 1) >> 1) & 1);               // of half hn - 1
+      const uint32_t keep = hn > 1 ? 1u : 0u;
+      await(DZ + (int)p, ph, 406);                                         // P^T, dz^T written: dV, dK, then the next half's S^T
+      if (elect_one()) {
+        accumulate(kDV, w2_of(p), L::ring + use.slot * L::kSlot + kHalfTile, keep);
+        if (!SELF) {
+          accumulate(kDK, w2_of(p) + 32, L::ring + use.slot * L::kSlot, keep);
+          mma_commit(bar(FREE + (int)use.slot));
+        }
+      }
+      __syncwarp();
+      if (!SELF) {
+        if (hn + 1 < halves) ask_s(p);
+        if (p == 1) {                                                    // both halves of the tile: dQ
+          if (hn > 2) await(ACC, 1u, 408);                          // dQ0 of the tile before has been read out
+          issue_dq(L::dz, L::k, DQ);
+        }
+      }
+      await(G + (int)p, ph, 407);                                          // g^T written: dK0, then the next half's L0^T
+      if (elect_one()) {
+        if (SELF) {
+          accumulate(kDK, w1_of(p), L::ring + use.slot * L::kSlot, keep);
+          mma_commit(bar(FREE + (int)use.slot));
+        } else {
+          accumulate(kDK0, w1_of(p), L::ring0 + use0.slot * kHalfTile, keep);
+          mma_commit(bar(FREE0 + (int)use0.slot));
+        }
+      }
+      __syncwarp();
+      next(use, R);
+      next(use0, 3);
+      if (hn + 1 < halves) {
+        if (SELF) ask_s(p);
+        else ask_l0(p);
+      }
+      if (p == 1) {
+        if (SELF) {
+          if (hn > 2) await(ACC, ph ^ 1u, 408);                     // dQ of the tile before
+          issue_dq(L::dz, L::k, DQ);
+        } else {
+          await(ACC, 0u, 409);                                      // dQ of this tile
+          issue_dq(L::g, L::k0, DQ0);
+        }
+      }
+    }
+    if (elect_one()) mma_commit(bar(FIN));
+    __syncwarp();
+  } else if (warp < 12) {
+    // ==================== read-out of dQ, dQ0: lanes are queries, a warp's 32 rows at a time ====================
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    uint8_t* stage = smem + L::out + (warp - 8) * 8192;           // two [32 queries][32 floats] boxes, 128-byte swizzle
+    const int n_reads = SELF ? n_iter : n_half;
+    for (int r = 0; r < n_reads; ++r) {
+      const int t = SELF ? r : r >> 1;
+      const bool second = !SELF && (r & 1);
+      wait(bar(second ? DQ0 : DQ), (uint32_t)(t & 1), 413);
+      tc_fence_after_sync();
+      if (lane == 0) bulk_wait_read();                            // the last reduce-add has read the staging boxes
+#pragma unroll 1
+      for (int x = 0; x < 2; ++x) {
+        uint32_t a[32];
+        tmem_ld32(lane_base + kDQ + 32 * x, a);
+        tmem_ld_wait();
+        if (x == 1) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(ACC));                   // the accumulator may be overwritten
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          *reinterpret_cast<float4*>(stage + x * 4096 + swz_off(lane, c)) =
+              make_float4(__uint_as_float(a[4 * c]) * scale, __uint_as_float(a[4 * c + 1]) * scale,
+                          __uint_as_float(a[4 * c + 2]) * scale, __uint_as_float(a[4 * c + 3]) * scale);
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        const CUtensorMap* map = second ? &map_dq0 : &map_dq;
+        const int row = second ? b * dq0_rows : n, q0 = (mi_top - t) * kTile + (warp - 8) * 32;
+        if (q0 < seq) {
+          tma_reduce_add_4d(map, stage, 0, q0, row, 0);
+          tma_reduce_add_4d(map, stage + 4096, 32, q0, row, 0);
+          bulk_commit();
+        }
+      }
+    }
+    if (!SELF) {                                                  // this head's share of dK0
+      wait(bar(FIN), 0, 415);
+      tc_fence_after_sync();
+      const int j = nj * kTile + (warp - 8) * 32 + lane;
+      float* row = dk0 + ((int64_t)b * seq + j) * D;
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        uint32_t r0[32];
+        tmem_ld32(lane_base + kDK0 + 32 * x, r0);
+        tmem_ld_wait();
+        if (j < seq) store_key_grads<false, 32>(nullptr, nullptr, r0, scale, nullptr, nullptr, row + 32 * x, false);
+      }
+    }
+    if (lane == 0) bulk_wait_all();                               // the last reduce-adds must land before the CTA exits
+    __syncwarp();
+  }
+  } else {
+    regs_grow<kChainRegs>();
+    // ============================================ the two chains ============================================
+    const int c = warp >> 2, row = tid & 127, other = c ^ 1;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);   // a warp reaches lanes 32 (warp % 4) ..
+    const uint32_t w1 = lane_base + w1_of(c), w2 = lane_base + w2_of(c);
+    const int j = nj * kTile + row;
+    const float c1 = scale * kLog2e;
+    const float c1_hist = (j >= exempt) ? c1 : 0.f;                // an exempt key has no history and no gate
+    const float shut = (j >= exempt) ? -1.4e-45f : -INFINITY;
+    // this thread's row in its chain's query half of the dz tile (the g tile lies kG further on); chunk x of it is at ^ 16 x
+    constexpr uint32_t kG = SELF ? 0 : L::g - L::dz;
+    const uint32_t my_row = sa + L::dz + (1 - c) * kRowTile + row * 128 + ((row & 7) << 4);
+    const uint32_t run_addr = smem_u32(&run_s[row]);
+    auto put8 = [&](uint32_t at, int chunk, const uint32_t* w) {             // eight queries of this thread's key
+      st_shared16(at ^ (uint32_t)(chunk << 4), w[0], w[1], w[2], w[3]);
+    };
+    auto arrive = [&](int id) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(id));
+    };
+    // chain 0 starts from the carry after the tile, chain 1 from the carry before it plus its own half's sum
+    auto fetch_carry = [&](int mi) {
+      return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1 - c) * seq + j) : 0.f;
+    };
+    float next_carry = fetch_carry(mi_top);
+
+    if (SELF) {                                                    // K (chain 0) and V (chain 1) rows into TMEM as bf16 pairs
+      wait(bar(KV), 0, 409);
+      const uint8_t* src = smem + (c == 0 ? L::k : L::v);
+      uint32_t w32[32];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint4 v4 = *reinterpret_cast<const uint4*>(src + swz_off(row, u));
+        w32[4 * u] = v4.x; w32[4 * u + 1] = v4.y; w32[4 * u + 2] = v4.z; w32[4 * u + 3] = v4.w;
+      }
+      tmem_st32(lane_base + (c == 0 ? kKA : kVA), w32);
       tmem_st_wait();
       tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_setup);
+      arrive(SETUP);
     }
 
-    // The shared accumulator (here the lane is a QUERY row, columns are d) -> scaled fp32 staging tile -> TMA reduce-add.
-    auto read_out = [&](uint64_t* done_bar, const CUtensorMap* map, int i0, int row_index) {
-      const int c0 = wg * kChunk;
-      uint32_t r[16];
-      tmem_ld16(lane_base + kColDQ + c0, r);
-      tmem_ld_wait();
-      uint8_t* sq = smem + L::out + (wg >> 1) * kRowTile;     // [128 queries][32 floats] tiles, 128-byte swizzle
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<float4*>(sq + swz_off(row, (wg & 1) * 4 + c)) =
-            make_float4(__uint_as_float(r[4 * c]) * scale, __uint_as_float(r[4 * c + 1]) * scale,
-                        __uint_as_float(r[4 * c + 2]) * scale, __uint_as_float(r[4 * c + 3]) * scale);
-      fence_async_smem();
-      tc_fence_before_sync();
-      named_barrier(kComputeBarrier, kComputeThreads);
-      if (tid == 0) {
-        mbar_arrive(done_bar);                                // the accumulator may be overwritten
-        tma_reduce_add_4d(map, smem + L::out, 0, i0, row_index, 0);
-        tma_reduce_add_4d(map, smem + L::out + kRowTile, 32, i0, row_index, 0);
-        bulk_commit();
-      }
-    };
-
-    HalfState st;
-    // One query tile.  The diagonal tile (the only one that needs the causal mask inside the tile) is the LAST of the
-    // walk, so the loop runs the unmasked form only and the masked form follows it once.
-    auto tile = [&](int it, auto diag_tag) {
+    int slot = c;
+    uint32_t ld_par = 0;
+    auto half = [&](int it, auto diag_tag) {
       constexpr bool kDiag = decltype(diag_tag)::value;
       const int mi = mi_top - it;
-      const int i0 = mi * kTile;
       const uint32_t ph = (uint32_t)(it & 1);
-      if (tid < kTile) {
-        lse_s[tid] = -next_lse;                                // negated: both enter packed adds directly
-        dbar_s[tid] = -next_dbar;
-      }
-      const float cnl = next_carry * kLog2e;
-      if (it + 1 < n_iter) {
-        next_lse = fetch_lse(mi - 1);
-        next_dbar = fetch_dbar(mi - 1);
-        next_carry = fetch_carry(mi - 1);
-      }
-      float sel_state = 0.f;         // selection of the tile's queries already visited, this key (raw logit units)
+      const int diag = row - (1 - c) * 64;                         // kDiag: query e of the half is this key itself
+      const uint32_t stat = sa + L::stat + slot * kStatBytes;
+      const float carry_log2 = next_carry * kLog2e;
+      if (it + 1 < n_iter) next_carry = fetch_carry(mi - 1);
 
-#pragma unroll   // both halves inline: with the masked form out of the loop this is worth 4.5 % (7 % for one head per selector)
-      for (int hf = 1; hf >= 0; --hf) {
-        const uint32_t hp = (uint32_t)(1 - hf);               // parity of this half's barrier phases
-        // the staging tile is written next at the read-out that follows this half's dz pass (dQ0 of the previous
-        // tile after the upper half, dQ of this tile after the lower half): its last reduce-add must have read it
-        const bool drain = SELF ? (hf == 1 && it > 0) : ((it > 0) || (hf == 0));
-        half_scores<kDiag, SELF>(ctx, hf, hp, cnl, sel_state, st, &bar_l0, &bar_sel, &bar_s, &bar_dp, &bar_early, drain, true);
-        if (hf == 1 && it > 0) {                               // the previous tile's last product, issued a half-tile ago:
-          if (SELF) {                                          //   dQ = (dz + g) K, or dQ0 = g K0
-            mbar_wait(&bar_dq, (uint32_t)((it - 1) & 1), status, 413);
-            tc_fence_after_sync();
-            read_out(&bar_dqread, &map_dq, i0 + kTile, n);
+      // ---- selection: relu(L0^T), the gate, and the sums of eight queries at a time ------------------------------
+      float v[64];
+      uint32_t off[SELF ? 2 : 32];                                 // where the gate is shut: bits, or masks of bf16 pairs
+      float part[8];
+      wait(bar((SELF ? S : L0) + c), ph, 410);
+      tc_fence_after_sync();
+      {
+        uint32_t r[2][32];
+        tmem_ld32((SELF ? w2 : w1), r[0]);
+        tmem_ld32((SELF ? w2 : w1) + 32, r[1]);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        if (!SELF) arrive(SEL + c);                             // W1 may take dP^T
+        if (SELF) off[0] = off[1] = 0u;
+#pragma unroll
+        for (int e = 0; e < 64; e += 2) {
+          float l0 = __uint_as_float(r[e >> 5][e & 31]), l1 = __uint_as_float(r[e >> 5][(e & 31) + 1]);
+          if (kDiag) {                                             // key strictly before the query
+            if (e <= diag) l0 = -1.f;
+            if (e + 1 <= diag) l1 = -1.f;
+          }
+          // the gate is open for l0 > 0: the sign of l0 minus the smallest number (an exempt key: minus infinity)
+          const float2 t = __fadd2_rn(make_float2(l0, l1), make_float2(shut, shut));
+          if constexpr (SELF) {
+            off[e >> 5] = __funnelshift_l(__float_as_uint(t.x), off[e >> 5], 1);      // query e ends up at bit 31 - e % 32
+            off[e >> 5] = __funnelshift_l(__float_as_uint(t.y), off[e >> 5], 1);
           } else {
-            mbar_wait(&bar_dq0, (uint32_t)((it - 1) & 1), status, 412);
-            tc_fence_after_sync();
-            read_out(&bar_dq0read, &map_dq0, i0 + kTile, b);
+            off[e >> 1] = sign_masks(t.x, t.y);
+          }
+          v[e] = fmaxf(l0, 0.f);
+          v[e + 1] = fmaxf(l1, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          float2 s = __fadd2_rn(make_float2(v[8 * u], v[8 * u + 1]), make_float2(v[8 * u + 2], v[8 * u + 3]));
+          s = __fadd2_rn(s, __fadd2_rn(make_float2(v[8 * u + 4], v[8 * u + 5]), make_float2(v[8 * u + 6], v[8 * u + 7])));
+          part[u] = s.x + s.y;
+        }
+      }
+#pragma unroll
+      for (int u = 6; u >= 0; --u) part[u] += part[u + 1];         // part[u]: the sum from query 8 u on
+      // F log2e = cb - c1 * (sum from the query on)
+      const float ncb = (c == 0) ? -carry_log2 : -fmaf(c1_hist, part[0], carry_log2);
+
+      // ---- probabilities: P = exp2(c1 (S + suffix) - cb - lse) -----------------------------------------------------
+      if (!SELF) {
+        wait(bar(S + c), ph, 416);
+        tc_fence_after_sync();
+      }
+      wait(bar(LD + slot), ld_par, 417);               // (complete by now) the statistics are in place
+      const float2 cc = make_float2(c1, c1), ch = make_float2(c1_hist, c1_hist), nb = make_float2(ncb, ncb);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t r[16], w8[8];
+        tmem_ld16(w2 + 16 * q, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 2 * q; u < 2 * q + 2; ++u) {                  // inclusive suffix sums of eight queries
+          float run = (u < 7) ? part[u + 1] : 0.f;
+#pragma unroll
+          for (int e = 8 * u + 7; e >= 8 * u; --e) {
+            run += v[e];
+            v[e] = run;
           }
         }
-        half_gate<SELF>(ctx, hf, dz_state, st, true);
-        fence_async_smem();                                    // g half tile -> visible to the MMAs
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_g);
+#pragma unroll
+        for (int e4 = 0; e4 < 16; e4 += 4) {
+          const float4 nl = ld_shared_f4(stat + 4 * (16 * q + e4));
+          const float2 nls[2] = {make_float2(nl.x, nl.y), make_float2(nl.z, nl.w)};
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int e = 16 * q + e4 + 2 * k;
+            const float2 hist = __ffma2_rn(make_float2(v[e], v[e + 1]), ch, __fadd2_rn(nls[k], nb));
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])), cc, hist);
+            v[e] = ex2(x.x);
+            v[e + 1] = ex2(x.y);
+            if (kDiag) {                                           // key after the query
+              if (e < diag) v[e] = 0.f;
+              if (e + 1 < diag) v[e + 1] = 0.f;
+            }
+            w8[(e4 >> 1) + k] = pack_bf16(v[e], v[e + 1]);
+          }
+        }
+        tmem_st8(w2 + 8 * q, w8);                                  // over S^T columns that have been read
       }
-      if (!SELF) {
-        mbar_wait(&bar_dq, ph, status, 413);                   // dQ of this tile, issued before the last g pass
-        tc_fence_after_sync();
-        read_out(&bar_dqread, &map_dq, i0, n);
-      }
-    };
-    for (int it = 0; it + 1 < n_iter; ++it) tile(it, std::false_type{});
-    tile(n_iter - 1, std::true_type{});
-    {                                                          // the first query tile's last product, visited last
-      mbar_wait(SELF ? &bar_dq : &bar_dq0, (uint32_t)((n_iter - 1) & 1), status, 414);
-      tc_fence_after_sync();
-      if (tid == 0) bulk_wait_read();
-      named_barrier(kComputeBarrier, kComputeThreads);
-      if (SELF) read_out(&bar_dqread, &map_dq, nj * kTile, n);
-      else read_out(&bar_dq0read, &map_dq0, nj * kTile, b);
-    }
 
-    // ---- epilogue: dV, dK (this head) and this head's share of dK0 ------------------------------------------
-    mbar_wait(&bar_fin, 0, status, 415);
+      // ---- dz = P (dP - dbar) ------------------------------------------------------------------------------------
+      wait(bar(DP + c), ph, 411);
+      tc_fence_after_sync();
+      if (!SELF && it > 0) wait(bar(DQ), ph ^ 1u, 418);   // dQ of the tile before has read the dz tile
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t r[16], w8[8];
+        tmem_ld16(w1 + 16 * q, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e4 = 0; e4 < 16; e4 += 4) {
+          const float4 nd = ld_shared_f4(stat + 4 * (64 + 16 * q + e4));
+          const float2 nds[2] = {make_float2(nd.x, nd.y), make_float2(nd.z, nd.w)};
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int e = 16 * q + e4 + 2 * k;
+            const float2 d = __fmul2_rn(make_float2(v[e], v[e + 1]),
+                                        __fadd2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])),
+                                                   nds[k]));
+            v[e] = d.x;
+            v[e + 1] = d.y;
+            if (!SELF) w8[(e4 >> 1) + k] = pack_bf16(d.x, d.y);
+          }
+        }
+#pragma unroll
+        for (int u = 2 * q; u < 2 * q + 2; ++u) {
+          float2 s = __fadd2_rn(make_float2(v[8 * u], v[8 * u + 1]), make_float2(v[8 * u + 2], v[8 * u + 3]));
+          s = __fadd2_rn(s, __fadd2_rn(make_float2(v[8 * u + 4], v[8 * u + 5]), make_float2(v[8 * u + 6], v[8 * u + 7])));
+          part[u] = s.x + s.y;
+        }
+        if (!SELF) {                                               // dz: to TMEM (A of dK) and shared memory (A of dQ)
+          tmem_st8(w2 + 32 + 8 * q, w8);
+          put8(my_row, 2 * q, w8);
+          put8(my_row, 2 * q + 1, w8 + 4);
+        }
+      }
+      if (!SELF) fence_async_smem();                               // dz half tile -> visible to the MMAs
+      tmem_st_wait();
+      tc_fence_before_sync();
+      arrive(DZ + c);
+#pragma unroll
+      for (int u = 6; u >= 0; --u) part[u] += part[u + 1];
+
+      // ---- the sum of dz over later queries, handed from half to half ----------------------------------------------
+      float base = 0.f;
+      if (c == 1 || it > 0) {
+        wait(bar(TOK + other), c == 1 ? ph : ph ^ 1u, 419);
+        base = run_s[row];
+      }
+      run_s[row] = base + part[0];
+      arrive(TOK + c);
+
+      // ---- g = gate ? -(sum of dz over later queries) : 0; SELF: dz + g --------------------------------------------
+      if (it > 0) wait(bar(SELF ? DQ : DQ0), ph ^ 1u, 420);   // the tile before has been read
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t w8[8];
+#pragma unroll
+        for (int u = 2 * q; u < 2 * q + 2; ++u) {
+          float run = -base - ((u < 7) ? part[u + 1] : 0.f);
+#pragma unroll
+          for (int e = 8 * u + 7; e >= 8 * u; --e) {
+            const float dz = v[e];
+            if constexpr (SELF) v[e] = ((off[e >> 5] >> (31 - (e & 31))) & 1u) ? dz : dz + run;
+            else v[e] = run;
+            run -= dz;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          w8[e] = pack_bf16(v[16 * q + 2 * e], v[16 * q + 2 * e + 1]);
+          if constexpr (!SELF) w8[e] &= ~off[8 * q + e];
+        }
+        tmem_st8(w1 + 8 * q, w8);                                  // over dP^T columns that have been read
+        put8(my_row + kG, 2 * q, w8);
+        put8(my_row + kG, 2 * q + 1, w8 + 4);
+      }
+      fence_async_smem();
+      tmem_st_wait();
+      tc_fence_before_sync();
+      arrive(G + c);
+      slot += 2;
+      if (slot >= R) { slot -= R; ld_par ^= 1u; }
+    };
+    for (int it = 0; it + 1 < n_iter; ++it) half(it, std::false_type{});
+    half(n_iter - 1, std::true_type{});
+
+    // ---- epilogue: dV (chain 0) and dK (chain 1) of this key tile -------------------------------------------------
+    wait(bar(FIN), 0, 415);
     tc_fence_after_sync();
-    {
-      const int c0 = wg * kChunk;
-      __nv_bfloat16* dv_row = dv + dv_rows.at(b, h, j) + c0;
-      float* dk_row = dk_acc + ((int64_t)n * seq + j) * D + c0;
-      float* dk0_row = dk0 + ((int64_t)b * seq + j) * D + c0;
-      uint32_t rv[16], rk[16], r0[16];
-      tmem_ld16(lane_base + kColDV + c0, rv);
-      tmem_ld16(lane_base + kColDK + c0, rk);
-      if (!SELF) tmem_ld16(lane_base + kColDK0 + c0, r0);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      uint32_t r[32];
+      tmem_ld32(lane_base + (c == 0 ? kDV : kDK) + 32 * x, r);
       tmem_ld_wait();
       if (j < seq) {
-#pragma unroll
-        for (int e = 0; e < 16; e += 8) {
-          uint4 w = make_uint4(pack_bf16(__uint_as_float(rv[e]), __uint_as_float(rv[e + 1])),
-                               pack_bf16(__uint_as_float(rv[e + 2]), __uint_as_float(rv[e + 3])),
-                               pack_bf16(__uint_as_float(rv[e + 4]), __uint_as_float(rv[e + 5])),
-                               pack_bf16(__uint_as_float(rv[e + 6]), __uint_as_float(rv[e + 7])));
-          *reinterpret_cast<uint4*>(dv_row + e) = w;
-        }
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          *reinterpret_cast<float4*>(dk_row + e) =
-              make_float4(__uint_as_float(rk[e]) * scale, __uint_as_float(rk[e + 1]) * scale,
-                          __uint_as_float(rk[e + 2]) * scale, __uint_as_float(rk[e + 3]) * scale);
-          if (!SELF)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dk0_row + e),
-                       "f"(__uint_as_float(r0[e]) * scale), "f"(__uint_as_float(r0[e + 1]) * scale),
-                       "f"(__uint_as_float(r0[e + 2]) * scale), "f"(__uint_as_float(r0[e + 3]) * scale)
-                       : "memory");
-        }
+        if (c == 0)
+          store_key_grads<SELF, 32>(r, nullptr, nullptr, scale, dv + dv_rows.at(b, h, j) + 32 * x, nullptr, nullptr, false);
+        else
+          store_key_grads<SELF, 32>(nullptr, r, nullptr, scale, nullptr, dk + dk_rows.at(b, h, j) + 32 * x,
+                                    dk0 + ((int64_t)b * seq + j) * D + 32 * x, SELF || (h == 0 && dq0_rows != 1));
       }
     }
-    if (tid == 0) bulk_wait_all();                            // the last reduce-adds must land before the CTA exits
   }
+  wait.end(status);
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
@@ -472,8 +634,8 @@ __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
 
 }  // namespace
 
-int backward(const Problem& p, const float* lse2, const float* carry, const float* dbar, const void* d_out_bf16,
-             float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
+int backward(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+             float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s) {
   if (p.head_dim != 64) return SA_ERR_UNSUPPORTED;
   const int ntiles = (p.seq + kTile - 1) / kTile;
   const int nrows = p.batch * p.heads;
@@ -484,11 +646,11 @@ int backward(const Problem& p, const float* lse2, const float* carry, const floa
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_v, p.v.ptr, 64, p.seq, p.heads, p.batch, p.v.st, p.v.sh, p.v.sb, kTile);
   if (st != SA_OK) return st;
-  st = make_map_16bit(&map_do, d_out_bf16, 64, p.seq, nrows, 1, 64, (int64_t)p.seq * 64, (int64_t)nrows * p.seq * 64, 64);
+  st = make_map_16bit(&map_do, d_out, 64, p.seq, p.heads, p.batch, d_out_rows.st, d_out_rows.sh, d_out_rows.sb, 64);
   if (st != SA_OK) return st;
   st = make_map_f32_rows(&map_dq, dq_acc, p.seq, nrows);
   if (st != SA_OK) return st;
-  st = make_map_f32_rows(&map_dq0, dq0, p.seq, p.batch);
+  st = dq0 != nullptr ? make_map_f32_rows(&map_dq0, dq0, p.seq, p.batch) : make_map_f32_rows(&map_dq0, dq_acc, p.seq, nrows);
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_q0, p.q0.ptr, 64, p.seq, 1, p.batch, p.q0.st, 0, p.q0.sb, 64);
   if (st != SA_OK) return st;
@@ -497,16 +659,17 @@ int backward(const Problem& p, const float* lse2, const float* carry, const floa
   WaitCtx status;
   st = wait_ctx(&status);
   if (st != SA_OK) return st;
-  const int smem = Smem::total + 1024;
-  const bool self = (p.heads == 1) && !p.external_selector;   // one head per selector: the selection logits are the head's own
+  const bool self = self_selecting(p);
+  const int smem = (self ? PairSmem<true>::total : PairSmem<false>::total) + 1024;
   const uint8_t* alive = static_cast<const uint8_t*>(p.tile_table);
   auto launch = [&](auto kernel) -> int {
     SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     ProfileScope prof(SA_KERNEL_TC_BACKWARD, s);
     count_launch();
-    kernel<<<(unsigned)ntiles * nrows, kThreads, smem, s>>>(
-        map_q, map_k, map_v, map_do, map_dq, map_dq0, map_q0, map_k0, lse2, carry, dbar, dk_acc, dk0,
-        static_cast<__nv_bfloat16*>(dv), p.heads, p.seq, ntiles, p.exempt, p.scale, status, p.dv_rows, alive);
+    kernel<<<(unsigned)ntiles * nrows, kPairThreads, smem, s>>>(
+        map_q, map_k, map_v, map_do, map_dq, map_dq0, map_q0, map_k0, stats, carry, static_cast<__nv_bfloat16*>(dk), dk0,
+        static_cast<__nv_bfloat16*>(dv), p.heads, dq0 != nullptr ? 1 : p.heads, p.seq, ntiles, p.exempt, p.scale, status,
+        p.dk_rows, p.dv_rows, alive);
     return SA_OK;
   };
   if (alive != nullptr) st = self ? launch(backward_kernel<true, true>) : launch(backward_kernel<false, true>);

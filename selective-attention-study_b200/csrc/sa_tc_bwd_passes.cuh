@@ -68,6 +68,45 @@ __device__ __forceinline__ void find_top_tile(const uint8_t* alive, int n, int n
   if (lane == 0) *top = found;
 }
 
+// N columns of one key row's gradients from the accumulators: dV in bf16, dK and dK0 scaled.  dK0 is added to the selecting
+// head's fp32 rows (every head of the sequence adds its share); `own` says that dK belongs there too (head 0, whose dk is
+// that sum), otherwise dK goes out in bf16.  SELF: dK holds both gradient paths and no one else adds to the row.
+template <bool SELF, int N>
+__device__ __forceinline__ void store_key_grads(const uint32_t* rv, const uint32_t* rk, const uint32_t* r0, float scale,
+                                                __nv_bfloat16* dv_row, __nv_bfloat16* dk_row, float* dk0_row, bool own) {
+#pragma unroll
+  for (int e = 0; e < N; e += 8) {
+    auto f = [&](const uint32_t* r, int u) { return __uint_as_float(r[e + u]); };
+    if (rv != nullptr)
+      *reinterpret_cast<uint4*>(dv_row + e) = make_uint4(pack_bf16(f(rv, 0), f(rv, 1)), pack_bf16(f(rv, 2), f(rv, 3)),
+                                                         pack_bf16(f(rv, 4), f(rv, 5)), pack_bf16(f(rv, 6), f(rv, 7)));
+    if (rk != nullptr && !own)
+      *reinterpret_cast<uint4*>(dk_row + e) =
+          make_uint4(pack_bf16(f(rk, 0) * scale, f(rk, 1) * scale), pack_bf16(f(rk, 2) * scale, f(rk, 3) * scale),
+                     pack_bf16(f(rk, 4) * scale, f(rk, 5) * scale), pack_bf16(f(rk, 6) * scale, f(rk, 7) * scale));
+#pragma unroll
+    for (int q = 0; q < 8; q += 4) {
+      if (SELF) {
+        if (rk != nullptr)
+          *reinterpret_cast<float4*>(dk0_row + e + q) =
+              make_float4(f(rk, q) * scale, f(rk, q + 1) * scale, f(rk, q + 2) * scale, f(rk, q + 3) * scale);
+        continue;
+      }
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      if (rk == nullptr && r0 == nullptr) continue;
+      if (r0 == nullptr && !own) continue;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (r0 != nullptr) a[u] += f(r0, q + u) * scale;
+        if (rk != nullptr && own) a[u] += f(rk, q + u) * scale;
+      }
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dk0_row + e + q), "f"(a[0]), "f"(a[1]), "f"(a[2]),
+                   "f"(a[3])
+                   : "memory");
+    }
+  }
+}
+
 // TMEM columns of the three score-shaped tiles (the same in both kernels)
 constexpr uint32_t kColZ = 256, kColX = 320, kColY = 384;
 

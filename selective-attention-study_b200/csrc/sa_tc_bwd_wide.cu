@@ -53,10 +53,9 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_q0, const __grid_constant__ CUtensorMap map_k0,
-    const float* __restrict__ lse2, const float* __restrict__ carry, const float* __restrict__ dbar,
-    float* __restrict__ dq_acc, float* __restrict__ dq0, float* __restrict__ dk_acc, float* __restrict__ dk0,
-    __nv_bfloat16* __restrict__ dv, int heads, int seq, int ntiles, int exempt, float scale, WaitCtx status,
-    RowLayout dv_rows, const uint8_t* __restrict__ alive) {
+    const float* __restrict__ stats, const float* __restrict__ carry, float* __restrict__ dq_acc, float* __restrict__ dq0,
+    __nv_bfloat16* __restrict__ dk, float* __restrict__ dk0, __nv_bfloat16* __restrict__ dv, int heads, int seq, int ntiles,
+    int exempt, float scale, WaitCtx status, RowLayout dk_rows, RowLayout dv_rows, const uint8_t* __restrict__ alive) {
   using L = Layout<SELF>;
   constexpr int D = 128;
   constexpr int kRingQD = L::ring_qd;
@@ -132,8 +131,8 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
         mbar_expect_tx(&bar_ldqd[slot], 2 * kOpTile);
         tma_load_4d(st, &map_q, &bar_ldqd[slot], 0, row0, h, b);
         tma_load_4d(st + kHalfTile, &map_q, &bar_ldqd[slot], 64, row0, h, b);
-        tma_load_4d(st + kOpTile, &map_do, &bar_ldqd[slot], 0, row0, n, 0);
-        tma_load_4d(st + kOpTile + kHalfTile, &map_do, &bar_ldqd[slot], 64, row0, n, 0);
+        tma_load_4d(st + kOpTile, &map_do, &bar_ldqd[slot], 0, row0, h, b);
+        tma_load_4d(st + kOpTile + kHalfTile, &map_do, &bar_ldqd[slot], 64, row0, h, b);
       };
       auto load_q0 = [&](int hn) {
         const int row0 = row_of(hn), slot = hn % kRing0;
@@ -286,14 +285,10 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
     ctx.dz_tot = dz_tot;
     ctx.status = status;
 
-    auto fetch_lse = [&](int mi) {
-      const int i = mi * kTile + tid;
-      return (tid < kTile && i < seq) ? load_ahead(lse2 + (int64_t)n * seq + i) : INFINITY;   // +inf: P = 0 for padded queries
-    };
-    auto fetch_dbar = [&](int mi) {
-      const int i = mi * kTile + tid;
-      return (tid < kTile && i < seq) ? load_ahead(dbar + (int64_t)n * seq + i) : 0.f;
-    };
+    // -lse2 and -dbar of a tile's 128 queries: two blocks of [64 of the one, 64 of the other]; padded queries hold -inf and 0
+    const float* const stat_row = stats + (int64_t)n * ntiles * (2 * kTile) + (tid >> 6) * kTile + (tid & 63);
+    auto fetch_lse = [&](int mi) { return tid < kTile ? load_ahead(stat_row + (int64_t)mi * (2 * kTile)) : 0.f; };
+    auto fetch_dbar = [&](int mi) { return tid < kTile ? load_ahead(stat_row + (int64_t)mi * (2 * kTile) + 64) : 0.f; };
     auto fetch_carry = [&](int mi) {
       return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1) * seq + j) : 0.f;
     };
@@ -319,7 +314,8 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
 
     // dQ^T (or dQ0^T) of one half: the lane is d, this warpgroup's 16 columns are queries; one query column of a warp
     // is 32 consecutive floats of the fp32 gradient row
-    float* const grad_rows = (SELF || dh == 0) ? dq_acc + (int64_t)n * seq * D : dq0 + (int64_t)b * seq * D;
+    float* const grad_rows = (SELF || dh == 0) ? dq_acc + (int64_t)n * seq * D
+                                               : (dq0 != nullptr ? dq0 + (int64_t)b * seq * D : dq_acc + (int64_t)b * heads * seq * D);
     auto read_out = [&](int hn) {
       const int i_first = (mi_top - (hn >> 1)) * kTile + (1 - (hn & 1)) * 64 + wg * kChunk;
       uint32_t r[16];
@@ -338,8 +334,8 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
       constexpr bool kDiag = decltype(diag_tag)::value;
       const int mi = mi_top - it;
       if (tid < kTile) {
-        lse_s[tid] = -next_lse;                                // negated: both enter packed adds directly
-        dbar_s[tid] = -next_dbar;
+        lse_s[tid] = next_lse;                                 // negated already: both enter packed adds directly
+        dbar_s[tid] = next_dbar;
       }
       const float cnl = next_carry * kLog2e;
       if (it + 1 < n_iter) {
@@ -384,34 +380,14 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
     {
       const int c0 = wg * kChunk;
       __nv_bfloat16* dv_row = dv + dv_rows.at(b, h, j) + dh * 64 + c0;
-      float* dk_row = dk_acc + ((int64_t)n * seq + j) * D + dh * 64 + c0;
-      float* dk0_row = dk0 + ((int64_t)b * seq + j) * D + dh * 64 + c0;
       uint32_t rv[16], rk[16], r0[16];
       tmem_ld16(lane_base + kColDV + c0, rv);
       tmem_ld16(lane_base + kColDK + c0, rk);
       if (!SELF) tmem_ld16(lane_base + kColDK0 + c0, r0);
       tmem_ld_wait();
-      if (j < seq) {
-#pragma unroll
-        for (int e = 0; e < 16; e += 8) {
-          uint4 w = make_uint4(pack_bf16(__uint_as_float(rv[e]), __uint_as_float(rv[e + 1])),
-                               pack_bf16(__uint_as_float(rv[e + 2]), __uint_as_float(rv[e + 3])),
-                               pack_bf16(__uint_as_float(rv[e + 4]), __uint_as_float(rv[e + 5])),
-                               pack_bf16(__uint_as_float(rv[e + 6]), __uint_as_float(rv[e + 7])));
-          *reinterpret_cast<uint4*>(dv_row + e) = w;
-        }
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          *reinterpret_cast<float4*>(dk_row + e) =
-              make_float4(__uint_as_float(rk[e]) * scale, __uint_as_float(rk[e + 1]) * scale,
-                          __uint_as_float(rk[e + 2]) * scale, __uint_as_float(rk[e + 3]) * scale);
-          if (!SELF)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dk0_row + e),
-                       "f"(__uint_as_float(r0[e]) * scale), "f"(__uint_as_float(r0[e + 1]) * scale),
-                       "f"(__uint_as_float(r0[e + 2]) * scale), "f"(__uint_as_float(r0[e + 3]) * scale)
-                       : "memory");
-        }
-      }
+      if (j < seq)
+        store_key_grads<SELF, 16>(rv, rk, r0, scale, dv_row, dk + dk_rows.at(b, h, j) + dh * 64 + c0,
+                                  dk0 + ((int64_t)b * seq + j) * D + dh * 64 + c0, SELF || (h == 0 && dq0 == nullptr));
     }
   }
   tc_fence_before_sync();
@@ -421,8 +397,8 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
 
 }  // namespace
 
-int backward_wide(const Problem& p, const float* lse2, const float* carry, const float* dbar, const void* d_out_bf16,
-                  float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
+int backward_wide(const Problem& p, const float* stats, const float* carry, const void* d_out, const RowLayout& d_out_rows,
+                  float* dq_acc, float* dq0, float* dk0, void* dk, void* dv, cudaStream_t s) {
   if (p.head_dim != 128) return SA_ERR_UNSUPPORTED;
   const int ntiles = (p.seq + kTile - 1) / kTile;
   const int nrows = p.batch * p.heads;
@@ -433,7 +409,7 @@ int backward_wide(const Problem& p, const float* lse2, const float* carry, const
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_v, p.v.ptr, 128, p.seq, p.heads, p.batch, p.v.st, p.v.sh, p.v.sb, kTile);
   if (st != SA_OK) return st;
-  st = make_map_16bit(&map_do, d_out_bf16, 128, p.seq, nrows, 1, 128, (int64_t)p.seq * 128, (int64_t)nrows * p.seq * 128, 64);
+  st = make_map_16bit(&map_do, d_out, 128, p.seq, p.heads, p.batch, d_out_rows.st, d_out_rows.sh, d_out_rows.sb, 64);
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_q0, p.q0.ptr, 128, p.seq, 1, p.batch, p.q0.st, 0, p.q0.sb, 64);
   if (st != SA_OK) return st;
@@ -442,7 +418,7 @@ int backward_wide(const Problem& p, const float* lse2, const float* carry, const
   WaitCtx status;
   st = wait_ctx(&status);
   if (st != SA_OK) return st;
-  const bool self = (p.heads == 1) && !p.external_selector;   // one head per selector: the selection logits are the head's own
+  const bool self = self_selecting(p);
   const int smem = (self ? Layout<true>::total : Layout<false>::total) + 1024;
   const uint8_t* alive = static_cast<const uint8_t*>(p.tile_table);
   const unsigned grid = 2u * (unsigned)ntiles * (unsigned)nrows;
@@ -450,9 +426,9 @@ int backward_wide(const Problem& p, const float* lse2, const float* carry, const
     SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     ProfileScope prof(SA_KERNEL_TC_BACKWARD, s);
     count_launch();
-    kernel<<<grid, kThreads, smem, s>>>(map_q, map_k, map_v, map_do, map_q0, map_k0, lse2, carry, dbar, dq_acc, dq0, dk_acc,
-                                        dk0, static_cast<__nv_bfloat16*>(dv), p.heads, p.seq, ntiles, p.exempt, p.scale,
-                                        status, p.dv_rows, alive);
+    kernel<<<grid, kThreads, smem, s>>>(map_q, map_k, map_v, map_do, map_q0, map_k0, stats, carry, dq_acc, dq0,
+                                        static_cast<__nv_bfloat16*>(dk), dk0, static_cast<__nv_bfloat16*>(dv), p.heads, p.seq,
+                                        ntiles, p.exempt, p.scale, status, p.dk_rows, p.dv_rows, alive);
     return SA_OK;
   };
   if (alive != nullptr) st = self ? launch(backward_wide_kernel<true, true>) : launch(backward_wide_kernel<false, true>);
