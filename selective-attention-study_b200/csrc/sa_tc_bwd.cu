@@ -2,9 +2,9 @@
 //
 // One CTA owns one 128-key tile of one head and walks the query tiles LAST TO FIRST in 64-query halves.  All
 // score-shaped tiles are computed transposed, KEYS on the TMEM lanes (S^T = K Q^T, dP^T = V dO^T, L0^T = K0 Q0^T), so
-// one thread owns one key and sees all 64 queries of a half along its registers.  The two running sums down the query
+// one thread owns one key and sees all 64 queries of a half along its registers, the last one first.  The two running sums down the query
 // axis are then thread-local fp32 recurrences walked from the last query to the first:
-//     F[i]  = carry_after_half - sum_{r >= i} sel[r]          (history term rebuilt per key)
+//     F[i]  = carry_after_tile - sum_{r >= i} sel[r]          (history term rebuilt per key)
 //     U[i]  = suffix + sum_{i' > i} dz[i']                      (logit gradient of later queries)
 // with  P = exp2(z - lse),  dz = P (dP - dbar),  g = gate ? -U : 0.
 //
@@ -12,13 +12,13 @@
 // them) whose links are hand-overs between the arithmetic warps and the tensor pipe.  With all warps on one half at a time
 // the SM idles at each of them: 10.4 k cycles per 128 x 128 tile of which ~3.8 k were issue slots.  Here the upper halves
 // (chain 0) and the lower halves (chain 1) of the tiles belong to one warpgroup each, with their own two score tiles in TMEM,
-// so that one chain computes while the other waits.  What couples them is little: the history of a half starts from a
-// checkpoint of its own (the carry after the tile, or the carry before it plus the half's own sum), and the running sum
-// of dz is handed from half to half, per key, through one shared-memory word (`run_s`).
+// so that one chain computes while the other waits.  What couples them is little: the per key, the upper half
+// hands the sum of its selection to the lower half of the same tile (`sel_s`), and the running sum of dz goes from half to
+// half (`run_s`).
 //
 // Roles.  Warps 0-3 and 4-7: the two chains.  Warps 8-11: read dQ and dQ0 out of TMEM, scale, stage and TMA-reduce-add them
-// into fp32 global rows.  Warp 12 issues every MMA, in the order in which the events of two chains half a tile apart come.
-// Warp 13, one lane: TMA loads.
+// into fp32 global rows.  Warps 12, 14, 15: MMA issue (per-key accumulators and L0^T; dQ and dQ0; S^T and dP^T).  Warp 13, one
+// lane: TMA loads.
 //
 // TMEM, 512 columns: dV | dK | one accumulator shared by dQ and dQ0 | per chain W1 and W2 | dK0 (64 each).
 //     W1: L0^T of half n -> (read) -> dP^T of half n -> (read) -> g^T as bf16 pairs -> dK0 -> L0^T of half n + 2
@@ -31,9 +31,10 @@
 // 48, dQ, dQ0 operands 96, dz and g written 64, dQ, dQ0 staged and reduced 128, loads 48 = 4.2 k cycles; the tensor pipe needs
 // 2.7 k, the issue slots ~3 k.  And the INSTRUCTION CACHE: everything that runs at one time has to fit 32 KB (measured: what
 // does not fit is fetched at 2.7 cycles an instruction, for each chain separately since they are half a tile apart).  The
-// first form of this kernel, with 45 KB of loops, ran at 15.5 k cycles a tile; hence the compact waits (Waiter), the rolled
-// MMA loop over halves (its order is the same for both chains), low words of descriptors, 32-bit shared addresses.
-// Measured at B = 4, H = 16, T = 16384: 16.6 ms with sixteen warps in lock step, 12.3 ms with two chains (SELF: 12.3, 9.3).
+// first form of this kernel, with 45 KB of loops, ran at 15.5 k cycles a tile; hence the compact waits (Waiter), rolled MMA
+// loops over halves (the order is the same for both chains), low words of descriptors, 32-bit shared addresses.
+// Measured at B = 4, H = 16, T = 16384: 16.6 ms with sixteen warps in lock step, 12.1 ms with two chains and one MMA warp,
+// 10.5 ms (5.0 k cycles a tile) with three (SELF: 12.3, 8.7, 8.0).
 //
 // SELF variant (one head per selector, i.e. the per-head form reshaped to (B H, 1, T, D)): the selection logits are the
 // head's own logits, so S^T serves as L0^T (read twice), and since Q0 = Q and K0 = K the two gradient paths add before the
@@ -63,10 +64,10 @@ using bwd::load_ahead;
 using bwd::store_key_grads;
 using bwd::tile_of_block;
 
-constexpr int kPairThreads = 512;     // two chains, the read-out warpgroup, the MMA and load warps (two warps idle)
+constexpr int kPairThreads = 512;     // two chains, the read-out warpgroup, three MMA warps and a load warp
 // Registers: 512 x 128 at launch; the chains keep 64 values and their masks, the rest needs little: 256 x 168 + 256 x 88.
 constexpr int kChainRegs = 168, kOtherRegs = 88;
-constexpr int kMmaWarp = 12, kLoadWarp = 13;
+constexpr int kMmaWarp = 12, kLoadWarp = 13, kDqWarp = 14, kScoreWarp = 15;
 constexpr int kStatBytes = 512;       // -lse2 and -dbar of 64 queries
 
 template <bool SELF>
@@ -91,11 +92,14 @@ constexpr uint32_t kDV = 0, kDK = 64, kDQ = 128, kW = 192, kDK0 = 448, kKA = 448
 __device__ __forceinline__ constexpr uint32_t w1_of(uint32_t chain) { return kW + 128 * chain; }
 __device__ __forceinline__ constexpr uint32_t w2_of(uint32_t chain) { return kW + 128 * chain + 64; }
 
-// The signs of two floats as a pair of 16-bit masks (0xffff where the sign bit is set).
-__device__ __forceinline__ uint32_t sign_masks(float lo, float hi) {
-  uint32_t m;
-  asm("prmt.b32 %0, %1, %2, 0xffbb;" : "=r"(m) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
-  return m;
+// The gate of two selection logits, l > 0, as a bf16 pair: masks of 16 bits, or 1 and 0.  The comparison is made on the bf16
+// roundings: they have the sign of the logit, and are zero only below 2^-134.
+template <bool MASK>
+__device__ __forceinline__ uint32_t gate_pair(float lo, float hi) {
+  const __nv_bfloat162 x = __floats2bfloat162_rn(lo, hi), zero = __floats2bfloat162_rn(0.f, 0.f);
+  if (MASK) return __hgt2_mask(x, zero);
+  const __nv_bfloat162 g = __hgt2(x, zero);
+  return *reinterpret_cast<const uint32_t*>(&g);
 }
 
 template <bool SELF, bool LIVE>   // LIVE: a table of live tiles is given (sa_tc_skip.cu)
@@ -120,12 +124,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // Barriers.  Completion: LD, LD0 TMA loads; L0, S, DP score products of a chain's half; FREE, FREE0 the last MMA that reads
   // a slot; DQ, DQ0 a tile's query-side product.  Arrival, one arrival per warp: SEL L0^T read; DZ P^T and dz^T written, S^T
-  // and dP^T read; G g^T written; TOK the running sum of dz handed on; ACC the shared accumulator read.
+  // and dP^T read; G g^T written; TOK the running sum of dz handed on; SUM the upper
+  // half's selection handed to the lower; ACC the shared accumulator read.
   enum : int { KV = 0, SETUP = 1, FIN = 2, DQ = 3, DQ0 = 4, ACC = 5, L0 = 6, S = 8, DP = 10, SEL = 12, DZ = 14, G = 16, TOK = 18,
-               LD = 20, FREE = 25, LD0 = 30, FREE0 = 33, kBars = 36 };
+               SUM = 20, LD = 21, FREE = 26, LD0 = 31, FREE0 = 34, kBars = 37 };
   __shared__ uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
-  __shared__ float run_s[kTile];
+  __shared__ float run_s[kTile], sel_s[2][kTile];
   __shared__ int top_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -134,6 +139,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
     for (int u = 0; u < kBars; ++u) mbar_init(&bars[u], u == SETUP ? 8 : (u == ACC || (u >= SEL && u < LD)) ? 4 : 1);
     mbar_init_fence();
   }
+  if (tid < kTile) run_s[tid] = 0.f;
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
   tc_fence_before_sync();
   __syncthreads();
@@ -186,9 +192,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
       }
     }
     __syncwarp();
-  } else if (warp == kMmaWarp) {
+  } else if (warp >= 12) {
     // ========================================== MMA issue ==================================================
-    // The whole warp walks this code, so that addresses and descriptors stay in uniform registers; one elected lane issues.
+    // A whole warp walks this code and one elected lane issues.  Issuing is slow enough (an await that finds its phase
+    // complete ~120 cycles, four MMAs ~300) that one warp for the 64 MMAs of a tile was the bottleneck at 6.2 k cycles a tile.
+    // Products that must follow one another in the pipe (what reads a column range, then what overwrites it) are issued by
+    // the same warp, or wait for the commit of the first.
     const uint32_t idesc_t = instr_desc_bf16(128, 64, false, false);     // keys x 64 queries, K = D
     const uint32_t idesc_acc = instr_desc_bf16(128, 64, false, true);    // A K-major (keys x queries), B MN-major
     const uint32_t idesc_dq = instr_desc_bf16(128, 64, true, true);      // A MN-major (queries x keys), B MN-major
@@ -251,84 +260,102 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
     auto next = [](Ring& x, uint32_t ring) {
       if (++x.slot == ring) { x.slot = 0; x.par ^= 1u; }
     };
-    Ring s_ring{0, 0}, l_ring{0, 0};                                     // of the next S^T and L0^T to issue
-    Ring use{0, 0}, use0{0, 0}, sel{0, 0};                               // of the half whose products are served (dz, g; selection)
-    auto ask_s = [&](uint32_t c) {                                       // S^T (SELF: and dP^T) of the chain's next half
-      await(LD + (int)s_ring.slot, s_ring.par, 403);
-      issue_s(c, s_ring.slot);
-      if (SELF) issue_dp(c, s_ring.slot);
-      next(s_ring, R);
-    };
-    auto ask_l0 = [&](uint32_t c) {
-      await(LD0 + (int)l_ring.slot, l_ring.par, 404);
-      issue_l0(c, l_ring.slot);
-      next(l_ring, 3);
-    };
-    // Chain 1 runs half a tile behind chain 0: while half hn is in its selection, the half before it, of the other chain,
-    // comes to its dz and g.  The order below is the order in which their events come then.
-    await(SELF ? SETUP : KV, 0, 400);                          // K, V (and K0) in place
-    ask_s(0);
-    if (!SELF) ask_l0(0);
-    ask_s(1);
-    if (!SELF) ask_l0(1);
     const int halves = 2 * tiles;
+    await(SELF ? SETUP : KV, 0, 400);                                    // K, V (and K0) in place
+    if (warp == kMmaWarp) {
+      // -- the per-key accumulators, and the products whose columns they free: L0^T (SELF: S^T and dP^T) of the half after next
+      Ring use{0, 0}, use0{0, 0}, ahead{0, 0};
+      auto ask_l0 = [&](uint32_t c) {
+        await(LD0 + (int)ahead.slot, ahead.par, 404);
+        issue_l0(c, ahead.slot);
+        next(ahead, 3);
+      };
+      auto ask_s = [&](uint32_t c) {
+        await(LD + (int)ahead.slot, ahead.par, 403);
+        issue_s(c, ahead.slot);
+      };
+      auto ask_dp = [&](uint32_t c) {
+        issue_dp(c, ahead.slot);
+        next(ahead, R);
+      };
 #pragma unroll 1
-    for (int hn = 0; hn <= halves; ++hn) {
-      const uint32_t c = (uint32_t)(hn & 1), p = c ^ 1u;                 // chain of half hn, and of the half before it
-      if (!SELF && hn < halves) {                                        // L0^T read: dP^T takes its columns
+      for (uint32_t c = 0; c < 2; ++c) {
+        if (SELF) ask_s(c), ask_dp(c);
+        else ask_l0(c);
+      }
+#pragma unroll 1
+      for (int hn = 0; hn < halves; ++hn) {
+        const uint32_t c = (uint32_t)(hn & 1), ph = (uint32_t)((hn >> 1) & 1), keep = hn > 0 ? 1u : 0u;
+        await(DZ + (int)c, ph, 406);                                     // P^T (and dz^T) written: dV, dK
+        if (elect_one()) {
+          accumulate(kDV, w2_of(c) + 32, L::ring + use.slot * L::kSlot + kHalfTile, keep);
+          if (!SELF) {
+            accumulate(kDK, w2_of(c), L::ring + use.slot * L::kSlot, keep);
+            mma_commit(bar(FREE + (int)use.slot));
+          }
+        }
+        __syncwarp();
+        if (SELF && hn + 2 < halves) ask_s(c);
+        await(G + (int)c, ph, 407);                                      // g^T written: dK0
+        if (elect_one()) {
+          if (SELF) {
+            accumulate(kDK, w1_of(c), L::ring + use.slot * L::kSlot, keep);
+            mma_commit(bar(FREE + (int)use.slot));
+          } else {
+            accumulate(kDK0, w1_of(c), L::ring0 + use0.slot * kHalfTile, keep);
+            mma_commit(bar(FREE0 + (int)use0.slot));
+          }
+        }
+        __syncwarp();
+        if (hn + 2 < halves) {
+          if (SELF) ask_dp(c);
+          else ask_l0(c);
+        }
+        next(use, R);
+        next(use0, 3);
+      }
+      if (elect_one()) mma_commit(bar(FIN));
+      __syncwarp();
+    } else if (warp == kDqWarp) {
+      // -- the query-side products of a tile, once both halves are there and the accumulator has been read
+#pragma unroll 1
+      for (int t = 0; t < tiles; ++t) {
+        const uint32_t ph = (uint32_t)(t & 1);
+        if (!SELF) {
+          await(DZ, ph, 408);
+          await(DZ + 1, ph, 408);
+          await(ACC, 1u, 409);                                           // (the first passes) dQ0 of the tile before
+          issue_dq(L::dz, L::k, DQ);
+        }
+        await(G, ph, 410);
+        await(G + 1, ph, 410);
+        await(ACC, SELF ? ph ^ 1u : 0u, 411);                            // dQ of this tile; SELF: of the tile before
+        issue_dq(SELF ? L::dz : L::g, SELF ? L::k : L::k0, SELF ? DQ : DQ0);
+      }
+    } else if (!SELF && warp == kScoreWarp) {
+      // -- dP^T of half hn when its L0^T has been read, S^T of half hn + 1 when dV, dK of half hn - 1 are done
+      Ring ahead{0, 0}, freed{0, 0}, sel{0, 0};
+      auto ask_s = [&](uint32_t c) {
+        await(LD + (int)ahead.slot, ahead.par, 403);
+        issue_s(c, ahead.slot);
+        next(ahead, R);
+      };
+      ask_s(0);
+      ask_s(1);
+#pragma unroll 1
+      for (int hn = 0; hn < halves; ++hn) {
+        const uint32_t c = (uint32_t)(hn & 1);
         await(SEL + (int)c, (uint32_t)((hn >> 1) & 1), 405);
         issue_dp(c, sel.slot);
         next(sel, R);
-      }
-      if (hn == 0) continue;
-      const uint32_t ph = (uint32_t)(((hn - 1) >> 1) & 1);               // of half hn - 1
-      const uint32_t keep = hn > 1 ? 1u : 0u;
-      await(DZ + (int)p, ph, 406);                                         // P^T, dz^T written: dV, dK, then the next half's S^T
-      if (elect_one()) {
-        accumulate(kDV, w2_of(p), L::ring + use.slot * L::kSlot + kHalfTile, keep);
-        if (!SELF) {
-          accumulate(kDK, w2_of(p) + 32, L::ring + use.slot * L::kSlot, keep);
-          mma_commit(bar(FREE + (int)use.slot));
-        }
-      }
-      __syncwarp();
-      if (!SELF) {
-        if (hn + 1 < halves) ask_s(p);
-        if (p == 1) {                                                    // both halves of the tile: dQ
-          if (hn > 2) await(ACC, 1u, 408);                          // dQ0 of the tile before has been read out
-          issue_dq(L::dz, L::k, DQ);
-        }
-      }
-      await(G + (int)p, ph, 407);                                          // g^T written: dK0, then the next half's L0^T
-      if (elect_one()) {
-        if (SELF) {
-          accumulate(kDK, w1_of(p), L::ring + use.slot * L::kSlot, keep);
-          mma_commit(bar(FREE + (int)use.slot));
-        } else {
-          accumulate(kDK0, w1_of(p), L::ring0 + use0.slot * kHalfTile, keep);
-          mma_commit(bar(FREE0 + (int)use0.slot));
-        }
-      }
-      __syncwarp();
-      next(use, R);
-      next(use0, 3);
-      if (hn + 1 < halves) {
-        if (SELF) ask_s(p);
-        else ask_l0(p);
-      }
-      if (p == 1) {
-        if (SELF) {
-          if (hn > 2) await(ACC, ph ^ 1u, 408);                     // dQ of the tile before
-          issue_dq(L::dz, L::k, DQ);
-        } else {
-          await(ACC, 0u, 409);                                      // dQ of this tile
-          issue_dq(L::g, L::k0, DQ0);
+        if (hn > 0 && hn + 1 < halves) {
+          await(FREE + (int)freed.slot, freed.par, 412);
+          next(freed, R);
+          ask_s(c ^ 1u);
         }
       }
     }
-    if (elect_one()) mma_commit(bar(FIN));
-    __syncwarp();
-  } else if (warp < 12) {
+  } else {
     // ==================== read-out of dQ, dQ0: lanes are queries, a warp's 32 rows at a time ====================
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint8_t* stage = smem + L::out + (warp - 8) * 8192;           // two [32 queries][32 floats] boxes, 128-byte swizzle
@@ -391,12 +418,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
     const uint32_t w1 = lane_base + w1_of(c), w2 = lane_base + w2_of(c);
     const int j = nj * kTile + row;
     const float c1 = scale * kLog2e;
-    const float c1_hist = (j >= exempt) ? c1 : 0.f;                // an exempt key has no history and no gate
-    const float shut = (j >= exempt) ? -1.4e-45f : -INFINITY;
+    const float inv_scale = 1.f / scale;
+    const float shut = (j >= exempt) ? 0.f : -INFINITY;            // an exempt key is never selected
     // this thread's row in its chain's query half of the dz tile (the g tile lies kG further on); chunk x of it is at ^ 16 x
     constexpr uint32_t kG = SELF ? 0 : L::g - L::dz;
     const uint32_t my_row = sa + L::dz + (1 - c) * kRowTile + row * 128 + ((row & 7) << 4);
-    const uint32_t run_addr = smem_u32(&run_s[row]);
     auto put8 = [&](uint32_t at, int chunk, const uint32_t* w) {             // eight queries of this thread's key
       st_shared16(at ^ (uint32_t)(chunk << 4), w[0], w[1], w[2], w[3]);
     };
@@ -404,9 +430,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(id));
     };
-    // chain 0 starts from the carry after the tile, chain 1 from the carry before it plus its own half's sum
     auto fetch_carry = [&](int mi) {
-      return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1 - c) * seq + j) : 0.f;
+      return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1) * seq + j) : 0.f;
     };
     float next_carry = fetch_carry(mi_top);
 
@@ -429,17 +454,17 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
     uint32_t ld_par = 0;
     auto half = [&](int it, auto diag_tag) {
       constexpr bool kDiag = decltype(diag_tag)::value;
-      const int mi = mi_top - it;
       const uint32_t ph = (uint32_t)(it & 1);
       const int diag = row - (1 - c) * 64;                         // kDiag: query e of the half is this key itself
       const uint32_t stat = sa + L::stat + slot * kStatBytes;
-      const float carry_log2 = next_carry * kLog2e;
-      if (it + 1 < n_iter) next_carry = fetch_carry(mi - 1);
+      float run = next_carry;
+      asm volatile("" : "+f"(run));                                // (the scaling stays here: next to the load it would wait for it)
+      run *= -inv_scale;                                           // minus the history after the tile, in units of q . k
+      if (it + 1 < n_iter) next_carry = fetch_carry(mi_top - it - 1);
 
-      // ---- selection: relu(L0^T), the gate, and the sums of eight queries at a time ------------------------------
+      // ---- selection: relu(L0^T) and the gate ---------------------------------------------------------
       float v[64];
-      uint32_t off[SELF ? 2 : 32];                                 // where the gate is shut: bits, or masks of bf16 pairs
-      float part[8];
+      uint32_t gate[32];                                           // bf16 pairs
       wait(bar((SELF ? S : L0) + c), ph, 410);
       tc_fence_after_sync();
       {
@@ -448,8 +473,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
         tmem_ld32((SELF ? w2 : w1) + 32, r[1]);
         tmem_ld_wait();
         tc_fence_before_sync();
-        if (!SELF) arrive(SEL + c);                             // W1 may take dP^T
-        if (SELF) off[0] = off[1] = 0u;
+        if (!SELF) arrive(SEL + c);                                // W1 may take dP^T
 #pragma unroll
         for (int e = 0; e < 64; e += 2) {
           float l0 = __uint_as_float(r[e >> 5][e & 31]), l1 = __uint_as_float(r[e >> 5][(e & 31) + 1]);
@@ -457,152 +481,121 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
             if (e <= diag) l0 = -1.f;
             if (e + 1 <= diag) l1 = -1.f;
           }
-          // the gate is open for l0 > 0: the sign of l0 minus the smallest number (an exempt key: minus infinity)
           const float2 t = __fadd2_rn(make_float2(l0, l1), make_float2(shut, shut));
-          if constexpr (SELF) {
-            off[e >> 5] = __funnelshift_l(__float_as_uint(t.x), off[e >> 5], 1);      // query e ends up at bit 31 - e % 32
-            off[e >> 5] = __funnelshift_l(__float_as_uint(t.y), off[e >> 5], 1);
-          } else {
-            off[e >> 1] = sign_masks(t.x, t.y);
-          }
-          v[e] = fmaxf(l0, 0.f);
-          v[e + 1] = fmaxf(l1, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          float2 s = __fadd2_rn(make_float2(v[8 * u], v[8 * u + 1]), make_float2(v[8 * u + 2], v[8 * u + 3]));
-          s = __fadd2_rn(s, __fadd2_rn(make_float2(v[8 * u + 4], v[8 * u + 5]), make_float2(v[8 * u + 6], v[8 * u + 7])));
-          part[u] = s.x + s.y;
+          gate[e >> 1] = gate_pair<!SELF>(t.x, t.y);
+          v[e] = fmaxf(t.x, 0.f);
+          v[e + 1] = fmaxf(t.y, 0.f);
         }
       }
-#pragma unroll
-      for (int u = 6; u >= 0; --u) part[u] += part[u + 1];         // part[u]: the sum from query 8 u on
-      // F log2e = cb - c1 * (sum from the query on)
-      const float ncb = (c == 0) ? -carry_log2 : -fmaf(c1_hist, part[0], carry_log2);
 
-      // ---- probabilities: P = exp2(c1 (S + suffix) - cb - lse) -----------------------------------------------------
+      // ---- probabilities, last query first: P = exp2(c1 (S + run) - lse), run growing by the selection ---------------
       if (!SELF) {
         wait(bar(S + c), ph, 416);
         tc_fence_after_sync();
       }
-      wait(bar(LD + slot), ld_par, 417);               // (complete by now) the statistics are in place
-      const float2 cc = make_float2(c1, c1), ch = make_float2(c1_hist, c1_hist), nb = make_float2(ncb, ncb);
+      mbar_try_wait(&bars[LD + slot], ld_par);                    // (complete: S^T was made from the slot) its statistics are visible
+      if (c == 1) {                                                // the upper half's selection comes first
+        wait(bar(SUM), ph, 421);
+        run += sel_s[ph][row];
+      }
+      const float2 cc = make_float2(c1, c1);
+      const float run_in = run;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t r[16], w8[8];
-        tmem_ld16(w2 + 16 * q, r);
+      for (int q = 1; q >= 0; --q) {
+        uint32_t r[32], w[16];
+        tmem_ld32(w2 + 32 * q, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 2 * q; u < 2 * q + 2; ++u) {                  // inclusive suffix sums of eight queries
-          float run = (u < 7) ? part[u + 1] : 0.f;
+        for (int e4 = 28; e4 >= 0; e4 -= 4) {
+          const float4 nl = ld_shared_f4(stat + 4 * (32 * q + e4));
 #pragma unroll
-          for (int e = 8 * u + 7; e >= 8 * u; --e) {
-            run += v[e];
-            v[e] = run;
-          }
-        }
-#pragma unroll
-        for (int e4 = 0; e4 < 16; e4 += 4) {
-          const float4 nl = ld_shared_f4(stat + 4 * (16 * q + e4));
-          const float2 nls[2] = {make_float2(nl.x, nl.y), make_float2(nl.z, nl.w)};
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int e = 16 * q + e4 + 2 * k;
-            const float2 hist = __ffma2_rn(make_float2(v[e], v[e + 1]), ch, __fadd2_rn(nls[k], nb));
-            const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])), cc, hist);
+          for (int k = 1; k >= 0; --k) {
+            const int e = 32 * q + e4 + 2 * k;
+            const float hi = run + v[e + 1];
+            run = hi + v[e];
+            const float2 s = __fadd2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])),
+                                        make_float2(run, hi));
+            const float2 x = __ffma2_rn(s, cc, k ? make_float2(nl.z, nl.w) : make_float2(nl.x, nl.y));
             v[e] = ex2(x.x);
             v[e + 1] = ex2(x.y);
             if (kDiag) {                                           // key after the query
               if (e < diag) v[e] = 0.f;
               if (e + 1 < diag) v[e + 1] = 0.f;
             }
-            w8[(e4 >> 1) + k] = pack_bf16(v[e], v[e + 1]);
+            w[(e4 >> 1) + k] = pack_bf16(v[e], v[e + 1]);
           }
         }
-        tmem_st8(w2 + 8 * q, w8);                                  // over S^T columns that have been read
+        tmem_st16(w2 + 32 + 16 * q, w);                            // over S^T columns that have been read
+      }
+      if (c == 0) {
+        sel_s[ph][row] = run - run_in;
+        arrive(SUM);
       }
 
       // ---- dz = P (dP - dbar) ------------------------------------------------------------------------------------
       wait(bar(DP + c), ph, 411);
       tc_fence_after_sync();
-      if (!SELF && it > 0) wait(bar(DQ), ph ^ 1u, 418);   // dQ of the tile before has read the dz tile
+      if (!SELF) wait(bar(DQ0), ph ^ 1u, 418);                     // dQ and dQ0 of the tile before have read dz and g
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t r[16], w8[8];
-        tmem_ld16(w1 + 16 * q, r);
+      for (int q = 0; q < 2; ++q) {
+        uint32_t r[32], w[16];
+        tmem_ld32(w1 + 32 * q, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int e4 = 0; e4 < 16; e4 += 4) {
-          const float4 nd = ld_shared_f4(stat + 4 * (64 + 16 * q + e4));
-          const float2 nds[2] = {make_float2(nd.x, nd.y), make_float2(nd.z, nd.w)};
+        for (int e4 = 0; e4 < 32; e4 += 4) {
+          const float4 nd = ld_shared_f4(stat + 4 * (64 + 32 * q + e4));
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const int e = 16 * q + e4 + 2 * k;
+            const int e = 32 * q + e4 + 2 * k;
             const float2 d = __fmul2_rn(make_float2(v[e], v[e + 1]),
                                         __fadd2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])),
-                                                   nds[k]));
+                                                   k ? make_float2(nd.z, nd.w) : make_float2(nd.x, nd.y)));
             v[e] = d.x;
             v[e + 1] = d.y;
-            if (!SELF) w8[(e4 >> 1) + k] = pack_bf16(d.x, d.y);
+            if (!SELF) w[(e4 >> 1) + k] = pack_bf16(d.x, d.y);
           }
         }
-#pragma unroll
-        for (int u = 2 * q; u < 2 * q + 2; ++u) {
-          float2 s = __fadd2_rn(make_float2(v[8 * u], v[8 * u + 1]), make_float2(v[8 * u + 2], v[8 * u + 3]));
-          s = __fadd2_rn(s, __fadd2_rn(make_float2(v[8 * u + 4], v[8 * u + 5]), make_float2(v[8 * u + 6], v[8 * u + 7])));
-          part[u] = s.x + s.y;
-        }
         if (!SELF) {                                               // dz: to TMEM (A of dK) and shared memory (A of dQ)
-          tmem_st8(w2 + 32 + 8 * q, w8);
-          put8(my_row, 2 * q, w8);
-          put8(my_row, 2 * q + 1, w8 + 4);
+          tmem_st16(w2 + 16 * q, w);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) put8(my_row, 4 * q + u, w + 4 * u);
         }
       }
       if (!SELF) fence_async_smem();                               // dz half tile -> visible to the MMAs
       tmem_st_wait();
       tc_fence_before_sync();
       arrive(DZ + c);
-#pragma unroll
-      for (int u = 6; u >= 0; --u) part[u] += part[u + 1];
 
-      // ---- the sum of dz over later queries, handed from half to half ----------------------------------------------
-      float base = 0.f;
-      if (c == 1 || it > 0) {
-        wait(bar(TOK + other), c == 1 ? ph : ph ^ 1u, 419);
-        base = run_s[row];
-      }
-      run_s[row] = base + part[0];
-      arrive(TOK + c);
-
-      // ---- g = gate ? -(sum of dz over later queries) : 0; SELF: dz + g --------------------------------------------
-      if (it > 0) wait(bar(SELF ? DQ : DQ0), ph ^ 1u, 420);   // the tile before has been read
+      // ---- g = gate ? -(sum of dz over later queries) : 0; SELF: dz + g.  The sum goes from half to half --------------
+      wait(bar(TOK + other), ph ^ (uint32_t)other, 419);
+      float later = run_s[row];                                    // minus the sum of dz over later queries
+      if (SELF) wait(bar(DQ), ph ^ 1u, 420);                       // dQ of the tile before has read dz + g
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t w8[8];
+      for (int q = 1; q >= 0; --q) {
+        uint32_t w[16];
 #pragma unroll
-        for (int u = 2 * q; u < 2 * q + 2; ++u) {
-          float run = -base - ((u < 7) ? part[u + 1] : 0.f);
-#pragma unroll
-          for (int e = 8 * u + 7; e >= 8 * u; --e) {
-            const float dz = v[e];
-            if constexpr (SELF) v[e] = ((off[e >> 5] >> (31 - (e & 31))) & 1u) ? dz : dz + run;
-            else v[e] = run;
-            run -= dz;
-          }
+        for (int e = 32 * q + 30; e >= 32 * q; e -= 2) {
+          const float hi = later, lo = later - v[e + 1];
+          later = lo - v[e];
+          const uint32_t m = gate[e >> 1];
+          if constexpr (SELF)
+            w[(e >> 1) & 15] = pack_bf16(fmaf(__uint_as_float(m << 16), lo, v[e]), fmaf(__uint_as_float(m & 0xffff0000u), hi, v[e + 1]));
+          else
+            w[(e >> 1) & 15] = pack_bf16(lo, hi) & m;
         }
+        tmem_st16(w1 + 16 * q, w);                                 // over dP^T columns that have been read
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          w8[e] = pack_bf16(v[16 * q + 2 * e], v[16 * q + 2 * e + 1]);
-          if constexpr (!SELF) w8[e] &= ~off[8 * q + e];
-        }
-        tmem_st8(w1 + 8 * q, w8);                                  // over dP^T columns that have been read
-        put8(my_row + kG, 2 * q, w8);
-        put8(my_row + kG, 2 * q + 1, w8 + 4);
+        for (int u = 0; u < 4; ++u) put8(my_row + kG, 4 * q + u, w + 4 * u);
       }
+      run_s[row] = later;
       fence_async_smem();
       tmem_st_wait();
       tc_fence_before_sync();
-      arrive(G + c);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bar(G + c));
+        mbar_arrive(bar(TOK + c));
+      }
       slot += 2;
       if (slot >= R) { slot -= R; ld_par ^= 1u; }
     };

@@ -61,32 +61,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-// Non-blocking form, for a thread that watches several barriers.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// The limit of a loop that watches several barriers: `expired` is called after each round without progress.
-struct PollLimit {
-  long long start = 0;
-  int spins = 0;
-  __device__ __forceinline__ void progress() { spins = 0; }
-  __device__ __forceinline__ bool expired(const WaitCtx& w, unsigned int site) {
-    if (spins++ == 0) start = clock64();
-    if ((spins & 63) != 0) return false;
-    if (*reinterpret_cast<volatile unsigned int*>(w.word + 1) == w.epoch) return true;
-    if (clock64() - start <= ((long long)w.limit_kcycles << 10)) return false;
-    report(w, site);
-    return true;
-  }
-};
 // Waits for the phase with the given parity to complete.  Gives up after the context's limit, or at once
 // when another wait of the same launch sequence has already given up, so a broken kernel ends quickly.
 // Callable by a single thread of a warp: it contains no warp-wide operation.
