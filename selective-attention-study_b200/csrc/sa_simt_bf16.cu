@@ -11,6 +11,6 @@ int simt_carry_bf16(const Problem& p, float* carry, float* total, cudaStream_t s
 int simt_backward_bf16(const Problem& p, const float* lse2, const float* carry, const float* dbar,
                          const float* d_out, float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv,
                          cudaStream_t s) {
-  return simt::backward_by_dim<__nv_bfloat16, float>(p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, dv, s);
+  return simt::backward_by_dim<__nv_bfloat16>(p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, dv, s);
 }
 }  // namespace sa
