@@ -18,8 +18,7 @@
 // Reference for the arithmetic: src/selective_attention/kernels.py:100-194 (selection, carry, forward).
 #include <type_traits>
 
-#include "sa_tc_host.cuh"
-#include "sa_tc_ptx.cuh"
+#include "sa_tc_fwd.cuh"
 
 namespace sa {
 namespace tc {
@@ -27,20 +26,6 @@ namespace {
 
 constexpr int kTile = 128;          // query rows per CTA; also the carry checkpoint spacing
 constexpr int kRowTile = 16384;     // bytes of a [128][64] bf16 operand tile
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// A global load the compiler must issue where it is written (volatile asm keeps its place among the other
-// volatile asm statements), so a value fetched one step ahead is really in flight during that step.
-__device__ __forceinline__ float load_ahead(const float* p) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
 
 // ---------------------------------------------------------------------------------------------------
 // selection column sums
@@ -215,7 +200,6 @@ struct WideSmem {
 constexpr int kWideCompute = 512;                      // four warpgroups: 32 of a step's 128 key columns, D / 4 of the d each
 constexpr int kWideThreads = kWideCompute + 32;        // + the control warp: one lane issues every TMA load and MMA
 constexpr int kWideBarrier = 1;                        // hardware barrier id of the arithmetic warps
-constexpr int kMaxLiveTiles = 1024;                    // key tiles of a sequence when dead tiles are left out (sa_tc_skip.cu)
 
 template <int D, bool SELF, bool LIVE>   // LIVE: a table of live key tiles is given and the dead ones are left out
 __global__ void __launch_bounds__(kWideThreads, 1)
@@ -629,17 +613,17 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   const int ntiles = (p.seq + kTile - 1) / kTile;
   const int q_rows = p.seq - p.q_offset;                 // rows of the query tensor (all of them unless continuing a prefill)
   const int mi_first = p.q_offset / kTile;               // first query tile with a row to compute
-  CUtensorMap map_q, map_k128, map_v128;                 // boxes of 128 rows x 64 columns
-  int st = make_map_16bit(&map_q, p.q.ptr, D, q_rows, p.heads, p.batch, p.q.st, p.q.sh, p.q.sb, kTile);
+  ForwardMaps m;
+  int st = make_map_16bit(&m.q, p.q.ptr, D, q_rows, p.heads, p.batch, p.q.st, p.q.sh, p.q.sb, kTile);
   if (st != SA_OK) return st;
-  st = make_map_16bit(&map_k128, p.k.ptr, D, p.seq, p.heads, p.batch, p.k.st, p.k.sh, p.k.sb, kTile);
+  st = make_map_16bit(&m.k, p.k.ptr, D, p.seq, p.heads, p.batch, p.k.st, p.k.sh, p.k.sb, kTile);
   if (st != SA_OK) return st;
-  st = make_map_16bit(&map_v128, p.v.ptr, D, p.seq, p.heads, p.batch, p.v.st, p.v.sh, p.v.sb, kTile);
+  st = make_map_16bit(&m.v, p.v.ptr, D, p.seq, p.heads, p.batch, p.v.st, p.v.sh, p.v.sb, kTile);
   if (st != SA_OK) return st;
-  CUtensorMap map_q0, map_k0;                            // the selector's rows: (d, token, 1, batch)
-  st = make_map_16bit(&map_q0, p.q0.ptr, D, q_rows, 1, p.batch, p.q0.st, 0, p.q0.sb, kTile);
+  // the selector's rows: (d, token, 1, batch)
+  st = make_map_16bit(&m.q0, p.q0.ptr, D, q_rows, 1, p.batch, p.q0.st, 0, p.q0.sb, kTile);
   if (st != SA_OK) return st;
-  st = make_map_16bit(&map_k0, p.k0.ptr, D, p.seq, 1, p.batch, p.k0.st, 0, p.k0.sb, kTile);
+  st = make_map_16bit(&m.k0, p.k0.ptr, D, p.seq, 1, p.batch, p.k0.st, 0, p.k0.sb, kTile);
   if (st != SA_OK) return st;
   WaitCtx status;
   st = wait_ctx(&status);
@@ -652,7 +636,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   {
     ProfileScope prof(SA_KERNEL_TC_COLSUM, s);
     count_launch();
-    colsum_kernel<D><<<gc, 128, colsum_smem, s>>>(map_q0, map_k0, carry, p.seq, ntiles, p.exempt, p.scale, status,
+    colsum_kernel<D><<<gc, 128, colsum_smem, s>>>(m.q0, m.k0, carry, p.seq, ntiles, p.exempt, p.scale, status,
                                                   p.q_offset, mi_first);
   }
   SA_CUDA_CHECK(cudaGetLastError());
@@ -670,14 +654,18 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
     if (st != SA_OK) return st;
     alive = static_cast<const uint8_t*>(p.tile_table);
   }
+  const bool self = self_selecting(p);
+  // Heads that share a selector go two to a CTA: its selection is made once and the two overlap (1.3x a head-tile).  While
+  // one head a CTA still fits the GPU in one wave, that is faster: a step of it takes 3.2 k cycles, of a pair 4.3 k.
+  const int64_t ctas = (int64_t)(ntiles - mi_first) * p.batch * p.heads;
+  if (D == 64 && !self && p.heads % 2 == 0 && ctas > kSms) return forward_pair(p, m, carry, out, lse2, status, alive, s);
   const unsigned grid = (unsigned)(ntiles - mi_first) * p.batch * p.heads;
-  const bool self = (p.heads == 1) && !p.external_selector;   // one head per selector: the selection logits are the head's own
   const int wide_smem = WideSmem<D>::total + 1024;
   auto launch = [&](auto kernel) -> int {
     SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem));
     ProfileScope prof(SA_KERNEL_TC_FORWARD, s);
     count_launch();
-    kernel<<<grid, kWideThreads, wide_smem, s>>>(map_q, map_k128, map_v128, map_q0, map_k0, carry, out, lse2, p.heads, p.seq,
+    kernel<<<grid, kWideThreads, wide_smem, s>>>(m.q, m.k, m.v, m.q0, m.k0, carry, out, lse2, p.heads, p.seq,
                                                  ntiles, p.exempt, p.scale, status, static_cast<__nv_bfloat16*>(p.out_lowp),
                                                  p.out_lowp_rows, p.q_offset, alive);
     return SA_OK;

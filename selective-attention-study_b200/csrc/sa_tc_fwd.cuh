@@ -1,0 +1,34 @@
+// Tensor-core engine, forward: what its translation units share.
+#pragma once
+
+#include "sa_tc_host.cuh"
+#include "sa_tc_ptx.cuh"
+
+namespace sa {
+namespace tc {
+
+constexpr int kMaxLiveTiles = 1024;   // key tiles of a sequence when dead tiles are left out (sa_tc_skip.cu)
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// A global load the compiler must issue where it is written (volatile asm keeps its place among the other
+// volatile asm statements), so a value fetched one step ahead is really in flight during that step.
+__device__ __forceinline__ float load_ahead(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+struct ForwardMaps {                  // boxes of 128 rows x 64 columns
+  CUtensorMap q, k, v, q0, k0;
+};
+// Two heads a CTA (sa_tc_fwd_pair.cu): head_dim 64, an even number of heads sharing a selector.
+int forward_pair(const Problem& p, const ForwardMaps& m, const float* carry, float* out, float* lse2, const WaitCtx& status,
+                 const uint8_t* alive, cudaStream_t s);
+
+}  // namespace tc
+}  // namespace sa
