@@ -306,6 +306,33 @@ int sa_decode_step_live_keys(int dtype, int batch, int heads, int groups, int le
                              float* selected, float* key_norms, float* y, void* workspace, size_t workspace_bytes,
                              void* stream);
 
+/* The decode step from a block of arguments that a caller keeps with its cache and updates (q1, k1, v1, y, length, stream)
+ * from step to step.  key_norms may be NULL.  y_dtype: SA_F32, or dtype for y in the cache's own type. */
+typedef struct sa_decode {
+  int32_t struct_bytes;   /* sizeof(sa_decode) */
+  int32_t dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt;
+  const void *q1, *k1, *v1;
+  void *k_cache, *v_cache;
+  float *selected, *key_norms;
+  void *y, *workspace;
+  uint64_t workspace_bytes;
+  void *stream;
+} sa_decode;
+int sa_decode_run(const sa_decode* d);
+
+/* A prompt, or a further chunk of one, for a decode cache (tensor-core engine; replaces mixers.py:105-113 around the
+ * kernels).  p->seq counts the cached tokens and the new ones; q holds the queries from position `cached` on, k and v all
+ * p->seq keys.  `selected` (batch, >= p->seq at selected_stride) is read where cached > 0 and receives the totals in place; y
+ * receives the new rows in the operand type.  carry, lse2 and the table (may be NULL) are scratch. */
+int sa_prefill_rows(const sa_problem* p, int cached, const void* q, const void* k, const void* v, float* selected,
+                    int64_t selected_stride, const sa_tensor* y, float* lse2, float* carry, void* tile_table,
+                    size_t tile_table_bytes, void* stream);
+/* Stores `seq` new keys and values, rows of head_dim elements at the strides of k and v (batch, head, token), into the
+ * (batch, heads, capacity, head_dim) caches from position `at` on.  With `begin` also zeros every row behind them and, where
+ * given, the history sums `selected` (batch, groups, capacity) from at + seq on. */
+int sa_cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, int begin,
+                   const sa_tensor* k, const sa_tensor* v, void* k_cache, void* v_cache, float* selected, void* stream);
+
 /* Per-kernel device timing for benchmarks.  sa_profile_enable(id) makes every later launch of that
  * kernel record a CUDA event pair on its stream (id 0 disables); sa_profile_collect waits for the
  * recorded pairs, writes their durations in milliseconds (launch order) to ms_host, forgets them and

@@ -76,6 +76,7 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   p->q_offset = 0;
   p->carry_init = nullptr;
   p->carry_init_stride = 0;
+  p->total_stride = in->seq;
   p->tile_table = nullptr;
   p->out_lowp = nullptr;
   p->out_lowp_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
@@ -524,18 +525,73 @@ int sa_decode_step_live_keys(int dtype, int batch, int heads, int groups, int le
                              int exempt, const void* q1, const void* k1, const void* v1, void* k_cache, void* v_cache,
                              float* selected, float* key_norms, float* y, void* workspace, size_t workspace_bytes,
                              void* stream) {
-  if (!dtype_ok(dtype) || batch < 1 || heads < 1 || groups < 1 || heads % groups != 0 || length < 0 || exempt < 1)
+  sa_decode d{};
+  d.struct_bytes = sizeof(sa_decode);
+  d.dtype = dtype; d.y_dtype = SA_F32; d.batch = batch; d.heads = heads; d.groups = groups; d.length = length;
+  d.capacity = capacity; d.head_dim = head_dim; d.exempt = exempt;
+  d.q1 = q1; d.k1 = k1; d.v1 = v1; d.k_cache = k_cache; d.v_cache = v_cache; d.selected = selected; d.key_norms = key_norms;
+  d.y = y; d.workspace = workspace; d.workspace_bytes = workspace_bytes; d.stream = stream;
+  return sa_decode_run(&d);
+}
+
+int sa_decode_run(const sa_decode* d) {
+  if (d == nullptr || d->struct_bytes != (int32_t)sizeof(sa_decode)) return SA_ERR_BAD_ARGUMENT;
+  if (!dtype_ok(d->dtype) || d->batch < 1 || d->heads < 1 || d->groups < 1 || d->heads % d->groups != 0 || d->length < 0 ||
+      d->exempt < 1 || (d->y_dtype != SA_F32 && d->y_dtype != d->dtype))
+    return SA_ERR_BAD_ARGUMENT;
+  if (!dim_ok(d->head_dim)) return SA_ERR_UNSUPPORTED;
+  if (d->length >= d->capacity) return SA_ERR_BAD_ARGUMENT;
+  if (!d->q1 || !d->k1 || !d->v1 || !d->k_cache || !d->v_cache || !d->selected || !d->y || !d->workspace)
+    return SA_ERR_BAD_ARGUMENT;
+  if ((int64_t)d->batch * d->heads * ((d->length + 512) / 512) > 0x7fffffffLL) return SA_ERR_TOO_LARGE;   // 1-D grid
+  for (const void* ptr : {d->q1, d->k1, d->v1, (const void*)d->k_cache, (const void*)d->v_cache})   // 16-byte loads, bulk copies
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0) return SA_ERR_ALIGNMENT;
+  if (d->workspace_bytes < sa_decode_workspace_bytes(d->batch, d->heads, d->groups, d->length, d->head_dim))
+    return SA_ERR_WORKSPACE;
+  if (tc::timeout_pending()) return SA_ERR_DEVICE_TIMEOUT;
+  const DecodeStep step{d->dtype, d->y_dtype, d->batch, d->heads, d->groups, d->length, d->capacity, d->head_dim, d->exempt,
+                        d->q1, d->k1, d->v1, d->k_cache, d->v_cache, d->selected, d->key_norms, d->y,
+                        static_cast<float*>(d->workspace)};
+  return decode_step(step, static_cast<cudaStream_t>(d->stream));
+}
+
+int sa_prefill_rows(const sa_problem* in, int cached, const void* q, const void* k, const void* v, float* selected,
+                    int64_t selected_stride, const sa_tensor* y, float* lse2, float* carry, void* tile_table,
+                    size_t tile_table_bytes, void* stream) {
+  Problem p;
+  int st = to_problem(in, q, k, v, nullptr, &p);
+  if (st != SA_OK) return st;
+  if (!q || !k || !v || !selected || !lse2 || !carry) return SA_ERR_BAD_ARGUMENT;
+  if (cached < 0 || cached >= in->seq || selected_stride < in->seq) return SA_ERR_BAD_ARGUMENT;
+  if (in->engine != SA_ENGINE_TCGEN05) return SA_ERR_UNSUPPORTED;
+  st = tc_supported(p);
+  if (st == SA_OK) st = rows_of(y, in->dtype, &p.out_lowp_rows);
+  if (st != SA_OK) return st;
+  if (tc::timeout_pending()) return SA_ERR_DEVICE_TIMEOUT;
+  if (tile_table != nullptr) {
+    const size_t need = tc::tile_table_bytes(p);
+    if (need == 0) return SA_ERR_UNSUPPORTED;
+    if (tile_table_bytes < need) return SA_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(tile_table) & 255) != 0) return SA_ERR_ALIGNMENT;
+    p.tile_table = tile_table;
+  }
+  p.out_lowp = y->ptr;
+  p.q_offset = cached;
+  p.carry_init = cached > 0 ? selected : nullptr;
+  p.carry_init_stride = selected_stride;
+  p.total_stride = selected_stride;
+  return tc_forward(p, nullptr, lse2, carry, selected, static_cast<cudaStream_t>(stream));
+}
+
+int sa_cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, int begin,
+                   const sa_tensor* k, const sa_tensor* v, void* k_cache, void* v_cache, float* selected, void* stream) {
+  if (!dtype_ok(dtype) || batch < 1 || heads < 1 || groups < 1 || seq < 1 || at < 0 || (int64_t)at + seq > capacity ||
+      !k || !v || !k->ptr || !v->ptr || k->dtype != dtype || v->dtype != dtype || !k_cache || !v_cache)
     return SA_ERR_BAD_ARGUMENT;
   if (!dim_ok(head_dim)) return SA_ERR_UNSUPPORTED;
-  if (length >= capacity) return SA_ERR_BAD_ARGUMENT;
-  if (!q1 || !k1 || !v1 || !k_cache || !v_cache || !selected || !y || !workspace) return SA_ERR_BAD_ARGUMENT;
-  if ((int64_t)batch * heads * ((length + 512) / 512) > 0x7fffffffLL) return SA_ERR_TOO_LARGE;   // 1-D grid
-  for (const void* ptr : {q1, k1, v1, (const void*)k_cache, (const void*)v_cache})            // 16-byte loads, bulk copies
-    if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0) return SA_ERR_ALIGNMENT;
-  if (workspace_bytes < sa_decode_workspace_bytes(batch, heads, groups, length, head_dim)) return SA_ERR_WORKSPACE;
-  if (tc::timeout_pending()) return SA_ERR_DEVICE_TIMEOUT;
-  return decode_step(dtype, batch, heads, groups, length, capacity, head_dim, exempt, q1, k1, v1, k_cache, v_cache,
-                     selected, y, static_cast<float*>(workspace), key_norms, static_cast<cudaStream_t>(stream));
+  const RowLayout kr{k->stride[0], k->stride[1], k->stride[2]}, vr{v->stride[0], v->stride[1], v->stride[2]};
+  return cache_store(dtype, batch, heads, groups, seq, capacity, head_dim, at, begin != 0, k->ptr, kr, v->ptr, vr, k_cache, v_cache,
+                     selected, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -6,6 +6,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "../../include/selective_attention_b200.h"
 
 namespace sa {
@@ -57,6 +61,7 @@ struct Problem {
   int q_offset;
   const float* carry_init;
   int64_t carry_init_stride;
+  int64_t total_stride;  // of the per-key totals (tensor-core engine; default seq)
   void* out_lowp;        // null: not requested
   RowLayout out_lowp_rows;
   RowLayout dv_rows;     // where dv rows go (default: contiguous (batch, heads, seq, head_dim))
@@ -105,9 +110,38 @@ int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, 
                      const RowLayout* dst_rows, cudaStream_t s);
 
 size_t decode_workspace_floats(int batch, int heads, int groups, int length, int head_dim);
-int decode_step(int dtype, int batch, int heads, int groups, int length, int capacity, int head_dim, int exempt,
-                const void* q1, const void* k1, const void* v1, void* kc, void* vc, float* selected, float* y,
-                float* ws, float* knorm, cudaStream_t s);   // knorm: per-key norms, or null (every key is read)
+// One cached decode step; y in fp32 or in the cache's type, key_norms null when every key is read.
+struct DecodeStep {
+  int dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt;
+  const void *q1, *k1, *v1;
+  void *k_cache, *v_cache;
+  float *selected, *key_norms;
+  void* y;
+  float* workspace;
+};
+int decode_step(const DecodeStep& d, cudaStream_t s);
+
+// New rows of a decode cache from position `at` on; `begin`: and zeros behind them (also in `selected`, may be null).
+int cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, bool begin, const void* k,
+                const RowLayout& k_rows, const void* v, const RowLayout& v_rows, void* k_cache, void* v_cache, float* selected,
+                cudaStream_t s);
+
+// Lets a kernel use `bytes` of dynamic shared memory, once per kernel and device (the attribute outlives the call).
+template <typename K>
+inline cudaError_t allow_smem(K kernel, size_t bytes) {
+  static std::mutex mutex;
+  static std::map<std::pair<const void*, int>, size_t> allowed;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  const std::pair<const void*, int> key(reinterpret_cast<const void*>(kernel), dev);
+  std::lock_guard<std::mutex> lock(mutex);
+  auto it = allowed.find(key);
+  if (it != allowed.end() && it->second >= bytes) return cudaSuccess;
+  err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err == cudaSuccess) allowed[key] = bytes;
+  return err;
+}
 
 void set_last_cuda_error(int code);
 void count_launch();   // every kernel launch of the library calls this once (sa_launch_count)

@@ -3,6 +3,8 @@
 //   row stats the tensor-core engine's form of it: -lse2 and -dbar in blocks, dO in bf16, zeroed accumulators
 //   fold/cast dq = cast(dq_acc + [head 0] dq0)            (reference: kernels.py:662-666)
 //   decode    one cached decode step                       (reference: src/selective_attention/mixers.py:115-130)
+#include <type_traits>
+
 #include "sa_common.cuh"
 #include "sa_tc_host.cuh"
 #include "sa_tc_ptx.cuh"
@@ -147,19 +149,22 @@ __global__ void __launch_bounds__(256) fold_cast_kernel(const float* __restrict_
 
 // ---- decode -----------------------------------------------------------------------------------------
 constexpr int kDecThreads = 128;
-constexpr int kDecSplitMin = 512;             // keys per CTA: a multiple of 512, at least 512
+constexpr int kDecSplitMin = 128;             // keys per CTA: a multiple of 128, at least 128
+constexpr int kDecSplitsMax = 256;            // of a long cache: more would make the merge long
 constexpr int kDecCtasPerSm = 4;              // attend CTAs resident per SM (48 KB of stages each)
 
 // Keys per CTA for `t` cached keys and `rows` = batch * heads query rows: the grid is about one full wave of
-// resident CTAs, so no SM is left with a straggler and the combine pass stays short.
+// resident CTAs, so no SM is left with a straggler and the combine pass stays short.  With 512 keys at least, 96 rows of
+// 1,500 keys were 288 CTAs of three ring refills each and took 13.9 us; with 256 they fill the wave.
 static int decode_split_keys(int t, int rows) {
-  int target_splits = 148 * kDecCtasPerSm / rows;
-  if (target_splits < 1) target_splits = 1;
-  int keys = (t + target_splits - 1) / target_splits;
-  keys = (keys + kDecSplitMin - 1) / kDecSplitMin * kDecSplitMin;
-  if (keys < kDecSplitMin) keys = kDecSplitMin;
-  return keys;
+  const int target_splits = max(1, min(148 * kDecCtasPerSm / rows, kDecSplitsMax));
+  const int keys = (t + target_splits - 1) / target_splits;
+  return (keys + kDecSplitMin - 1) / kDecSplitMin * kDecSplitMin;
 }
+
+// The attend kernel is launched while the append kernel runs (programmatic stream serialization): what does not depend
+// on the new key or the tickets goes ahead of this wait.
+__device__ __forceinline__ void wait_for_append() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Writes the new key and value into the cache and clears the tickets the attend kernel counts CTAs with.
 // With `knorm` (the per-key norms a decode that leaves out dead keys relies on) also stores the new key's norm.
@@ -167,6 +172,7 @@ template <typename T>
 __global__ void append_kernel(const T* __restrict__ k1, const T* __restrict__ v1, T* __restrict__ kc,
                               T* __restrict__ vc, int rows, int capacity, int length, int D,
                               unsigned int* __restrict__ tickets, int n_tickets, float* __restrict__ knorm) {
+  asm volatile("griddepcontrol.launch_dependents;");
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < n_tickets) tickets[idx] = 0u;
   if (knorm != nullptr && idx < rows) {
@@ -215,7 +221,8 @@ constexpr float kDecDeadMargin = 150.f;         // binades below the newest key'
 // maximum is found first so that the weighted sums over splits have no serial dependence: warp w folds splits
 // w, w + 4, ... (lane l owns output columns l, l + 32, ...), then the four warps are added through shared memory.
 // The partials were written by other CTAs: they are read past the L1 cache.
-__device__ __forceinline__ void decode_combine_row(const float* prow, float* yrow, int splits, int D,
+template <typename TY>
+__device__ __forceinline__ void decode_combine_row(const float* prow, TY* yrow, int splits, int D,
                                                    float (*part)[128 + 1], float* red) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float m = -INFINITY;
@@ -250,7 +257,7 @@ __device__ __forceinline__ void decode_combine_row(const float* prow, float* yro
   if (d < D) {
     const float nn = part[0][d] + part[1][d] + part[2][d] + part[3][d];
     const float dd = part[0][128] + part[1][128] + part[2][128] + part[3][128];
-    yrow[d] = nn / dd;
+    yrow[d] = from_float<TY>(nn / dd);
   }
 }
 
@@ -266,11 +273,11 @@ __device__ __forceinline__ void decode_combine_row(const float* prow, float* yro
 // history term is zero, and the row maximum is at least that).  A CTA first marks the 64-key stages of its range that
 // hold a live key (it reads 8 bytes per key for that instead of the 2 x 128 or 256 of K and V) and then streams
 // only those.  The CTAs of a selecting head stay dense: the new query's selection is needed for every key.
-template <typename T, int D, bool LIVE>
+template <typename T, typename TY, int D, bool LIVE>
 __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     const T* __restrict__ q1, const T* __restrict__ kc, const T* __restrict__ vc, float* selected,
     float* __restrict__ partial, float* __restrict__ sel_new, int heads, int groups, int t, int capacity,
-    int exempt, float scale, int split_keys, tc::WaitCtx status, float* __restrict__ y, unsigned int* __restrict__ row_tickets, unsigned int* __restrict__ split_tickets, int splits,
+    int exempt, float scale, int split_keys, tc::WaitCtx status, TY* __restrict__ y, unsigned int* __restrict__ row_tickets, unsigned int* __restrict__ split_tickets, int splits,
     const float* __restrict__ knorm) {
   constexpr int kLanes = D / 8;                                   // lanes per key
   constexpr int kGroups = kDecThreads / kLanes;                   // keys the CTA covers per step
@@ -317,6 +324,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
   const float* selb = selected + ((int64_t)b * groups + g) * capacity;
   float* selnb = sel_new + ((int64_t)b * groups + g) * t;
   int n_iter = n_stages;
+  if (sparse || c1 == t) wait_for_append();                       // the new key's norm, or the new key itself
   if (sparse) {
     // |q| and the newest key's logit, by every group of lanes (each holds the whole of q between its lanes)
     float kx[8], ss = 0.f, dot = 0.f;
@@ -475,6 +483,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     prow[D + 1] = red[0];
   }
 
+  wait_for_append();                                              // the tickets are cleared
   // The last CTA of a query row merges the row's partials into y; the last of the `per` heads that share a
   // history vector to finish a key range adds the new selection of that range to it (every reader is done).
   __threadfence();                                                // partials and sel_new visible before the ticket
@@ -510,61 +519,107 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     decode_combine_row(partial + (int64_t)n * splits * (D + 2), y + (int64_t)n * D, splits, D, part, red);
 }
 
-template <typename T>
-int decode_impl(int batch, int heads, int groups, int length, int capacity, int D, int exempt, const void* q1,
-                const void* k1, const void* v1, void* kc, void* vc, float* selected, float* y, float* ws,
-                float* knorm, cudaStream_t s) {
-  const int rows = batch * heads, t = length + 1;
+template <typename T, typename TY, int D, bool LIVE>
+int launch_attend(unsigned grid, cudaStream_t s, const T* q, const T* kc, const T* vc, float* selected, float* partial,
+                  float* sel_new, int heads, int groups, int t, int capacity, int exempt, int split_keys,
+                  const tc::WaitCtx& status, TY* y, unsigned int* row_tickets, unsigned int* split_tickets, int splits,
+                  const float* knorm) {
+  auto kernel = decode_attend_kernel<T, TY, D, LIVE>;
+  SA_CUDA_CHECK(allow_smem(kernel, kDecSmemBytes));
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(kDecThreads);
+  config.dynamicSmemBytes = kDecSmemBytes;
+  config.stream = s;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  count_launch();
+  SA_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, q, kc, vc, selected, partial, sel_new, heads, groups, t, capacity, exempt,
+                                   1.0f / sqrtf((float)D), split_keys, status, y, row_tickets, split_tickets, splits, knorm));
+  return SA_OK;
+}
+
+template <typename T, typename TY>
+int decode_impl(const DecodeStep& d, cudaStream_t s) {
+  const int rows = d.batch * d.heads, t = d.length + 1, D = d.head_dim;
   // With key norms most CTAs find nothing to stream and only the selecting heads stay dense: short key ranges (1024
   // keys; 512 and 2048 measured slower) then spread those heads over the whole GPU.
-  const int split_keys = (knorm != nullptr) ? 2 * kDecSplitMin : decode_split_keys(t, rows);
+  const int split_keys = (d.key_norms != nullptr) ? 1024 : decode_split_keys(t, rows);
   const int splits = (t + split_keys - 1) / split_keys;
-  float* partial = ws;
+  float* partial = d.workspace;
   float* sel_new = partial + (size_t)rows * splits * (D + 2);
-  unsigned int* row_tickets = reinterpret_cast<unsigned int*>(sel_new + (size_t)batch * groups * t);
+  unsigned int* row_tickets = reinterpret_cast<unsigned int*>(sel_new + (size_t)d.batch * d.groups * t);
   unsigned int* split_tickets = row_tickets + rows;
-  const int n_tickets = rows + batch * groups * splits;
+  const int n_tickets = rows + d.batch * d.groups * splits;
   const int append_threads = rows * D > n_tickets ? rows * D : n_tickets;
+  tc::WaitCtx status;
+  if (int st = tc::wait_ctx(&status)) return st;
   ProfileScope prof(SA_KERNEL_DECODE, s);   // the whole step: append, then attend with its merge and update
   count_launch();
   append_kernel<T><<<(append_threads + 255) / 256, 256, 0, s>>>(
-      static_cast<const T*>(k1), static_cast<const T*>(v1), static_cast<T*>(kc), static_cast<T*>(vc), rows, capacity,
-      length, D, row_tickets, n_tickets, knorm);
+      static_cast<const T*>(d.k1), static_cast<const T*>(d.v1), static_cast<T*>(d.k_cache), static_cast<T*>(d.v_cache), rows,
+      d.capacity, d.length, D, row_tickets, n_tickets, d.key_norms);
   SA_CUDA_CHECK(cudaGetLastError());
-  const unsigned grid = (unsigned)rows * (unsigned)splits;
-  const float scale = 1.0f / sqrtf((float)D);
-  const T* q = static_cast<const T*>(q1);
-  const T* kk = static_cast<const T*>(kc);
-  const T* vv = static_cast<const T*>(vc);
-  tc::WaitCtx status;
-  if (int st = tc::wait_ctx(&status)) return st;
   // dead stages are left out when the norms are given and a CTA's range fits the stage list
-  const bool live = knorm != nullptr && split_keys / (kDecStageBytes / (D * (int)sizeof(T))) <= kDecMaxLive;
-#define SA_DECODE_LAUNCH_ONE(DIM, LIVE_)                                                                           \
-  do {                                                                                                             \
-    SA_CUDA_CHECK(cudaFuncSetAttribute(decode_attend_kernel<T, DIM, LIVE_>,                                        \
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecSmemBytes));          \
-    count_launch();                                                                                                \
-    decode_attend_kernel<T, DIM, LIVE_><<<grid, kDecThreads, kDecSmemBytes, s>>>(                                  \
-        q, kk, vv, selected, partial, sel_new, heads, groups, t, capacity, exempt, scale, split_keys, status,      \
-        y, row_tickets, split_tickets, splits, knorm);                                                            \
-  } while (0)
-#define SA_DECODE_LAUNCH(DIM)                                                                                      \
-  do {                                                                                                             \
-    if (live) SA_DECODE_LAUNCH_ONE(DIM, true);                                                                     \
-    else SA_DECODE_LAUNCH_ONE(DIM, false);                                                                         \
-  } while (0)
+  const bool live = d.key_norms != nullptr && split_keys / (kDecStageBytes / (D * (int)sizeof(T))) <= kDecMaxLive;
+  auto attend = [&](auto dim, auto live_tag) {
+    return launch_attend<T, TY, decltype(dim)::value, decltype(live_tag)::value>(
+        (unsigned)rows * (unsigned)splits, s, static_cast<const T*>(d.q1), static_cast<const T*>(d.k_cache),
+        static_cast<const T*>(d.v_cache), d.selected, partial, sel_new, d.heads, d.groups, t, d.capacity, d.exempt, split_keys,
+        status, static_cast<TY*>(d.y), row_tickets, split_tickets, splits, d.key_norms);
+  };
+  auto by_live = [&](auto dim) { return live ? attend(dim, std::true_type{}) : attend(dim, std::false_type{}); };
   switch (D) {
-    case 16: SA_DECODE_LAUNCH(16); break;
-    case 32: SA_DECODE_LAUNCH(32); break;
-    case 64: SA_DECODE_LAUNCH(64); break;
-    case 128: SA_DECODE_LAUNCH(128); break;
-    default: return SA_ERR_UNSUPPORTED;
+    case 16: return by_live(std::integral_constant<int, 16>{});
+    case 32: return by_live(std::integral_constant<int, 32>{});
+    case 64: return by_live(std::integral_constant<int, 64>{});
+    case 128: return by_live(std::integral_constant<int, 128>{});
   }
-#undef SA_DECODE_LAUNCH
-#undef SA_DECODE_LAUNCH_ONE
-  SA_CUDA_CHECK(cudaGetLastError());
-  return SA_OK;
+  return SA_ERR_UNSUPPORTED;
+}
+
+// ---- new rows of a decode cache ---------------------------------------------------------------------
+// blockIdx.y is the (batch, head) row, blockIdx.z 0: keys, 1: values, 2: the history sums behind the prompt.  Units are 16
+// bytes of a cache row.  Bound by memory: one read and one write of the new rows, one write of the zeros; the same in torch
+// is two fills and two strided copies (1.0 ms for 131,072 tokens of 16 heads).
+__global__ void __launch_bounds__(256) cache_store_kernel(const uint8_t* k, RowLayout k_rows, const uint8_t* v, RowLayout v_rows,
+                                                          uint8_t* kc, uint8_t* vc, float* selected, int heads, int groups, int seq,
+                                                          int capacity, int row_bytes, int elem_bytes, int at, bool begin, bool vec) {
+  const int n = blockIdx.y, b = n / heads, h = n - b * heads;
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  if (blockIdx.z == 2) {
+    if (h >= groups) return;
+    float* sel = selected + ((int64_t)b * groups + h) * capacity;
+    for (int64_t j = at + seq + first; j < capacity; j += step) sel[j] = 0.f;
+    return;
+  }
+  const RowLayout& rows = blockIdx.z == 0 ? k_rows : v_rows;
+  const uint8_t* src = (blockIdx.z == 0 ? k : v) + (rows.at(b, h, 0)) * elem_bytes;
+  uint8_t* dst = (blockIdx.z == 0 ? kc : vc) + (int64_t)n * capacity * row_bytes;
+  const int units = row_bytes / 16;
+  const int64_t last = (int64_t)(begin ? capacity : at + seq) * units;
+  for (int64_t u = (int64_t)at * units + first; u < last; u += step) {
+    const int t = (int)(u / units), c = (int)(u - (int64_t)t * units);
+    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+    if (t < at + seq) {
+      const uint8_t* from = src + (int64_t)(t - at) * rows.st * elem_bytes + c * 16;
+      if (vec) {
+        x = *reinterpret_cast<const uint4*>(from);
+      } else {                                       // rows at a multiple of the element size only
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          w[e] = elem_bytes == 4 ? *reinterpret_cast<const uint32_t*>(from + 4 * e)
+                                 : ((uint32_t)*reinterpret_cast<const uint16_t*>(from + 4 * e) |
+                                    ((uint32_t)*reinterpret_cast<const uint16_t*>(from + 4 * e + 2) << 16));
+        x = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+    *reinterpret_cast<uint4*>(dst + u * 16) = x;
+  }
 }
 
 }  // namespace
@@ -647,6 +702,34 @@ int launch_fold_cast(const float* acc, const float* acc0, void* dst, int dtype, 
   return SA_OK;
 }
 
+int cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, bool begin, const void* k,
+                const RowLayout& k_rows, const void* v, const RowLayout& v_rows, void* k_cache, void* v_cache, float* selected,
+                cudaStream_t s) {
+  if (((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0) return SA_ERR_ALIGNMENT;
+  if ((int64_t)batch * heads > 65535) return SA_ERR_UNSUPPORTED;
+  const int es = dtype == SA_F32 ? 4 : 2;
+  // A chunk whose rows are dense per head, heads at one pitch, is a plain 2-D copy: no kernel of ours.
+  auto pitched = [&](const RowLayout& r) { return r.st == head_dim && (batch == 1 || r.sb == heads * r.sh); };
+  if (!begin && pitched(k_rows) && pitched(v_rows)) {
+    const size_t row = (size_t)head_dim * es, width = seq * row, dst_pitch = capacity * row, nrows = (size_t)batch * heads;
+    const size_t k_pitch = nrows == 1 ? width : k_rows.sh * (size_t)es, v_pitch = nrows == 1 ? width : v_rows.sh * (size_t)es;
+    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(k_cache) + at * row, dst_pitch, k, k_pitch, width, nrows,
+                                    cudaMemcpyDeviceToDevice, s));
+    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(v_cache) + at * row, dst_pitch, v, v_pitch, width, nrows,
+                                    cudaMemcpyDeviceToDevice, s));
+    return SA_OK;
+  }
+  const bool vec = aligned_rows(k, k_rows, es, 16) && aligned_rows(v, v_rows, es, 16);
+  const int64_t units = (int64_t)((begin ? capacity : at + seq) - at) * head_dim * es / 16;
+  const unsigned blocks = (unsigned)max((int64_t)1, min((int64_t)256, (units + 1023) / 1024));
+  count_launch();
+  cache_store_kernel<<<dim3(blocks, batch * heads, begin && selected != nullptr ? 3 : 2), 256, 0, s>>>(
+      static_cast<const uint8_t*>(k), k_rows, static_cast<const uint8_t*>(v), v_rows, static_cast<uint8_t*>(k_cache),
+      static_cast<uint8_t*>(v_cache), selected, heads, groups, seq, capacity, head_dim * es, es, at, begin, vec);
+  SA_CUDA_CHECK(cudaGetLastError());
+  return SA_OK;
+}
+
 size_t decode_workspace_floats(int batch, int heads, int groups, int length, int head_dim) {
   const int t = length + 1;
   const size_t splits = (size_t)(t + kDecSplitMin - 1) / kDecSplitMin;       // upper bound: the smallest split size
@@ -654,19 +737,12 @@ size_t decode_workspace_floats(int batch, int heads, int groups, int length, int
          + (size_t)batch * heads + (size_t)batch * groups * splits;                       // tickets
 }
 
-int decode_step(int dtype, int batch, int heads, int groups, int length, int capacity, int head_dim, int exempt,
-                const void* q1, const void* k1, const void* v1, void* kc, void* vc, float* selected, float* y,
-                float* ws, float* knorm, cudaStream_t s) {
-  switch (dtype) {
-    case SA_F32:
-      return decode_impl<float>(batch, heads, groups, length, capacity, head_dim, exempt, q1, k1, v1, kc, vc, selected,
-                                y, ws, knorm, s);
-    case SA_BF16:
-      return decode_impl<__nv_bfloat16>(batch, heads, groups, length, capacity, head_dim, exempt, q1, k1, v1, kc, vc,
-                                        selected, y, ws, knorm, s);
-    case SA_F16:
-      return decode_impl<__half>(batch, heads, groups, length, capacity, head_dim, exempt, q1, k1, v1, kc, vc, selected,
-                                 y, ws, knorm, s);
+int decode_step(const DecodeStep& d, cudaStream_t s) {
+  const bool y_low = d.y_dtype != SA_F32;             // y in the cache's own type
+  switch (d.dtype) {
+    case SA_F32: return decode_impl<float, float>(d, s);
+    case SA_BF16: return y_low ? decode_impl<__nv_bfloat16, __nv_bfloat16>(d, s) : decode_impl<__nv_bfloat16, float>(d, s);
+    case SA_F16: return y_low ? decode_impl<__half, __half>(d, s) : decode_impl<__half, float>(d, s);
   }
   return SA_ERR_BAD_ARGUMENT;
 }

@@ -589,7 +589,7 @@ inline bool vector_rows(const Problem& p) {
 template <typename T, int D>
 int carry_impl(const Problem& p, float* carry, float* total, cudaStream_t s) {
   const int nb = (p.seq + kQ - 1) / kQ;
-  SA_CUDA_CHECK(cudaFuncSetAttribute(colsum_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)colsum_smem<D>()));
+  SA_CUDA_CHECK(allow_smem(colsum_kernel<T, D>, colsum_smem<D>()));
   count_launch();
   colsum_kernel<T, D><<<dim3((p.seq + kKF - 1) / kKF, nb, p.batch), kThreads, colsum_smem<D>(), s>>>(p, carry, nb, vector_rows(p));
   SA_CUDA_CHECK(cudaGetLastError());
@@ -603,7 +603,7 @@ template <typename T, int D>
 int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float* total, cudaStream_t s) {
   if (int st = carry_impl<T, D>(p, carry, total, s)) return st;
   const int nb = (p.seq + kQ - 1) / kQ;
-  SA_CUDA_CHECK(cudaFuncSetAttribute(forward_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)forward_smem<D>()));
+  SA_CUDA_CHECK(allow_smem(forward_kernel<T, D>, forward_smem<D>()));
   count_launch();
   forward_kernel<T, D><<<dim3(nb, p.batch * p.heads), kThreads, forward_smem<D>(), s>>>(p, carry, out, lse2, nb, vector_rows(p));
   SA_CUDA_CHECK(cudaGetLastError());
@@ -614,7 +614,7 @@ template <typename T, int D>
 int backward_impl(const Problem& p, const float* lse2, const float* carry, const float* dbar, const float* d_out,
                   float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
   const int nb = (p.seq + kQ - 1) / kQ;
-  SA_CUDA_CHECK(cudaFuncSetAttribute(backward_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)backward_smem<D>()));
+  SA_CUDA_CHECK(allow_smem(backward_kernel<T, D>, backward_smem<D>()));
   count_launch();
   backward_kernel<T, D><<<dim3((p.seq + kKB - 1) / kKB, p.batch * p.heads), kThreads, backward_smem<D>(), s>>>(
       p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, static_cast<T*>(dv), nb, vector_rows(p));

@@ -656,7 +656,7 @@ int backward(const Problem& p, const float* stats, const float* carry, const voi
   const int smem = (self ? PairSmem<true>::total : PairSmem<false>::total) + 1024;
   const uint8_t* alive = static_cast<const uint8_t*>(p.tile_table);
   auto launch = [&](auto kernel) -> int {
-    SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SA_CUDA_CHECK(allow_smem(kernel, smem));
     ProfileScope prof(SA_KERNEL_TC_BACKWARD, s);
     count_launch();
     kernel<<<(unsigned)ntiles * nrows, kPairThreads, smem, s>>>(

@@ -423,7 +423,7 @@ int backward_wide(const Problem& p, const float* stats, const float* carry, cons
   const uint8_t* alive = static_cast<const uint8_t*>(p.tile_table);
   const unsigned grid = 2u * (unsigned)ntiles * (unsigned)nrows;
   auto launch = [&](auto kernel) -> int {
-    SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SA_CUDA_CHECK(allow_smem(kernel, smem));
     ProfileScope prof(SA_KERNEL_TC_BACKWARD, s);
     count_launch();
     kernel<<<grid, kThreads, smem, s>>>(map_q, map_k, map_v, map_do, map_q0, map_k0, stats, carry, dq_acc, dq0,

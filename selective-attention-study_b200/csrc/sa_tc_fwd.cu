@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(128) colsum_kernel(const __grid_constant__ CUt
 
 // One thread per key column: CARRY[b][mi][j] = sum of COLSUM[b][m'][j] over m' < mi, in place; row `ntiles`
 // and total[b][j] receive the sum over all query tiles.  Only rows mi >= j / 128 exist.
-__global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, float* __restrict__ total, int seq,
-                                                   int ntiles, int mi_first, const float* __restrict__ init,
+__global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, float* total, int64_t total_stride, int seq,
+                                                   int ntiles, int mi_first, const float* init,
                                                    int64_t init_stride) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, fl
     run += x;
   }
   col[(int64_t)ntiles * seq] = run;
-  total[(int64_t)b * seq + j] = run;
+  total[(int64_t)b * total_stride + j] = run;                    // (a continued prefill: where `init` was)
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -586,11 +586,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     if (i < seq && i >= q_offset) {                            // rows before q_offset belong to an earlier call
       const int iq = i - q_offset;                             // row inside the query tensor
       const int q_rows = seq - q_offset;
-      float4* orow = reinterpret_cast<float4*>(out + ((int64_t)n * q_rows + iq) * D + wg * DH);
+      if (out != nullptr) {
+        float4* orow = reinterpret_cast<float4*>(out + ((int64_t)n * q_rows + iq) * D + wg * DH);
 #pragma unroll
-      for (int d = 0; d < DH; d += 4)
-        orow[d >> 2] = make_float4(__uint_as_float(r[d]) * inv, __uint_as_float(r[d + 1]) * inv,
-                                   __uint_as_float(r[d + 2]) * inv, __uint_as_float(r[d + 3]) * inv);
+        for (int d = 0; d < DH; d += 4)
+          orow[d >> 2] = make_float4(__uint_as_float(r[d]) * inv, __uint_as_float(r[d + 1]) * inv,
+                                     __uint_as_float(r[d + 2]) * inv, __uint_as_float(r[d + 3]) * inv);
+      }
       if (wg == 0) lse2[(int64_t)n * q_rows + iq] = run_max + log2f(den);
       if (out_lowp != nullptr) {                               // the same rows in the operand dtype, in the caller's layout
         uint4* lrow = reinterpret_cast<uint4*>(out_lowp + out_lowp_rows.at(b, h, iq) + wg * DH);
@@ -631,7 +633,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
 
   constexpr int DK = D / 64;
   const int colsum_smem = 3 * DK * kRowTile + 1024;
-  SA_CUDA_CHECK(cudaFuncSetAttribute(colsum_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, colsum_smem));
+  SA_CUDA_CHECK(allow_smem(colsum_kernel<D>, colsum_smem));
   dim3 gc(ntiles, (ntiles - mi_first + kColsumChunk - 1) / kColsumChunk, p.batch);
   {
     ProfileScope prof(SA_KERNEL_TC_COLSUM, s);
@@ -644,7 +646,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   {
     ProfileScope prof(SA_KERNEL_TC_SCAN, s);
     count_launch();
-    scan_kernel<<<gs, 256, 0, s>>>(carry, total, p.seq, ntiles, mi_first, p.carry_init, p.carry_init_stride);
+    scan_kernel<<<gs, 256, 0, s>>>(carry, total, p.total_stride, p.seq, ntiles, mi_first, p.carry_init, p.carry_init_stride);
   }
   SA_CUDA_CHECK(cudaGetLastError());
 
@@ -662,7 +664,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   const unsigned grid = (unsigned)(ntiles - mi_first) * p.batch * p.heads;
   const int wide_smem = WideSmem<D>::total + 1024;
   auto launch = [&](auto kernel) -> int {
-    SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem));
+    SA_CUDA_CHECK(allow_smem(kernel, wide_smem));
     ProfileScope prof(SA_KERNEL_TC_FORWARD, s);
     count_launch();
     kernel<<<grid, kWideThreads, wide_smem, s>>>(m.q, m.k, m.v, m.q0, m.k0, carry, out, lse2, p.heads, p.seq,

@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
       if (mine) {
         float* orow = out + (n * q_rows + iq) * D + 32 * c;
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(orow + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+        for (int e = 0; e < 32 && out != nullptr; e += 4) *reinterpret_cast<float4*>(orow + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
         if (out_lowp != nullptr) {                             // the same rows in the operand dtype, in the caller's layout
           uint4* lrow = reinterpret_cast<uint4*>(out_lowp + out_lowp_rows.at(b, h0 + x, iq) + 32 * c);
 #pragma unroll
@@ -421,7 +421,7 @@ int forward_pair(const Problem& p, const ForwardMaps& m, const float* carry, flo
   const unsigned grid = (unsigned)(ntiles - p.q_offset / kTile) * p.batch * (p.heads / 2);
   const int smem = PairSmem::total;
   auto launch = [&](auto kernel) -> int {
-    SA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SA_CUDA_CHECK(allow_smem(kernel, smem));
     ProfileScope prof(SA_KERNEL_TC_FORWARD, s);
     count_launch();
     kernel<<<grid, kThreads, smem, s>>>(m.q, m.k, m.v, m.q0, m.k0, carry, out, lse2, p.heads, p.seq, ntiles, p.exempt, p.scale,

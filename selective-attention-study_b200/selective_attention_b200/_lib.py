@@ -24,7 +24,8 @@ EXPORTS = ("sa_abi_version", "sa_status_string", "sa_last_cuda_error", "sa_engin
            "sa_backward_workspace_bytes", "sa_backward", "sa_decode_workspace_bytes", "sa_decode_step", "sa_device_status", "sa_selftest_tcgen05", "sa_profile_enable",
            "sa_profile_collect", "sa_static_scratch_floats", "sa_forward_static_scratch", "sa_forward_selector",
            "sa_backward_selector", "sa_forward_fused", "sa_backward_fused", "sa_prefill_extend", "sa_selection_carry", "sa_launch_count", "sa_selftest_wait_timeout",
-           "sa_tile_table_bytes", "sa_forward_live_tiles", "sa_backward_live_tiles", "sa_prefill_extend_live_tiles", "sa_decode_step_live_keys")
+           "sa_tile_table_bytes", "sa_forward_live_tiles", "sa_backward_live_tiles", "sa_prefill_extend_live_tiles", "sa_decode_step_live_keys",
+           "sa_decode_run", "sa_prefill_rows", "sa_cache_store")
 
 
 class Problem(ctypes.Structure):
@@ -44,6 +45,15 @@ class Tensor(ctypes.Structure):
     """sa_tensor: rows of head_dim contiguous elements at batch / head / token strides."""
     _fields_ = [("ptr", ctypes.c_void_p), ("dtype", ctypes.c_int32), ("reserved", ctypes.c_int32),
                 ("stride", ctypes.c_int64 * 3)]
+
+
+class Decode(ctypes.Structure):
+    """sa_decode: the arguments of a decode step, kept with its cache."""
+    _fields_ = ([(name, ctypes.c_int32) for name in ("struct_bytes", "dtype", "y_dtype", "batch", "heads", "groups", "length",
+                                                     "capacity", "head_dim", "exempt")] +
+                [(name, ctypes.c_void_p) for name in ("q1", "k1", "v1", "k_cache", "v_cache", "selected", "key_norms", "y",
+                                                      "workspace")] +
+                [("workspace_bytes", ctypes.c_uint64), ("stream", ctypes.c_void_p)])
 
 
 class LibraryError(RuntimeError):
@@ -118,6 +128,12 @@ def load() -> ctypes.CDLL:
     lib.sa_decode_step.argtypes = [i32] * 8 + [vp] * 8 + [sz, vp]
     lib.sa_decode_step_live_keys.restype = i32
     lib.sa_decode_step_live_keys.argtypes = [i32] * 8 + [vp] * 9 + [sz, vp]
+    lib.sa_decode_run.restype = i32
+    lib.sa_decode_run.argtypes = [vp]
+    lib.sa_prefill_rows.restype = i32
+    lib.sa_prefill_rows.argtypes = [pp, i32, vp, vp, vp, f32p, ctypes.c_int64, tp, f32p, f32p, vp, sz, vp]
+    lib.sa_cache_store.restype = i32
+    lib.sa_cache_store.argtypes = [i32] * 9 + [tp, tp, vp, vp, f32p, vp]
     lib.sa_device_status.restype = i32
     lib.sa_device_status.argtypes = [ctypes.POINTER(ctypes.c_uint), i32]
     lib.sa_selftest_tcgen05.restype = i32

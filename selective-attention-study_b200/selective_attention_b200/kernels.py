@@ -19,6 +19,7 @@ There is no fallback: without the library every kernel entry raises.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
@@ -179,8 +180,16 @@ def _check_selector(selector, q: torch.Tensor):
     return tuple(out)
 
 
+_NO_GUARD = contextlib.nullcontext()
+
+
+def _on(device):
+    """``torch.cuda.device(device)`` where it is not the current device already."""
+    return _NO_GUARD if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def _prepare(q, k, v, lowp: bool):
@@ -227,7 +236,7 @@ def _selection_carry32(q, k, sel, exempt: int, zero: bool):
     total = torch.empty(b, t, device=q.device, dtype=torch.float32)
     prob = _problem(q, k, q, _lib.ENGINE_SIMT, exempt)
     sel_ref = ctypes.byref(_selector_struct(*sel)) if sel is not None else None
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         st = lib.sa_selection_carry(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), sel_ref, carry.data_ptr(),
                                     total.data_ptr(), _stream(q.device))
     _lib.check("sa_selection_carry", st)
@@ -258,7 +267,7 @@ def _forward(q, k, v, lowp: bool, exempt: int, damp: int, train_len: int, select
         need = lib.sa_tile_table_bytes(ctypes.byref(prob))
         if need:
             table = torch.empty(need, device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = lib.sa_forward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), sel_ref,
                                        out.data_ptr(), None, lse2.data_ptr(), carry.data_ptr(), total.data_ptr(),
                                        table.data_ptr() if table is not None else None,
@@ -344,7 +353,7 @@ def _backward_call(ctx, dout, dq0=None, dk0=None):
     dq, dk, dv = (torch.empty(q.shape, device=dev, dtype=q.dtype) for _ in range(3))
     sel_ref = ctypes.byref(_selector_struct(*sel)) if sel is not None else None
     table = getattr(ctx, "tile_table", None)
-    with torch.cuda.device(dev):
+    with _on(dev):
         if table is not None:           # the forward left out dead tiles: the backward walks the same live ones
             descs = [_tensor_struct(x) for x in (dout, dq, dk, dv)]
             st = lib.sa_backward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), sel_ref,
@@ -507,7 +516,7 @@ class _SelectiveAttentionPackedFn(torch.autograd.Function):
         need = lib.sa_tile_table_bytes(ctypes.byref(prob)) if skip_dead_tiles else 0
         if need:
             table = torch.empty(need, device=dev, dtype=torch.uint8)
-        with torch.cuda.device(dev):
+        with _on(dev):
             st = lib.sa_forward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), None,
                                            out.data_ptr(), ctypes.byref(low), lse2.data_ptr(), carry.data_ptr(),
                                            total.data_ptr(), table.data_ptr() if need else None, need, _stream(dev))
@@ -534,7 +543,7 @@ class _SelectiveAttentionPackedFn(torch.autograd.Function):
         workspace = torch.empty(max(need, 1), device=dev, dtype=torch.uint8)
         descs = [_tensor_struct(x) for x in (d_merged.view(b, t, h, d).transpose(1, 2), dq, dk, dv)]
         table = ctx.tile_table
-        with torch.cuda.device(dev):
+        with _on(dev):
             st = lib.sa_backward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), None,
                                             out.data_ptr(), lse2.data_ptr(), carry.data_ptr(),
                                             *(ctypes.byref(x) for x in descs), None, None, workspace.data_ptr(), need,
@@ -555,6 +564,62 @@ def selective_attention_packed(qkv: torch.Tensor, exempt: int = 1, *, skip_dead_
 
 # ---- cached decode ------------------------------------------------------------------------------------
 
+def _store_rows(cache: dict, k: torch.Tensor, v: torch.Tensor, at: int, begin: bool) -> None:
+    """New keys and values into the cache from position ``at`` on; ``begin``: the first ones, with zeros behind them (and in
+    ``selected``).  One launch where the rows are of the cache's type and contiguous along head_dim."""
+    kc, vc, selected = cache["k"], cache["v"], cache["selected"]
+    b, h, cap, d = kc.shape
+    t = k.shape[2]
+    if not (kc.is_cuda and k.dtype == v.dtype == kc.dtype and k.device == v.device == kc.device and k.stride(3) == v.stride(3) == 1
+            and kc.is_contiguous() and vc.is_contiguous() and selected.is_contiguous() and b * h <= 65535 and d in HEAD_DIMS):
+        kc[:, :, at:at + t] = k
+        vc[:, :, at:at + t] = v
+        if begin:
+            for x in (kc, vc, selected):
+                x[:, :, at + t:] = 0
+        return
+    with _on(kc.device):
+        st = _lib.load().sa_cache_store(_DTYPE_CODE[kc.dtype], b, h, selected.shape[1], t, cap, d, at, int(begin),
+                                        ctypes.byref(_tensor_struct(k)), ctypes.byref(_tensor_struct(v)), kc.data_ptr(),
+                                        vc.data_ptr(), selected.data_ptr(), _stream(kc.device))
+    _lib.check("sa_cache_store", st)
+
+
+def _prefill_rows(q, k, v, cached: int, selected: torch.Tensor, exempt: int, skip_dead_tiles: bool = False) -> torch.Tensor:
+    """Rows ``cached`` .. of a prompt in bf16, (B, H, Tn, D), and the totals of its keys into ``selected`` (B, G, capacity).
+    q holds the new queries; k, v all keys, or a cache of them.  G = 1, or G = H with every head its own selector."""
+    lib = _lib.load()
+    b, h, tn, d = q.shape
+    total_len, cap = cached + tn, selected.shape[2]
+    if selected.shape[1] == h and h > 1:         # every head is its own one-head sequence
+        q, k, v = (x.reshape(b * h, 1, x.shape[2], d) for x in (q, k, v))
+    q, k, v = (_strided(x, True) for x in (q, k, v))
+    bb, hh = q.shape[:2]
+    dev, engine = q.device, _lib.ENGINE_TCGEN05
+    y = torch.empty(b, h, tn, d, device=dev, dtype=torch.bfloat16)
+    # one allocation for the scratch: log-sum-exp rows, then the checkpoints (256-byte aligned)
+    lse_bytes = (bb * hh * tn * 4 + 255) // 256 * 256
+    scratch = torch.empty(lse_bytes + bb * lib.sa_carry_checkpoints(engine, total_len) * total_len * 4, device=dev, dtype=torch.uint8)
+    prob = _problem(q, k, v, engine, exempt)
+    prob.seq = total_len
+    need = lib.sa_tile_table_bytes(ctypes.byref(prob)) if skip_dead_tiles else 0
+    table = torch.empty(need, device=dev, dtype=torch.uint8) if need else None
+    rows = _tensor_struct(y.view(bb, hh, tn, d))
+    with _on(dev):
+        st = lib.sa_prefill_rows(ctypes.byref(prob), cached, q.data_ptr(), k.data_ptr(), v.data_ptr(), selected.data_ptr(), cap,
+                                 ctypes.byref(rows), scratch.data_ptr(), scratch.data_ptr() + lse_bytes,
+                                 table.data_ptr() if need else None, need, _stream(dev))
+    _lib.check("sa_prefill_rows", st)
+    return y
+
+
+def _prompt_in_place(q: torch.Tensor, v: torch.Tensor, dot_precision: str | None, damp: str, groups: int) -> bool:
+    """Whether ``_prefill_rows`` gives what a forward with its output cast to v's type would: bf16 throughout, on the
+    tensor-core engine, one selector per sequence or per head."""
+    return (q.dtype == v.dtype == torch.bfloat16 and _lowp(dot_precision, q.dtype) and damp == "none" and groups in (1, q.shape[1])
+            and _engine(True, q.shape[3], False) == _lib.ENGINE_TCGEN05)
+
+
 def prefill_extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, exempt: int = 1, *,
                    skip_dead_tiles: bool = False) -> torch.Tensor:
     """Continues a prefill: appends a chunk of new tokens to the cache and returns their outputs, (B, H, Tn, D)
@@ -566,6 +631,11 @@ def prefill_extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
     (head 0 selects) or G = H (every head its own selector).  q, k, v: (B, H, Tn, D).  bf16 operands on the
     tensor-core engine only (head_dim 64 or 128).  ``skip_dead_tiles``: as in ``selective_attention``; the part of
     the cache whose probabilities are all exactly zero for the new queries is not read."""
+    return _extend(cache, q, k, v, exempt, skip_dead_tiles, torch.float32)
+
+
+def _extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, exempt: int, skip_dead_tiles: bool,
+            out_dtype: torch.dtype) -> torch.Tensor:
     lib = _lib.load()
     exempt = _check_exempt(exempt)
     kc, vc, selected = cache["k"], cache["v"], cache["selected"]
@@ -584,11 +654,14 @@ def prefill_extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
                          "per sequence or per head")
     if cached == 0:
         raise ValueError("the cache is empty: use selective_attention_forward(return_aux=True) for the first chunk")
-    kc[:, :, cached:total_len] = k
-    vc[:, :, cached:total_len] = v
+    _store_rows(cache, k, v, cached, begin=False)
     if cache.get("key_norms") is not None:
         cache["key_norms"][:, :, cached:total_len] = key_norms(k.to(kc.dtype))
     qn = q.to(torch.bfloat16)
+    if out_dtype == torch.bfloat16:
+        y = _prefill_rows(qn, kc, vc, cached, selected, exempt, skip_dead_tiles)
+        cache["len"] = total_len
+        return y
     if groups == h and h > 1:             # every head is its own one-head sequence
         qn = qn.reshape(b * h, 1, tn, d)
         kv, vv = kc.view(b * h, 1, cap, d), vc.view(b * h, 1, cap, d)
@@ -606,7 +679,7 @@ def prefill_extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
     prob.seq = total_len
     need = lib.sa_tile_table_bytes(ctypes.byref(prob)) if skip_dead_tiles else 0
     table = torch.empty(need, device=dev, dtype=torch.uint8) if need else None
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = lib.sa_prefill_extend_live_tiles(ctypes.byref(prob), cached, qn.data_ptr(), kv.data_ptr(), vv.data_ptr(),
                                               selected.data_ptr(), cap, out.data_ptr(), lse2.data_ptr(),
                                               carry.data_ptr(), total.data_ptr(),
@@ -634,38 +707,67 @@ def decode_step(cache: dict, q1: torch.Tensor, k1: torch.Tensor, v1: torch.Tenso
     When the cache also holds ``"key_norms"`` (B, H, capacity) fp32 (``key_norms(k)`` of the cached keys; the slot's
     ``begin_cache(..., live_keys=True)`` creates it), the step leaves out the part of the cache whose weights are
     below 2^-150 for this query and keeps the norms up to date."""
-    lib = _lib.load()
+    return _decode(cache, q1, k1, v1, exempt, torch.float32)
+
+
+class _DecodePlan:
+    """What a decode step finds out about its cache: checked once, kept with the cache for as long as it holds the same
+    tensors.  A step then only fills in its own pointers and position."""
+
+    def __init__(self, cache: dict):
+        kc, vc, selected = self.tensors = (cache["k"], cache["v"], cache["selected"])
+        norms = self.norms = cache.get("key_norms")
+        b, h, cap, d = kc.shape
+        if not (kc.is_cuda and kc.is_contiguous() and vc.is_contiguous() and selected.is_contiguous()):
+            raise ValueError("the cache must be contiguous CUDA tensors")
+        if kc.dtype not in _DTYPE_CODE or vc.dtype != kc.dtype or selected.dtype != torch.float32:
+            raise ValueError("cache dtype must be float16, bfloat16 or float32 with fp32 `selected`")
+        if d not in HEAD_DIMS:
+            raise ValueError(f"head_dim must be one of {HEAD_DIMS}; got {d}")
+        if norms is not None and not (norms.is_cuda and norms.dtype == torch.float32 and norms.is_contiguous()
+                                      and tuple(norms.shape) == (b, h, cap)):
+            raise ValueError("cache['key_norms'] must be a contiguous fp32 CUDA tensor (B, H, capacity)")
+        self.shape, self.token = (b, h, d), (b, h, 1, d)
+        self.capacity, self.dtype, self.device = cap, kc.dtype, kc.device
+        groups = selected.shape[1]
+        # scratch for the longest step that the cache can take
+        need = _lib.load().sa_decode_workspace_bytes(b, h, groups, max(cap - 1, 0), d)
+        self.workspace = torch.empty(need, device=kc.device, dtype=torch.uint8)
+        a = self.args = _lib.Decode()
+        a.struct_bytes = ctypes.sizeof(_lib.Decode)
+        a.dtype, a.batch, a.heads, a.groups, a.capacity, a.head_dim = _DTYPE_CODE[kc.dtype], b, h, groups, cap, d
+        a.k_cache, a.v_cache, a.selected = kc.data_ptr(), vc.data_ptr(), selected.data_ptr()
+        a.key_norms = norms.data_ptr() if norms is not None else None
+        a.workspace, a.workspace_bytes = self.workspace.data_ptr(), need
+        self.address = ctypes.addressof(a)
+
+    def holds(self, cache: dict) -> bool:
+        kc, vc, selected = self.tensors
+        a = self.args
+        return (cache["k"] is kc and cache["v"] is vc and cache["selected"] is selected and cache.get("key_norms") is self.norms
+                and kc.data_ptr() == a.k_cache and vc.data_ptr() == a.v_cache and selected.data_ptr() == a.selected)
+
+
+def _decode(cache: dict, q1: torch.Tensor, k1: torch.Tensor, v1: torch.Tensor, exempt: int, out_dtype: torch.dtype) -> torch.Tensor:
+    """The step with y in fp32 or in the cache's own type."""
     exempt = _check_exempt(exempt)
-    kc, vc, selected = cache["k"], cache["v"], cache["selected"]
-    b, h, cap, d = kc.shape
+    plan = cache.get("_plan")
+    if plan is None or not plan.holds(cache):
+        plan = cache["_plan"] = _DecodePlan(cache)
     length = int(cache["len"])
-    if length >= cap:
+    if length >= plan.capacity:
         raise ValueError("decode step past the cache capacity (context_length)")
-    if not (kc.is_cuda and kc.is_contiguous() and vc.is_contiguous() and selected.is_contiguous()):
-        raise ValueError("the cache must be contiguous CUDA tensors")
-    if kc.dtype not in _DTYPE_CODE or vc.dtype != kc.dtype or selected.dtype != torch.float32:
-        raise ValueError("cache dtype must be float16, bfloat16 or float32 with fp32 `selected`")
-    if d not in HEAD_DIMS:
-        raise ValueError(f"head_dim must be one of {HEAD_DIMS}; got {d}")
-    groups = selected.shape[1]
-    q1, k1, v1 = (t.reshape(b, h, d) for t in (q1, k1, v1))
-    q1, k1, v1 = (t if (t.dtype == kc.dtype and t.is_contiguous()) else t.to(kc.dtype).contiguous() for t in (q1, k1, v1))
-    dev = kc.device
-    y = torch.empty(b, h, 1, d, device=dev, dtype=torch.float32)
-    need = lib.sa_decode_workspace_bytes(b, h, groups, length, d)
-    ws = cache.get("_workspace")                  # scratch of the step, kept with the cache and grown when needed
-    if ws is None or ws.numel() < need or ws.device != dev:
-        ws = torch.empty(max(2 * need, 1 << 16), device=dev, dtype=torch.uint8)
-        cache["_workspace"] = ws
-    norms = cache.get("key_norms")
-    if norms is not None and not (norms.is_cuda and norms.dtype == torch.float32 and norms.is_contiguous()
-                                  and tuple(norms.shape) == (b, h, cap)):
-        raise ValueError("cache['key_norms'] must be a contiguous fp32 CUDA tensor (B, H, capacity)")
-    with torch.cuda.device(dev):
-        st = lib.sa_decode_step_live_keys(_DTYPE_CODE[kc.dtype], b, h, groups, length, cap, d, exempt, q1.data_ptr(),
-                                          k1.data_ptr(), v1.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-                                          selected.data_ptr(), norms.data_ptr() if norms is not None else None,
-                                          y.data_ptr(), ws.data_ptr(), need, _stream(dev))
-    _lib.check("sa_decode_step", st)
+    dtype, token, dev = plan.dtype, plan.token, plan.device
+    q1, k1, v1 = (t if (t.dtype == dtype and t.shape == token and t.device == dev and t.is_contiguous())
+                  else t.reshape(plan.shape).to(dtype).contiguous() for t in (q1, k1, v1))
+    y = torch.empty(token, device=dev, dtype=out_dtype)
+    a = plan.args
+    a.y_dtype, a.length, a.exempt = _DTYPE_CODE[out_dtype], length, exempt
+    a.q1, a.k1, a.v1, a.y = q1.data_ptr(), k1.data_ptr(), v1.data_ptr(), y.data_ptr()
+    a.stream = _stream(dev)
+    with _on(dev):
+        st = _lib.load().sa_decode_run(plan.address)
+    if st:
+        _lib.check("sa_decode_step", st)
     cache["len"] = length + 1
     return y

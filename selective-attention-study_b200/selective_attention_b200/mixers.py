@@ -71,14 +71,24 @@ class SelectiveAttentionSlot:
         """Prefill: outputs plus the decode cache {"k", "v", "len", "selected"}.  ``live_keys`` adds ``"key_norms"``,
         with which the decode steps leave out the part of the cache that no longer carries weight."""
         b, h, t, d = k.shape
-        y, total = self.attend(q, k, v, want_total=True)
         capacity = max(capacity if capacity is not None else self.context_length, t)
-        cache = {"k": k.new_zeros(b, h, capacity, d), "v": v.new_zeros(b, h, capacity, d), "len": t}
-        cache["k"][:, :, :t] = k
-        cache["v"][:, :, :t] = v
-        selected = torch.zeros(b, self.groups, capacity, device=k.device, dtype=torch.float32)
-        selected[:, :, :t] = total.float()
-        cache["selected"] = selected
+        if not (self._kernel_ok(q) and k.device == v.device == q.device and k.dtype == v.dtype):
+            y, total = self.attend(q, k, v, want_total=True)
+            cache = {"k": k.new_zeros(b, h, capacity, d), "v": v.new_zeros(b, h, capacity, d), "len": t,
+                     "selected": torch.zeros(b, self.groups, capacity, device=k.device, dtype=torch.float32)}
+            cache["k"][:, :, :t] = k
+            cache["v"][:, :, :t] = v
+            cache["selected"][:, :, :t] = total.float()
+        else:
+            cache = {"k": k.new_empty(b, h, capacity, d), "v": v.new_empty(b, h, capacity, d), "len": t,
+                     "selected": torch.empty(b, self.groups, capacity, device=k.device, dtype=torch.float32)}
+            kernels.check_inputs(q, k, v)
+            kernels._store_rows(cache, k, v, 0, begin=True)
+            if kernels._prompt_in_place(q, v, self.dot_precision, self.history_damp, self.groups):
+                y = kernels._prefill_rows(q, k, v, 0, cache["selected"], self.exempt)
+            else:
+                y, total = self.attend(q, k, v, want_total=True)
+                cache["selected"][:, :, :t] = total
         if live_keys:
             norms = torch.zeros(b, h, capacity, device=k.device, dtype=torch.float32)
             norms[:, :, :t] = kernels.key_norms(k)
@@ -89,12 +99,16 @@ class SelectiveAttentionSlot:
         """A further chunk of prompt tokens: (B, H, Tn, D) outputs in v's dtype; appends to the cache and moves
         ``selected`` on.  Equals the rows a single prefill over all tokens would produce.  ``skip_dead_tiles``: the
         part of the cache whose probabilities are all exactly zero for these queries is not read (same rows)."""
-        return kernels.prefill_extend(cache, q, k, v, self.exempt, skip_dead_tiles=skip_dead_tiles).to(v.dtype)
+        out_dtype = torch.bfloat16 if v.dtype == torch.bfloat16 else torch.float32
+        y = kernels._extend(cache, q, k, v, self.exempt, skip_dead_tiles, out_dtype)
+        return y if y.dtype == v.dtype else y.to(v.dtype)
 
     def step_cache(self, q1, k1, v1, cache: dict):
         """One token: (B, H, 1, D) in q1's dtype; appends to the cache and updates ``selected``."""
         if cache["len"] >= cache["k"].shape[2]:
             raise ValueError("decode step past the cache capacity (context_length)")
         if cache["k"].is_cuda and kernels.HAS_KERNELS and self.use_kernel:
-            return kernels.decode_step(cache, q1, k1, v1, self.exempt).to(q1.dtype)
+            out_dtype = q1.dtype if q1.dtype == cache["k"].dtype else torch.float32
+            y = kernels._decode(cache, q1, k1, v1, self.exempt, out_dtype)
+            return y if y.dtype == q1.dtype else y.to(q1.dtype)
         raise RuntimeError("cached decode needs CUDA tensors and the built library (no CPU path)")
