@@ -49,26 +49,13 @@
 // selection-gradient products).
 #include <type_traits>
 
-#include "sa_tc_bwd_passes.cuh"
+#include "sa_tc_bwd_chain.cuh"
 
 namespace sa {
 namespace tc {
 namespace {
 
-using bwd::ex2;
-using bwd::find_top_tile;
-using bwd::kHalfTile;
-using bwd::kRowTile;
-using bwd::kTile;
-using bwd::load_ahead;
-using bwd::store_key_grads;
-using bwd::tile_of_block;
-
-constexpr int kPairThreads = 512;     // two chains, the read-out warpgroup, three MMA warps and a load warp
-// Registers: 512 x 128 at launch; the chains keep 64 values and their masks, the rest needs little: 256 x 168 + 256 x 88.
-constexpr int kChainRegs = 168, kOtherRegs = 88;
-constexpr int kMmaWarp = 12, kLoadWarp = 13, kDqWarp = 14, kScoreWarp = 15;
-constexpr int kStatBytes = 512;       // -lse2 and -dbar of 64 queries
+using namespace bwd;
 
 template <bool SELF>
 struct PairSmem {
@@ -87,23 +74,12 @@ struct PairSmem {
   static constexpr int total = stat + kRing * kStatBytes;
 };
 
-// TMEM columns
-constexpr uint32_t kDV = 0, kDK = 64, kDQ = 128, kW = 192, kDK0 = 448, kKA = 448, kVA = 480;
-__device__ __forceinline__ constexpr uint32_t w1_of(uint32_t chain) { return kW + 128 * chain; }
-__device__ __forceinline__ constexpr uint32_t w2_of(uint32_t chain) { return kW + 128 * chain + 64; }
-
-// The gate of two selection logits, l > 0, as a bf16 pair: masks of 16 bits, or 1 and 0.  The comparison is made on the bf16
-// roundings: they have the sign of the logit, and are zero only below 2^-134.
-template <bool MASK>
-__device__ __forceinline__ uint32_t gate_pair(float lo, float hi) {
-  const __nv_bfloat162 x = __floats2bfloat162_rn(lo, hi), zero = __floats2bfloat162_rn(0.f, 0.f);
-  if (MASK) return __hgt2_mask(x, zero);
-  const __nv_bfloat162 g = __hgt2(x, zero);
-  return *reinterpret_cast<const uint32_t*>(&g);
-}
+// TMEM columns (W1, W2: sa_tc_bwd_chain.cuh)
+constexpr uint32_t kDV = 0, kDK = 64, kDQ = 128, kDK0 = 448, kKA = 448, kVA = 480;
+constexpr int DQ0 = DQ + 1;           // completes per tile like DQ
 
 template <bool SELF, bool LIVE>   // LIVE: a table of live tiles is given (sa_tc_skip.cu)
-__global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
+__global__ void __launch_bounds__(kThreads, 1) backward_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dq0,
@@ -122,22 +98,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // Barriers.  Completion: LD, LD0 TMA loads; L0, S, DP score products of a chain's half; FREE, FREE0 the last MMA that reads
-  // a slot; DQ, DQ0 a tile's query-side product.  Arrival, one arrival per warp: SEL L0^T read; DZ P^T and dz^T written, S^T
-  // and dP^T read; G g^T written; TOK the running sum of dz handed on; SUM the upper
-  // half's selection handed to the lower; ACC the shared accumulator read.
-  enum : int { KV = 0, SETUP = 1, FIN = 2, DQ = 3, DQ0 = 4, ACC = 5, L0 = 6, S = 8, DP = 10, SEL = 12, DZ = 14, G = 16, TOK = 18,
-               SUM = 20, LD = 21, FREE = 26, LD0 = 31, FREE0 = 34, kBars = 37 };
   __shared__ uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
-  __shared__ float run_s[kTile], sel_s[2][kTile];
+  __shared__ float run_s[kTile], sel_s[2 * kTile];
   __shared__ int top_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (LIVE && warp == 1) find_top_tile(alive, n, nj, ntiles, lane, &top_s);
   if (tid == 0) {
-    for (int u = 0; u < kBars; ++u) mbar_init(&bars[u], u == SETUP ? 8 : (u == ACC || (u >= SEL && u < LD)) ? 4 : 1);
-    mbar_init_fence();
+    init_bars(bars);
   }
   if (tid < kTile) run_s[tid] = 0.f;
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
@@ -413,30 +382,33 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
   } else {
     regs_grow<kChainRegs>();
     // ============================================ the two chains ============================================
-    const int c = warp >> 2, row = tid & 127, other = c ^ 1;
+    const int c = warp >> 2, row = tid & 127;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);   // a warp reaches lanes 32 (warp % 4) ..
-    const uint32_t w1 = lane_base + w1_of(c), w2 = lane_base + w2_of(c);
     const int j = nj * kTile + row;
-    const float c1 = scale * kLog2e;
-    const float inv_scale = 1.f / scale;
-    const float shut = (j >= exempt) ? 0.f : -INFINITY;            // an exempt key is never selected
-    // this thread's row in its chain's query half of the dz tile (the g tile lies kG further on); chunk x of it is at ^ 16 x
-    constexpr uint32_t kG = SELF ? 0 : L::g - L::dz;
-    const uint32_t my_row = sa + L::dz + (1 - c) * kRowTile + row * 128 + ((row & 7) << 4);
-    auto put8 = [&](uint32_t at, int chunk, const uint32_t* w) {             // eight queries of this thread's key
-      st_shared16(at ^ (uint32_t)(chunk << 4), w[0], w[1], w[2], w[3]);
-    };
-    auto arrive = [&](int id) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(id));
-    };
-    auto fetch_carry = [&](int mi) {
-      return (j < seq) ? load_ahead(carry + ((int64_t)b * (ntiles + 1) + mi + 1) * seq + j) : 0.f;
-    };
-    float next_carry = fetch_carry(mi_top);
+    Chain ch;
+    ch.c = c; ch.row = row; ch.lane = lane; ch.j = j; ch.n_iter = n_iter;
+    ch.w1 = lane_base + w1_of(c);
+    ch.w2 = lane_base + w2_of(c);
+    ch.bar0 = bar0;
+    ch.stat0 = sa + L::stat;
+    ch.dz_row = sa + L::dz + (1 - c) * kRowTile + row * 128 + ((row & 7) << 4);
+    ch.g_row = ch.dz_row + (SELF ? 0 : L::g - L::dz);              // (SELF: dz + g go to the dz tile, in the g pass)
+    ch.keep_dz = ch.keep_g = true;
+    ch.free_bar = SELF ? DQ : DQ0;                                 // of the tile before: has read dz and, later, g
+    ch.c1 = scale * kLog2e;
+    ch.inv_scale = 1.f / scale;
+    ch.shut = (j >= exempt) ? 0.f : -INFINITY;                     // an exempt key is never selected
+    ch.carry = (j < seq) ? carry + ((int64_t)b * (ntiles + 1) + mi_top + 1) * seq + j : nullptr;
+    ch.carry_step = seq;
+    ch.run_s = run_s;
+    ch.sel_s = sel_s;
+    ch.slot = c;
+    ch.ld_par = 0;
+    ch.wait = wait;
+    ch.fetch_carry();
 
     if (SELF) {                                                    // K (chain 0) and V (chain 1) rows into TMEM as bf16 pairs
-      wait(bar(KV), 0, 409);
+      ch.wait(bar(KV), 0, 409);
       const uint8_t* src = smem + (c == 0 ? L::k : L::v);
       uint32_t w32[32];
 #pragma unroll
@@ -447,160 +419,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) backward_kernel(
       tmem_st32(lane_base + (c == 0 ? kKA : kVA), w32);
       tmem_st_wait();
       tc_fence_before_sync();
-      arrive(SETUP);
+      ch.arrive(SETUP);
     }
-
-    int slot = c;
-    uint32_t ld_par = 0;
-    auto half = [&](int it, auto diag_tag) {
-      constexpr bool kDiag = decltype(diag_tag)::value;
-      const uint32_t ph = (uint32_t)(it & 1);
-      const int diag = row - (1 - c) * 64;                         // kDiag: query e of the half is this key itself
-      const uint32_t stat = sa + L::stat + slot * kStatBytes;
-      float run = next_carry;
-      asm volatile("" : "+f"(run));                                // (the scaling stays here: next to the load it would wait for it)
-      run *= -inv_scale;                                           // minus the history after the tile, in units of q . k
-      if (it + 1 < n_iter) next_carry = fetch_carry(mi_top - it - 1);
-
-      // ---- selection: relu(L0^T) and the gate ---------------------------------------------------------
-      float v[64];
-      uint32_t gate[32];                                           // bf16 pairs
-      wait(bar((SELF ? S : L0) + c), ph, 410);
-      tc_fence_after_sync();
-      {
-        uint32_t r[2][32];
-        tmem_ld32((SELF ? w2 : w1), r[0]);
-        tmem_ld32((SELF ? w2 : w1) + 32, r[1]);
-        tmem_ld_wait();
-        tc_fence_before_sync();
-        if (!SELF) arrive(SEL + c);                                // W1 may take dP^T
-#pragma unroll
-        for (int e = 0; e < 64; e += 2) {
-          float l0 = __uint_as_float(r[e >> 5][e & 31]), l1 = __uint_as_float(r[e >> 5][(e & 31) + 1]);
-          if (kDiag) {                                             // key strictly before the query
-            if (e <= diag) l0 = -1.f;
-            if (e + 1 <= diag) l1 = -1.f;
-          }
-          const float2 t = __fadd2_rn(make_float2(l0, l1), make_float2(shut, shut));
-          gate[e >> 1] = gate_pair<!SELF>(t.x, t.y);
-          v[e] = fmaxf(t.x, 0.f);
-          v[e + 1] = fmaxf(t.y, 0.f);
-        }
-      }
-
-      // ---- probabilities, last query first: P = exp2(c1 (S + run) - lse), run growing by the selection ---------------
-      if (!SELF) {
-        wait(bar(S + c), ph, 416);
-        tc_fence_after_sync();
-      }
-      mbar_try_wait(&bars[LD + slot], ld_par);                    // (complete: S^T was made from the slot) its statistics are visible
-      if (c == 1) {                                                // the upper half's selection comes first
-        wait(bar(SUM), ph, 421);
-        run += sel_s[ph][row];
-      }
-      const float2 cc = make_float2(c1, c1);
-      const float run_in = run;
-#pragma unroll
-      for (int q = 1; q >= 0; --q) {
-        uint32_t r[32], w[16];
-        tmem_ld32(w2 + 32 * q, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e4 = 28; e4 >= 0; e4 -= 4) {
-          const float4 nl = ld_shared_f4(stat + 4 * (32 * q + e4));
-#pragma unroll
-          for (int k = 1; k >= 0; --k) {
-            const int e = 32 * q + e4 + 2 * k;
-            const float hi = run + v[e + 1];
-            run = hi + v[e];
-            const float2 s = __fadd2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])),
-                                        make_float2(run, hi));
-            const float2 x = __ffma2_rn(s, cc, k ? make_float2(nl.z, nl.w) : make_float2(nl.x, nl.y));
-            v[e] = ex2(x.x);
-            v[e + 1] = ex2(x.y);
-            if (kDiag) {                                           // key after the query
-              if (e < diag) v[e] = 0.f;
-              if (e + 1 < diag) v[e + 1] = 0.f;
-            }
-            w[(e4 >> 1) + k] = pack_bf16(v[e], v[e + 1]);
-          }
-        }
-        tmem_st16(w2 + 32 + 16 * q, w);                            // over S^T columns that have been read
-      }
-      if (c == 0) {
-        sel_s[ph][row] = run - run_in;
-        arrive(SUM);
-      }
-
-      // ---- dz = P (dP - dbar) ------------------------------------------------------------------------------------
-      wait(bar(DP + c), ph, 411);
-      tc_fence_after_sync();
-      if (!SELF) wait(bar(DQ0), ph ^ 1u, 418);                     // dQ and dQ0 of the tile before have read dz and g
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        uint32_t r[32], w[16];
-        tmem_ld32(w1 + 32 * q, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e4 = 0; e4 < 32; e4 += 4) {
-          const float4 nd = ld_shared_f4(stat + 4 * (64 + 32 * q + e4));
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int e = 32 * q + e4 + 2 * k;
-            const float2 d = __fmul2_rn(make_float2(v[e], v[e + 1]),
-                                        __fadd2_rn(make_float2(__uint_as_float(r[e4 + 2 * k]), __uint_as_float(r[e4 + 2 * k + 1])),
-                                                   k ? make_float2(nd.z, nd.w) : make_float2(nd.x, nd.y)));
-            v[e] = d.x;
-            v[e + 1] = d.y;
-            if (!SELF) w[(e4 >> 1) + k] = pack_bf16(d.x, d.y);
-          }
-        }
-        if (!SELF) {                                               // dz: to TMEM (A of dK) and shared memory (A of dQ)
-          tmem_st16(w2 + 16 * q, w);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) put8(my_row, 4 * q + u, w + 4 * u);
-        }
-      }
-      if (!SELF) fence_async_smem();                               // dz half tile -> visible to the MMAs
-      tmem_st_wait();
-      tc_fence_before_sync();
-      arrive(DZ + c);
-
-      // ---- g = gate ? -(sum of dz over later queries) : 0; SELF: dz + g.  The sum goes from half to half --------------
-      wait(bar(TOK + other), ph ^ (uint32_t)other, 419);
-      float later = run_s[row];                                    // minus the sum of dz over later queries
-      if (SELF) wait(bar(DQ), ph ^ 1u, 420);                       // dQ of the tile before has read dz + g
-#pragma unroll
-      for (int q = 1; q >= 0; --q) {
-        uint32_t w[16];
-#pragma unroll
-        for (int e = 32 * q + 30; e >= 32 * q; e -= 2) {
-          const float hi = later, lo = later - v[e + 1];
-          later = lo - v[e];
-          const uint32_t m = gate[e >> 1];
-          if constexpr (SELF)
-            w[(e >> 1) & 15] = pack_bf16(fmaf(__uint_as_float(m << 16), lo, v[e]), fmaf(__uint_as_float(m & 0xffff0000u), hi, v[e + 1]));
-          else
-            w[(e >> 1) & 15] = pack_bf16(lo, hi) & m;
-        }
-        tmem_st16(w1 + 16 * q, w);                                 // over dP^T columns that have been read
-#pragma unroll
-        for (int u = 0; u < 4; ++u) put8(my_row + kG, 4 * q + u, w + 4 * u);
-      }
-      run_s[row] = later;
-      fence_async_smem();
-      tmem_st_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar(G + c));
-        mbar_arrive(bar(TOK + c));
-      }
-      slot += 2;
-      if (slot >= R) { slot -= R; ld_par ^= 1u; }
-    };
-    for (int it = 0; it + 1 < n_iter; ++it) half(it, std::false_type{});
-    half(n_iter - 1, std::true_type{});
+    for (int it = 0; it + 1 < n_iter; ++it) half_pass<SELF, false, R>(ch, it);
+    half_pass<SELF, true, R>(ch, n_iter - 1);
+    wait = ch.wait;
 
     // ---- epilogue: dV (chain 0) and dK (chain 1) of this key tile -------------------------------------------------
     wait(bar(FIN), 0, 415);
@@ -641,9 +464,10 @@ int backward(const Problem& p, const float* stats, const float* carry, const voi
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_do, d_out, 64, p.seq, p.heads, p.batch, d_out_rows.st, d_out_rows.sh, d_out_rows.sb, 64);
   if (st != SA_OK) return st;
-  st = make_map_f32_rows(&map_dq, dq_acc, p.seq, nrows);
+  st = make_map_f32_rows(&map_dq, dq_acc, p.seq, nrows, 64, true);
   if (st != SA_OK) return st;
-  st = dq0 != nullptr ? make_map_f32_rows(&map_dq0, dq0, p.seq, p.batch) : make_map_f32_rows(&map_dq0, dq_acc, p.seq, nrows);
+  st = dq0 != nullptr ? make_map_f32_rows(&map_dq0, dq0, p.seq, p.batch, 64, true)
+                      : make_map_f32_rows(&map_dq0, dq_acc, p.seq, nrows, 64, true);
   if (st != SA_OK) return st;
   st = make_map_16bit(&map_q0, p.q0.ptr, 64, p.seq, 1, p.batch, p.q0.st, 0, p.q0.sb, 64);
   if (st != SA_OK) return st;
@@ -659,7 +483,7 @@ int backward(const Problem& p, const float* stats, const float* carry, const voi
     SA_CUDA_CHECK(allow_smem(kernel, smem));
     ProfileScope prof(SA_KERNEL_TC_BACKWARD, s);
     count_launch();
-    kernel<<<(unsigned)ntiles * nrows, kPairThreads, smem, s>>>(
+    kernel<<<(unsigned)ntiles * nrows, kThreads, smem, s>>>(
         map_q, map_k, map_v, map_do, map_dq, map_dq0, map_q0, map_k0, stats, carry, static_cast<__nv_bfloat16*>(dk), dk0,
         static_cast<__nv_bfloat16*>(dv), p.heads, dq0 != nullptr ? 1 : p.heads, p.seq, ntiles, p.exempt, p.scale, status,
         p.dk_rows, p.dv_rows, alive);

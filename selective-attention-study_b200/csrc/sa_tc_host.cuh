@@ -50,18 +50,19 @@ inline int make_map_16bit(CUtensorMap* map, const void* base, int head_dim, int 
   return SA_OK;
 }
 
-// 4-D map over (d, token, row, 1) of a contiguous fp32 tensor (rows x seq x 64); box = (32 floats, 32
-// tokens, 1, 1) with the 128-byte swizzle: the target of the TMA reduce-add of one warp's rows of a dQ tile.
-inline int make_map_f32_rows(CUtensorMap* map, const void* base, int seq, int rows) {
+// 4-D map over (d, token, row, 1) of a contiguous fp32 tensor (rows x seq x dim); box = (32 floats, 32 tokens, 1, 1): the
+// target of the TMA reduce-add of one warp's rows of a dQ tile.  `swizzled`: the 128-byte swizzle in shared memory.
+inline int make_map_f32_rows(CUtensorMap* map, const void* base, int seq, int rows, int dim, bool swizzled) {
   auto fn = encode_fn();
   if (fn == nullptr) return SA_ERR_CUDA;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return SA_ERR_ALIGNMENT;
-  cuuint64_t dims[4] = {64, (cuuint64_t)seq, (cuuint64_t)rows, 1};
-  cuuint64_t strides[3] = {64 * 4, (cuuint64_t)seq * 64 * 4, (cuuint64_t)rows * seq * 64 * 4};
+  const cuuint64_t row = (cuuint64_t)dim * 4;
+  cuuint64_t dims[4] = {(cuuint64_t)dim, (cuuint64_t)seq, (cuuint64_t)rows, 1};
+  cuuint64_t strides[3] = {row, (cuuint64_t)seq * row, (cuuint64_t)rows * seq * row};
   cuuint32_t box[4] = {32, 32, 1, 1};
   cuuint32_t elem[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, strides, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_last_cuda_error(10000 + (int)r);
