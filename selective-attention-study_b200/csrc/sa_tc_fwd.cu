@@ -30,35 +30,40 @@ constexpr int kRowTile = 16384;     // bytes of a [128][64] bf16 operand tile
 // ---------------------------------------------------------------------------------------------------
 // selection column sums
 // ---------------------------------------------------------------------------------------------------
-constexpr int kColsumChunk = 8;     // query tiles per CTA
+// 128 threads own a key each; a fifth warp's elected lane issues the loads and MMAs, one tile ahead.  Bound by latency and
+// issue: 128 compares and 64 packed additions a thread and tile.  (One accumulator and a block-wide barrier a tile, with the
+// issuing thread among the 128, took 2.1 k cycles a tile and CTA: the additions alone were a chain of 512.)
+constexpr int kColsumThreads = 160;
 
 template <int D>
-__global__ void __launch_bounds__(128) colsum_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                     const __grid_constant__ CUtensorMap map_k, float* __restrict__ carry,
-                                                     int seq, int ntiles, int exempt, float scale,
-                                                     WaitCtx status, int q_offset, int mi_first) {
+__global__ void __launch_bounds__(kColsumThreads) colsum_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                const __grid_constant__ CUtensorMap map_k,
+                                                                float* __restrict__ carry, int seq, int ntiles, int exempt,
+                                                                float scale, WaitCtx status, int q_offset, int mi_first,
+                                                                int chunk) {
   constexpr int DK = D / 64;
   const int nj = blockIdx.x, b = blockIdx.z;
   // Query tiles from the key tile's own (the diagonal) on; in a prefill continuation from the first tile that holds a
   // new query on (rows before q_offset are not in the query tensor: TMA fills them with zeros, which select nothing).
-  const int mi0 = max(nj, mi_first) + blockIdx.y * kColsumChunk;
+  const int mi0 = max(nj, mi_first) + blockIdx.y * chunk;
   if (mi0 >= ntiles) return;
-  const int count = min(kColsumChunk, ntiles - mi0);
+  const int count = min(chunk, ntiles - mi0);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* k0s = smem;                               // DK tiles [128 keys][64]
   uint8_t* q0s = smem + DK * kRowTile;               // 2 stages x DK tiles [128 queries][64]
-  __shared__ uint64_t bar_k, bar_q[2], bar_mma[2];
+  __shared__ uint64_t bar_k, bar_q[2], bar_mma[2], bar_read[2];
   __shared__ uint32_t tmem_base_s;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     mbar_init(&bar_k, 1);
-    mbar_init(&bar_q[0], 1);
-    mbar_init(&bar_q[1], 1);
-    mbar_init(&bar_mma[0], 1);
-    mbar_init(&bar_mma[1], 1);
+    for (int u = 0; u < 2; ++u) {
+      mbar_init(&bar_q[u], 1);
+      mbar_init(&bar_mma[u], 1);
+      mbar_init(&bar_read[u], 4);
+    }
     mbar_init_fence();
   }
   if (warp == 0) tmem_alloc(&tmem_base_s, 256);
@@ -66,61 +71,79 @@ __global__ void __launch_bounds__(128) colsum_kernel(const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-  const uint32_t idesc = instr_desc_bf16(128, 128, false, false);
-  const uint32_t k0a = smem_u32(k0s), q0a = smem_u32(q0s);
 
-  auto load_q = [&](int it) {
-    uint64_t* bar = &bar_q[it & 1];
-    mbar_expect_tx(bar, DK * kRowTile);
-    for (int s = 0; s < DK; ++s)
-      tma_load_4d(q0s + ((it & 1) * DK + s) * kRowTile, &map_q, bar, s * 64, (mi0 + it) * kTile - q_offset, 0, b);
-  };
-  auto issue = [&](int it) {
-    mbar_wait(&bar_q[it & 1], (it >> 1) & 1, status, 200);
-    tc_fence_after_sync();
-    for (int ks = 0; ks < 4 * DK; ++ks)
-      mma_ss(tmem + (it & 1) * 128, smem_desc(k0a + (ks >> 2) * kRowTile + (ks & 3) * 32, 16, 1024),
-             smem_desc(q0a + ((it & 1) * DK + (ks >> 2)) * kRowTile + (ks & 3) * 32, 16, 1024), idesc, ks > 0);
-    mma_commit(&bar_mma[it & 1]);
-  };
-
-  if (tid == 0) {
-    mbar_expect_tx(&bar_k, DK * kRowTile);
-    for (int s = 0; s < DK; ++s) tma_load_4d(k0s + s * kRowTile, &map_k, &bar_k, s * 64, nj * kTile, 0, b);
-    load_q(0);
-    if (count > 1) load_q(1);
-    mbar_wait(&bar_k, 0, status, 201);
-    issue(0);
-  }
-  const int j = nj * kTile + tid;
-  for (int it = 0; it < count; ++it) {
-    if (tid == 0 && it + 1 < count) issue(it + 1);
-    mbar_wait(&bar_mma[it & 1], (it >> 1) & 1, status, 202);
-    tc_fence_after_sync();
-    if (tid == 0 && it + 2 < count) load_q(it + 2);     // stage (it & 1) is free: its MMA has completed
-    const int mi = mi0 + it;
-    const int i0 = mi * kTile;
-    const bool diag = (mi == nj);
-    float sum = 0.f;
-#pragma unroll
-    for (int c0 = 0; c0 < 128; c0 += 32) {
-      uint32_t r[32];
-      tmem_ld32(lane_base + (it & 1) * 128 + c0, r);
-      tmem_ld_wait();
-      if (diag) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) sum += (j < i0 + c0 + e) ? fmaxf(__uint_as_float(r[e]), 0.f) : 0.f;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) sum += fmaxf(__uint_as_float(r[e]), 0.f);
+  if (warp == 4) {
+    if (lane == 0) {
+      const uint32_t idesc = instr_desc_bf16(128, 128, false, false);
+      const uint32_t k_low = desc_low(smem_u32(k0s), 16), q_low = desc_low(smem_u32(q0s), 16);
+      auto load_q = [&](int it) {
+        uint64_t* bar = &bar_q[it & 1];
+        mbar_expect_tx(bar, DK * kRowTile);
+        for (int s = 0; s < DK; ++s)
+          tma_load_4d(q0s + ((it & 1) * DK + s) * kRowTile, &map_q, bar, s * 64, (mi0 + it) * kTile - q_offset, 0, b);
+      };
+      mbar_expect_tx(&bar_k, DK * kRowTile);
+      for (int s = 0; s < DK; ++s) tma_load_4d(k0s + s * kRowTile, &map_k, &bar_k, s * 64, nj * kTile, 0, b);
+      load_q(0);
+      if (count > 1) load_q(1);
+      mbar_wait(&bar_k, 0, status, 201);
+#pragma unroll 1
+      for (int it = 0; it < count; ++it) {
+        const int st = it & 1;
+        const uint32_t ph = (uint32_t)((it >> 1) & 1);
+        if (it >= 2) mbar_wait(&bar_read[st], ph ^ 1u, status, 203);      // the columns' last tile has been read
+        mbar_wait(&bar_q[st], ph, status, 200);
+        tc_fence_after_sync();
+        for (int ks = 0; ks < 4 * DK; ++ks) {
+          const uint32_t off = (uint32_t)((ks >> 2) * kRowTile + (ks & 3) * 32) >> 4;
+          const uint32_t ql = q_low + (uint32_t)(st * DK * kRowTile >> 4) + off;
+          if (ks == 0) mma_ss_low<false>(tmem + st * 128, k_low + off, ql, idesc);
+          else mma_ss_low<true>(tmem + st * 128, k_low + off, ql, idesc);
+        }
+        mma_commit(&bar_mma[st]);
+        if (it >= 1 && it + 1 < count) {                                  // the other stage: its MMA has completed
+          mbar_wait(&bar_mma[st ^ 1], (uint32_t)(((it - 1) >> 1) & 1), status, 204);
+          load_q(it + 1);
+        }
       }
     }
-    if (j < exempt) sum = 0.f;
-    if (j < seq) carry[((int64_t)b * (ntiles + 1) + mi) * seq + j] = sum * scale;
-    tc_fence_before_sync();
-    __syncthreads();
+    __syncwarp();
+  } else {
+    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    const int j = nj * kTile + tid;
+    float* dst = carry + ((int64_t)b * (ntiles + 1) + mi0) * seq + j;
+#pragma unroll 1
+    for (int it = 0; it < count; ++it, dst += seq) {
+      mbar_wait(&bar_mma[it & 1], (uint32_t)((it >> 1) & 1), status, 202);
+      tc_fence_after_sync();
+      const bool diag = mi0 + it == nj;
+      float2 acc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int c0 = 0; c0 < 128; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32(lane_base + (it & 1) * 128 + c0, r);
+        tmem_ld_wait();
+        if (diag) {                                                        // (key and query count from the same position)
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (tid >= c0 + e) r[e] = 0u;
+        }
+#pragma unroll
+        for (int e = 0; e < 32; e += 2)
+          acc[(e >> 1) & 3] = __fadd2_rn(acc[(e >> 1) & 3], make_float2(fmaxf(__uint_as_float(r[e]), 0.f),
+                                                                        fmaxf(__uint_as_float(r[e + 1]), 0.f)));
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_read[it & 1]);
+      const float2 s2 = __fadd2_rn(__fadd2_rn(acc[0], acc[1]), __fadd2_rn(acc[2], acc[3]));
+      if (j < seq) *dst = (j < exempt) ? 0.f : (s2.x + s2.y) * scale;
+    }
   }
+  tc_fence_before_sync();
+  __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
@@ -634,12 +657,15 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   constexpr int DK = D / 64;
   const int colsum_smem = 3 * DK * kRowTile + 1024;
   SA_CUDA_CHECK(allow_smem(colsum_kernel<D>, colsum_smem));
-  dim3 gc(ntiles, (ntiles - mi_first + kColsumChunk - 1) / kColsumChunk, p.batch);
+  // query tiles per CTA: 8, or 32 where that still gives every SM several CTAs (the key tile and the set-up are paid per CTA)
+  const int64_t tiles = (int64_t)ntiles * (ntiles - mi_first) * p.batch;
+  const int chunk = tiles >= 32 * 16 * kSms ? 32 : 8;
+  dim3 gc(ntiles, (ntiles - mi_first + chunk - 1) / chunk, p.batch);
   {
     ProfileScope prof(SA_KERNEL_TC_COLSUM, s);
     count_launch();
-    colsum_kernel<D><<<gc, 128, colsum_smem, s>>>(m.q0, m.k0, carry, p.seq, ntiles, p.exempt, p.scale, status,
-                                                  p.q_offset, mi_first);
+    colsum_kernel<D><<<gc, kColsumThreads, colsum_smem, s>>>(m.q0, m.k0, carry, p.seq, ntiles, p.exempt, p.scale, status,
+                                                             p.q_offset, mi_first, chunk);
   }
   SA_CUDA_CHECK(cudaGetLastError());
   dim3 gs((p.seq + 255) / 256, p.batch);
