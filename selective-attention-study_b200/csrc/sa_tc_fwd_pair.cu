@@ -36,8 +36,8 @@ constexpr int kTile = 128;          // query rows per CTA; also the carry checkp
 constexpr int kRowTile = 16384;     // bytes of a [128][64] bf16 operand tile
 constexpr int kThreads = 512;       // two softmax warpgroups, the selection, four single warps (one idle)
 constexpr int kRing = 3;
-// Registers: 512 x 128 at launch; the softmax keeps 128 logits: 256 x 192 + 256 x 64.
-constexpr int kSoftmaxRegs = 192, kOtherRegs = 64;
+// Registers: 512 x 128 at launch; the softmax keeps 128 logits: 256 x 176 + 256 x 80.
+constexpr int kSoftmaxRegs = 176, kOtherRegs = 80;
 
 struct PairSmem {
   static constexpr int q = 0;                              // Q of the two heads, Q0
@@ -263,25 +263,28 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         const bool masked = t == 0 || j0 < exempt;
         wait(bar(L0F), (uint32_t)(t & 1), 530);
         tc_fence_after_sync();
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(lane_base + kF + 32 * c, r);
+        uint32_t r[2][16];                                     // 16 columns are converted while the next 16 arrive
+        tmem_ld16(lane_base + kF, r[0]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint32_t* cur = r[c & 1];
           tmem_ld_wait();
+          if (c + 1 < 8) tmem_ld16(lane_base + kF + 16 * (c + 1), r[(c + 1) & 1]);
           if (masked) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const int j = j0 + 32 * c + e;
-              if (!(j < i && j >= exempt)) r[e] = 0u;
+            for (int e = 0; e < 16; ++e) {
+              const int j = j0 + 16 * c + e;
+              if (!(j < i && j >= exempt)) cur[e] = 0u;
             }
           }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {                        // the relu rides on the bf16 conversion
+          for (int u = 0; u < 2; ++u) {                        // the relu rides on the bf16 conversion
             uint32_t w[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) w[e] = pack_bf16_relu(__uint_as_float(r[8 * u + 2 * e]), __uint_as_float(r[8 * u + 2 * e + 1]));
-            const uint32_t chunk = (uint32_t)(((c & 1) * 4 + u) << 4);
-            st_shared16(sa + L::sel + (c >> 1) * kRowTile + (row_off ^ chunk), w[0], w[1], w[2], w[3]);
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack_bf16_relu(__uint_as_float(cur[8 * u + 2 * e]), __uint_as_float(cur[8 * u + 2 * e + 1]));
+            const uint32_t chunk = (uint32_t)(((c & 3) * 2 + u) << 4);
+            st_shared16(sa + L::sel + (c >> 2) * kRowTile + (row_off ^ chunk), w[0], w[1], w[2], w[3]);
           }
         }
         fence_async_smem();
@@ -303,19 +306,25 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
       constexpr bool kFirst = decltype(first_tag)::value;      // the diagonal tile: causal mask inside it, nothing to rescale yet
       const uint32_t ph = (uint32_t)(t & 1);
       const uint32_t nc_at = carry_base + ph * (kTile * 4);
-      wait(bar(SELW), ph, 540);                                // the carry of the step's keys
-      wait(bar(SF + x), ph, 541);
+      // ---- logits z = ((F + S) * scale - carry) * log2(e), and the row maximum (packed fp32x2 arithmetic).  F is read as soon
+      // as it is there, not when S is: the next step's selection starts when both heads have it.
+      uint32_t z[4][32];
       wait(bar(FF), ph, 542);
       tc_fence_after_sync();
-      // ---- logits z = ((S + F) * scale - carry) * log2(e), and the row maximum (packed fp32x2 arithmetic) -----------
-      float2 z[64];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32(lane_base + kF + 32 * c, z[c]);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      arrive(FREAD);                                           // F may take the next step's L0
+      wait(bar(SELW), ph, 540);                                // the carry of the step's keys
+      wait(bar(SF + x), ph, 541);
+      tc_fence_after_sync();
       const float2 cc = make_float2(c1, c1);
       float tile_max = -INFINITY;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t s[32], f[32];
+        uint32_t s[32];
         tmem_ld32(s_cols + 32 * c, s);
-        tmem_ld32(lane_base + kF + 32 * c, f);
         tmem_ld_wait();
 #pragma unroll
         for (int e4 = 0; e4 < 32; e4 += 4) {
@@ -324,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
           for (int k = 0; k < 2; ++k) {
             const int e = e4 + 2 * k;
             const float2 y = __fadd2_rn(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])),
-                                        make_float2(__uint_as_float(f[e]), __uint_as_float(f[e + 1])));
+                                        make_float2(__uint_as_float(z[c][e]), __uint_as_float(z[c][e + 1])));
             float2 a = __ffma2_rn(y, cc, k ? make_float2(nc.z, nc.w) : make_float2(nc.x, nc.y));
             if (kFirst) {
               const int j = 32 * c + e;                        // key and query count from the same position
@@ -332,12 +341,11 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
               if (j + 1 > row) a.y = -INFINITY;
             }
             tile_max = fmaxf(tile_max, fmaxf(a.x, a.y));
-            z[16 * c + (e >> 1)] = a;
+            z[c][e] = __float_as_uint(a.x);
+            z[c][e + 1] = __float_as_uint(a.y);
           }
         }
       }
-      tc_fence_before_sync();
-      arrive(FREAD);                                           // F may take the next step's L0
       // every row has its own key in the diagonal tile, so the maximum is finite from the first step on
       const float new_max = fmaxf(run_max, tile_max);
       const float alpha = ex2(run_max - new_max);
@@ -350,7 +358,8 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         uint32_t w[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-          const float2 y = __fadd2_rn(z[32 * c + e], nm);
+          const uint32_t* zz = &z[2 * c + (e >> 4)][2 * (e & 15)];
+          const float2 y = __fadd2_rn(make_float2(__uint_as_float(zz[0]), __uint_as_float(zz[1])), nm);
           const float2 p = make_float2(ex2(y.x), ex2(y.y));
           sum = __fadd2_rn(sum, p);
           w[e] = pack_bf16(p.x, p.y);
