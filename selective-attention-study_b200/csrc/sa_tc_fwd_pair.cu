@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
                FREEV = 21, kBars = 24 };
   __shared__ uint64_t bars[kBars];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(16) float carry_s[2][kTile];
+  __shared__ __align__(16) float carry_s[kTile];
   __shared__ unsigned live_s[LIVE ? kMaxLiveTiles / 32 : 1];   // with a table of live tiles: bit nj of this query tile's row
   __shared__ int live_count_s;
 
@@ -255,14 +255,14 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
 #pragma unroll 1
       for (int t = 0; t < steps; ++t) {
         const int j0 = nj * kTile;
-        carry_s[t & 1][row] = -next_carry * kLog2e;            // negated: the softmax adds it in an FMA
-        if (t + 1 < steps) {
-          nj = step_back(nj);
-          next_carry = fetch_carry(nj);
-        }
         const bool masked = t == 0 || j0 < exempt;
         wait(bar(L0F), (uint32_t)(t & 1), 530);
         tc_fence_after_sync();
+        carry_s[row] = -next_carry * kLog2e;                   // negated: the softmax adds it in an FMA (both heads have read the
+        if (t + 1 < steps) {                                   //   last one, with F: L0 came after that)
+          nj = step_back(nj);
+          next_carry = fetch_carry(nj);
+        }
         uint32_t r[2][16];                                     // 16 columns are converted while the next 16 arrive
         tmem_ld16(lane_base + kF, r[0]);
 #pragma unroll
@@ -300,26 +300,36 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
     const uint32_t s_cols = lane_base + kS + 128 * x, o_cols = lane_base + kO + 64 * x;
     const uint32_t carry_base = smem_u32(carry_s);
     const float c1 = scale * kLog2e;
+    const float2 cc = make_float2(c1, c1);
     const int i = i0 + row;
     float run_max = -INFINITY, run_den = 0.f;
     auto step = [&](int t, auto first_tag) {
       constexpr bool kFirst = decltype(first_tag)::value;      // the diagonal tile: causal mask inside it, nothing to rescale yet
       const uint32_t ph = (uint32_t)(t & 1);
-      const uint32_t nc_at = carry_base + ph * (kTile * 4);
-      // ---- logits z = ((F + S) * scale - carry) * log2(e), and the row maximum (packed fp32x2 arithmetic).  F is read as soon
-      // as it is there, not when S is: the next step's selection starts when both heads have it.
-      uint32_t z[4][32];
+      // ---- the history part of the logits, F * scale - carry in log2 units, as soon as F is there and not when S is: the next
+      // step's selection starts when both heads have it (packed fp32x2 arithmetic throughout)
+      float2 z[64];
+      wait(bar(SELW), ph, 540);                                // (complete: F came after it) the carry of the step's keys
       wait(bar(FF), ph, 542);
       tc_fence_after_sync();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(lane_base + kF + 32 * c, z[c]);
-      tmem_ld_wait();
+      for (int c = 0; c < 4; ++c) {
+        uint32_t f[32];
+        tmem_ld32(lane_base + kF + 32 * c, f);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e4 = 0; e4 < 32; e4 += 4) {
+          const float4 nc = ld_shared_f4(carry_base + 4 * (32 * c + e4));
+          float2* zz = &z[16 * c + (e4 >> 1)];
+          zz[0] = __ffma2_rn(make_float2(__uint_as_float(f[e4]), __uint_as_float(f[e4 + 1])), cc, make_float2(nc.x, nc.y));
+          zz[1] = __ffma2_rn(make_float2(__uint_as_float(f[e4 + 2]), __uint_as_float(f[e4 + 3])), cc, make_float2(nc.z, nc.w));
+        }
+      }
       tc_fence_before_sync();
-      arrive(FREAD);                                           // F may take the next step's L0
-      wait(bar(SELW), ph, 540);                                // the carry of the step's keys
+      arrive(FREAD);                                           // F may take the next step's L0, carry_s its carry
+      // ---- logits and the row maximum -------------------------------------------------------------------------------
       wait(bar(SF + x), ph, 541);
       tc_fence_after_sync();
-      const float2 cc = make_float2(c1, c1);
       float tile_max = -INFINITY;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -327,23 +337,15 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         tmem_ld32(s_cols + 32 * c, s);
         tmem_ld_wait();
 #pragma unroll
-        for (int e4 = 0; e4 < 32; e4 += 4) {
-          const float4 nc = ld_shared_f4(nc_at + 4 * (32 * c + e4));
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int e = e4 + 2 * k;
-            const float2 y = __fadd2_rn(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])),
-                                        make_float2(__uint_as_float(z[c][e]), __uint_as_float(z[c][e + 1])));
-            float2 a = __ffma2_rn(y, cc, k ? make_float2(nc.z, nc.w) : make_float2(nc.x, nc.y));
-            if (kFirst) {
-              const int j = 32 * c + e;                        // key and query count from the same position
-              if (j > row) a.x = -INFINITY;
-              if (j + 1 > row) a.y = -INFINITY;
-            }
-            tile_max = fmaxf(tile_max, fmaxf(a.x, a.y));
-            z[c][e] = __float_as_uint(a.x);
-            z[c][e + 1] = __float_as_uint(a.y);
+        for (int e = 0; e < 16; ++e) {
+          float2 a = __ffma2_rn(make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), cc, z[16 * c + e]);
+          if (kFirst) {
+            const int j = 32 * c + 2 * e;                      // key and query count from the same position
+            if (j > row) a.x = -INFINITY;
+            if (j + 1 > row) a.y = -INFINITY;
           }
+          tile_max = fmaxf(tile_max, fmaxf(a.x, a.y));
+          z[16 * c + e] = a;
         }
       }
       // every row has its own key in the diagonal tile, so the maximum is finite from the first step on
@@ -362,8 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         uint32_t w[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-          const uint32_t* zz = &z[2 * c + (e >> 4)][2 * (e & 15)];
-          const float2 y = __fadd2_rn(make_float2(__uint_as_float(zz[0]), __uint_as_float(zz[1])), nm);
+          const float2 y = __fadd2_rn(z[32 * c + e], nm);
           const float2 p = make_float2(ex2(y.x), ex2(y.y));
           sum[e & 3] = __fadd2_rn(sum[e & 3], p);
           w[e] = pack_bf16(p.x, p.y);
