@@ -66,7 +66,20 @@ _lib = None
 
 
 def available() -> bool:
-    return os.path.exists(LIB_PATH)
+    return os.path.exists(LIB_PATH) and os.path.exists(os.path.join(HERE, "_native.so"))
+
+
+_native_module = None
+
+
+def native():
+    """The C++ host path (csrc/torch/sa_torch.cpp); loads the library first, so that both see the same one."""
+    global _native_module
+    if _native_module is None:
+        load()
+        from . import _native
+        _native_module = _native
+    return _native_module
 
 
 def load() -> ctypes.CDLL:

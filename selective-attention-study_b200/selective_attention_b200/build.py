@@ -17,6 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "csrc")
 LIB_NAME = "libselective_attention_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
+NATIVE_SRC = os.path.join(CSRC, "torch", "sa_torch.cpp")
+NATIVE_PATH = os.path.join(HERE, "_native.so")      # the torch side (C++), linked against the library beside it
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -38,6 +40,30 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(f) <= built for f in _inputs())
 
 
+def _native_command():
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
+    includes = [f"{root}/include", f"{root}/include/torch/csrc/api/include", f"{cuda}/include", sysconfig.get_paths()["include"]]
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in includes), NATIVE_SRC,
+            "-o", NATIVE_PATH, f"-L{HERE}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN", f"-L{root}/lib", "-ltorch", "-ltorch_cpu",
+            "-ltorch_python", "-lc10", "-lc10_cuda", "-ltorch_cuda"]
+
+
+def build_native(force: bool = False) -> str:
+    inputs = [NATIVE_SRC, os.path.join(os.path.dirname(os.path.dirname(HERE)), "include", "selective_attention_b200.h")]
+    if not force and os.path.exists(NATIVE_PATH) and all(os.path.getmtime(f) <= os.path.getmtime(NATIVE_PATH) for f in inputs):
+        return NATIVE_PATH
+    res = subprocess.run(_native_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {NATIVE_SRC}:\n{res.stdout}")
+    return NATIVE_PATH
+
+
 def nvcc_path() -> str:
     found = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(found):
@@ -47,6 +73,7 @@ def nvcc_path() -> str:
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
+        build_native(force)
         return LIB_PATH
     objs = []
     obj_dir = os.path.join(os.path.dirname(HERE), "build")
@@ -73,6 +100,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}")
+    build_native(force)
     return LIB_PATH
 
 

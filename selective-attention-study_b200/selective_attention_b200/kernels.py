@@ -373,28 +373,21 @@ def _backward_call(ctx, dout, dq0=None, dk0=None):
     return dq, dk, dv
 
 
-class _SelectiveAttentionFn(torch.autograd.Function):
+class _SelectiveAttentionFn:
+    """The differentiable operator; the autograd node is C++ (csrc/torch/sa_torch.cpp)."""
+
     @staticmethod
-    def forward(ctx, q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n, bwd_num_warps,
-                bwd_num_stages, group, bwd_group, num_stages, exempt, skip_dead_tiles=False):
+    def apply(q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n, bwd_num_warps, bwd_num_stages, group, bwd_group,
+              num_stages, exempt, skip_dead_tiles=False):
         check_inputs(q, k, v)
         exempt = _check_exempt(exempt)
         lowp = _lowp(dot_precision, q.dtype)
         _check_blocks(block_m, block_n)
-        out, lse2, carry, _, operands, _, engine, _, table = _forward(q, k, v, lowp, exempt, 0, 0,
-                                                                      live_tiles=skip_dead_tiles)
-        ctx.save_for_backward(*operands, out, lse2, carry)
-        ctx.engine, ctx.exempt, ctx.bwd_group, ctx.tile_table = engine, exempt, bwd_group, table
-        ctx.grad_dtypes = (q.dtype, k.dtype, v.dtype)
+        tc = _engine(lowp, q.shape[3], False) == _lib.ENGINE_TCGEN05
+        out = _lib.native().attend(q, k, v, exempt, lowp, tc, bool(skip_dead_tiles) and tc, False)
+        if bwd_group not in (None, 1, 2) and out.requires_grad:
+            out.register_hook(lambda _: _check_bwd_group(bwd_group))       # raised by the backward, whose knob it is
         return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, dout):
-        _check_bwd_group(ctx.bwd_group)
-        grads = _backward_call(ctx, dout)
-        grads = tuple(g if g.dtype == want else g.to(want) for g, want in zip(grads, ctx.grad_dtypes))
-        return grads + (None,) * 12
 
 
 class _SelectiveAttentionSelectorFn(torch.autograd.Function):
@@ -491,75 +484,15 @@ def packed_supported(qkv: torch.Tensor) -> bool:
             and qkv.shape[4] in (64, 128) and qkv.is_contiguous() and os.environ.get("SA_B200_ENGINE", "") != "simt")
 
 
-class _SelectiveAttentionPackedFn(torch.autograd.Function):
-    """The operator between a model's fused QKV projection and its output projection, without the copies around it:
-    q, k, v are read in place from the (B, T, 3, H, D) projection output (strided TMA descriptors), the result is
-    written by the forward kernel as (B, T, H * D) in the activation dtype, the cotangent is read in that layout,
-    and dq, dk, dv are written by the backward's kernels into one (B, T, 3, H, D) gradient."""
-
-    @staticmethod
-    def forward(ctx, qkv, exempt, skip_dead_tiles=False):
-        exempt = _check_exempt(exempt)
-        lib = _lib.load()
-        b, t, _, h, d = qkv.shape
-        q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))          # (B, H, T, D) views
-        dev = qkv.device
-        engine = _lib.ENGINE_TCGEN05
-        out = torch.empty(b, h, t, d, device=dev, dtype=torch.float32)       # kept for the backward's row sums
-        merged = torch.empty(b, t, h * d, device=dev, dtype=qkv.dtype)
-        lse2 = torch.empty(b, h, t, device=dev, dtype=torch.float32)
-        carry = torch.empty(b, lib.sa_carry_checkpoints(engine, t), t, device=dev, dtype=torch.float32)
-        total = torch.empty(b, t, device=dev, dtype=torch.float32)
-        prob = _problem(q, k, v, engine, exempt)
-        low = _tensor_struct(merged.view(b, t, h, d).transpose(1, 2))
-        table = None
-        need = lib.sa_tile_table_bytes(ctypes.byref(prob)) if skip_dead_tiles else 0
-        if need:
-            table = torch.empty(need, device=dev, dtype=torch.uint8)
-        with _on(dev):
-            st = lib.sa_forward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), None,
-                                           out.data_ptr(), ctypes.byref(low), lse2.data_ptr(), carry.data_ptr(),
-                                           total.data_ptr(), table.data_ptr() if need else None, need, _stream(dev))
-        _lib.check("sa_forward_fused", st)
-        ctx.save_for_backward(qkv, out, lse2, carry)
-        ctx.exempt, ctx.tile_table = exempt, table
-        return merged
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_merged):
-        qkv, out, lse2, carry = ctx.saved_tensors
-        lib = _lib.load()
-        b, t, _, h, d = qkv.shape
-        dev = qkv.device
-        q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
-        d_merged = d_merged.to(qkv.dtype)
-        if not d_merged.is_contiguous():
-            d_merged = d_merged.contiguous()
-        d_qkv = torch.empty_like(qkv)
-        dq, dk, dv = (d_qkv[:, :, i].transpose(1, 2) for i in range(3))
-        prob = _problem(q, k, v, _lib.ENGINE_TCGEN05, ctx.exempt)
-        need = lib.sa_backward_workspace_bytes(ctypes.byref(prob))
-        workspace = torch.empty(max(need, 1), device=dev, dtype=torch.uint8)
-        descs = [_tensor_struct(x) for x in (d_merged.view(b, t, h, d).transpose(1, 2), dq, dk, dv)]
-        table = ctx.tile_table
-        with _on(dev):
-            st = lib.sa_backward_live_tiles(ctypes.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), None,
-                                            out.data_ptr(), lse2.data_ptr(), carry.data_ptr(),
-                                            *(ctypes.byref(x) for x in descs), None, None, workspace.data_ptr(), need,
-                                            table.data_ptr() if table is not None else None, _stream(dev))
-        _lib.check("sa_backward_fused", st)
-        return d_qkv, None, None
-
-
 def selective_attention_packed(qkv: torch.Tensor, exempt: int = 1, *, skip_dead_tiles: bool = False) -> torch.Tensor:
     """Differentiable Selective Attention on a fused projection output.  qkv: (B, T, 3, H, D) bf16, contiguous
     (``packed_supported``); returns (B, T, H * D) bf16, ready for the output projection.  Head 0 selects for all
     heads.  Same arithmetic as ``selective_attention`` on the three (B, H, T, D) views; what is saved is every
-    copy between the projections and the kernels.  ``skip_dead_tiles``: as in ``selective_attention``."""
+    copy between the projections and the kernels (strided TMA descriptors read q, k, v in place; the forward kernel writes the
+    merged result, the backward's kernels one (B, T, 3, H, D) gradient).  ``skip_dead_tiles``: as in ``selective_attention``."""
     if not packed_supported(qkv):
         raise ValueError("qkv must be a contiguous bf16 CUDA tensor (B, T, 3, H, 64 or 128); use selective_attention otherwise")
-    return _SelectiveAttentionPackedFn.apply(qkv, exempt, bool(skip_dead_tiles))
+    return _lib.native().attend_packed(qkv, _check_exempt(exempt), bool(skip_dead_tiles))
 
 
 # ---- cached decode ------------------------------------------------------------------------------------
@@ -568,53 +501,27 @@ def _store_rows(cache: dict, k: torch.Tensor, v: torch.Tensor, at: int, begin: b
     """New keys and values into the cache from position ``at`` on; ``begin``: the first ones, with zeros behind them (and in
     ``selected``).  One launch where the rows are of the cache's type and contiguous along head_dim."""
     kc, vc, selected = cache["k"], cache["v"], cache["selected"]
-    b, h, cap, d = kc.shape
-    t = k.shape[2]
-    if not (kc.is_cuda and k.dtype == v.dtype == kc.dtype and k.device == v.device == kc.device and k.stride(3) == v.stride(3) == 1
-            and kc.is_contiguous() and vc.is_contiguous() and selected.is_contiguous() and b * h <= 65535 and d in HEAD_DIMS):
+    if not _lib.native().store_rows(kc, vc, selected, k, v, at, begin):
+        t = k.shape[2]
         kc[:, :, at:at + t] = k
         vc[:, :, at:at + t] = v
         if begin:
             for x in (kc, vc, selected):
                 x[:, :, at + t:] = 0
-        return
-    with _on(kc.device):
-        st = _lib.load().sa_cache_store(_DTYPE_CODE[kc.dtype], b, h, selected.shape[1], t, cap, d, at, int(begin),
-                                        ctypes.byref(_tensor_struct(k)), ctypes.byref(_tensor_struct(v)), kc.data_ptr(),
-                                        vc.data_ptr(), selected.data_ptr(), _stream(kc.device))
-    _lib.check("sa_cache_store", st)
 
 
-def _prefill_rows(q, k, v, cached: int, selected: torch.Tensor, exempt: int, skip_dead_tiles: bool = False) -> torch.Tensor:
-    """Rows ``cached`` .. of a prompt in bf16, (B, H, Tn, D), and the totals of its keys into ``selected`` (B, G, capacity).
-    q holds the new queries; k, v all keys, or a cache of them.  G = 1, or G = H with every head its own selector."""
-    lib = _lib.load()
-    b, h, tn, d = q.shape
-    total_len, cap = cached + tn, selected.shape[2]
-    if selected.shape[1] == h and h > 1:         # every head is its own one-head sequence
-        q, k, v = (x.reshape(b * h, 1, x.shape[2], d) for x in (q, k, v))
-    q, k, v = (_strided(x, True) for x in (q, k, v))
-    bb, hh = q.shape[:2]
-    dev, engine = q.device, _lib.ENGINE_TCGEN05
-    y = torch.empty(b, h, tn, d, device=dev, dtype=torch.bfloat16)
-    # one allocation for the scratch: log-sum-exp rows, then the checkpoints (256-byte aligned)
-    lse_bytes = (bb * hh * tn * 4 + 255) // 256 * 256
-    scratch = torch.empty(lse_bytes + bb * lib.sa_carry_checkpoints(engine, total_len) * total_len * 4, device=dev, dtype=torch.uint8)
-    prob = _problem(q, k, v, engine, exempt)
-    prob.seq = total_len
-    need = lib.sa_tile_table_bytes(ctypes.byref(prob)) if skip_dead_tiles else 0
-    table = torch.empty(need, device=dev, dtype=torch.uint8) if need else None
-    rows = _tensor_struct(y.view(bb, hh, tn, d))
-    with _on(dev):
-        st = lib.sa_prefill_rows(ctypes.byref(prob), cached, q.data_ptr(), k.data_ptr(), v.data_ptr(), selected.data_ptr(), cap,
-                                 ctypes.byref(rows), scratch.data_ptr(), scratch.data_ptr() + lse_bytes,
-                                 table.data_ptr() if need else None, need, _stream(dev))
-    _lib.check("sa_prefill_rows", st)
-    return y
+def _attend_low(q, k, v, dot_precision: str | None, exempt: int):
+    """The differentiable operator with its result in the operands' bf16 (the kernel writes both forms), and the cotangent read
+    in bf16; None where the result has to be cast by the caller."""
+    if not (q.dtype == k.dtype == v.dtype == torch.bfloat16 and _lowp(dot_precision, q.dtype)
+            and _engine(True, q.shape[3], False) == _lib.ENGINE_TCGEN05):
+        return None
+    check_inputs(q, k, v)
+    return _lib.native().attend(q, k, v, exempt, True, True, False, True)
 
 
 def _prompt_in_place(q: torch.Tensor, v: torch.Tensor, dot_precision: str | None, damp: str, groups: int) -> bool:
-    """Whether ``_prefill_rows`` gives what a forward with its output cast to v's type would: bf16 throughout, on the
+    """Whether ``prefill_rows`` (rows in bf16, totals into a cache) gives what a forward with its output cast to v's type would: bf16 throughout, on the
     tensor-core engine, one selector per sequence or per head."""
     return (q.dtype == v.dtype == torch.bfloat16 and _lowp(dot_precision, q.dtype) and damp == "none" and groups in (1, q.shape[1])
             and _engine(True, q.shape[3], False) == _lib.ENGINE_TCGEN05)
@@ -659,7 +566,7 @@ def _extend(cache: dict, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, exem
         cache["key_norms"][:, :, cached:total_len] = key_norms(k.to(kc.dtype))
     qn = q.to(torch.bfloat16)
     if out_dtype == torch.bfloat16:
-        y = _prefill_rows(qn, kc, vc, cached, selected, exempt, skip_dead_tiles)
+        y = _lib.native().prefill_rows(qn, kc, vc, cached, selected, exempt, bool(skip_dead_tiles))
         cache["len"] = total_len
         return y
     if groups == h and h > 1:             # every head is its own one-head sequence
@@ -727,8 +634,7 @@ class _DecodePlan:
         if norms is not None and not (norms.is_cuda and norms.dtype == torch.float32 and norms.is_contiguous()
                                       and tuple(norms.shape) == (b, h, cap)):
             raise ValueError("cache['key_norms'] must be a contiguous fp32 CUDA tensor (B, H, capacity)")
-        self.shape, self.token = (b, h, d), (b, h, 1, d)
-        self.capacity, self.dtype, self.device = cap, kc.dtype, kc.device
+        self.capacity = cap
         groups = selected.shape[1]
         # scratch for the longest step that the cache can take
         need = _lib.load().sa_decode_workspace_bytes(b, h, groups, max(cap - 1, 0), d)
@@ -757,17 +663,6 @@ def _decode(cache: dict, q1: torch.Tensor, k1: torch.Tensor, v1: torch.Tensor, e
     length = int(cache["len"])
     if length >= plan.capacity:
         raise ValueError("decode step past the cache capacity (context_length)")
-    dtype, token, dev = plan.dtype, plan.token, plan.device
-    q1, k1, v1 = (t if (t.dtype == dtype and t.shape == token and t.device == dev and t.is_contiguous())
-                  else t.reshape(plan.shape).to(dtype).contiguous() for t in (q1, k1, v1))
-    y = torch.empty(token, device=dev, dtype=out_dtype)
-    a = plan.args
-    a.y_dtype, a.length, a.exempt = _DTYPE_CODE[out_dtype], length, exempt
-    a.q1, a.k1, a.v1, a.y = q1.data_ptr(), k1.data_ptr(), v1.data_ptr(), y.data_ptr()
-    a.stream = _stream(dev)
-    with _on(dev):
-        st = _lib.load().sa_decode_run(plan.address)
-    if st:
-        _lib.check("sa_decode_step", st)
+    y = _lib.native().decode(plan.address, plan.tensors[0], q1, k1, v1, length, exempt, out_dtype != torch.float32)
     cache["len"] = length + 1
     return y

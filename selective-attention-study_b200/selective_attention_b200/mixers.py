@@ -60,8 +60,10 @@ class SelectiveAttentionSlot:
                     q, k, v, dot_precision=self.dot_precision, return_aux=True, exempt=self.exempt,
                     damp=self.history_damp, train_len=self.context_length)
                 return y.to(v.dtype), aux["selected_total"]
-            y = kernels.selective_attention(q, k, v, dot_precision=self.dot_precision, exempt=self.exempt)
-            return y.to(v.dtype), None
+            y = kernels._attend_low(q, k, v, self.dot_precision, self.exempt)
+            if y is None:
+                y = kernels.selective_attention(q, k, v, dot_precision=self.dot_precision, exempt=self.exempt).to(v.dtype)
+            return y, None
         # off-kernel path: the dense listing, exactly as the reference falls back (CPU tensors, dropout)
         with torch.autocast(q.device.type, enabled=False):
             logits, total = kernels.selective_logits(q, k, self.exempt)
@@ -85,7 +87,7 @@ class SelectiveAttentionSlot:
             kernels.check_inputs(q, k, v)
             kernels._store_rows(cache, k, v, 0, begin=True)
             if kernels._prompt_in_place(q, v, self.dot_precision, self.history_damp, self.groups):
-                y = kernels._prefill_rows(q, k, v, 0, cache["selected"], self.exempt)
+                y = kernels._lib.native().prefill_rows(q, k, v, 0, cache["selected"], self.exempt, False)
             else:
                 y, total = self.attend(q, k, v, want_total=True)
                 cache["selected"][:, :, :t] = total
