@@ -687,6 +687,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   // one head a CTA still fits the GPU in one wave, that is faster: a step of it takes 3.2 k cycles, of a pair 4.3 k.
   const int64_t ctas = (int64_t)(ntiles - mi_first) * p.batch * p.heads;
   if (D == 64 && !self && p.heads % 2 == 0 && ctas > kSms) return forward_pair(p, m, carry, out, lse2, status, alive, s);
+  if (D == 64 && self && p.batch % 2 == 0 && ctas > kSms) return forward_self(p, m, carry, out, lse2, status, alive, s);
   const unsigned grid = (unsigned)(ntiles - mi_first) * p.batch * p.heads;
   const int wide_smem = WideSmem<D>::total + 1024;
   auto launch = [&](auto kernel) -> int {

@@ -30,5 +30,9 @@ struct ForwardMaps {                  // boxes of 128 rows x 64 columns
 int forward_pair(const Problem& p, const ForwardMaps& m, const float* carry, float* out, float* lse2, const WaitCtx& status,
                  const uint8_t* alive, cudaStream_t s);
 
+// Two rows a CTA (sa_tc_fwd_self.cu): head_dim 64, one head per selector, an even number of rows.
+int forward_self(const Problem& p, const ForwardMaps& m, const float* carry, float* out, float* lse2, const WaitCtx& status,
+                 const uint8_t* alive, cudaStream_t s);
+
 }  // namespace tc
 }  // namespace sa
