@@ -235,19 +235,15 @@ __global__ void __launch_bounds__(kThreads, 1) forward_self_kernel(
       for (int n = 0; n < tiles; ++n) {
         const int j0 = nj * kTile;
         const bool masked = n < 2 || j0 < exempt;
+        if (n >= 2) wait(bar(FF + (r.slot == 2 ? 0 : r.slot + 1)), r.slot == 2 ? r.par : r.par ^ 1u, 631);   // tile n - 2: its selection has been read
         wait(bar(SF + r.slot), r.par, 630);
         tc_fence_after_sync();
-        carry_s[r.slot][row] = -next_carry * kLog2e;           // negated: the softmax adds it in an FMA (the slot's last carry has
-        if (n + 1 < tiles) {                                   //   been read: S came after P V of its last tile)
-          if (n & 1) nj = nj_next;
-          else if (n + 2 < tiles) nj_next = step_back(nj);
-          next_carry = fetch_carry((n + 1) & 1, nj);
-        }
-        if (n >= 2) wait(bar(FF + (r.slot == 2 ? 0 : r.slot + 1)), r.slot == 2 ? r.par : r.par ^ 1u, 631);   // tile n - 2: its selection has been read
         const uint32_t sel = sa + L::sel + (n & 1) * 2 * kRowTile;
         const uint32_t cols = lane_base + 128 * r.slot;
         uint32_t q[2][16];                                     // 16 columns are converted while the next 16 arrive
         tmem_ld16(cols, q[0]);
+        carry_s[r.slot][row] = -next_carry * kLog2e;           // negated: the softmax adds it in an FMA (the slot's last carry has
+                                                               //   been read: S came after P V of its last tile)
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t* cur = q[c & 1];
@@ -273,6 +269,11 @@ __global__ void __launch_bounds__(kThreads, 1) forward_self_kernel(
         fence_async_smem();
         tc_fence_before_sync();
         arrive(SELW + r.slot);
+        if (n + 1 < tiles) {                                   // the next tile's carry arrives while its S is awaited
+          if (n & 1) nj = nj_next;
+          else if (n + 2 < tiles) nj_next = step_back(nj);
+          next_carry = fetch_carry((n + 1) & 1, nj);
+        }
         r.next();
       }
     }
