@@ -31,8 +31,8 @@ constexpr int kTile = 128;          // query rows per CTA; also the carry checkp
 constexpr int kRowTile = 16384;     // bytes of a [128][64] bf16 operand tile
 constexpr int kThreads = 512;       // two softmax warpgroups, the selection, four single warps (one idle)
 constexpr int kRing = 3;            // tiles in flight
-// Registers: 512 x 128 at launch; the softmax keeps 128 logits: 256 x 176 + 256 x 80.
-constexpr int kSoftmaxRegs = 176, kOtherRegs = 80;
+// Registers: 512 x 128 at launch; the softmax keeps 128 logits: 256 x 168 + 256 x 88.
+constexpr int kSoftmaxRegs = 168, kOtherRegs = 88;
 constexpr int kMmaWarp = 12, kLoadWarp = 13, kSumWarp = 14;
 
 struct SelfSmem {
@@ -240,30 +240,30 @@ __global__ void __launch_bounds__(kThreads, 1) forward_self_kernel(
         tc_fence_after_sync();
         const uint32_t sel = sa + L::sel + (n & 1) * 2 * kRowTile;
         const uint32_t cols = lane_base + 128 * r.slot;
-        uint32_t q[2][16];                                     // 16 columns are converted while the next 16 arrive
-        tmem_ld16(cols, q[0]);
+        uint32_t q[2][32];                                     // 32 columns are converted while the next 32 arrive
+        tmem_ld32(cols, q[0]);
         carry_s[r.slot][row] = -next_carry * kLog2e;           // negated: the softmax adds it in an FMA (the slot's last carry has
                                                                //   been read: S came after P V of its last tile)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 4; ++c) {
           uint32_t* cur = q[c & 1];
           tmem_ld_wait();
-          if (c + 1 < 8) tmem_ld16(cols + 16 * (c + 1), q[(c + 1) & 1]);
+          if (c + 1 < 4) tmem_ld32(cols + 32 * (c + 1), q[(c + 1) & 1]);
           if (masked) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int j = j0 + 16 * c + e;
+            for (int e = 0; e < 32; ++e) {
+              const int j = j0 + 32 * c + e;
               if (!(j < i && j >= exempt)) cur[e] = 0u;
             }
           }
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {                        // the relu rides on the bf16 conversion
+          for (int u = 0; u < 4; ++u) {                        // the relu rides on the bf16 conversion
             uint32_t w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               w[e] = pack_bf16_relu(__uint_as_float(cur[8 * u + 2 * e]), __uint_as_float(cur[8 * u + 2 * e + 1]));
-            const uint32_t chunk = (uint32_t)(((c & 3) * 2 + u) << 4);
-            st_shared16(sel + (c >> 2) * kRowTile + (row_off ^ chunk), w[0], w[1], w[2], w[3]);
+            const uint32_t chunk = (uint32_t)(((c & 1) * 4 + u) << 4);
+            st_shared16(sel + (c >> 1) * kRowTile + (row_off ^ chunk), w[0], w[1], w[2], w[3]);
           }
         }
         fence_async_smem();
