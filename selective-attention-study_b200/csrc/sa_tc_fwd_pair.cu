@@ -258,13 +258,10 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         const bool masked = t == 0 || j0 < exempt;
         wait(bar(L0F), (uint32_t)(t & 1), 530);
         tc_fence_after_sync();
-        carry_s[row] = -next_carry * kLog2e;                   // negated: the softmax adds it in an FMA (both heads have read the
-        if (t + 1 < steps) {                                   //   last one, with F: L0 came after that)
-          nj = step_back(nj);
-          next_carry = fetch_carry(nj);
-        }
         uint32_t r[2][16];                                     // 16 columns are converted while the next 16 arrive
         tmem_ld16(lane_base + kF, r[0]);
+        carry_s[row] = -next_carry * kLog2e;                   // negated: the softmax adds it in an FMA (both heads have read the
+                                                               //   last one, with F: L0 came after that)
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t* cur = r[c & 1];
@@ -290,6 +287,10 @@ __global__ void __launch_bounds__(kThreads, 1) forward_pair_kernel(
         fence_async_smem();
         tc_fence_before_sync();
         arrive(SELW);
+        if (t + 1 < steps) {                                   // the next step's carry arrives while its L0 is awaited
+          nj = step_back(nj);
+          next_carry = fetch_carry(nj);
+        }
       }
     }
   } else {
