@@ -1,0 +1,67 @@
+"""The forward variants that only larger grids reach: two heads of a selector, or two rows that each select for
+themselves, in one CTA."""
+
+import pytest
+import torch
+
+import selective_oracle as oracle
+from selective_attention_b200 import kernels, mixers
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(batch, heads, seq, dim, scale, seed):
+    g = torch.Generator("cpu").manual_seed(seed)
+    qk = (scale * torch.randn(batch, heads, seq, dim, generator=g) for _ in range(2))
+    return tuple(x.bfloat16() for x in (*qk, *(torch.randn(batch, heads, seq, dim, generator=g) for _ in range(2))))
+
+
+def _rel(got, want):
+    return float((got.float().cpu() - want).norm() / want.norm().clamp_min(1e-30))
+
+
+# more than 148 (query tile, head) pairs: below that the forward takes one head a CTA
+@pytest.mark.parametrize("batch,heads,seq,exempt,scale", [
+    (1, 150, 50, 1, 1.0), (1, 76, 129, 3, 1.0), (2, 38, 257, 1, 0.3), (1, 22, 1000, 140, 0.3),          # two heads of a selector
+    (150, 1, 50, 1, 1.0), (76, 1, 129, 3, 1.0), (76, 1, 257, 1, 0.3), (22, 1, 1000, 140, 0.3),          # two rows, each its own
+])
+def test_two_heads_a_cta(batch, heads, seq, exempt, scale):
+    q, k, v, w = _inputs(batch, heads, seq, 64, scale, seq + heads)
+    want = oracle.attention_grads(q.float(), k.float(), v.float(), w.float(), exempt)
+    qq, kk, vv = (x.cuda().requires_grad_(True) for x in (q, k, v))
+    out = kernels.selective_attention(qq, kk, vv, exempt=exempt)
+    grads = torch.autograd.grad(out, (qq, kk, vv), w.cuda().float())
+    _, aux = kernels.selective_attention_forward(q.cuda(), k.cuda(), v.cuda(), return_aux=True, exempt=exempt)
+    for got, ref in zip((out.detach(), *grads), want):
+        assert _rel(got, ref) < 1e-2
+    _, total = kernels.selective_logits(q.float(), k.float(), exempt)
+    torch.testing.assert_close(aux["selected_total"].cpu(), total, atol=2e-3, rtol=2e-3)
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+def test_two_heads_a_cta_in_a_continued_prefill_and_in_bf16(per_head):
+    heads, first, total = 76, 200, 460
+    q, k, v, w = (x.cuda() for x in _inputs(1, heads, total, 64, 0.5, 7))
+    slot = mixers.SelectiveAttentionSlot(n_heads=heads, context_length=total, per_head=per_head)
+    whole, _ = slot.begin_cache(q, k, v)
+    y, cache = slot.begin_cache(*(x[:, :, :first] for x in (q, k, v)))
+    rows = slot.extend_cache(q[:, :, first:], k[:, :, first:], v[:, :, first:], cache)
+    assert whole.dtype == torch.bfloat16
+    torch.testing.assert_close(torch.cat([y, rows], dim=2).float(), whole.float(), atol=2e-2, rtol=2e-2)
+    qq, kk, vv = (x.clone().requires_grad_(True) for x in (q, k, v))
+    layer, _ = slot.attend(qq, kk, vv)                       # the kernels write bf16 and read a bf16 cotangent
+    assert layer.dtype == torch.bfloat16 and torch.equal(layer, whole)
+    got = torch.autograd.grad(layer, (qq, kk, vv), w)
+    views = [x.reshape(heads, 1, total, 64) if per_head else x for x in (qq, kk, vv)]
+    out = kernels.selective_attention(*views).reshape(q.shape)
+    want = torch.autograd.grad(out, (qq, kk, vv), w.float())
+    for a, b in zip(got, want):
+        assert _rel(a, b.float().cpu()) < 2e-3
+
+
+def test_a_second_differentiation_raises():
+    q, k, v, _ = (x.cuda().requires_grad_(True) for x in _inputs(1, 2, 70, 64, 1.0, 3))
+    out = kernels.selective_attention(q, k, v)
+    (dq,) = torch.autograd.grad(out.square().sum(), q, create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        dq.sum().backward()
