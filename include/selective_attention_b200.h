@@ -307,10 +307,12 @@ int sa_decode_step_live_keys(int dtype, int batch, int heads, int groups, int le
                              void* stream);
 
 /* The decode step from a block of arguments that a caller keeps with its cache and updates (q1, k1, v1, y, length, stream)
- * from step to step.  key_norms may be NULL.  y_dtype: SA_F32, or dtype for y in the cache's own type. */
+ * from step to step.  key_norms may be NULL.  y_dtype: SA_F32, or dtype for y in the cache's own type.  tickets_zero: the
+ * workspace, sized for the cache's last position (length = capacity - 1), was zeroed before the first step and is used by this
+ * cache's steps alone; a step then needs no memset. */
 typedef struct sa_decode {
   int32_t struct_bytes;   /* sizeof(sa_decode) */
-  int32_t dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt;
+  int32_t dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt, tickets_zero, reserved;
   const void *q1, *k1, *v1;
   void *k_cache, *v_cache;
   float *selected, *key_norms;

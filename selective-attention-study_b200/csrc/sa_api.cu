@@ -546,11 +546,12 @@ int sa_decode_run(const sa_decode* d) {
   if ((int64_t)d->batch * d->heads * ((d->length + 512) / 512) > 0x7fffffffLL) return SA_ERR_TOO_LARGE;   // 1-D grid
   for (const void* ptr : {d->q1, d->k1, d->v1, (const void*)d->k_cache, (const void*)d->v_cache})   // 16-byte loads, bulk copies
     if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0) return SA_ERR_ALIGNMENT;
-  if (d->workspace_bytes < sa_decode_workspace_bytes(d->batch, d->heads, d->groups, d->length, d->head_dim))
+  if (d->workspace_bytes < sa_decode_workspace_bytes(d->batch, d->heads, d->groups,
+                                                     d->tickets_zero ? d->capacity - 1 : d->length, d->head_dim))
     return SA_ERR_WORKSPACE;
   if (tc::timeout_pending()) return SA_ERR_DEVICE_TIMEOUT;
   const DecodeStep step{d->dtype, d->y_dtype, d->batch, d->heads, d->groups, d->length, d->capacity, d->head_dim, d->exempt,
-                        d->q1, d->k1, d->v1, d->k_cache, d->v_cache, d->selected, d->key_norms, d->y,
+                        d->tickets_zero != 0, d->q1, d->k1, d->v1, d->k_cache, d->v_cache, d->selected, d->key_norms, d->y,
                         static_cast<float*>(d->workspace)};
   return decode_step(step, static_cast<cudaStream_t>(d->stream));
 }

@@ -162,34 +162,6 @@ static int decode_split_keys(int t, int rows) {
   return (keys + kDecSplitMin - 1) / kDecSplitMin * kDecSplitMin;
 }
 
-// The attend kernel is launched while the append kernel runs (programmatic stream serialization): what does not depend
-// on the new key or the tickets goes ahead of this wait.
-__device__ __forceinline__ void wait_for_append() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// Writes the new key and value into the cache and clears the tickets the attend kernel counts CTAs with.
-// With `knorm` (the per-key norms a decode that leaves out dead keys relies on) also stores the new key's norm.
-template <typename T>
-__global__ void append_kernel(const T* __restrict__ k1, const T* __restrict__ v1, T* __restrict__ kc,
-                              T* __restrict__ vc, int rows, int capacity, int length, int D,
-                              unsigned int* __restrict__ tickets, int n_tickets, float* __restrict__ knorm) {
-  asm volatile("griddepcontrol.launch_dependents;");
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < n_tickets) tickets[idx] = 0u;
-  if (knorm != nullptr && idx < rows) {
-    float ss = 0.f;
-    for (int d = 0; d < D; ++d) {
-      const float x = to_float<T>(k1[(int64_t)idx * D + d]);
-      ss = fmaf(x, x, ss);
-    }
-    knorm[(int64_t)idx * capacity + length] = sqrtf(ss);
-  }
-  if (idx >= rows * D) return;
-  int n = idx / D, d = idx - n * D;
-  int64_t dst = ((int64_t)n * capacity + length) * D + d;
-  kc[dst] = k1[idx];
-  vc[dst] = v1[idx];
-}
-
 // 16-byte load of 8 (bf16 / fp16) or two 16-byte loads of 8 fp32 elements, converted to fp32.
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&x)[8]) {
@@ -275,16 +247,19 @@ __device__ __forceinline__ void decode_combine_row(const float* prow, TY* yrow, 
 // only those.  The CTAs of a selecting head stay dense: the new query's selection is needed for every key.
 template <typename T, typename TY, int D, bool LIVE>
 __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
-    const T* __restrict__ q1, const T* __restrict__ kc, const T* __restrict__ vc, float* selected,
+    const T* __restrict__ q1, const T* __restrict__ k1, const T* __restrict__ v1, T* kc, T* vc, float* selected,
     float* __restrict__ partial, float* __restrict__ sel_new, int heads, int groups, int t, int capacity,
     int exempt, float scale, int split_keys, tc::WaitCtx status, TY* __restrict__ y, unsigned int* __restrict__ row_tickets, unsigned int* __restrict__ split_tickets, int splits,
-    const float* __restrict__ knorm) {
+    float* knorm) {
   constexpr int kLanes = D / 8;                                   // lanes per key
   constexpr int kGroups = kDecThreads / kLanes;                   // keys the CTA covers per step
   constexpr int kRowBytes = D * (int)sizeof(T);
   constexpr int kStageKeys = kDecStageBytes / kRowBytes;
   constexpr int kPer = kStageKeys / kGroups;                      // keys per group per stage (4, fp32: 2)
   static_assert(kPer >= 1 && kPer * kGroups == kStageKeys, "stage layout");
+  // Launched while the step before is still running (programmatic stream serialization); its results from here on.
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   extern __shared__ uint8_t dec_smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dec_smem_raw) + 127) & ~uintptr_t(127));
   __shared__ uint64_t full[kDecStages];
@@ -307,15 +282,20 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
   const uint8_t* kb = reinterpret_cast<const uint8_t*>(kc + (int64_t)n * capacity * D);
   const uint8_t* vb = reinterpret_cast<const uint8_t*>(vc + (int64_t)n * capacity * D);
 
+  // The range that ends with the newest key: that key and value come from k1, v1, and this CTA writes them to the cache (in a
+  // launch of their own the append took 1.6 us of a 13 us step, and the launch as much on the host).
+  const bool tail = c1 == t;
+  const int c_mem = tail ? t - 1 : c1;                            // keys below come from the cache
   const bool sparse = LIVE && !selector;                          // this CTA leaves out dead stages
   auto stage_of = [&](int it) { return sparse ? (int)live_s[it] : it; };
   auto issue = [&](int it) {                                      // thread 0 only; `it` counts the stages this CTA streams
     const int st = it;
     const int j0 = c0 + stage_of(it) * kStageKeys;
-    const uint32_t bytes = (uint32_t)(min(kStageKeys, c1 - j0) * kRowBytes);
+    const uint32_t bytes = (uint32_t)(min(kStageKeys, c_mem - j0) * kRowBytes);      // 0: the newest key alone
     uint8_t* dst = ring + (size_t)(st % kDecStages) * 2 * kDecStageBytes;
     uint64_t* bar = &full[st % kDecStages];
     tc::mbar_expect_tx(bar, 2 * bytes);
+    if (bytes == 0) return;
     tc::bulk_load(dst, kb + (int64_t)j0 * kRowBytes, bytes, bar);
     tc::bulk_load(dst + kDecStageBytes, vb + (int64_t)j0 * kRowBytes, bytes, bar);
   };
@@ -324,11 +304,19 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
   const float* selb = selected + ((int64_t)b * groups + g) * capacity;
   float* selnb = sel_new + ((int64_t)b * groups + g) * t;
   int n_iter = n_stages;
-  if (sparse || c1 == t) wait_for_append();                       // the new key's norm, or the new key itself
+  if (knorm != nullptr && tail) {                                 // the newest key's norm
+    float kx[8], ss = 0.f;
+    load8<T>(k1 + (int64_t)n * D + lane * 8, kx);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss = fmaf(kx[e], kx[e], ss);
+#pragma unroll
+    for (int sft = kLanes / 2; sft > 0; sft >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sft);
+    if (threadIdx.x == 0) knorm[(int64_t)n * capacity + t - 1] = sqrtf(ss);
+  }
   if (sparse) {
     // |q| and the newest key's logit, by every group of lanes (each holds the whole of q between its lanes)
     float kx[8], ss = 0.f, dot = 0.f;
-    load8<T>(kc + ((int64_t)n * capacity + (t - 1)) * D + lane * 8, kx);
+    load8<T>(k1 + (int64_t)n * D + lane * 8, kx);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       ss = fmaf(qv[e], qv[e], ss);
@@ -350,13 +338,13 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         const int j = base + u * kDecThreads;
-        nrm[u] = (j < c1) ? __ldg(kn + j) : 0.f;
+        nrm[u] = (j < c_mem) ? __ldcg(kn + j) : 0.f;
         sel[u] = (j < c1) ? __ldcg(selb + j) : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         const int j = base + u * kDecThreads;
-        if (j < c1 && cq * nrm[u] - kLog2e * sel[u] >= thr) {
+        if (j < c1 && (j == t - 1 || cq * nrm[u] - kLog2e * sel[u] >= thr)) {
           const int st = (j - c0) / kStageKeys;
           atomicOr(&live_bits[st >> 5], 1u << (st & 31));
         }
@@ -405,6 +393,17 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     // the slot that stage st + kDecStages - 1 uses was read in iteration st - 1; every thread is past it
     if (threadIdx.x == 0 && st + kDecStages - 1 < n_iter) issue(st + kDecStages - 1);
     tc::mbar_wait(&full[st % kDecStages], (st / kDecStages) & 1, status, 600);
+    if (tail && st == n_iter - 1) {                               // the newest key and value: into their rows of the stage and the cache
+      constexpr int kChunks = kRowBytes / 16;
+      if (threadIdx.x < 2 * kChunks) {
+        const bool val = threadIdx.x >= kChunks;
+        const int c = (int)threadIdx.x - (val ? kChunks : 0);
+        const uint4 x = reinterpret_cast<const uint4*>((val ? v1 : k1) + (int64_t)n * D)[c];
+        reinterpret_cast<uint4*>(ring + ((size_t)(st % kDecStages) * 2 + (val ? 1 : 0)) * kDecStageBytes + (t - 1 - j0) * kRowBytes)[c] = x;
+        reinterpret_cast<uint4*>((val ? vc : kc) + ((int64_t)n * capacity + t - 1) * D)[c] = x;
+      }
+      __syncthreads();
+    }
     const uint8_t* ks = ring + (size_t)(st % kDecStages) * 2 * kDecStageBytes;
     const uint8_t* vs = ks + kDecStageBytes;
 
@@ -483,7 +482,6 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
     prow[D + 1] = red[0];
   }
 
-  wait_for_append();                                              // the tickets are cleared
   // The last CTA of a query row merges the row's partials into y; the last of the `per` heads that share a
   // history vector to finish a key range adds the new selection of that range to it (every reader is done).
   __threadfence();                                                // partials and sel_new visible before the ticket
@@ -497,6 +495,10 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
   const bool last_of_range = ticket_s[1] == (unsigned)per - 1;
   if (!last_of_row && !last_of_range) return;
   __threadfence();
+  if (threadIdx.x == 0) {                                          // zero again for the next step
+    if (last_of_row) row_tickets[n] = 0u;
+    if (last_of_range) split_tickets[((int64_t)b * groups + g) * splits + split] = 0u;
+  }
   if (last_of_range) {
     float* sel_rw = selected + ((int64_t)b * groups + g) * capacity;
     constexpr int kBatch = 8;                                     // independent loads in flight per thread
@@ -520,10 +522,10 @@ __global__ void __launch_bounds__(kDecThreads) decode_attend_kernel(
 }
 
 template <typename T, typename TY, int D, bool LIVE>
-int launch_attend(unsigned grid, cudaStream_t s, const T* q, const T* kc, const T* vc, float* selected, float* partial,
+int launch_attend(unsigned grid, cudaStream_t s, const T* q, const T* k1, const T* v1, T* kc, T* vc, float* selected, float* partial,
                   float* sel_new, int heads, int groups, int t, int capacity, int exempt, int split_keys,
                   const tc::WaitCtx& status, TY* y, unsigned int* row_tickets, unsigned int* split_tickets, int splits,
-                  const float* knorm) {
+                  float* knorm) {
   auto kernel = decode_attend_kernel<T, TY, D, LIVE>;
   SA_CUDA_CHECK(allow_smem(kernel, kDecSmemBytes));
   cudaLaunchAttribute attr;
@@ -537,7 +539,7 @@ int launch_attend(unsigned grid, cudaStream_t s, const T* q, const T* kc, const 
   config.attrs = &attr;
   config.numAttrs = 1;
   count_launch();
-  SA_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, q, kc, vc, selected, partial, sel_new, heads, groups, t, capacity, exempt,
+  SA_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, q, k1, v1, kc, vc, selected, partial, sel_new, heads, groups, t, capacity, exempt,
                                    1.0f / sqrtf((float)D), split_keys, status, y, row_tickets, split_tickets, splits, knorm));
   return SA_OK;
 }
@@ -549,26 +551,24 @@ int decode_impl(const DecodeStep& d, cudaStream_t s) {
   // keys; 512 and 2048 measured slower) then spread those heads over the whole GPU.
   const int split_keys = (d.key_norms != nullptr) ? 1024 : decode_split_keys(t, rows);
   const int splits = (t + split_keys - 1) / split_keys;
-  float* partial = d.workspace;
-  float* sel_new = partial + (size_t)rows * splits * (D + 2);
-  unsigned int* row_tickets = reinterpret_cast<unsigned int*>(sel_new + (size_t)d.batch * d.groups * t);
+  // Tickets first: with `tickets_zero` at a size that does not change from step to step, so that what the last CTAs leave at zero
+  // is where the next step looks.
+  const int ticket_splits = d.tickets_zero ? (d.capacity + kDecSplitMin - 1) / kDecSplitMin : splits;
+  unsigned int* row_tickets = reinterpret_cast<unsigned int*>(d.workspace);
   unsigned int* split_tickets = row_tickets + rows;
-  const int n_tickets = rows + d.batch * d.groups * splits;
-  const int append_threads = rows * D > n_tickets ? rows * D : n_tickets;
+  const size_t n_tickets = (size_t)rows + (size_t)d.batch * d.groups * ticket_splits;
+  float* partial = d.workspace + n_tickets;
+  float* sel_new = partial + (size_t)rows * splits * (D + 2);
   tc::WaitCtx status;
   if (int st = tc::wait_ctx(&status)) return st;
-  ProfileScope prof(SA_KERNEL_DECODE, s);   // the whole step: append, then attend with its merge and update
-  count_launch();
-  append_kernel<T><<<(append_threads + 255) / 256, 256, 0, s>>>(
-      static_cast<const T*>(d.k1), static_cast<const T*>(d.v1), static_cast<T*>(d.k_cache), static_cast<T*>(d.v_cache), rows,
-      d.capacity, d.length, D, row_tickets, n_tickets, d.key_norms);
-  SA_CUDA_CHECK(cudaGetLastError());
+  ProfileScope prof(SA_KERNEL_DECODE, s);
+  if (!d.tickets_zero) SA_CUDA_CHECK(cudaMemsetAsync(row_tickets, 0, n_tickets * 4, s));
   // dead stages are left out when the norms are given and a CTA's range fits the stage list
   const bool live = d.key_norms != nullptr && split_keys / (kDecStageBytes / (D * (int)sizeof(T))) <= kDecMaxLive;
   auto attend = [&](auto dim, auto live_tag) {
     return launch_attend<T, TY, decltype(dim)::value, decltype(live_tag)::value>(
-        (unsigned)rows * (unsigned)splits, s, static_cast<const T*>(d.q1), static_cast<const T*>(d.k_cache),
-        static_cast<const T*>(d.v_cache), d.selected, partial, sel_new, d.heads, d.groups, t, d.capacity, d.exempt, split_keys,
+        (unsigned)rows * (unsigned)splits, s, static_cast<const T*>(d.q1), static_cast<const T*>(d.k1),
+        static_cast<const T*>(d.v1), static_cast<T*>(d.k_cache), static_cast<T*>(d.v_cache), d.selected, partial, sel_new, d.heads, d.groups, t, d.capacity, d.exempt, split_keys,
         status, static_cast<TY*>(d.y), row_tickets, split_tickets, splits, d.key_norms);
   };
   auto by_live = [&](auto dim) { return live ? attend(dim, std::true_type{}) : attend(dim, std::false_type{}); };

@@ -50,7 +50,7 @@ class Tensor(ctypes.Structure):
 class Decode(ctypes.Structure):
     """sa_decode: the arguments of a decode step, kept with its cache."""
     _fields_ = ([(name, ctypes.c_int32) for name in ("struct_bytes", "dtype", "y_dtype", "batch", "heads", "groups", "length",
-                                                     "capacity", "head_dim", "exempt")] +
+                                                     "capacity", "head_dim", "exempt", "tickets_zero", "reserved")] +
                 [(name, ctypes.c_void_p) for name in ("q1", "k1", "v1", "k_cache", "v_cache", "selected", "key_norms", "y",
                                                       "workspace")] +
                 [("workspace_bytes", ctypes.c_uint64), ("stream", ctypes.c_void_p)])

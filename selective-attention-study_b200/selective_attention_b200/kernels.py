@@ -638,9 +638,9 @@ class _DecodePlan:
         groups = selected.shape[1]
         # scratch for the longest step that the cache can take
         need = _lib.load().sa_decode_workspace_bytes(b, h, groups, max(cap - 1, 0), d)
-        self.workspace = torch.empty(need, device=kc.device, dtype=torch.uint8)
+        self.workspace = torch.zeros(need, device=kc.device, dtype=torch.uint8)
         a = self.args = _lib.Decode()
-        a.struct_bytes = ctypes.sizeof(_lib.Decode)
+        a.struct_bytes, a.tickets_zero = ctypes.sizeof(_lib.Decode), 1
         a.dtype, a.batch, a.heads, a.groups, a.capacity, a.head_dim = _DTYPE_CODE[kc.dtype], b, h, groups, cap, d
         a.k_cache, a.v_cache, a.selected = kc.data_ptr(), vc.data_ptr(), selected.data_ptr()
         a.key_norms = norms.data_ptr() if norms is not None else None

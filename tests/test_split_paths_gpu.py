@@ -1,5 +1,5 @@
-"""The forward variants that only larger grids reach: two heads of a selector, or two rows that each select for
-themselves, in one CTA."""
+"""The forward variants that only larger grids reach (two heads of a selector, or two rows that each select for
+themselves, in one CTA), second differentiation, and the newest key of a decode step."""
 
 import pytest
 import torch
@@ -65,3 +65,29 @@ def test_a_second_differentiation_raises():
     (dq,) = torch.autograd.grad(out.square().sum(), q, create_graph=True)
     with pytest.raises(RuntimeError, match="once_differentiable"):
         dq.sum().backward()
+
+
+@pytest.mark.parametrize("dtype,dim,norms", [(torch.bfloat16, 64, False), (torch.bfloat16, 64, True), (torch.float16, 128, False),
+                                             (torch.float32, 16, False)])
+@pytest.mark.parametrize("start", [0, 1020])
+def test_the_newest_key_at_the_edges_of_a_decode_range(dtype, dim, norms, start):
+    """The newest key comes from the call, not from the cache: alone in its stage, alone in its range, after either."""
+    b, h, steps = 2, 3, 134
+    g = torch.Generator("cpu").manual_seed(start + dim)
+    q, k, v = ((s * torch.randn(b, h, start + steps, dim, generator=g)).to(dtype) for s in (0.5, 1.0, 1.0))
+    ref = {"k": torch.zeros_like(k), "v": torch.zeros_like(v), "len": start, "selected": torch.zeros(b, 1, start + steps)}
+    ref["k"][:, :, :start], ref["v"][:, :, :start] = k[:, :, :start], v[:, :, :start]
+    dev = {key: (val.cuda() if torch.is_tensor(val) else val) for key, val in ref.items()}
+    if norms:
+        dev["key_norms"] = dev["k"].float().norm(dim=-1)
+    slot = mixers.SelectiveAttentionSlot(n_heads=h, context_length=start + steps)
+    for t in range(start, start + steps):
+        step = [x[:, :, t:t + 1] for x in (q, k, v)]
+        want = oracle.decode_step(ref, *step, groups=1)
+        got = slot.step_cache(*(x.cuda() for x in step), dev)
+        tol = 2e-5 if dtype == torch.float32 else 2e-2
+        torch.testing.assert_close(got.float().cpu(), want, atol=tol, rtol=tol)
+    torch.testing.assert_close(dev["selected"].cpu(), ref["selected"], atol=1e-3, rtol=1e-3)
+    assert torch.equal(dev["k"].cpu(), k) and torch.equal(dev["v"].cpu(), v)
+    if norms:
+        torch.testing.assert_close(dev["key_norms"].cpu(), k.float().norm(dim=-1), rtol=1e-5, atol=1e-5)
