@@ -10,14 +10,19 @@
 //   backward per 32-key block of one head, query blocks last to first; dV, dK in registers; dQ and the
 //            head-0 selection gradients through fp32 reductions                                      (:196-268)
 //
-// Register tiles.  128 threads as 8 x 16; a thread owns 4 rows (4 ty ..) of a tile and the columns tx + 16 c, or 4 rows and
-// D / 16 output columns (256 threads with 2 rows each, 1.5 loads a FMA more, took 17 % longer).  Operands sit in shared
-// memory as fp32 rows of D + 4 floats (consecutive rows start 4 banks apart, so eight rows of a 16-byte load do not
-// conflict) and are read 16 bytes at a time along the contraction: 8 loads for 64 FMAs.  The contraction index runs upwards
-// in every product, one FMA after the other.
-// What bounds it: FFMA issue and the shared-memory loads that feed it, at about the same rate; with few (batch, head) rows
-// the longest walk.  With one load per FMA operand and thread, and the selection pass on T / 64 blocks, the case
-// B = 2, H = 4, T = 1024, D = 64 took 153 + 403 + 859 us (selection, forward, backward); this form takes 15 + 134 + 339 us.
+// Work split of forward and backward.  A team is 256 threads in two groups of 128, 8 x 16; a CTA has one team or two.
+//   logits    each group forms half of the contraction of the whole tile, 4 rows x 4 (backward 2) columns a thread, and hands
+//             the other group its half of the columns, so that what follows has one group for each half of the columns
+//   forward   a group has the softmax state and the output of its own 32 keys of every tile; a second team takes every other
+//             key tile; the two or four are merged at the end, and nothing else crosses groups
+//   backward  a second team takes every other query tile and shares the sums of dz per key, the one thing that is carried from
+//             tile to tile; key gradients: 4 x 4 a thread for any D, so 128 / D sets of threads take the queries in turn and
+//             are added up at the end; dQ and the selector's dQ0: a group each
+// Operands sit in shared memory as fp32 rows of D + 4 floats (consecutive rows start 4 banks apart) and are read 16 bytes at a
+// time; two FMAs an instruction, along the contraction in the logits (even and odd elements apart), else along the columns.
+// What bounds it: shared-memory loads (82 % of their rate in backward at D = 32) and FMAs at about the same rate; with few
+// (batch, head) rows the longest walk.  us for selection, forward, backward, at first / 128 threads a CTA, one FMA an
+// instruction / now:  (2, 4, 1024, 64) fp32  153, 403, 859 / 15, 134, 339 / 14, 78, 160;  (4, 8, 1000, 32) fp16 now 12, 170, 290.
 //
 // A head that is its own selector (head 0, unless the selector comes from outside) has its selection logits already, and
 // since Q0 = Q, K0 = K its two gradient paths add before the products: dK += (dz + g)^T Q, dQ += (dz + g) K.
@@ -27,7 +32,8 @@
 namespace sa {
 namespace simt {
 
-constexpr int kThreads = 128;
+constexpr int kTeam = 256;     // forward and backward: a CTA is two teams (forward, D = 128: one) of two groups of 128
+constexpr int kSelThreads = 128;
 constexpr int kQ = 32;         // query rows per tile (== kSimtCarryRows)
 constexpr int kKF = 64;        // keys per tile, selection and forward kernels
 constexpr int kKB = 32;        // keys per block, backward kernel
@@ -42,15 +48,15 @@ __device__ __forceinline__ const T* row_ptr(const Strided& s, int b, int h) {
 // ROWS rows of D elements from token t0 on, on their way to dst[ROWS][D + 4] as fp32, zero past seq.  fetch() has all of a
 // thread's loads in flight at once; between fetch() and store() they are covered by whatever is computed there.
 // `vec`: four elements at a time.
-template <typename T, int D, int ROWS>
+template <typename T, int D, int ROWS, int THREADS = kTeam>
 struct Tile {
-  static constexpr int C = D / 4, N = (ROWS * C + kThreads - 1) / kThreads;
+  static constexpr int C = D / 4, N = (ROWS * C + THREADS - 1) / THREADS;
   struct alignas(4 * sizeof(T)) Quad { T e[4]; };
   Quad x[N];
-  __device__ __forceinline__ void fetch(const T* base, int64_t st, int t0, int seq, bool vec) {
+  __device__ __forceinline__ void fetch(int id, const T* base, int64_t st, int t0, int seq, bool vec) {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-      const int idx = threadIdx.x + u * kThreads, r = idx / C, c = (idx - r * C) * 4, t = t0 + r;
+      const int idx = id + u * THREADS, r = idx / C, c = (idx - r * C) * 4, t = t0 + r;
 #pragma unroll
       for (int e = 0; e < 4; ++e) x[u].e[e] = from_float<T>(0.f);
       if (t >= seq || r >= ROWS) continue;
@@ -63,104 +69,152 @@ struct Tile {
       }
     }
   }
-  __device__ __forceinline__ void store(float* dst) const {
+  __device__ __forceinline__ void store(int id, float* dst) const {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-      const int idx = threadIdx.x + u * kThreads, r = idx / C, c = (idx - r * C) * 4;
+      const int idx = id + u * THREADS, r = idx / C, c = (idx - r * C) * 4;
       if (r < ROWS)
         *reinterpret_cast<float4*>(dst + r * (D + 4) + c) =
             make_float4(to_float<T>(x[u].e[0]), to_float<T>(x[u].e[1]), to_float<T>(x[u].e[2]), to_float<T>(x[u].e[3]));
     }
   }
 };
-// Whether the next tiles' elements are held in registers during the products of the tile at hand.
-template <typename T, int D> constexpr bool kAhead = D * (int)sizeof(T) <= 256;
-
-template <typename T, int D, int ROWS>
+template <typename T, int D, int ROWS, int THREADS>
 __device__ __forceinline__ void load_tile(float* dst, const T* base, int64_t st, int t0, int seq, bool vec) {
-  Tile<T, D, ROWS> x;
-  x.fetch(base, st, t0, seq, vec);
-  x.store(dst);
+  Tile<T, D, ROWS, THREADS> x;
+  x.fetch(threadIdx.x, base, st, t0, seq, vec);
+  x.store(threadIdx.x, dst);
 }
+
+// Thread `id` of a grid of X columns: neighbouring lanes take two rows of one column.  A 16-byte shared-memory load takes 2 cycles
+// a warp where lanes l and l ^ 1 (or l ^ 2) read the same address, and 4 where only l and l ^ 16 do, however few the addresses.
+template <int X> __device__ __forceinline__ int col_of(int id) { return (id >> 1) % X; }
+template <int X> __device__ __forceinline__ int row_of(int id) { return (id & 1) | (id / (2 * X) << 1); }
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// acc[u][c] += a[4 ty + u] . b[tx + 16 c] over D, in order
-template <int D, int NC>
-__device__ __forceinline__ void dot_rows(float (&acc)[kRows][NC], const float* a, const float* b, int ty, int tx) {
+// Two fp32 FMAs in one instruction: 118 FMAs a cycle and SM measured, where the single one reaches 85.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ ulonglong2 ld4x2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory"); }
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(3 + group) : "memory"); }
+
+// acc[u][c] = a[4 ty + u] . row tx + 16 c of `own` (the first half of the columns) or `other`, over DN elements: the even and the
+// odd ones each in order, then their sum
+template <int D, int DN, int NC>
+__device__ __forceinline__ void dot_rows(float (&acc)[kRows][NC], const float* a, const float* own, const float* other, int ty, int tx) {
   const float* ar = a + (ty * kRows) * (D + 4);
-  const float* br = b + tx * (D + 4);
+  const float* b0 = own + tx * (D + 4);
+  const float* b1 = other + tx * (D + 4);
+  f32x2 sum[kRows][NC];
+#pragma unroll
+  for (int u = 0; u < kRows; ++u)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sum[u][c] = 0ull;
 #pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
-    float4 x[kRows], y[NC];
+  for (int d = 0; d < DN; d += 4) {
+    ulonglong2 x[kRows], y[NC];
 #pragma unroll
-    for (int u = 0; u < kRows; ++u) x[u] = ld4(ar + u * (D + 4) + d);
+    for (int u = 0; u < kRows; ++u) x[u] = ld4x2(ar + u * (D + 4) + d);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) y[c] = ld4(br + 16 * c * (D + 4) + d);
+    for (int c = 0; c < NC; ++c) y[c] = ld4x2((c < NC / 2 ? b0 + 16 * c * (D + 4) : b1 + 16 * (c - NC / 2) * (D + 4)) + d);
 #pragma unroll
     for (int u = 0; u < kRows; ++u)
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        acc[u][c] = fmaf(x[u].x, y[c].x, acc[u][c]);
-        acc[u][c] = fmaf(x[u].y, y[c].y, acc[u][c]);
-        acc[u][c] = fmaf(x[u].z, y[c].z, acc[u][c]);
-        acc[u][c] = fmaf(x[u].w, y[c].w, acc[u][c]);
+        sum[u][c] = fma2(x[u].x, y[c].x, sum[u][c]);
+        sum[u][c] = fma2(x[u].y, y[c].y, sum[u][c]);
       }
   }
-}
-
-// The D / 16 output columns of a thread: in fours (D = 128: 4 tx .. and 64 + 4 tx ..), or 2 tx, 2 tx + 1, or tx.
-template <int CD>
-__device__ __forceinline__ void load_cols(const float* row, int tx, float (&x)[CD]) {
-  if constexpr (CD >= 4) {
 #pragma unroll
-    for (int f = 0; f < CD / 4; ++f) {
-      const float4 v = ld4(row + 64 * f + 4 * tx);
-      x[4 * f] = v.x; x[4 * f + 1] = v.y; x[4 * f + 2] = v.z; x[4 * f + 3] = v.w;
+  for (int u = 0; u < kRows; ++u)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float2 v = unpack2(sum[u][c]);
+      acc[u][c] = v.x + v.y;
     }
-  } else if constexpr (CD == 2) {
-    const float2 v = *reinterpret_cast<const float2*>(row + 2 * tx);
-    x[0] = v.x; x[1] = v.y;
-  } else {
-    x[0] = row[tx];
-  }
 }
-// dst += x: fp32 reductions in global memory, as wide as the columns are contiguous
-template <int CD>
-__device__ __forceinline__ void reduce_cols(float* row, int tx, const float (&x)[CD], float scale) {
-  if constexpr (CD >= 4) {
-#pragma unroll
-    for (int f = 0; f < CD / 4; ++f)
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + 64 * f + 4 * tx), "f"(x[4 * f] * scale),
-                   "f"(x[4 * f + 1] * scale), "f"(x[4 * f + 2] * scale), "f"(x[4 * f + 3] * scale)
-                   : "memory");
-  } else if constexpr (CD == 2) {
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(row + 2 * tx), "f"(x[0] * scale), "f"(x[1] * scale) : "memory");
-  } else {
-    atomicAdd(row + tx, x[0] * scale);
-  }
-}
-template <int CD>
-__device__ __forceinline__ int col_of(int tx, int c) { return CD >= 4 ? 64 * (c >> 2) + 4 * tx + (c & 3) : CD * tx + c; }
 
-// acc[u][:] += sum_j w[4 ty + u][j] rows[j][:] over N rows j, w with row stride WS
-template <int D, int N, int WS, int CD>
-__device__ __forceinline__ void weighted_rows(float (&acc)[kRows][CD], const float* w, const float* rows, int ty, int tx) {
-  const float* wr = w + (ty * kRows) * WS;
+// CD neighbouring output columns of one row (CD = 8: two runs of four, 64 columns apart).
+template <int CD>
+struct Cols {
+  f32x2 p[CD / 2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int k = 0; k < CD / 2; ++k) p[k] = 0ull;
+  }
+  __device__ __forceinline__ void load(const float* row, int tx) {
+    if constexpr (CD == 2) {
+      p[0] = *reinterpret_cast<const f32x2*>(row + 2 * tx);
+    } else {
+#pragma unroll
+      for (int f = 0; f < CD / 4; ++f) {
+        const ulonglong2 v = ld4x2(row + 64 * f + 4 * tx);
+        p[2 * f] = v.x; p[2 * f + 1] = v.y;
+      }
+    }
+  }
+  __device__ __forceinline__ void add(f32x2 w, const Cols& y) {
+#pragma unroll
+    for (int k = 0; k < CD / 2; ++k) p[k] = fma2(w, y.p[k], p[k]);
+  }
+  __device__ __forceinline__ void scale(float a) {
+    const f32x2 aa = pack2(a, a);
+#pragma unroll
+    for (int k = 0; k < CD / 2; ++k) p[k] = fma2(aa, p[k], 0ull);
+  }
+  __device__ __forceinline__ float get(int c) const {
+    const float2 v = unpack2(p[c >> 1]);
+    return (c & 1) ? v.y : v.x;
+  }
+};
+template <>
+struct Cols<1> {
+  float p;
+  __device__ __forceinline__ void zero() { p = 0.f; }
+  __device__ __forceinline__ void load(const float* row, int tx) { p = row[tx]; }
+  __device__ __forceinline__ void add(f32x2 w, const Cols& y) { p = fmaf(unpack2(w).x, y.p, p); }
+  __device__ __forceinline__ void scale(float a) { p *= a; }
+  __device__ __forceinline__ float get(int) const { return p; }
+};
+template <int CD>
+__device__ __forceinline__ int out_col(int tx, int c) { return CD >= 4 ? 64 * (c >> 2) + 4 * tx + (c & 3) : CD * tx + c; }
+__device__ __forceinline__ void reduce4(float* dst, float4 x) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+}
+
+// acc[u] += sum_j w[R y + u][j] rows[j][columns of x] over N rows j, w with row stride WS
+template <int D, int N, int WS, int R, int CD>
+__device__ __forceinline__ void weighted_rows(Cols<CD> (&acc)[R], const float* w, const float* rows, int y, int x) {
+  const float* wr = w + (y * R) * WS;
 #pragma unroll 2
   for (int j = 0; j < N; j += 4) {
-    float4 x[kRows];
+    float4 a[R];
 #pragma unroll
-    for (int u = 0; u < kRows; ++u) x[u] = ld4(wr + u * WS + j);
+    for (int u = 0; u < R; ++u) a[u] = ld4(wr + u * WS + j);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      float y[CD];
-      load_cols<CD>(rows + (j + v) * (D + 4), tx, y);
+      Cols<CD> b;
+      b.load(rows + (j + v) * (D + 4), x);
 #pragma unroll
-      for (int u = 0; u < kRows; ++u) {
-        const float xv = v == 0 ? x[u].x : v == 1 ? x[u].y : v == 2 ? x[u].z : x[u].w;
-#pragma unroll
-        for (int c = 0; c < CD; ++c) acc[u][c] = fmaf(xv, y[c], acc[u][c]);
+      for (int u = 0; u < R; ++u) {
+        const float av = v == 0 ? a[u].x : v == 1 ? a[u].y : v == 2 ? a[u].z : a[u].w;
+        acc[u].add(pack2(av, av), b);
       }
     }
   }
@@ -170,19 +224,19 @@ __device__ __forceinline__ void weighted_rows(float (&acc)[kRows][CD], const flo
 // selection: grid (key tiles of 64, query blocks of 32, batch); carry[b][block][key] <- the block's sum per key
 // ---------------------------------------------------------------------------------------------------
 template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) colsum_kernel(Problem p, float* __restrict__ carry, int nblocks, bool vec) {
+__global__ void __launch_bounds__(kSelThreads) colsum_kernel(Problem p, float* __restrict__ carry, int nblocks, bool vec) {
   extern __shared__ __align__(16) float smem[];
   float* k0s = smem;                       // [64][D + 4]
   float* q0s = k0s + kKF * (D + 4);        // [32][D + 4]
   float* part = q0s + kQ * (D + 4);        // [8][64]
   const int j0 = blockIdx.x * kKF, rb = blockIdx.y, b = blockIdx.z, m0 = rb * kQ;
   if (m0 + kQ <= j0) return;               // all keys of the tile come after all its queries
-  load_tile<T, D, kKF>(k0s, row_ptr<T>(p.k0, b, 0), p.k0.st, j0, p.seq, vec);
-  load_tile<T, D, kQ>(q0s, row_ptr<T>(p.q0, b, 0), p.q0.st, m0, p.seq, vec);
+  load_tile<T, D, kKF, kSelThreads>(k0s, row_ptr<T>(p.k0, b, 0), p.k0.st, j0, p.seq, vec);
+  load_tile<T, D, kQ, kSelThreads>(q0s, row_ptr<T>(p.q0, b, 0), p.q0.st, m0, p.seq, vec);
   __syncthreads();
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  float acc[kRows][4] = {};
-  dot_rows<D, 4>(acc, q0s, k0s, ty, tx);
+  const int ty = row_of<16>(threadIdx.x), tx = col_of<16>(threadIdx.x);
+  float acc[kRows][4];
+  dot_rows<D, D, 4>(acc, q0s, k0s, k0s + 32 * (D + 4), ty, tx);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int j = j0 + tx + 16 * c;
@@ -233,32 +287,34 @@ static __global__ void __launch_bounds__(128) scan_kernel(float* __restrict__ ca
 // ---------------------------------------------------------------------------------------------------
 // forward: grid (query tiles of 32 [heaviest first], batch * heads)
 // ---------------------------------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) forward_kernel(Problem p, const float* __restrict__ carry,
-                                                           float* __restrict__ out, float* __restrict__ lse2,
-                                                           int nblocks, bool vec) {
+template <int D> constexpr int kForwardTeamFloats = 3 * kKF * (D + 4) + kQ * (kKF + 4) + kGroups * kKF + 4 * kTeam * 4;
+
+template <typename T, int D, int TEAMS>
+__global__ void __launch_bounds__(kTeam * TEAMS, TEAMS == 1 && D < 128 ? 2 : 1) forward_kernel(Problem p, const float* __restrict__ carry,
+                                                                             float* __restrict__ out, float* __restrict__ lse2,
+                                                                             int nblocks, bool vec) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int P = D + 4, W = kKF + 4, CD = D / 16;
+  constexpr int P = D + 4, W = kKF + 4, CD = D / 16, kThreads = kTeam * TEAMS;
+  const int team = threadIdx.x / kTeam, id = threadIdx.x % kTeam, grp = id >> 7, ty = row_of<16>(id & 127), tx = col_of<16>(id);
   float* qs = smem;                        // [32][P]
   float* q0s = qs + kQ * P;
-  float* ks = q0s + kQ * P;                // [64][P]
+  float* ks = q0s + kQ * P + team * kForwardTeamFloats<D>;    // [64][P], from here on a team's own
   float* k0s = ks + kKF * P;
   float* vs = k0s + kKF * P;
   float* ps = vs + kKF * P;                // [32][W] exp2 tile
-  float* gs = ps + kQ * W;                 // [8][64]: selection of a row group, at [group][tx][c]
+  float* gs = ps + kQ * W;                 // [2][8][16][2]: selection of a row group
+  float4* ex = reinterpret_cast<float4*>(gs + kGroups * kKF);    // [4][256]: the products' other half, for the other group
 
-  const int mi = gridDim.x - 1 - blockIdx.x;
-  const int n = blockIdx.y;
+  const int rows = p.batch * p.heads, mi = nblocks - 1 - (int)blockIdx.x / rows, n = (int)blockIdx.x % rows;
   const int b = n / p.heads, h = n - b * p.heads;
   const int m0 = mi * kQ;
   const bool self = h == 0 && !p.external_selector;
   const T* kh = row_ptr<T>(p.k, b, h);
   const T* vh = row_ptr<T>(p.v, b, h);
   const T* k0 = row_ptr<T>(p.k0, b, 0);
-  load_tile<T, D, kQ>(qs, row_ptr<T>(p.q, b, h), p.q.st, m0, p.seq, vec);
-  if (!self) load_tile<T, D, kQ>(q0s, row_ptr<T>(p.q0, b, 0), p.q0.st, m0, p.seq, vec);
+  load_tile<T, D, kQ, kThreads>(qs, row_ptr<T>(p.q, b, h), p.q.st, m0, p.seq, vec);
+  if (!self) load_tile<T, D, kQ, kThreads>(q0s, row_ptr<T>(p.q0, b, 0), p.q0.st, m0, p.seq, vec);
 
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   float damp[kRows];
 #pragma unroll
   for (int u = 0; u < kRows; ++u) {
@@ -267,42 +323,64 @@ __global__ void __launch_bounds__(kThreads) forward_kernel(Problem p, const floa
     if (p.damp == SA_DAMP_LINEAR) damp[u] = fminf(1.f, (float)p.train_len / (float)(i + 1));
     if (p.damp == SA_DAMP_SQRT) damp[u] = fminf(1.f, sqrtf((float)p.train_len / (float)(i + 1)));
   }
-  float run_max[kRows], run_den[kRows], acc[kRows][CD] = {};
+  // A group keeps the running maximum, the denominator and the sums of its own 32 keys of every tile.
+  float run_max[kRows], run_den[kRows];
+  Cols<CD> acc[kRows];
 #pragma unroll
-  for (int u = 0; u < kRows; ++u) run_max[u] = -INFINITY, run_den[u] = 0.f;
+  for (int u = 0; u < kRows; ++u) run_max[u] = -INFINITY, run_den[u] = 0.f, acc[u].zero();
   const float* carry_row = carry + ((int64_t)b * nblocks + mi) * p.seq;
   const int last_key = min(m0 + kQ, p.seq);  // keys < last_key can be visible
 
+  // The next tile's keys are on their way while the values are weighted, the values while the products run.
   Tile<T, D, kKF> tk, tk0, tv;
-  float hist[4], next_hist[4];
+  float hist[2], next_hist[2];
   auto fetch = [&](int n0) {
-    tk.fetch(kh, p.k.st, n0, p.seq, vec);
-    if (!self) tk0.fetch(k0, p.k0.st, n0, p.seq, vec);
-    tv.fetch(vh, p.v.st, n0, p.seq, vec);
+    tk.fetch(id, kh, p.k.st, n0, p.seq, vec);
+    if (!self) tk0.fetch(id, k0, p.k0.st, n0, p.seq, vec);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = n0 + tx + 16 * c;
+    for (int c = 0; c < 2; ++c) {
+      const int j = n0 + 32 * grp + tx + 16 * c;
       next_hist[c] = (j < last_key) ? carry_row[j] : 0.f;
     }
   };
-  if (kAhead<T, D>) fetch(0);
-  for (int n0 = 0; n0 < last_key; n0 += kKF) {
-    if (!kAhead<T, D>) fetch(n0);
-    __syncthreads();
-    tk.store(ks);
-    if (!self) tk0.store(k0s);
-    tv.store(vs);
+  fetch(team * kKF);
+  __syncthreads();
+  for (int n0 = team * kKF; n0 < last_key; n0 += TEAMS * kKF) {
+    team_sync(team);
+    tk.store(id, ks);
+    if (!self) tk0.store(id, k0s);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) hist[c] = next_hist[c];
-    __syncthreads();
-    if (kAhead<T, D> && n0 + kKF < last_key) fetch(n0 + kKF);
-    float z[kRows][4] = {}, sel[kRows][4] = {};
-    dot_rows<D, 4>(z, qs, ks, ty, tx);
-    if (!self) dot_rows<D, 4>(sel, q0s, k0s, ty, tx);
-    float before[4];
+    for (int c = 0; c < 2; ++c) hist[c] = next_hist[c];
+    tv.fetch(id, vh, p.v.st, n0, p.seq, vec);
+    team_sync(team);
+    float z[kRows][2], sel[kRows][2];
+    {
+      const int d0 = grp * (D / 2), own = 32 * grp * P + d0, other = 32 * (1 - grp) * P + d0;
+      float t[kRows][4];
+      auto product = [&](float (&mine)[kRows][2], const float* a, const float* k, float4* to) {
+        dot_rows<D, D / 2, 4>(t, a + d0, k + own, k + other, ty, tx);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = n0 + tx + 16 * c;
+        for (int u = 0; u < kRows; ++u) mine[u][0] = t[u][0], mine[u][1] = t[u][1];
+        to[id] = make_float4(t[0][2], t[0][3], t[1][2], t[1][3]);
+        to[kTeam + id] = make_float4(t[2][2], t[2][3], t[3][2], t[3][3]);
+      };
+      product(z, qs, ks, ex);
+      if (!self) product(sel, q0s, k0s, ex + 2 * kTeam);
+      tv.store(id, vs);
+      team_sync(team);
+      auto join = [&](float (&mine)[kRows][2], const float4* from) {
+        const float4 x = from[id ^ 128], y = from[kTeam + (id ^ 128)];
+        mine[0][0] += x.x; mine[0][1] += x.y; mine[1][0] += x.z; mine[1][1] += x.w;
+        mine[2][0] += y.x; mine[2][1] += y.y; mine[3][0] += y.z; mine[3][1] += y.w;
+      };
+      join(z, ex);
+      if (!self) join(sel, ex + 2 * kTeam);
+    }
+    if (n0 + TEAMS * kKF < last_key) fetch(n0 + TEAMS * kKF);
+    float before[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int j = n0 + 32 * grp + tx + 16 * c;
       float sum = 0.f;
 #pragma unroll
       for (int u = 0; u < kRows; ++u) {          // sel becomes the exclusive prefix inside the row group
@@ -314,85 +392,134 @@ __global__ void __launch_bounds__(kThreads) forward_kernel(Problem p, const floa
       }
       before[c] = sum;
     }
-    *reinterpret_cast<float4*>(gs + ty * kKF + tx * 4) = make_float4(before[0], before[1], before[2], before[3]);
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 4; ++c) before[c] = 0.f;
+    float* gsel = gs + grp * (kGroups * 32) + tx * 2;
+    *reinterpret_cast<float2*>(gsel + ty * 32) = make_float2(before[0], before[1]);
+    group_sync(2 * team + grp);
+    before[0] = before[1] = 0.f;
     for (int g = 0; g < ty; ++g) {
-      const float4 x = ld4(gs + g * kKF + tx * 4);
-      before[0] += x.x; before[1] += x.y; before[2] += x.z; before[3] += x.w;
+      const float2 x = *reinterpret_cast<const float2*>(gsel + g * 32);
+      before[0] += x.x; before[1] += x.y;
     }
 #pragma unroll
     for (int u = 0; u < kRows; ++u) {
       const int i = m0 + ty * kRows + u;
       float tile_max = -INFINITY;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int j = n0 + tx + 16 * c;
+      for (int c = 0; c < 2; ++c) {
+        const int j = n0 + 32 * grp + tx + 16 * c;
         const bool causal = (j <= i) && (i < p.seq);
         const float f = (hist[c] + (before[c] + sel[u][c])) * damp[u];
         z[u][c] = causal ? (z[u][c] * p.scale - f) * kLog2e : -INFINITY;
         tile_max = fmaxf(tile_max, z[u][c]);
       }
 #pragma unroll
-      for (int s = 1; s < 16; s <<= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, s));
+      for (int s = 2; s < 32; s <<= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, s));
       const float new_max = fmaxf(run_max[u], tile_max);
       const float alpha = (new_max == -INFINITY) ? 1.f : exp2f(run_max[u] - new_max);
       float sum = 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
         const float e = (z[u][c] == -INFINITY) ? 0.f : exp2f(z[u][c] - new_max);
-        ps[(ty * kRows + u) * W + tx + 16 * c] = e;
+        ps[(ty * kRows + u) * W + 32 * grp + tx + 16 * c] = e;
         sum += e;
       }
       run_den[u] = run_den[u] * alpha + sum;  // this thread's columns only; the rows are added up at the end
       run_max[u] = new_max;
-#pragma unroll
-      for (int c = 0; c < CD; ++c) acc[u][c] *= alpha;
+      acc[u].scale(alpha);
     }
-    __syncwarp();                             // a row's 16 threads are in one warp: its P row is read by them alone
-    weighted_rows<D, kKF, W, CD>(acc, ps, vs, ty, tx);
+    __syncwarp();                             // a group's P row is written and read by the 16 threads of one warp alone
+    weighted_rows<D, 32, W, kRows, CD>(acc, ps + 32 * grp, vs + 32 * grp * P, ty, tx);
   }
+  // the groups' sums, at a common maximum: group g > 0 hands over [32][D], then maxima [32] and denominators [32]
+  __syncthreads();
+  const int g = threadIdx.x >> 7;
+  constexpr int kHanded = kQ * (D + 2);
 #pragma unroll
   for (int u = 0; u < kRows; ++u) {
 #pragma unroll
-    for (int s = 1; s < 16; s <<= 1) run_den[u] += __shfl_xor_sync(0xffffffffu, run_den[u], s);
-    const int i = m0 + ty * kRows + u;
+    for (int s = 2; s < 32; s <<= 1) run_den[u] += __shfl_xor_sync(0xffffffffu, run_den[u], s);
+    const int r = ty * kRows + u;
+    if (g > 0) {
+      float* to = smem + (g - 1) * kHanded;
+#pragma unroll
+      for (int c = 0; c < CD; ++c) to[r * D + out_col<CD>(tx, c)] = acc[u].get(c);
+      if (tx == 0) to[kQ * D + r] = run_max[u], to[kQ * D + kQ + r] = run_den[u];
+    }
+  }
+  __syncthreads();
+  if (g > 0) return;
+#pragma unroll
+  for (int u = 0; u < kRows; ++u) {
+    const int r = ty * kRows + u, i = m0 + r;
     if (i >= p.seq) continue;
-    const float inv = 1.f / run_den[u];
+    float top = run_max[u];                                     // finite: a visible row sees key 0, which is group 0's
+#pragma unroll
+    for (int k = 0; k < 2 * TEAMS - 1; ++k) top = fmaxf(top, smem[k * kHanded + kQ * D + r]);
+    const float a = exp2f(run_max[u] - top);
+    float den = run_den[u] * a, y[CD];
+#pragma unroll
+    for (int c = 0; c < CD; ++c) y[c] = acc[u].get(c) * a;
+#pragma unroll
+    for (int k = 0; k < 2 * TEAMS - 1; ++k) {
+      const float* from = smem + k * kHanded;
+      const float o = exp2f(from[kQ * D + r] - top);
+      den += from[kQ * D + kQ + r] * o;
+#pragma unroll
+      for (int c = 0; c < CD; ++c) y[c] += from[r * D + out_col<CD>(tx, c)] * o;
+    }
+    const float inv = 1.f / den;
     float* orow = out + ((int64_t)n * p.seq + i) * D;
 #pragma unroll
-    for (int c = 0; c < CD; ++c) orow[col_of<CD>(tx, c)] = acc[u][c] * inv;
-    if (tx == 0) lse2[(int64_t)n * p.seq + i] = run_max[u] + log2f(run_den[u]);
+    for (int c = 0; c < CD; ++c) orow[out_col<CD>(tx, c)] = y[c] * inv;
+    if (tx == 0) lse2[(int64_t)n * p.seq + i] = top + log2f(den);
   }
 }
 
 // ---------------------------------------------------------------------------------------------------
 // backward: grid (key blocks of 32, batch * heads); query blocks last to first
 // ---------------------------------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) backward_kernel(
+// dst rows += scale * w rows, R rows and 4 columns a thread, `id` counting the threads
+template <int D, int R>
+__device__ __forceinline__ void query_grads(const float* w, const float* rows, float* dst, int left, float scale, int id) {
+  const int x = col_of<D / 4>(id), y = row_of<D / 4>(id);
+  if (y * R >= kQ) return;
+  Cols<4> acc[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) acc[u].zero();
+  weighted_rows<D, kKB, kKB + 4, R, 4>(acc, w, rows, y, x);
+#pragma unroll
+  for (int u = 0; u < R; ++u)
+    if (y * R + u < left)
+      reduce4(dst + (int64_t)(y * R + u) * D + 4 * x, make_float4(acc[u].get(0) * scale, acc[u].get(1) * scale,
+                                                                  acc[u].get(2) * scale, acc[u].get(3) * scale));
+}
+
+template <int D> constexpr int kBackwardTeamFloats = 3 * kQ * (D + 4) + 3 * kQ * (kKB + 4) + 3 * kTeam * 4 + kGroups * kKB + 2 * kQ;
+
+template <typename T, int D, int TEAMS>
+__global__ void __launch_bounds__(kTeam * TEAMS, 2 / TEAMS) backward_kernel(
     Problem p, const float* __restrict__ lse2, const float* __restrict__ carry, const float* __restrict__ dbar,
     const float* __restrict__ d_out, float* __restrict__ dq_acc, float* __restrict__ dk_acc,
     float* __restrict__ dq0, float* __restrict__ dk0, T* __restrict__ dv, int nblocks, bool vec) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int P = D + 4, W = kKB + 4, CD = D / 16;
+  constexpr int P = D + 4, W = kKB + 4;
+  const int team = threadIdx.x / kTeam, id = threadIdx.x % kTeam;
   float* ks = smem;                 // [32][P] keys of this head
   float* vs = ks + kKB * P;
   float* k0s = vs + kKB * P;
-  float* qs = k0s + kKB * P;        // [32][P] query tile of this head
+  float* gdz = k0s + kKB * P;       // [2][row groups of all teams][32] dz of a row group, by the parity of the step
+  float* qs = gdz + 2 * TEAMS * kGroups * kKB + team * kBackwardTeamFloats<D>;   // [32][P] query tile of this head, from here on a team's own
   float* q0s = qs + kQ * P;
   float* dos = q0s + kQ * P;
   float* as = dos + kQ * P;         // [32 queries][W] attention
   float* zs = as + kQ * W;          // [32][W] dz; a head that is its own selector: dz + g
   float* gs = zs + kQ * W;          // [32][W] g
-  float* gsel = gs + kQ * W;        // [8][32] selection of a row group, at [group][tx][c]
-  float* gdz = gsel + kGroups * kKB;   // [8][32] dz of a row group
-  float* lse_s = gdz + kGroups * kKB;  // [32]
+  float4* ex = reinterpret_cast<float4*>(gs + kQ * W);   // [3][256]: the products' other half, for the other group
+  float* gsel = gs + kQ * W + 3 * kTeam * 4;             // [8][32] selection of a row group
+  float* lse_s = gsel + kGroups * kKB; // [32]
   float* dbar_s = lse_s + kQ;          // [32]
 
-  const int kb = blockIdx.x;
-  const int n = blockIdx.y;
+  const int heads_all = p.batch * p.heads, kb = (int)blockIdx.x / heads_all, n = (int)blockIdx.x % heads_all;
   const int b = n / p.heads, h = n - b * p.heads;
   const int j0 = kb * kKB;
   const bool self = h == 0 && !p.external_selector;
@@ -400,180 +527,195 @@ __global__ void __launch_bounds__(kThreads) backward_kernel(
   const T* q0 = row_ptr<T>(p.q0, b, 0);
   const float* doh = d_out + (int64_t)n * p.seq * D;
   const bool vec_do = (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
-  load_tile<T, D, kKB>(ks, row_ptr<T>(p.k, b, h), p.k.st, j0, p.seq, vec);
-  load_tile<T, D, kKB>(vs, row_ptr<T>(p.v, b, h), p.v.st, j0, p.seq, vec);
-  if (!self) load_tile<T, D, kKB>(k0s, row_ptr<T>(p.k0, b, 0), p.k0.st, j0, p.seq, vec);
+  load_tile<T, D, kKB, kTeam * TEAMS>(ks, row_ptr<T>(p.k, b, h), p.k.st, j0, p.seq, vec);
+  load_tile<T, D, kKB, kTeam * TEAMS>(vs, row_ptr<T>(p.v, b, h), p.v.st, j0, p.seq, vec);
+  if (!self) load_tile<T, D, kKB, kTeam * TEAMS>(k0s, row_ptr<T>(p.k0, b, 0), p.k0.st, j0, p.seq, vec);
 
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;   // 4 rows 4 ty .. (queries, or keys of the accumulators)
-  float dk_r[kRows][CD] = {}, dv_r[kRows][CD] = {}, dk0_r[kRows][CD] = {};
-  float suffix[2] = {0.f, 0.f};     // sum of dz over queries in later tiles, keys tx and tx + 16
+  // logits: 4 queries 4 ty .. and key col of a thread, of which its group forms half of the contraction
+  const int grp = id >> 7, ty = row_of<16>(id & 127), tx = col_of<16>(id), col = 16 * grp + tx;
+  const int j = j0 + col;
+  // key gradients: D / 4 queries of every tile (`part`), 4 keys 4 ky .. and 4 columns 4 kx ..
+  constexpr int kParts = 128 / D, kPartRows = kQ / kParts;
+  const int part = id / (2 * D), ky = row_of<D / 4>(id % (2 * D)), kx = col_of<D / 4>(id);
+  Cols<4> dk_r[kRows], dv_r[kRows], dk0_r[kRows];
+#pragma unroll
+  for (int u = 0; u < kRows; ++u) dk_r[u].zero(), dv_r[u].zero(), dk0_r[u].zero();
+  float suffix = 0.f;               // sum of dz over queries in later tiles
 
   Tile<T, D, kQ> tq, tq0;
   Tile<float, D, kQ> tdo;
-  float next_lse = 0.f, next_dbar = 0.f, next_hist[2];
+  float next_lse = 0.f, next_dbar = 0.f, next_hist;
   auto fetch = [&](int rb) {
     const int m0 = rb * kQ;
-    tq.fetch(qh, p.q.st, m0, p.seq, vec);
-    if (!self) tq0.fetch(q0, p.q0.st, m0, p.seq, vec);
-    tdo.fetch(doh, D, m0, p.seq, vec_do);
-    if (threadIdx.x < kQ) {
-      const int t = m0 + threadIdx.x;
+    tq.fetch(id, qh, p.q.st, m0, p.seq, vec);
+    if (!self) tq0.fetch(id, q0, p.q0.st, m0, p.seq, vec);
+    tdo.fetch(id, doh, D, m0, p.seq, vec_do);
+    if (id < kQ) {
+      const int t = m0 + id;
       next_lse = (t < p.seq) ? lse2[(int64_t)n * p.seq + t] : 0.f;
       next_dbar = (t < p.seq) ? dbar[(int64_t)n * p.seq + t] : 0.f;
     }
-    const float* carry_row = carry + ((int64_t)b * nblocks + rb) * p.seq;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int j = j0 + tx + 16 * c;
-      next_hist[c] = (j < p.seq && j < m0 + kQ) ? carry_row[j] : 0.f;
-    }
+    next_hist = (j < p.seq && j < m0 + kQ) ? carry[((int64_t)b * nblocks + rb) * p.seq + j] : 0.f;
   };
-  if (kAhead<T, D>) fetch(nblocks - 1);
-  for (int rb = nblocks - 1; rb >= 0 && rb * kQ + kQ > j0; --rb) {
+  // A query tile for each team in a step, last to first: team 0 takes the later one.
+  if (nblocks - 1 - team >= kb) fetch(nblocks - 1 - team);
+  __syncthreads();
+  for (int rb = nblocks - 1 - team, step = 0; rb + team >= kb; rb -= TEAMS, ++step) {
+    if (rb < kb) {                  // an odd number of tiles: team 1 has none in the last step
+      __syncthreads();
+      break;
+    }
     const int m0 = rb * kQ;
-    if (!kAhead<T, D>) fetch(rb);
-    __syncthreads();
-    tq.store(qs);
-    if (!self) tq0.store(q0s);
-    tdo.store(dos);
-    if (threadIdx.x < kQ) {
-      lse_s[threadIdx.x] = next_lse;
-      dbar_s[threadIdx.x] = next_dbar;
+    team_sync(team);
+    tq.store(id, qs);
+    if (!self) tq0.store(id, q0s);
+    tdo.store(id, dos);
+    if (id < kQ) {
+      lse_s[id] = next_lse;
+      dbar_s[id] = next_dbar;
     }
-    const float hist[2] = {next_hist[0], next_hist[1]};
-    __syncthreads();
-    if (kAhead<T, D> && rb > 0 && rb * kQ > j0) fetch(rb - 1);
+    const float hist = next_hist;
+    team_sync(team);
 
-    float aff[kRows][2] = {}, sel[kRows][2] = {}, dov[kRows][2] = {};
-    dot_rows<D, 2>(aff, qs, ks, ty, tx);
-    if (!self) dot_rows<D, 2>(sel, q0s, k0s, ty, tx);
-    dot_rows<D, 2>(dov, dos, vs, ty, tx);
+    float aff[kRows], sel[kRows], dov[kRows];
+    {
+      const int d0 = grp * (D / 2), own = 16 * grp * P + d0, other = 16 * (1 - grp) * P + d0;
+      auto product = [&](float (&mine)[kRows], const float* a, const float* k, float4* to) {
+        float t[kRows][2];
+        dot_rows<D, D / 2, 2>(t, a + d0, k + own, k + other, ty, tx);
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) mine[u] = t[u][0];
+        to[id] = make_float4(t[0][1], t[1][1], t[2][1], t[3][1]);
+      };
+      product(aff, qs, ks, ex);
+      if (!self) product(sel, q0s, k0s, ex + kTeam);
+      product(dov, dos, vs, ex + 2 * kTeam);
+      team_sync(team);
+      auto join = [&](float (&mine)[kRows], const float4* from) {
+        const float4 x = from[id ^ 128];
+        mine[0] += x.x; mine[1] += x.y; mine[2] += x.z; mine[3] += x.w;
+      };
+      join(aff, ex);
+      if (!self) join(sel, ex + kTeam);
+      join(dov, ex + 2 * kTeam);
+    }
     unsigned gates = 0u;
-    float before[2];
+    float sum = 0.f;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int j = j0 + tx + 16 * c;
-      float sum = 0.f;
-#pragma unroll
-      for (int u = 0; u < kRows; ++u) {          // sel becomes the exclusive prefix inside the row group
-        const int i = m0 + ty * kRows + u;
-        const float l0 = (self ? aff[u][c] : sel[u][c]) * p.scale;
-        const bool gate = (j < i) && (j >= p.exempt) && (i < p.seq) && (l0 > 0.f);
-        gates |= (gate ? 1u : 0u) << (u * 2 + c);
-        sel[u][c] = sum;
-        sum += gate ? l0 : 0.f;
-      }
-      before[c] = sum;
+    for (int u = 0; u < kRows; ++u) {            // sel becomes the exclusive prefix inside the row group
+      const int i = m0 + ty * kRows + u;
+      const float l0 = (self ? aff[u] : sel[u]) * p.scale;
+      const bool gate = (j < i) && (j >= p.exempt) && (i < p.seq) && (l0 > 0.f);
+      gates |= (gate ? 1u : 0u) << u;
+      sel[u] = sum;
+      sum += gate ? l0 : 0.f;
     }
-    *reinterpret_cast<float2*>(gsel + ty * kKB + tx * 2) = make_float2(before[0], before[1]);
-    __syncthreads();
-    before[0] = before[1] = 0.f;
-    for (int g = 0; g < ty; ++g) {
-      const float2 x = *reinterpret_cast<const float2*>(gsel + g * kKB + tx * 2);
-      before[0] += x.x; before[1] += x.y;
-    }
-    float dz[kRows][2], dz_sum[2] = {0.f, 0.f};
+    gsel[ty * kKB + col] = sum;
+    group_sync(2 * team + grp);
+    float before = 0.f;
+    for (int g = 0; g < ty; ++g) before += gsel[g * kKB + col];
+    float dz[kRows], dz_sum = 0.f;
 #pragma unroll
     for (int u = 0; u < kRows; ++u) {
       const int r = ty * kRows + u, i = m0 + r;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int j = j0 + tx + 16 * c;
-        const bool causal = (j <= i) && (i < p.seq);
-        float attn = 0.f;
-        dz[u][c] = 0.f;
-        if (causal) {
-          attn = exp2f((aff[u][c] * p.scale - (hist[c] + (before[c] + sel[u][c]))) * kLog2e - lse_s[r]);
-          dz[u][c] = attn * (dov[u][c] - dbar_s[r]);
-        }
-        as[r * W + tx + 16 * c] = attn;
-        dz_sum[c] += dz[u][c];
+      const bool causal = (j <= i) && (i < p.seq);
+      float attn = 0.f;
+      dz[u] = 0.f;
+      if (causal) {
+        attn = exp2f((aff[u] * p.scale - (hist + (before + sel[u]))) * kLog2e - lse_s[r]);
+        dz[u] = attn * (dov[u] - dbar_s[r]);
       }
+      as[r * W + col] = attn;
+      dz_sum += dz[u];
     }
-    *reinterpret_cast<float2*>(gdz + ty * kKB + tx * 2) = make_float2(dz_sum[0], dz_sum[1]);
-    __syncthreads();
-    float later[2] = {suffix[0], suffix[1]};
-    for (int g = kGroups - 1; g >= 0; --g) {
-      const float2 x = *reinterpret_cast<const float2*>(gdz + g * kKB + tx * 2);
-      if (g > ty) { later[0] += x.x; later[1] += x.y; }
-      suffix[0] += x.x; suffix[1] += x.y;
+    const int order = (TEAMS - 1 - team) * kGroups + ty;        // of the step's row groups, first query first
+    float* dz_groups = gdz + (step & 1) * (TEAMS * kGroups * kKB);
+    dz_groups[order * kKB + col] = dz_sum;
+    if constexpr (TEAMS == 1) group_sync(grp); else __syncthreads();
+    float later = suffix;
+    const int first = TEAMS == 2 && rb == kb && team == 0 ? kGroups : 0;      // without a tile of team 1
+#pragma unroll 8
+    for (int g = TEAMS * kGroups - 1; g >= first; --g) {
+      const float x = dz_groups[g * kKB + col];
+      if (g > order) later += x;
+      suffix += x;
     }
 #pragma unroll
     for (int u = kRows - 1; u >= 0; --u) {
       const int r = ty * kRows + u;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const float g = ((gates >> (u * 2 + c)) & 1u) ? -later[c] : 0.f;
-        later[c] += dz[u][c];
-        zs[r * W + tx + 16 * c] = self ? dz[u][c] + g : dz[u][c];
-        if (!self) gs[r * W + tx + 16 * c] = g;
-      }
+      const float g = ((gates >> u) & 1u) ? -later : 0.f;
+      later += dz[u];
+      zs[r * W + col] = self ? dz[u] + g : dz[u];
+      if (!self) gs[r * W + col] = g;
     }
-    __syncthreads();
+    team_sync(team);
+    if (rb - TEAMS >= kb) fetch(rb - TEAMS);            // covered by the products below
 
     // key rows: dV += A^T dO, dK += Z^T Q, dK0 += G^T Q0
-#pragma unroll 2
-    for (int r = 0; r < kQ; ++r) {
-      const float4 a = ld4(as + r * W + ty * kRows), z = ld4(zs + r * W + ty * kRows);
-      const float av[kRows] = {a.x, a.y, a.z, a.w}, zv[kRows] = {z.x, z.y, z.z, z.w};
-      float y[CD];
-      load_cols<CD>(dos + r * P, tx, y);
-#pragma unroll
-      for (int u = 0; u < kRows; ++u)
-#pragma unroll
-        for (int c = 0; c < CD; ++c) dv_r[u][c] = fmaf(av[u], y[c], dv_r[u][c]);
-      load_cols<CD>(qs + r * P, tx, y);
-#pragma unroll
-      for (int u = 0; u < kRows; ++u)
-#pragma unroll
-        for (int c = 0; c < CD; ++c) dk_r[u][c] = fmaf(zv[u], y[c], dk_r[u][c]);
-      if (!self) {
-        const float4 g = ld4(gs + r * W + ty * kRows);
-        const float gv[kRows] = {g.x, g.y, g.z, g.w};
-        load_cols<CD>(q0s + r * P, tx, y);
-#pragma unroll
-        for (int u = 0; u < kRows; ++u)
-#pragma unroll
-          for (int c = 0; c < CD; ++c) dk0_r[u][c] = fmaf(gv[u], y[c], dk0_r[u][c]);
-      }
+    auto key_grads = [&](Cols<4> (&acc)[kRows], const float* w, const float* rows, int r) {
+      const float4 a = ld4(w + r * W + ky * kRows);
+      Cols<4> y;
+      y.load(rows + r * P, kx);
+      acc[0].add(pack2(a.x, a.x), y);
+      acc[1].add(pack2(a.y, a.y), y);
+      acc[2].add(pack2(a.z, a.z), y);
+      acc[3].add(pack2(a.w, a.w), y);
+    };
+#pragma unroll 4
+    for (int r = part * kPartRows; r < (part + 1) * kPartRows; ++r) {
+      key_grads(dv_r, as, dos, r);
+      key_grads(dk_r, zs, qs, r);
+      if (!self) key_grads(dk0_r, gs, q0s, r);
     }
     // query rows: dQ += Z K, dQ0 += G K0, reduced across the key blocks in global memory
-    {
-      float x[kRows][CD] = {};
-      weighted_rows<D, kKB, W, CD>(x, zs, ks, ty, tx);
-#pragma unroll
-      for (int u = 0; u < kRows; ++u)
-        if (m0 + ty * kRows + u < p.seq) reduce_cols<CD>(dq_acc + ((int64_t)n * p.seq + m0 + ty * kRows + u) * D, tx, x[u], p.scale);
-    }
-    if (!self) {
-      float x[kRows][CD] = {};
-      weighted_rows<D, kKB, W, CD>(x, gs, k0s, ty, tx);
-#pragma unroll
-      for (int u = 0; u < kRows; ++u)
-        if (m0 + ty * kRows + u < p.seq) reduce_cols<CD>(dq0 + ((int64_t)b * p.seq + m0 + ty * kRows + u) * D, tx, x[u], p.scale);
+    float* dq_tile = dq_acc + ((int64_t)n * p.seq + m0) * D;
+    float* dq0_tile = dq0 + ((int64_t)b * p.seq + m0) * D;
+    if (self) {
+      query_grads<D, (D >= 64 ? D / 32 : 1)>(zs, ks, dq_tile, p.seq - m0, p.scale, id);
+    } else if constexpr (D == 128) {
+      query_grads<D, 4>(zs, ks, dq_tile, p.seq - m0, p.scale, id);
+      query_grads<D, 4>(gs, k0s, dq0_tile, p.seq - m0, p.scale, id);
+    } else {                                    // one product a group
+      query_grads<D, D / 16>(grp ? gs : zs, grp ? k0s : ks, grp ? dq0_tile : dq_tile, p.seq - m0, p.scale, id & 127);
     }
   }
+  // the parts' sums of a key row, over the tiles' place in shared memory: [parts of all teams][32][D]
+  auto finish = [&](const Cols<4> (&acc)[kRows], auto&& out) {
+    __syncthreads();
 #pragma unroll
-  for (int u = 0; u < kRows; ++u) {
-    const int j = j0 + ty * kRows + u;
-    if (j >= p.seq) continue;
-    float* dk_row = dk_acc + ((int64_t)n * p.seq + j) * D;
-    T* dv_row = dv + ((int64_t)n * p.seq + j) * D;
+    for (int u = 0; u < kRows; ++u)
+      *reinterpret_cast<float4*>(smem + ((team * kParts + part) * kKB + ky * kRows + u) * D + 4 * kx) =
+          make_float4(acc[u].get(0), acc[u].get(1), acc[u].get(2), acc[u].get(3));
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < kKB * D / 4; idx += kTeam * TEAMS) {
+      const int r = idx / (D / 4), c = idx % (D / 4) * 4;
+      if (j0 + r >= p.seq) break;
+      float4 x = ld4(smem + r * D + c);
 #pragma unroll
-    for (int c = 0; c < CD; ++c) {
-      dk_row[col_of<CD>(tx, c)] = dk_r[u][c] * p.scale;
-      dv_row[col_of<CD>(tx, c)] = from_float<T>(dv_r[u][c]);
+      for (int k = 1; k < TEAMS * kParts; ++k) {
+        const float4 y = ld4(smem + (k * kKB + r) * D + c);
+        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+      }
+      out(j0 + r, c, x);
     }
-    if (!self) reduce_cols<CD>(dk0 + ((int64_t)b * p.seq + j) * D, tx, dk0_r[u], p.scale);
-  }
+  };
+  auto scaled = [&](float4 x) { return make_float4(x.x * p.scale, x.y * p.scale, x.z * p.scale, x.w * p.scale); };
+  finish(dk_r, [&](int t, int c, float4 x) {
+    const float4 y = scaled(x);
+    float* dst = dk_acc + ((int64_t)n * p.seq + t) * D + c;
+    dst[0] = y.x; dst[1] = y.y; dst[2] = y.z; dst[3] = y.w;
+  });
+  finish(dv_r, [&](int t, int c, float4 x) {
+    T* dst = dv + ((int64_t)n * p.seq + t) * D + c;
+    dst[0] = from_float<T>(x.x); dst[1] = from_float<T>(x.y); dst[2] = from_float<T>(x.z); dst[3] = from_float<T>(x.w);
+  });
+  if (!self) finish(dk0_r, [&](int t, int c, float4 x) { reduce4(dk0 + ((int64_t)b * p.seq + t) * D + c, scaled(x)); });
 }
 
 template <int D> constexpr size_t colsum_smem() { return sizeof(float) * ((kKF + kQ) * (D + 4) + kGroups * kKF); }
-template <int D> constexpr size_t forward_smem() {
-  return sizeof(float) * ((2 * kQ + 3 * kKF) * (D + 4) + kQ * (kKF + 4) + kGroups * kKF);
-}
-template <int D> constexpr size_t backward_smem() {
-  return sizeof(float) * ((3 * kKB + 3 * kQ) * (D + 4) + 3 * kQ * (kKB + 4) + 2 * kGroups * kKB + 2 * kQ);
+template <int D, int TEAMS> constexpr size_t forward_smem() { return sizeof(float) * (2 * kQ * (D + 4) + TEAMS * kForwardTeamFloats<D>); }
+template <int D, int TEAMS> constexpr size_t backward_smem() {
+  return sizeof(float) * (3 * kKB * (D + 4) + TEAMS * (2 * kGroups * kKB + kBackwardTeamFloats<D>));
 }
 
 // Four consecutive elements of every row start at a 16-byte (fp32) or 8-byte boundary.
@@ -591,7 +733,7 @@ int carry_impl(const Problem& p, float* carry, float* total, cudaStream_t s) {
   const int nb = (p.seq + kQ - 1) / kQ;
   SA_CUDA_CHECK(allow_smem(colsum_kernel<T, D>, colsum_smem<D>()));
   count_launch();
-  colsum_kernel<T, D><<<dim3((p.seq + kKF - 1) / kKF, nb, p.batch), kThreads, colsum_smem<D>(), s>>>(p, carry, nb, vector_rows(p));
+  colsum_kernel<T, D><<<dim3((p.seq + kKF - 1) / kKF, nb, p.batch), kSelThreads, colsum_smem<D>(), s>>>(p, carry, nb, vector_rows(p));
   SA_CUDA_CHECK(cudaGetLastError());
   count_launch();
   scan_kernel<<<dim3((p.seq + 127) / 128, p.batch), 128, 0, s>>>(carry, total, p.seq, nb);
@@ -599,27 +741,52 @@ int carry_impl(const Problem& p, float* carry, float* total, cudaStream_t s) {
   return SA_OK;
 }
 
+template <typename T, int D, int TEAMS>
+int launch_forward(const Problem& p, const float* carry, float* out, float* lse2, cudaStream_t s) {
+  const int nb = (p.seq + kQ - 1) / kQ;
+  constexpr size_t smem = forward_smem<D, TEAMS>();
+  SA_CUDA_CHECK(allow_smem(forward_kernel<T, D, TEAMS>, smem));
+  count_launch();
+  forward_kernel<T, D, TEAMS><<<(unsigned)nb * (unsigned)(p.batch * p.heads), kTeam * TEAMS, smem, s>>>(p, carry, out, lse2, nb, vector_rows(p));
+  SA_CUDA_CHECK(cudaGetLastError());
+  return SA_OK;
+}
+
+template <typename T, int D, int TEAMS>
+int launch_backward(const Problem& p, const float* lse2, const float* carry, const float* dbar, const float* d_out,
+                    float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
+  const int nb = (p.seq + kQ - 1) / kQ;
+  constexpr size_t smem = backward_smem<D, TEAMS>();
+  SA_CUDA_CHECK(allow_smem(backward_kernel<T, D, TEAMS>, smem));
+  count_launch();
+  backward_kernel<T, D, TEAMS><<<(unsigned)nb * (unsigned)(p.batch * p.heads), kTeam * TEAMS, smem, s>>>(
+      p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, static_cast<T*>(dv), nb, vector_rows(p));
+  SA_CUDA_CHECK(cudaGetLastError());
+  return SA_OK;
+}
+
+// Two teams a CTA and one CTA an SM where one-team CTAs, two an SM, would all be resident at once: the hardware then pairs them
+// as it likes, and the fullest SM had twice the mean.  (B, H, T, D) = (2, 4, 1024, 64) takes 76 + 160 us with two teams, 110 +
+// 235 us with one.  With more CTAs than that the SMs that finish early take the rest, and teams without a common barrier are
+// the faster ones: 292 + 540 against 328 + 588 us at (4, 8, 1000, 64), 192 + 345 against 209 + 363 us at (1, 12, 1280, 64).
+inline bool two_teams(const Problem& p) {
+  return (int64_t)p.batch * p.heads * ((p.seq + kQ - 1) / kQ) <= 2 * 148;
+}
+
 template <typename T, int D>
 int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float* total, cudaStream_t s) {
   if (int st = carry_impl<T, D>(p, carry, total, s)) return st;
-  const int nb = (p.seq + kQ - 1) / kQ;
-  SA_CUDA_CHECK(allow_smem(forward_kernel<T, D>, forward_smem<D>()));
-  count_launch();
-  forward_kernel<T, D><<<dim3(nb, p.batch * p.heads), kThreads, forward_smem<D>(), s>>>(p, carry, out, lse2, nb, vector_rows(p));
-  SA_CUDA_CHECK(cudaGetLastError());
-  return SA_OK;
+  if constexpr (D < 128)                     // a second team's tiles do not fit at D = 128
+    if (two_teams(p)) return launch_forward<T, D, 2>(p, carry, out, lse2, s);
+  return launch_forward<T, D, 1>(p, carry, out, lse2, s);
 }
 
 template <typename T, int D>
 int backward_impl(const Problem& p, const float* lse2, const float* carry, const float* dbar, const float* d_out,
                   float* dq_acc, float* dk_acc, float* dq0, float* dk0, void* dv, cudaStream_t s) {
-  const int nb = (p.seq + kQ - 1) / kQ;
-  SA_CUDA_CHECK(allow_smem(backward_kernel<T, D>, backward_smem<D>()));
-  count_launch();
-  backward_kernel<T, D><<<dim3((p.seq + kKB - 1) / kKB, p.batch * p.heads), kThreads, backward_smem<D>(), s>>>(
-      p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, static_cast<T*>(dv), nb, vector_rows(p));
-  SA_CUDA_CHECK(cudaGetLastError());
-  return SA_OK;
+  if constexpr (D < 128)                     // two CTAs do not fit on an SM at D = 128
+    if (!two_teams(p)) return launch_backward<T, D, 1>(p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, dv, s);
+  return launch_backward<T, D, 2>(p, lse2, carry, dbar, d_out, dq_acc, dk_acc, dq0, dk0, dv, s);
 }
 
 template <typename T>

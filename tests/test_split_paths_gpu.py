@@ -1,5 +1,6 @@
 """The forward variants that only larger grids reach (two heads of a selector, or two rows that each select for
-themselves, in one CTA), second differentiation, and the newest key of a decode step."""
+themselves, in one CTA), second differentiation, the newest key of a decode step, and
+the exact-product engine with one and two teams a CTA."""
 
 import pytest
 import torch
@@ -91,3 +92,19 @@ def test_the_newest_key_at_the_edges_of_a_decode_range(dtype, dim, norms, start)
     assert torch.equal(dev["k"].cpu(), k) and torch.equal(dev["v"].cpu(), v)
     if norms:
         torch.testing.assert_close(dev["key_norms"].cpu(), k.float().norm(dim=-1), rtol=1e-5, atol=1e-5)
+
+
+# up to 296 (32-token block, head) pairs a CTA has two teams, and the last step of an odd number of blocks only one of them
+@pytest.mark.parametrize("dim,dtype", [(16, torch.float32), (32, torch.float16), (64, torch.float32), (128, torch.float32)])
+@pytest.mark.parametrize("batch,heads,seq,exempt", [(1, 2, 1, 1), (2, 3, 33, 1), (1, 2, 64, 5), (2, 2, 65, 1), (1, 3, 161, 40),
+                                                    (50, 3, 33, 1), (60, 2, 97, 3)])
+def test_exact_products_with_one_and_two_teams(dim, dtype, batch, heads, seq, exempt):
+    g = torch.Generator("cpu").manual_seed(seq + dim)
+    q, k, v, w = ((s * torch.randn(batch, heads, seq, dim, generator=g)).to(dtype) for s in (0.5, 0.5, 1.0, 1.0))
+    want = oracle.attention_grads(q.float(), k.float(), v.float(), w.float(), exempt)
+    qq, kk, vv = (x.cuda().requires_grad_(True) for x in (q, k, v))
+    out = kernels.selective_attention(qq, kk, vv, exempt=exempt, dot_precision="ieee")
+    grads = torch.autograd.grad(out, (qq, kk, vv), w.cuda().float())
+    tol = 1e-5 if dtype == torch.float32 else 2e-3
+    for got, ref in zip((out.detach(), *grads), want):
+        torch.testing.assert_close(got.float().cpu(), ref, atol=tol * float(ref.abs().max()) + 1e-6, rtol=tol)
