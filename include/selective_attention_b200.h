@@ -325,10 +325,12 @@ int sa_decode_run(const sa_decode* d);
 /* A prompt, or a further chunk of one, for a decode cache (tensor-core engine; replaces mixers.py:105-113 around the
  * kernels).  p->seq counts the cached tokens and the new ones; q holds the queries from position `cached` on, k and v all
  * p->seq keys.  `selected` (batch, >= p->seq at selected_stride) is read where cached > 0 and receives the totals in place; y
- * receives the new rows in the operand type.  carry, lse2 and the table (may be NULL) are scratch. */
+ * receives the new rows in the operand type.  carry, lse2, the table (may be NULL) and `scratch` are scratch; with
+ * sa_prefill_scratch_bytes (0: not needed) of the last, a few rows after many keys are spread over the whole GPU (may be NULL). */
+size_t sa_prefill_scratch_bytes(const sa_problem* p, int cached);
 int sa_prefill_rows(const sa_problem* p, int cached, const void* q, const void* k, const void* v, float* selected,
                     int64_t selected_stride, const sa_tensor* y, float* lse2, float* carry, void* tile_table,
-                    size_t tile_table_bytes, void* stream);
+                    size_t tile_table_bytes, void* scratch, size_t scratch_bytes, void* stream);
 /* Stores `seq` new keys and values, rows of head_dim elements at the strides of k and v (batch, head, token), into the
  * (batch, heads, capacity, head_dim) caches from position `at` on.  With `begin` also zeros every row behind them and, where
  * given, the history sums `selected` (batch, groups, capacity) from at + seq on. */

@@ -78,6 +78,7 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   p->carry_init_stride = 0;
   p->total_stride = in->seq;
   p->tile_table = nullptr;
+  p->split_scratch = nullptr;
   p->out_lowp = nullptr;
   p->out_lowp_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
   p->dv_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
@@ -556,9 +557,17 @@ int sa_decode_run(const sa_decode* d) {
   return decode_step(step, static_cast<cudaStream_t>(d->stream));
 }
 
+size_t sa_prefill_scratch_bytes(const sa_problem* in, int cached) {
+  Problem p;
+  if (to_problem(in, nullptr, nullptr, nullptr, nullptr, &p) != SA_OK || in->engine != SA_ENGINE_TCGEN05) return 0;
+  if (cached < 0 || cached >= in->seq) return 0;
+  p.q_offset = cached;
+  return tc::prefill_split_floats(p) * 4;
+}
+
 int sa_prefill_rows(const sa_problem* in, int cached, const void* q, const void* k, const void* v, float* selected,
                     int64_t selected_stride, const sa_tensor* y, float* lse2, float* carry, void* tile_table,
-                    size_t tile_table_bytes, void* stream) {
+                    size_t tile_table_bytes, void* scratch, size_t scratch_bytes, void* stream) {
   Problem p;
   int st = to_problem(in, q, k, v, nullptr, &p);
   if (st != SA_OK) return st;
@@ -581,6 +590,11 @@ int sa_prefill_rows(const sa_problem* in, int cached, const void* q, const void*
   p.carry_init = cached > 0 ? selected : nullptr;
   p.carry_init_stride = selected_stride;
   p.total_stride = selected_stride;
+  if (scratch != nullptr) {
+    if (scratch_bytes < tc::prefill_split_floats(p) * 4) return SA_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return SA_ERR_ALIGNMENT;
+    p.split_scratch = static_cast<float*>(scratch);
+  }
   return tc_forward(p, nullptr, lse2, carry, selected, static_cast<cudaStream_t>(stream));
 }
 

@@ -69,6 +69,7 @@ struct Problem {
   // Tensor-core engine, optional: the table of live (query tile, key tile) pairs (sa_tc_skip.cu).  The forward
   // fills it after its selection pass and leaves out the dead tiles; the backward of the same call reads it.
   void* tile_table;      // null: every causal tile is computed
+  float* split_scratch;  // null: a query tile's keys are one walk (else prefill_split_pieces of them)
 };
 
 // ---- engine entry points (host) -------------------------------------------------------------------
@@ -81,6 +82,12 @@ int simt_backward(const Problem& p, const float* lse2, const float* carry, const
 namespace tc {
 size_t tile_table_bytes(const Problem& p);                                     // 0: not offered for this problem
 int build_tile_table(const Problem& p, const float* carry, cudaStream_t s);
+int prefill_split_pieces(const Problem& p);                                     // 1: not split
+constexpr int kSplitTickets = 128;                                             // no split has more walks (half the SMs)
+inline size_t prefill_split_floats(const Problem& p) {
+  const int pieces = prefill_split_pieces(p);
+  return pieces > 1 ? kSplitTickets + (size_t)pieces * p.batch * p.heads * (p.seq - p.q_offset) * (p.head_dim + 1) : 0;
+}
 }  // namespace tc
 
 int tc_available();

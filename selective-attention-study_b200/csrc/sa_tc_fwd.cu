@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(kColsumThreads) colsum_kernel(const __grid_con
 // and total[b][j] receive the sum over all query tiles.  Only rows mi >= j / 128 exist.
 __global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, float* total, int64_t total_stride, int seq,
                                                    int ntiles, int mi_first, const float* init,
-                                                   int64_t init_stride) {
+                                                   int64_t init_stride, unsigned int* tickets, int n_tickets) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && (int)threadIdx.x < n_tickets) tickets[threadIdx.x] = 0u;   // of a split forward
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (j >= seq) return;
@@ -224,6 +225,14 @@ constexpr int kWideCompute = 512;                      // four warpgroups: 32 of
 constexpr int kWideThreads = kWideCompute + 32;        // + the control warp: one lane issues every TMA load and MMA
 constexpr int kWideBarrier = 1;                        // hardware barrier id of the arithmetic warps
 
+// With pieces > 1 a CTA walks one piece of its query tile's key tiles (nothing goes from key tile to key tile but the softmax
+// state: the history at the query tile is given) and leaves its rows, normalised, and their lse2 in [piece][batch * heads].
+struct SplitWalk {
+  int pieces;
+  unsigned int* tickets;       // one per (query tile, row), zero
+  float *part, *lse;
+};
+
 template <int D, bool SELF, bool LIVE>   // LIVE: a table of live key tiles is given and the dead ones are left out
 __global__ void __launch_bounds__(kWideThreads, 1)
     forward_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -231,7 +240,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                         const __grid_constant__ CUtensorMap map_k0, const float* __restrict__ carry,
                         float* __restrict__ out, float* __restrict__ lse2, int heads, int seq, int ntiles, int exempt,
                         float scale, WaitCtx status, __nv_bfloat16* __restrict__ out_lowp, RowLayout out_lowp_rows,
-                        int q_offset, const uint8_t* __restrict__ alive) {
+                        int q_offset, const uint8_t* __restrict__ alive, SplitWalk split) {
   using L = WideSmem<D>;
   constexpr int DK = D / 64, DH = D / 4, NC = 32, ST = L::kStages;
   // TMEM columns: S and L0 (fp32, 128 each), the output accumulator (D), Q and Q0 as bf16 pairs (D / 2 each)
@@ -241,11 +250,15 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   constexpr bool kTmemAB = (D == 64);
   constexpr uint32_t kColTri = 384, kColP = 448;
 
-  const int nrows = gridDim.x / (ntiles - q_offset / kTile);  // batch * heads (the grid covers the query tiles with rows to compute)
-  const int mi = ntiles - 1 - (int)(blockIdx.x / nrows);      // heaviest query tiles first
-  const int n = blockIdx.x % nrows;
+  const int piece = (int)blockIdx.x % split.pieces, cta = (int)blockIdx.x / split.pieces;
+  const int nrows = gridDim.x / split.pieces / (ntiles - q_offset / kTile);  // batch * heads (the grid covers the query tiles with rows to compute)
+  const int mi = ntiles - 1 - cta / nrows;                    // heaviest query tiles first
+  const int n = cta % nrows;
   const int b = n / heads, h = n - b * heads;
   const int i0 = mi * kTile;
+  // this piece's key tiles: last, last - 1, .. lowest (the last pieces may have none)
+  const int piece_tiles = (mi + split.pieces) / split.pieces;
+  const int last = mi - piece * piece_tiles, lowest = max(0, last - piece_tiles + 1);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -258,14 +271,15 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   __shared__ float rmax_s[4][kTile];
   __shared__ uint16_t live_s[kMaxLiveTiles + 1];              // with a table of live tiles: this query tile's key tiles,
   __shared__ int live_count_s;                                //   nearest first
+  __shared__ bool last_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (LIVE && warp == 1) {
     const uint8_t* live_row = alive + ((int64_t)n * ntiles + mi) * ntiles;
     int cnt = 0;
-    for (int base = mi; base >= 0; base -= 32) {
+    for (int base = last; base >= lowest; base -= 32) {
       const int nj = base - lane;
-      const bool f = nj >= 0 && live_row[nj] != 0;
+      const bool f = nj >= lowest && live_row[nj] != 0;
       const unsigned m = __ballot_sync(0xffffffffu, f);
       if (f) live_s[cnt + __popc(m & ((1u << lane) - 1u))] = (uint16_t)nj;
       cnt += __popc(m);
@@ -296,10 +310,14 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   const uint32_t sa = smem_u32(smem);
   // 128-key steps: every key tile up to and including the diagonal one, or the live ones only.  Step index `it`
   // counts from the diagonal (it = 0) back towards key 0; key_tile(it) is the tile it covers.
-  const int steps = LIVE ? live_count_s : mi + 1;
-  auto key_tile = [&](int it) { return LIVE ? (it < steps ? (int)live_s[it] : 0) : steps - 1 - it; };
+  const int steps = LIVE ? live_count_s : last - lowest + 1;
+  auto key_tile = [&](int it) { return LIVE ? (it < steps ? (int)live_s[it] : 0) : last - it; };
+  const int q_rows = seq - q_offset;
 
-  if (warp == kWideCompute / 32) {
+  if (steps <= 0) {                                            // a piece without keys
+    if (tid < kTile && i0 + tid < seq && i0 + tid >= q_offset)
+      split.lse[((int64_t)piece * nrows + n) * q_rows + i0 + tid - q_offset] = -INFINITY;
+  } else if (warp == kWideCompute / 32) {
     // =============================== control warp: TMA loads and MMA issue ===============================
     if (lane == 0) {
       // A tile of step it lives in stage slot(it); the j-th fill of a stage completes its barrier's phase j.
@@ -608,16 +626,18 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     tmem_ld_wait();
     if (i < seq && i >= q_offset) {                            // rows before q_offset belong to an earlier call
       const int iq = i - q_offset;                             // row inside the query tensor
-      const int q_rows = seq - q_offset;
-      if (out != nullptr) {
-        float4* orow = reinterpret_cast<float4*>(out + ((int64_t)n * q_rows + iq) * D + wg * DH);
+      const bool whole = split.pieces == 1;
+      const int64_t nr = ((int64_t)piece * nrows + n) * q_rows + iq;
+      float* rows_to = whole ? out : split.part;
+      if (rows_to != nullptr) {
+        float4* orow = reinterpret_cast<float4*>(rows_to + nr * D + wg * DH);
 #pragma unroll
         for (int d = 0; d < DH; d += 4)
           orow[d >> 2] = make_float4(__uint_as_float(r[d]) * inv, __uint_as_float(r[d + 1]) * inv,
                                      __uint_as_float(r[d + 2]) * inv, __uint_as_float(r[d + 3]) * inv);
       }
-      if (wg == 0) lse2[(int64_t)n * q_rows + iq] = run_max + log2f(den);
-      if (out_lowp != nullptr) {                               // the same rows in the operand dtype, in the caller's layout
+      if (wg == 0) (whole ? lse2 : split.lse)[nr] = run_max + log2f(den);
+      if (whole && out_lowp != nullptr) {                               // the same rows in the operand dtype, in the caller's layout
         uint4* lrow = reinterpret_cast<uint4*>(out_lowp + out_lowp_rows.at(b, h, iq) + wg * DH);
 #pragma unroll
         for (int d = 0; d < DH; d += 8)
@@ -628,9 +648,47 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       }
     }
   }
+  if (split.pieces > 1) __threadfence();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
+  if (split.pieces == 1) return;
+  // The CTA that finishes last merges the pieces of its 128 rows, D / 8 threads a row.
+  if (tid == 0) last_s = atomicAdd(split.tickets + cta, 1u) == (unsigned)split.pieces - 1;
+  __syncthreads();
+  if (!last_s || tid >= kWideCompute) return;
+  __threadfence();
+  constexpr int kLanes = D / 8;
+  const int64_t stride = (int64_t)nrows * q_rows;              // rows of a piece
+  for (int r = tid / kLanes; r < kTile; r += kWideCompute / kLanes) {
+    const int iq = i0 + r - q_offset, d = tid % kLanes * 8;
+    if (iq < 0 || iq >= q_rows) continue;
+    const int64_t at = (int64_t)n * q_rows + iq;
+    float top = -INFINITY;
+    for (int s2 = 0; s2 < split.pieces; ++s2) top = fmaxf(top, __ldcg(split.lse + s2 * stride + at));
+    float acc[8] = {}, den = 0.f;
+    for (int s2 = 0; s2 < split.pieces; ++s2) {
+      const float l = __ldcg(split.lse + s2 * stride + at);
+      if (l == -INFINITY) continue;                            // no keys, and no rows written
+      const float w = ex2(l - top);
+      const float4* src = reinterpret_cast<const float4*>(split.part + (s2 * stride + at) * D + d);
+      const float4 x = __ldcg(src), y = __ldcg(src + 1);
+      den += w;
+      acc[0] = fmaf(w, x.x, acc[0]); acc[1] = fmaf(w, x.y, acc[1]); acc[2] = fmaf(w, x.z, acc[2]); acc[3] = fmaf(w, x.w, acc[3]);
+      acc[4] = fmaf(w, y.x, acc[4]); acc[5] = fmaf(w, y.y, acc[5]); acc[6] = fmaf(w, y.z, acc[6]); acc[7] = fmaf(w, y.w, acc[7]);
+    }
+    const float inv = 1.f / den;
+    if (d == 0) lse2[at] = top + log2f(den);
+    if (out != nullptr) {
+      float4* dst = reinterpret_cast<float4*>(out + at * D + d);
+      dst[0] = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+      dst[1] = make_float4(acc[4] * inv, acc[5] * inv, acc[6] * inv, acc[7] * inv);
+    }
+    if (out_lowp != nullptr)
+      *reinterpret_cast<uint4*>(out_lowp + out_lowp_rows.at(b, h, iq) + d) =
+          make_uint4(pack_bf16(acc[0] * inv, acc[1] * inv), pack_bf16(acc[2] * inv, acc[3] * inv),
+                     pack_bf16(acc[4] * inv, acc[5] * inv), pack_bf16(acc[6] * inv, acc[7] * inv));
+  }
 }
 
 template <int D>
@@ -668,11 +726,20 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
                                                              p.q_offset, mi_first, chunk);
   }
   SA_CUDA_CHECK(cudaGetLastError());
+  const int pieces = p.split_scratch != nullptr ? prefill_split_pieces(p) : 1;
+  const int64_t rows = (int64_t)p.batch * p.heads * q_rows;
+  SplitWalk split{pieces, nullptr, nullptr, nullptr};
+  if (pieces > 1) {
+    split.tickets = reinterpret_cast<unsigned int*>(p.split_scratch);
+    split.part = p.split_scratch + kSplitTickets;
+    split.lse = split.part + pieces * rows * D;
+  }
   dim3 gs((p.seq + 255) / 256, p.batch);
   {
     ProfileScope prof(SA_KERNEL_TC_SCAN, s);
     count_launch();
-    scan_kernel<<<gs, 256, 0, s>>>(carry, total, p.total_stride, p.seq, ntiles, mi_first, p.carry_init, p.carry_init_stride);
+    scan_kernel<<<gs, 256, 0, s>>>(carry, total, p.total_stride, p.seq, ntiles, mi_first, p.carry_init, p.carry_init_stride,
+                                    split.tickets, pieces > 1 ? kSplitTickets : 0);
   }
   SA_CUDA_CHECK(cudaGetLastError());
 
@@ -688,15 +755,16 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   const int64_t ctas = (int64_t)(ntiles - mi_first) * p.batch * p.heads;
   if (D == 64 && !self && p.heads % 2 == 0 && ctas > kSms) return forward_pair(p, m, carry, out, lse2, status, alive, s);
   if (D == 64 && self && p.batch % 2 == 0 && ctas > kSms) return forward_self(p, m, carry, out, lse2, status, alive, s);
-  const unsigned grid = (unsigned)(ntiles - mi_first) * p.batch * p.heads;
+  const unsigned grid = (unsigned)(ntiles - mi_first) * p.batch * p.heads * pieces;
   const int wide_smem = WideSmem<D>::total + 1024;
   auto launch = [&](auto kernel) -> int {
     SA_CUDA_CHECK(allow_smem(kernel, wide_smem));
     ProfileScope prof(SA_KERNEL_TC_FORWARD, s);
     count_launch();
     kernel<<<grid, kWideThreads, wide_smem, s>>>(m.q, m.k, m.v, m.q0, m.k0, carry, out, lse2, p.heads, p.seq,
-                                                 ntiles, p.exempt, p.scale, status, static_cast<__nv_bfloat16*>(p.out_lowp),
-                                                 p.out_lowp_rows, p.q_offset, alive);
+                                                 ntiles, p.exempt, p.scale, status,
+                                                 static_cast<__nv_bfloat16*>(p.out_lowp), p.out_lowp_rows,
+                                                 p.q_offset, alive, split);
     return SA_OK;
   };
   if (alive != nullptr) st = self ? launch(forward_wide_kernel<D, true, true>) : launch(forward_wide_kernel<D, false, true>);
@@ -707,6 +775,17 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
 }
 
 }  // namespace
+
+// A short chunk after a long cache has few (query tile, head) pairs, each with a long walk: where half of the SMs or more would
+// have nothing to do, a walk is cut into as many pieces as give each its SM, of at least 4 steps of 128 keys (a piece pays a
+// set-up of about two, and the last one reads all of them).  A prompt is not cut: its rows do not depend on what follows them.
+int prefill_split_pieces(const Problem& p) {
+  if (p.q_offset == 0) return 1;
+  const int ntiles = (p.seq + kTile - 1) / kTile;
+  const int64_t ctas = (int64_t)(ntiles - p.q_offset / kTile) * p.batch * p.heads;
+  const int64_t pieces = ctas > 0 ? kSms / ctas : 1;
+  return (int)(pieces < ntiles / 4 ? (pieces > 1 ? pieces : 1) : (ntiles / 4 > 1 ? ntiles / 4 : 1));
+}
 
 int forward(const Problem& p, float* out, float* lse2, float* carry, float* total, cudaStream_t s) {
   if (p.head_dim == 64) return forward_impl<64>(p, out, lse2, carry, total, s);

@@ -266,7 +266,8 @@ Tensor prefill_rows(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, 
   const size_t lse = round_up((size_t)b * h * tn * 4);
   const size_t carry = round_up((size_t)p.batch * sa_carry_checkpoints(p.engine, p.seq) * p.seq * 4);
   const size_t table = skip ? sa_tile_table_bytes(&p) : 0;
-  const Tensor scratch = bytes_on(q, lse + carry + table);
+  const size_t split = sa_prefill_scratch_bytes(&p, (int)cached), table_room = round_up(table);
+  const Tensor scratch = bytes_on(q, lse + carry + table_room + split);
   char* s = static_cast<char*>(scratch.data_ptr());
   sa_tensor rows{};
   rows.ptr = y.data_ptr();
@@ -275,7 +276,7 @@ Tensor prefill_rows(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, 
   check("sa_prefill_rows",
         sa_prefill_rows(&p, (int)cached, q.data_ptr(), k.data_ptr(), v.data_ptr(), selected.data_ptr<float>(), selected.size(2), &rows,
                         reinterpret_cast<float*>(s), reinterpret_cast<float*>(s + lse), table ? s + lse + carry : nullptr, table,
-                        stream_of(q)));
+                        split ? s + lse + carry + table_room : nullptr, split, stream_of(q)));
   return y;
 }
 

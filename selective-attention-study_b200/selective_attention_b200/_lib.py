@@ -25,7 +25,7 @@ EXPORTS = ("sa_abi_version", "sa_status_string", "sa_last_cuda_error", "sa_engin
            "sa_profile_collect", "sa_static_scratch_floats", "sa_forward_static_scratch", "sa_forward_selector",
            "sa_backward_selector", "sa_forward_fused", "sa_backward_fused", "sa_prefill_extend", "sa_selection_carry", "sa_launch_count", "sa_selftest_wait_timeout",
            "sa_tile_table_bytes", "sa_forward_live_tiles", "sa_backward_live_tiles", "sa_prefill_extend_live_tiles", "sa_decode_step_live_keys",
-           "sa_decode_run", "sa_prefill_rows", "sa_cache_store")
+           "sa_decode_run", "sa_prefill_scratch_bytes", "sa_prefill_rows", "sa_cache_store")
 
 
 class Problem(ctypes.Structure):
@@ -143,8 +143,10 @@ def load() -> ctypes.CDLL:
     lib.sa_decode_step_live_keys.argtypes = [i32] * 8 + [vp] * 9 + [sz, vp]
     lib.sa_decode_run.restype = i32
     lib.sa_decode_run.argtypes = [vp]
+    lib.sa_prefill_scratch_bytes.restype = sz
+    lib.sa_prefill_scratch_bytes.argtypes = [pp, i32]
     lib.sa_prefill_rows.restype = i32
-    lib.sa_prefill_rows.argtypes = [pp, i32, vp, vp, vp, f32p, ctypes.c_int64, tp, f32p, f32p, vp, sz, vp]
+    lib.sa_prefill_rows.argtypes = [pp, i32, vp, vp, vp, f32p, ctypes.c_int64, tp, f32p, f32p, vp, sz, vp, sz, vp]
     lib.sa_cache_store.restype = i32
     lib.sa_cache_store.argtypes = [i32] * 9 + [tp, tp, vp, vp, f32p, vp]
     lib.sa_device_status.restype = i32

@@ -1,12 +1,13 @@
 """The forward variants that only larger grids reach (two heads of a selector, or two rows that each select for
-themselves, in one CTA), second differentiation, the newest key of a decode step, and
+themselves, in one CTA), second differentiation, the newest key of a decode step, the split
+walk of a short chunk after a long cache, and
 the exact-product engine with one and two teams a CTA."""
 
 import pytest
 import torch
 
 import selective_oracle as oracle
-from selective_attention_b200 import kernels, mixers
+from selective_attention_b200 import _lib, kernels, mixers
 
 pytestmark = pytest.mark.gpu
 
@@ -108,3 +109,22 @@ def test_exact_products_with_one_and_two_teams(dim, dtype, batch, heads, seq, ex
     tol = 1e-5 if dtype == torch.float32 else 2e-3
     for got, ref in zip((out.detach(), *grads), want):
         torch.testing.assert_close(got.float().cpu(), ref, atol=tol * float(ref.abs().max()) + 1e-6, rtol=tol)
+
+
+# few new rows: the walk over the cached keys is cut into pieces, of which a short one's last has no keys or no live ones
+@pytest.mark.parametrize("heads,dim,first,second,per_head", [(2, 64, 1020, 3, False), (3, 128, 1152, 128, False), (2, 64, 4100, 300, True),
+                                                             (1, 128, 2200, 1, False), (12, 64, 3000, 129, False)])
+@pytest.mark.parametrize("scale", [1.0, 0.2])
+def test_a_short_chunk_after_a_long_cache(heads, dim, first, second, per_head, scale):
+    total = first + second
+    q, k, v, _ = (x.cuda() for x in _inputs(1, heads, total, dim, scale, total))
+    slot = mixers.SelectiveAttentionSlot(n_heads=heads, context_length=total, per_head=per_head)
+    whole, sums = slot.attend(q, k, v, want_total=True)
+    got = []
+    for skip in (False, True):
+        _, cache = slot.begin_cache(*(x[:, :, :first] for x in (q, k, v)))
+        got.append(slot.extend_cache(*(x[:, :, first:] for x in (q, k, v)), cache, skip_dead_tiles=skip))
+        torch.testing.assert_close(cache["selected"], sums, atol=1e-3, rtol=1e-4)
+    assert _lib.device_status() == 0
+    assert torch.equal(got[0], got[1])
+    assert _rel(got[0], whole[:, :, first:].float().cpu()) < 4e-3
