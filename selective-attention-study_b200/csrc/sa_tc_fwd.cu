@@ -319,107 +319,120 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       split.lse[((int64_t)piece * nrows + n) * q_rows + i0 + tid - q_offset] = -INFINITY;
   } else if (warp == kWideCompute / 32) {
     // =============================== control warp: TMA loads and MMA issue ===============================
-    if (lane == 0) {
-      // A tile of step it lives in stage slot(it); the j-th fill of a stage completes its barrier's phase j.
-      auto slot = [](int it) { return ST == 2 ? (it & 1) : 0; };
-      auto fill = [](int it) { return (uint32_t)((ST == 2 ? (it >> 1) : it) & 1); };
-      auto load_tile = [&](int off, const CUtensorMap* map, uint64_t* bars, int it, int head) {
+    // The warp stays converged and one elected lane issues: inside a divergent branch an MMA took about 75 cycles to issue.
+    Waiter wait;
+    wait.begin(status);
+    // A tile of step it lives in stage slot(it); the j-th fill of a stage completes its barrier's phase j.
+    auto slot = [](int it) { return ST == 2 ? (it & 1) : 0; };
+    auto fill = [](int it) { return (uint32_t)((ST == 2 ? (it >> 1) : it) & 1); };
+    auto await = [&](uint64_t* bar, uint32_t parity, int site) { wait.left = wait_call(smem_u32(bar), parity, site, wait.left); };
+    auto load_tile = [&](int off, const CUtensorMap* map, uint64_t* bars, int it, int head) {
+      const int j0 = key_tile(it) * kTile;
+      if (elect_one()) {
         uint64_t* bar = &bars[slot(it)];
         mbar_expect_tx(bar, L::kTileBytes);
         for (int s2 = 0; s2 < DK; ++s2)
-          tma_load_4d(smem + off + slot(it) * L::kTileBytes + s2 * kRowTile, map, bar, s2 * 64, key_tile(it) * kTile, head, b);
-      };
-      auto load_k = [&](int it) { load_tile(L::k, &map_k, bar_k, it, h); };
-      auto load_k0 = [&](int it) { if (!SELF) load_tile(L::k0, &map_k0, bar_k0, it, 0); };   // SELF: K0 is K
-      auto load_v = [&](int it) { load_tile(L::v, &map_v, bar_v, it, h); };
-      const uint32_t idesc_s = instr_desc_bf16(128, 128, false, false);
-      const uint32_t idesc_tri = instr_desc_bf16(128, 128, false, true, /*negate_a=*/true);
-      const uint32_t idesc_pv = instr_desc_bf16(128, D, false, true);
-      auto issue_l0 = [&](int it) {                            // L0 = Q0 K0^T
-        mbar_wait(SELF ? &bar_k[slot(it)] : &bar_k0[slot(it)], fill(it), status, 311);
-        tc_fence_after_sync();
-        const uint32_t tile = sa + (SELF ? L::k : L::k0) + slot(it) * L::kTileBytes;
+          tma_load_4d(smem + off + slot(it) * L::kTileBytes + s2 * kRowTile, map, bar, s2 * 64, j0, head, b);
+      }
+      __syncwarp();
+    };
+    auto load_k = [&](int it) { load_tile(L::k, &map_k, bar_k, it, h); };
+    auto load_k0 = [&](int it) { if (!SELF) load_tile(L::k0, &map_k0, bar_k0, it, 0); };   // SELF: K0 is K
+    auto load_v = [&](int it) { load_tile(L::v, &map_v, bar_v, it, h); };
+    const uint32_t idesc_s = instr_desc_bf16(128, 128, false, false);
+    const uint32_t idesc_tri = instr_desc_bf16(128, 128, false, true, /*negate_a=*/true);
+    const uint32_t idesc_pv = instr_desc_bf16(128, D, false, true);
+    const uint32_t kBase = desc_low(sa, 16);                   // K-major views (rows = M or N index)
+    const uint32_t mBase = desc_low(sa, kRowTile);             // MN-major views (rows = K index)
+    auto at = [](uint32_t low, uint32_t byte_off) { return low + (byte_off >> 4); };
+    auto kstep = [](int ks) { return (uint32_t)((ks >> 2) * kRowTile + (ks & 3) * 32); };
+    auto issue_l0 = [&](int it) {                              // L0 = Q0 K0^T
+      await(SELF ? &bar_k[slot(it)] : &bar_k0[slot(it)], fill(it), 311);
+      if (elect_one()) {
+        const uint32_t tile = at(kBase, (SELF ? L::k : L::k0) + slot(it) * L::kTileBytes);
+#pragma unroll
         for (int ks = 0; ks < 4 * DK; ++ks)
-          mma_ts(tmem + kColL, tmem + (SELF ? kColQ : kColQ0) + ks * 8,
-                 smem_desc(tile + (ks >> 2) * kRowTile + (ks & 3) * 32, 16, 1024), idesc_s, ks > 0);
+          mma_ts_low(tmem + kColL, tmem + (SELF ? kColQ : kColQ0) + ks * 8, at(tile, kstep(ks)), idesc_s, ks > 0);
         mma_commit(&bar_l0);
-      };
-      auto issue_s_tri = [&](int it) {                         // S = Q K^T, then S -= TRI x selection
-        mbar_wait(&bar_k[slot(it)], fill(it), status, 312);
-        tc_fence_after_sync();
-        const uint32_t tile = sa + L::k + slot(it) * L::kTileBytes;
-        for (int ks = 0; ks < 4 * DK; ++ks)
-          mma_ts(tmem + kColS, tmem + kColQ + ks * 8, smem_desc(tile + (ks >> 2) * kRowTile + (ks & 3) * 32, 16, 1024),
-                 idesc_s, ks > 0);
+      }
+      __syncwarp();
+    };
+    auto issue_s_tri = [&](int it) {                           // S = Q K^T, then S -= TRI x selection
+      await(&bar_k[slot(it)], fill(it), 312);
+      if (elect_one()) {
+        const uint32_t tile = at(kBase, L::k + slot(it) * L::kTileBytes);
+#pragma unroll
+        for (int ks = 0; ks < 4 * DK; ++ks) mma_ts_low(tmem + kColS, tmem + kColQ + ks * 8, at(tile, kstep(ks)), idesc_s, ks > 0);
+#pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          if (kTmemAB)
-            mma_ts(tmem + kColS, tmem + kColTri + ks * 8, smem_desc(sa + L::sel + ks * 2048, kRowTile, 1024), idesc_tri, 1);
-          else
-            mma_ss(tmem + kColS, smem_desc(sa + L::q + (ks >> 2) * kRowTile + (ks & 3) * 32, 16, 1024),
-                   smem_desc(sa + L::sel + ks * 2048, kRowTile, 1024), idesc_tri, 1);
+          if (kTmemAB) mma_ts_low(tmem + kColS, tmem + kColTri + ks * 8, at(mBase, L::sel + ks * 2048), idesc_tri, 1u);
+          else mma_ss_low<true>(tmem + kColS, at(kBase, L::q + kstep(ks)), at(mBase, L::sel + ks * 2048), idesc_tri);
         }
         mma_commit(&bar_tri);
-      };
-      auto issue_pv = [&](int it, uint64_t* bar) {             // O += P V
-        mbar_wait(&bar_v[slot(it)], fill(it), status, 315);
-        tc_fence_after_sync();
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](int it, uint64_t* bar) {               // O += P V
+      await(&bar_v[slot(it)], fill(it), 315);
+      if (elect_one()) {
+        const uint32_t v = at(mBase, L::v + slot(it) * L::kTileBytes);
+        const uint32_t more = it > 0 ? 1u : 0u;
+#pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t vdesc = smem_desc(sa + L::v + slot(it) * L::kTileBytes + ks * 2048, kRowTile, 1024);
-          if (kTmemAB)
-            mma_ts(tmem + kColO, tmem + kColP + ks * 8, vdesc, idesc_pv, (it > 0 || ks > 0) ? 1u : 0u);
-          else
-            mma_ss(tmem + kColO, smem_desc(sa + L::p + (ks >> 2) * kRowTile + (ks & 3) * 32, 16, 1024), vdesc, idesc_pv,
-                   (it > 0 || ks > 0) ? 1u : 0u);
+          if (kTmemAB) mma_ts_low(tmem + kColO, tmem + kColP + ks * 8, at(v, ks * 2048), idesc_pv, ks > 0 ? 1u : more);
+          else if (ks > 0) mma_ss_low<true>(tmem + kColO, at(kBase, L::p + kstep(ks)), at(v, ks * 2048), idesc_pv);
+          else if (it > 0) mma_ss_low<true>(tmem + kColO, at(kBase, L::p), v, idesc_pv);
+          else mma_ss_low<false>(tmem + kColO, at(kBase, L::p), v, idesc_pv);
         }
         mma_commit(bar);
-      };
+      }
+      __syncwarp();
+    };
 
+    if (elect_one()) {
       mbar_expect_tx(&bar_q, (SELF ? 1 : 2) * DK * kRowTile);
       for (int s2 = 0; s2 < DK; ++s2) {
         tma_load_4d(smem + L::q + s2 * kRowTile, &map_q, &bar_q, s2 * 64, i0 - q_offset, h, b);
         if (!SELF) tma_load_4d(smem + L::q0_landing + s2 * kRowTile, &map_q0, &bar_q, s2 * 64, i0 - q_offset, 0, b);
       }
-      load_k0(0);
-      load_k(0);
-      load_v(0);
-      if (ST == 2 && steps > 1) {
-        load_k0(1);
-        load_k(1);
-        load_v(1);
-      }
-      mbar_wait(&bar_setup, 0, status, 317);                   // Q, Q0 in TMEM and the triangular tile in place
-      tc_fence_after_sync();
-      issue_l0(0);
-#pragma unroll(D == 64 ? 2 : 1)   // head_dim 64: the stage and phase parities become constants (-2.6 %); head_dim 128: +11 %
-      for (int it = 0; it < steps; ++it) {
-        mbar_wait(&bar_sel, it & 1, status, 318);              // selection of step it written; logits of it - 1 read;
-        tc_fence_after_sync();                                 //   L0 of step it consumed: its K0 tile is free
-        if (it + ST < steps) load_k0(it + ST);
-        issue_s_tri(it);
-        const bool l0_now = !(SELF && ST == 1);                // one-stage SELF: K of the next step is not loaded yet
-        if (l0_now && it + 1 < steps) issue_l0(it + 1);
-        if (it > 0) {
-          mbar_wait(&bar_p, (it - 1) & 1, status, 320);        // P of step it - 1 written, O rescaled
-          tc_fence_after_sync();
-          if (ST == 2 && it >= 2) {                            // before this barrier's next commit: P V of it - 2 done,
-            mbar_wait(&bar_pv, it & 1, status, 321);           //   so its V tile may be refilled
-            load_v(it);
-          }
-          issue_pv(it - 1, &bar_pv);
-        }
-        mbar_wait(&bar_tri, it & 1, status, 319);              // S of step it done: its K tile is free
-        if (it + ST < steps) load_k(it + ST);
-        if (!l0_now && it + 1 < steps) issue_l0(it + 1);
-        if (ST == 1 && it > 0) {                               // the single V tile: refilled with V of step it (for the
-          mbar_wait(&bar_pv, (it - 1) & 1, status, 321);       //   P V issued in the next iteration) once P V of step
-          load_v(it);                                          //   it - 1 has completed
-        }
-      }
-      mbar_wait(&bar_p, (steps - 1) & 1, status, 322);
-      tc_fence_after_sync();
-      issue_pv(steps - 1, &bar_fin);
     }
     __syncwarp();
+    load_k0(0);
+    load_k(0);
+    load_v(0);
+    if (ST == 2 && steps > 1) {
+      load_k0(1);
+      load_k(1);
+      load_v(1);
+    }
+    await(&bar_setup, 0, 317);                                 // Q, Q0 in TMEM and the triangular tile in place
+    issue_l0(0);
+#pragma unroll(D == 64 ? 2 : 1)   // head_dim 64: the stage and phase parities become constants
+    for (int it = 0; it < steps; ++it) {
+      await(&bar_sel, it & 1, 318);                            // selection of step it written; logits of it - 1 read;
+      if (it + ST < steps) load_k0(it + ST);                   //   L0 of step it consumed: its K0 tile is free
+      issue_s_tri(it);
+      const bool l0_now = !(SELF && ST == 1);                  // one-stage SELF: K of the next step is not loaded yet
+      if (l0_now && it + 1 < steps) issue_l0(it + 1);
+      if (it > 0) {
+        await(&bar_p, (it - 1) & 1, 320);                      // P of step it - 1 written, O rescaled
+        if (ST == 2 && it >= 2) {                              // before this barrier's next commit: P V of it - 2 done,
+          await(&bar_pv, it & 1, 321);                         //   so its V tile may be refilled
+          load_v(it);
+        }
+        issue_pv(it - 1, &bar_pv);
+      }
+      await(&bar_tri, it & 1, 319);                            // S of step it done: its K tile is free
+      if (it + ST < steps) load_k(it + ST);
+      if (!l0_now && it + 1 < steps) issue_l0(it + 1);
+      if (ST == 1 && it > 0) {                                 // the single V tile: refilled with V of step it (for the
+        await(&bar_pv, (it - 1) & 1, 321);                     //   P V issued in the next iteration) once P V of step
+        load_v(it);                                            //   it - 1 has completed
+      }
+    }
+    await(&bar_p, (steps - 1) & 1, 322);
+    issue_pv(steps - 1, &bar_fin);
+    if (lane == 0) wait.end(status);
   } else {
     // ======================================= arithmetic warps ============================================
     const int row = tid & 127, wg = tid >> 7;
