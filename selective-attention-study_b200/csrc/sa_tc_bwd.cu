@@ -34,7 +34,7 @@
 // first form of this kernel, with 45 KB of loops, ran at 15.5 k cycles a tile; hence the compact waits (Waiter), rolled MMA
 // loops over halves (the order is the same for both chains), low words of descriptors, 32-bit shared addresses.
 // Measured at B = 4, H = 16, T = 16384: 16.6 ms with sixteen warps in lock step, 12.1 ms with two chains and one MMA warp,
-// 10.5 ms (5.0 k cycles a tile) with three (SELF: 12.3, 8.7, 8.0).
+// 10.3 ms (5.0 k cycles a tile) with three (SELF: 12.3, 8.7, 8.0).
 //
 // SELF variant (one head per selector, i.e. the per-head form reshaped to (B H, 1, T, D)): the selection logits are the
 // head's own logits, so S^T serves as L0^T (read twice), and since Q0 = Q and K0 = K the two gradient paths add before the

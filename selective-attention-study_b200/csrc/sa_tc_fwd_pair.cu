@@ -15,13 +15,14 @@
 // heads (64 each).  Shared memory, 224 KB: Q, Q of the two heads and Q0 48 KB, TRI 32, selection 32, K and V rings of three
 // tiles 48 each (the heads alternate), K0 16.
 //
-// What bounds it: latency around F.  The step of both heads takes 4.3 k cycles: F read by both -> L0 -> selection -> running
-// sum -> F read by both is 2.6 k of hand-overs plus the read, and a head's own chain is as long (S after P V of the step
-// before 1.2 k, read 0.8 k, 128 exponentials a thread 1.5 - 1.8 k).  The exponential unit (16 ex2 a clock and SM) needs 2.0 k
-// of them, the tensor pipe 1.8 k, shared memory 2.4 k, the issue slots 1.4 k.  TMEM is full, so neither S nor F can have a
-// second buffer; S in two halves of 64 keys around P V (N = 64 products read shared memory 1.5 times as much) was no faster.
-// Measured at B = 4, H = 16, T = 16384: 4.74 ms (forward_wide_kernel, which makes the selection and its running sum for each
-// head and keeps its sixteen warps in step: 6.06 ms); B = 1, H = 16, T = 131072: 95.1 -> 71.6 ms.
+// What bounds it: latency around F.  The step of both heads takes 3.9 k cycles: F read by both -> L0 -> selection -> running
+// sum -> F read by both is a chain of hand-overs, and a head's own chain is as long (S after P V of the step before 1.2 k, read
+// 0.8 k, 128 exponentials a thread 1.5 k).  The exponential unit (16 ex2 a clock and SM) needs 2.0 k of them and is busy 48 % of
+// the time, the tensor pipe 41 %, the issue slots 42 %.  TMEM is full, so neither S nor F can have a second buffer; S in two halves
+// of 64 keys around P V (N = 64 products read shared memory 1.5 times as much), four softmax warpgroups and two for the
+// selection were slower.
+// Measured at B = 4, H = 16, T = 16384: 4.25 ms (forward_wide_kernel, which makes the selection and its running sum for each
+// head and keeps its sixteen warps in step: 6.06 ms); B = 1, H = 16, T = 131072: 95.1 -> 66.2 ms.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:140-194 (one head), :366-424 (heads sharing S and F).
 #include <type_traits>
