@@ -20,7 +20,7 @@
 //             are added up at the end; dQ and the selector's dQ0: a group each
 // Operands sit in shared memory as fp32 rows of D + 4 floats (consecutive rows start 4 banks apart) and are read 16 bytes at a
 // time; two FMAs an instruction, along the contraction in the logits (even and odd elements apart), else along the columns.
-// What bounds it: shared-memory loads (82 % of their rate in backward at D = 32) and FMAs at about the same rate; with few
+// What bounds it: shared-memory loads (71 % of their rate in backward at D = 32) and FMAs at about the same rate; with few
 // (batch, head) rows the longest walk.  us for selection, forward, backward, at first / 128 threads a CTA, one FMA an
 // instruction / now:  (2, 4, 1024, 64) fp32  153, 403, 859 / 15, 134, 339 / 14, 78, 160;  (4, 8, 1000, 32) fp16 now 12, 170, 290.
 //
