@@ -28,61 +28,80 @@ namespace {
 constexpr int kTile = 128;
 constexpr float kDeadMargin = 150.f;
 
-// Largest row norm of each 128-row tile of q (z = 0) and k (z = 1): one block per (tile, row n, tensor), one thread
-// per token.  Tiles are counted in absolute positions; the query tensor starts at position q_offset (a prefill that
-// continues from a cache), the key tensor at 0.
+// Largest row norm of each 128-row tile of q (z = 0) and k (z = 1): one block per (tile, row n, tensor), D / 8 lanes per
+// token, so that a warp's load is contiguous, and eight (D = 128: sixteen) of them in flight a thread.  Bound by HBM; with a
+// thread per token 16 heads of T = 16384 took 21 us.  Tiles are counted in absolute positions; the query tensor
+// starts at position q_offset (a prefill that continues from a cache), the key tensor at 0.
 template <int D>
 __global__ void __launch_bounds__(kTile) tile_norms_kernel(const __nv_bfloat16* __restrict__ q, RowLayout q_rows,
                                                            const __nv_bfloat16* __restrict__ k, RowLayout k_rows,
                                                            int heads, int seq, int ntiles, int q_offset,
                                                            float* __restrict__ qn, float* __restrict__ kn) {
+  constexpr int kLanes = D / 8, kRows = kTile / kLanes, kPasses = kTile / kRows;
   const int tile = blockIdx.x, n = blockIdx.y, which = blockIdx.z;
   const int b = n / heads, h = n - b * heads;
-  const int t = tile * kTile + threadIdx.x;
-  float ss = 0.f;
-  if (t < seq && (which == 1 || t >= q_offset)) {
-    const __nv_bfloat16* row = which == 0 ? q + q_rows.at(b, h, t - q_offset) : k + k_rows.at(b, h, t);
+  const int lane = threadIdx.x % kLanes, t0 = tile * kTile + threadIdx.x / kLanes;
+  uint4 v[kPasses];
 #pragma unroll
-    for (int c = 0; c < D / 8; ++c) {
-      const uint4 v = *reinterpret_cast<const uint4*>(row + c * 8);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xffff0000u);
-        ss = fmaf(lo, lo, fmaf(hi, hi, ss));
-      }
-    }
+  for (int u = 0; u < kPasses; ++u) {
+    const int t = t0 + u * kRows;
+    v[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < seq && (which == 1 || t >= q_offset))
+      v[u] = *reinterpret_cast<const uint4*>((which == 0 ? q + q_rows.at(b, h, t - q_offset) : k + k_rows.at(b, h, t)) + lane * 8);
   }
-  float m = sqrtf(ss);
+  float m = 0.f;                                                  // of the squares
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int u = 0; u < kPasses; ++u) {
+    const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xffff0000u);
+      ss = fmaf(lo, lo, fmaf(hi, hi, ss));
+    }
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    m = fmaxf(m, ss);
+  }
+#pragma unroll
+  for (int o = 16; o >= kLanes; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   __shared__ float part[4];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0)
-    (which == 0 ? qn : kn)[(int64_t)n * ntiles + tile] = fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3]));
+    (which == 0 ? qn : kn)[(int64_t)n * ntiles + tile] = sqrtf(fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])));
 }
 
-// alive[n][mi][nj] for nj <= mi: one block per (query tile mi >= mi_first, sequence b); a warp takes every fourth key
-// tile, finds the smallest carry over its 128 keys, and its lanes write the verdict for the heads of the sequence.
+// alive[n][mi][nj] for nj <= mi: one block per (query tile mi >= mi_first, 16 key tiles, sequence b); a warp takes every fourth
+// of them, finds the smallest carry over its 128 keys, and its lanes write the verdict for the heads of the sequence.
+// (Bound by latency; with a query tile's key tiles all in one block T = 16384 took 20 us.)
+constexpr int kTableChunk = 16;
 __global__ void __launch_bounds__(kTile) tile_table_kernel(const float* __restrict__ carry, const float* __restrict__ qn,
                                                            const float* __restrict__ kn, int heads, int seq, int ntiles,
                                                            int mi_first, float c1, uint8_t* __restrict__ alive) {
-  const int mi = mi_first + blockIdx.x, b = blockIdx.y;
+  const int mi = mi_first + blockIdx.x, b = blockIdx.z, nj0 = blockIdx.y * kTableChunk;
+  if (nj0 > mi) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* carry_row = carry + ((int64_t)b * (ntiles + 1) + mi) * seq;
-  for (int nj = warp; nj <= mi; nj += 4) {
-    float fmin = FLT_MAX;
+  float fmin[kTableChunk / 4];
+#pragma unroll
+  for (int u = 0; u < kTableChunk / 4; ++u) {
+    fmin[u] = FLT_MAX;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int j = nj * kTile + c * 32 + lane;
-      if (j < seq) fmin = fminf(fmin, carry_row[j]);
+      const int nj = nj0 + warp + 4 * u, j = nj * kTile + c * 32 + lane;
+      if (nj <= mi && j < seq) fmin[u] = fminf(fmin[u], carry_row[j]);
     }
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) fmin = fminf(fmin, __shfl_xor_sync(0xffffffffu, fmin, o));
+  for (int u = 0; u < kTableChunk / 4; ++u) {
+    const int nj = nj0 + warp + 4 * u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) fmin[u] = fminf(fmin[u], __shfl_xor_sync(0xffffffffu, fmin[u], o));
+    if (nj > mi) continue;
     for (int h = lane; h < heads; h += 32) {
       const int64_t n = (int64_t)b * heads + h;
-      const float bound = c1 * qn[n * ntiles + mi] * (kn[n * ntiles + nj] + kn[n * ntiles + mi]) - kLog2e * fmin;
+      const float bound = c1 * qn[n * ntiles + mi] * (kn[n * ntiles + nj] + kn[n * ntiles + mi]) - kLog2e * fmin[u];
       alive[(n * ntiles + mi) * ntiles + nj] = (nj == mi || !(bound < -kDeadMargin)) ? 1 : 0;
     }
   }
@@ -122,7 +141,7 @@ int build_tile_table(const Problem& p, const float* carry, cudaStream_t s) {
   SA_CUDA_CHECK(cudaGetLastError());
   count_launch();
   const int mi_first = p.q_offset / kTile;                // a continued prefill computes the query tiles from here on
-  tile_table_kernel<<<dim3(ntiles - mi_first, p.batch), kTile, 0, s>>>(carry, qn, kn, p.heads, p.seq, ntiles, mi_first,
+  tile_table_kernel<<<dim3(ntiles - mi_first, (ntiles + kTableChunk - 1) / kTableChunk, p.batch), kTile, 0, s>>>(carry, qn, kn, p.heads, p.seq, ntiles, mi_first,
                                                                        p.scale * kLog2e, alive);
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;
