@@ -19,6 +19,8 @@
 //                   P V): 3.2 k cycles at head_dim 64, 5.3 k at 128, of which the tensor pipe needs 0.8 k and 1.1 k.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:100-194 (selection, carry, forward).
+#include <float.h>
+
 #include <type_traits>
 
 #include "sa_tc_fwd.cuh"
@@ -538,7 +540,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       arrive(&bar_sel);
     };
 
-    float run_max = -INFINITY, run_den = 0.f;                  // run_den: this warpgroup's share of the denominator
+    // run_den: this warpgroup's share of the denominator.  The maximum starts at the lowest finite value: a later piece of a walk
+    // can begin with key tiles whose history is infinite (keys taken out by their caller), and -inf - (-inf) is not a number.
+    float run_max = -FLT_MAX, run_den = 0.f;
     selection(0, fetch_carry(0));
     float next_carry = fetch_carry(1);
     // One 128-key step.  The diagonal step (it = 0: causal mask inside the tile, nothing to wait for or rescale yet) is
@@ -579,7 +583,6 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         rmax_s[wg][row] = tile_max;
       }
       named_barrier(kWideBarrier, kWideCompute);
-      // every row has its own key in the diagonal tile, so the maximum is finite from the first step on
       const float new_max =
           fmaxf(fmaxf(run_max, fmaxf(rmax_s[0][row], rmax_s[1][row])), fmaxf(rmax_s[2][row], rmax_s[3][row]));
       const float alpha = ex2(run_max - new_max);

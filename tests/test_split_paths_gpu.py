@@ -128,3 +128,21 @@ def test_a_short_chunk_after_a_long_cache(heads, dim, first, second, per_head, s
     assert _lib.device_status() == 0
     assert torch.equal(got[0], got[1])
     assert _rel(got[0], whole[:, :, first:].float().cpu()) < 4e-3
+
+
+@pytest.mark.parametrize("heads,dim,per_head", [(2, 64, False), (2, 64, True), (2, 128, False)])
+@pytest.mark.parametrize("gone", [(1, 2000), (0, 3968), (1500, 1501)])
+def test_a_split_walk_over_keys_with_an_infinite_history(heads, dim, per_head, gone):
+    """A key whose history is infinite has no weight; a piece of the walk may hold nothing else, or begin with it."""
+    first, total = 4000, 4008
+    q, k, v, _ = (x.cuda() for x in _inputs(1, heads, total, dim, 0.3, dim))
+    slot = mixers.SelectiveAttentionSlot(n_heads=heads, context_length=total, per_head=per_head)
+    _, cache = slot.begin_cache(*(x[:, :, :first] for x in (q, k, v)))
+    cache["selected"][:, :, gone[0]:gone[1]] = float("inf")
+    whole = {key: (x.clone() if torch.is_tensor(x) else x) for key, x in cache.items()}
+    new = [x[:, :, first:] for x in (q, k, v)]
+    got = slot.extend_cache(*new, cache)
+    want = kernels.prefill_extend(whole, *new)                   # fp32 rows: one walk over all keys
+    assert torch.isfinite(want).all()
+    assert _rel(got, want.cpu()) < 4e-3                          # the rounding of the rows to bf16
+    assert torch.equal(cache["selected"], whole["selected"])
