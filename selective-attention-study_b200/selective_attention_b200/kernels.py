@@ -373,21 +373,37 @@ def _backward_call(ctx, dout, dq0=None, dk0=None):
     return dq, dk, dv
 
 
-class _SelectiveAttentionFn:
-    """The differentiable operator; the autograd node is C++ (csrc/torch/sa_torch.cpp)."""
+class _SelectiveAttentionFn(torch.autograd.Function):
+    """The differentiable operator as an autograd function that tracing records; ``selective_attention`` takes the node in
+    C++ (csrc/torch/sa_torch.cpp) where nothing records."""
 
     @staticmethod
-    def apply(q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n, bwd_num_warps, bwd_num_stages, group, bwd_group,
-              num_stages, exempt, skip_dead_tiles=False):
+    def forward(ctx, q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n, bwd_num_warps,
+                bwd_num_stages, group, bwd_group, num_stages, exempt, skip_dead_tiles=False):
         check_inputs(q, k, v)
         exempt = _check_exempt(exempt)
         lowp = _lowp(dot_precision, q.dtype)
         _check_blocks(block_m, block_n)
-        tc = _engine(lowp, q.shape[3], False) == _lib.ENGINE_TCGEN05
-        out = _lib.native().attend(q, k, v, exempt, lowp, tc, bool(skip_dead_tiles) and tc, False)
-        if bwd_group not in (None, 1, 2) and out.requires_grad:
-            out.register_hook(lambda _: _check_bwd_group(bwd_group))       # raised by the backward, whose knob it is
+        out, lse2, carry, _, operands, _, engine, _, table = _forward(q, k, v, lowp, exempt, 0, 0,
+                                                                      live_tiles=skip_dead_tiles)
+        ctx.save_for_backward(*operands, out, lse2, carry)
+        ctx.engine, ctx.exempt, ctx.bwd_group, ctx.tile_table = engine, exempt, bwd_group, table
+        ctx.grad_dtypes = (q.dtype, k.dtype, v.dtype)
         return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dout):
+        _check_bwd_group(ctx.bwd_group)
+        grads = _backward_call(ctx, dout)
+        grads = tuple(g if g.dtype == want else g.to(want) for g, want in zip(grads, ctx.grad_dtypes))
+        return grads + (None,) * 12
+
+
+def _recorded() -> bool:
+    """A trace is being recorded: it sees an autograd function, but not a call into ``_native``, whose result it would keep as
+    a constant."""
+    return torch._C._get_tracing_state() is not None
 
 
 class _SelectiveAttentionSelectorFn(torch.autograd.Function):
@@ -462,9 +478,19 @@ def selective_attention(
         _check_bwd_group(bwd_group)
         q0, k0 = selector
         return _SelectiveAttentionSelectorFn.apply(q, k, v, q0, k0, dot_precision, exempt, bool(skip_dead_tiles))
-    return _SelectiveAttentionFn.apply(q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n,
-                                       bwd_num_warps, bwd_num_stages, group, bwd_group, num_stages, exempt,
-                                       bool(skip_dead_tiles))
+    if _recorded():
+        return _SelectiveAttentionFn.apply(q, k, v, dot_precision, block_m, block_n, num_warps, bwd_block_n,
+                                           bwd_num_warps, bwd_num_stages, group, bwd_group, num_stages, exempt,
+                                           bool(skip_dead_tiles))
+    check_inputs(q, k, v)
+    exempt = _check_exempt(exempt)
+    lowp = _lowp(dot_precision, q.dtype)
+    _check_blocks(block_m, block_n)
+    tc = _engine(lowp, q.shape[3], False) == _lib.ENGINE_TCGEN05
+    out = _lib.native().attend(q, k, v, exempt, lowp, tc, bool(skip_dead_tiles) and tc, False)
+    if bwd_group not in (None, 1, 2) and out.requires_grad:
+        out.register_hook(lambda _: _check_bwd_group(bwd_group))       # raised by the backward, whose knob it is
+    return out
 
 
 # ---- layout-fused form for a model's attention layer -------------------------------------------------
@@ -492,6 +518,10 @@ def selective_attention_packed(qkv: torch.Tensor, exempt: int = 1, *, skip_dead_
     merged result, the backward's kernels one (B, T, 3, H, D) gradient).  ``skip_dead_tiles``: as in ``selective_attention``."""
     if not packed_supported(qkv):
         raise ValueError("qkv must be a contiguous bf16 CUDA tensor (B, T, 3, H, 64 or 128); use selective_attention otherwise")
+    if _recorded():
+        b, t, _, h, d = qkv.shape
+        y = selective_attention(*(qkv[:, :, i].transpose(1, 2) for i in range(3)), exempt=exempt, skip_dead_tiles=skip_dead_tiles)
+        return y.to(qkv.dtype).transpose(1, 2).reshape(b, t, h * d)
     return _lib.native().attend_packed(qkv, _check_exempt(exempt), bool(skip_dead_tiles))
 
 
@@ -513,8 +543,8 @@ def _store_rows(cache: dict, k: torch.Tensor, v: torch.Tensor, at: int, begin: b
 def _attend_low(q, k, v, dot_precision: str | None, exempt: int):
     """The differentiable operator with its result in the operands' bf16 (the kernel writes both forms), and the cotangent read
     in bf16; None where the result has to be cast by the caller."""
-    if not (q.dtype == k.dtype == v.dtype == torch.bfloat16 and _lowp(dot_precision, q.dtype)
-            and _engine(True, q.shape[3], False) == _lib.ENGINE_TCGEN05):
+    if _recorded() or not (q.dtype == k.dtype == v.dtype == torch.bfloat16 and _lowp(dot_precision, q.dtype)
+                           and _engine(True, q.shape[3], False) == _lib.ENGINE_TCGEN05):
         return None
     check_inputs(q, k, v)
     return _lib.native().attend(q, k, v, exempt, True, True, False, True)
