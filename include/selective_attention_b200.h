@@ -307,9 +307,9 @@ int sa_decode_step_live_keys(int dtype, int batch, int heads, int groups, int le
                              void* stream);
 
 /* The decode step from a block of arguments that a caller keeps with its cache and updates (q1, k1, v1, y, length, stream)
- * from step to step.  key_norms may be NULL.  y_dtype: SA_F32, or dtype for y in the cache's own type.  tickets_zero: the
- * workspace, sized for the cache's last position (length = capacity - 1), was zeroed before the first step and is used by this
- * cache's steps alone; a step then needs no memset. */
+ * from step to step.  key_norms may be NULL.  y_dtype: SA_F32, or dtype for y in the cache's own type.  tickets_zero: 0, the
+ * workspace holds anything and its tickets are cleared by a memset; otherwise it is sized for the cache's last position (length =
+ * capacity - 1) and kept for this cache's steps alone, on one stream: 2 in the first of them, which clears it, then 1. */
 typedef struct sa_decode {
   int32_t struct_bytes;   /* sizeof(sa_decode) */
   int32_t dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt, tickets_zero, reserved;

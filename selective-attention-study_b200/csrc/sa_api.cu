@@ -538,7 +538,7 @@ int sa_decode_step_live_keys(int dtype, int batch, int heads, int groups, int le
 int sa_decode_run(const sa_decode* d) {
   if (d == nullptr || d->struct_bytes != (int32_t)sizeof(sa_decode)) return SA_ERR_BAD_ARGUMENT;
   if (!dtype_ok(d->dtype) || d->batch < 1 || d->heads < 1 || d->groups < 1 || d->heads % d->groups != 0 || d->length < 0 ||
-      d->exempt < 1 || (d->y_dtype != SA_F32 && d->y_dtype != d->dtype))
+      d->exempt < 1 || d->tickets_zero < 0 || d->tickets_zero > 2 || (d->y_dtype != SA_F32 && d->y_dtype != d->dtype))
     return SA_ERR_BAD_ARGUMENT;
   if (!dim_ok(d->head_dim)) return SA_ERR_UNSUPPORTED;
   if (d->length >= d->capacity) return SA_ERR_BAD_ARGUMENT;
@@ -552,7 +552,7 @@ int sa_decode_run(const sa_decode* d) {
     return SA_ERR_WORKSPACE;
   if (tc::timeout_pending()) return SA_ERR_DEVICE_TIMEOUT;
   const DecodeStep step{d->dtype, d->y_dtype, d->batch, d->heads, d->groups, d->length, d->capacity, d->head_dim, d->exempt,
-                        d->tickets_zero != 0, d->q1, d->k1, d->v1, d->k_cache, d->v_cache, d->selected, d->key_norms, d->y,
+                        d->tickets_zero, d->q1, d->k1, d->v1, d->k_cache, d->v_cache, d->selected, d->key_norms, d->y,
                         static_cast<float*>(d->workspace)};
   return decode_step(step, static_cast<cudaStream_t>(d->stream));
 }

@@ -120,7 +120,7 @@ size_t decode_workspace_floats(int batch, int heads, int groups, int length, int
 // One cached decode step; y in fp32 or in the cache's type, key_norms null when every key is read.
 struct DecodeStep {
   int dtype, y_dtype, batch, heads, groups, length, capacity, head_dim, exempt;
-  bool tickets_zero;
+  int tickets_zero;            // 0: clear them; 1: kept at zero from step to step; 2: the first of such steps, which clears them
   const void *q1, *k1, *v1;
   void *k_cache, *v_cache;
   float *selected, *key_norms;

@@ -551,7 +551,7 @@ int decode_impl(const DecodeStep& d, cudaStream_t s) {
   // keys; 512 and 2048 measured slower) then spread those heads over the whole GPU.
   const int split_keys = (d.key_norms != nullptr) ? 1024 : decode_split_keys(t, rows);
   const int splits = (t + split_keys - 1) / split_keys;
-  // Tickets first: with `tickets_zero` at a size that does not change from step to step, so that what the last CTAs leave at zero
+  // Tickets first: where they are kept (`tickets_zero`), at a size that does not change from step to step, so that what the last CTAs leave at zero
   // is where the next step looks.
   const int ticket_splits = d.tickets_zero ? (d.capacity + kDecSplitMin - 1) / kDecSplitMin : splits;
   unsigned int* row_tickets = reinterpret_cast<unsigned int*>(d.workspace);
@@ -562,7 +562,7 @@ int decode_impl(const DecodeStep& d, cudaStream_t s) {
   tc::WaitCtx status;
   if (int st = tc::wait_ctx(&status)) return st;
   ProfileScope prof(SA_KERNEL_DECODE, s);
-  if (!d.tickets_zero) SA_CUDA_CHECK(cudaMemsetAsync(row_tickets, 0, n_tickets * 4, s));
+  if (d.tickets_zero != 1) SA_CUDA_CHECK(cudaMemsetAsync(row_tickets, 0, n_tickets * 4, s));
   // dead stages are left out when the norms are given and a CTA's range fits the stage list
   const bool live = d.key_norms != nullptr && split_keys / (kDecStageBytes / (D * (int)sizeof(T))) <= kDecMaxLive;
   auto attend = [&](auto dim, auto live_tag) {

@@ -297,24 +297,68 @@ bool store_rows(const Tensor& kc, const Tensor& vc, const Tensor& selected, cons
   return true;
 }
 
-// A decode step with the arguments that the caller keeps with its cache (their address) and the token's own.
-Tensor decode(int64_t address, const Tensor& kc, Tensor q1, Tensor k1, Tensor v1, int64_t length, int64_t exempt, bool y_low) {
+// A decode step.  Everything about the cache is looked at in every step.  What stays with it is the step's scratch: (tensor,
+// address of `selected`, stream, tickets), good for steps that have all three alike, since the tickets are at zero only between
+// steps of one order and a copy of a cache, or another stream, must not share them.  Returns y and the scratch to be kept,
+// None where the one that was given is.
+pybind11::tuple decode(const Tensor& kc, const Tensor& vc, const Tensor& selected, const std::optional<Tensor>& norms,
+                       const pybind11::object& kept, Tensor q1, Tensor k1, Tensor v1, int64_t length, int64_t exempt, bool y_low) {
+  TORCH_CHECK_VALUE(kc.dim() == 4 && selected.dim() == 3, "the cache must be (B, H, capacity, D) with (B, G, capacity) `selected`");
+  const int64_t b = kc.size(0), h = kc.size(1), capacity = kc.size(2), d = kc.size(3), groups = selected.size(1);
+  TORCH_CHECK_VALUE(length < capacity, "decode step past the cache capacity (context_length)");
+  TORCH_CHECK_VALUE(kc.is_cuda() && kc.is_contiguous() && vc.is_contiguous() && selected.is_contiguous() && vc.device() == kc.device() &&
+                        selected.device() == kc.device() && vc.numel() >= kc.numel() && selected.numel() >= b * groups * capacity,
+                    "the cache must be contiguous CUDA tensors");
+  TORCH_CHECK_VALUE(code_of(kc) >= 0 && vc.scalar_type() == kc.scalar_type() && selected.scalar_type() == at::kFloat,
+                    "cache dtype must be float16, bfloat16 or float32 with fp32 `selected`");
+  TORCH_CHECK_VALUE(d == 16 || d == 32 || d == 64 || d == 128, "head_dim must be one of (16, 32, 64, 128); got ", d);
+  TORCH_CHECK_VALUE(!norms || (norms->device() == kc.device() && norms->scalar_type() == at::kFloat && norms->is_contiguous() &&
+                               norms->sizes() == kc.sizes().slice(0, 3)),
+                    "cache['key_norms'] must be a contiguous fp32 CUDA tensor (B, H, capacity)");
   const at::NoGradGuard no_grad;
   const c10::cuda::CUDAGuard guard(kc.device());
-  sa_decode a = *reinterpret_cast<const sa_decode*>(address);
-  const int64_t b = a.batch, h = a.heads, d = a.head_dim;
-  for (Tensor* t : {&q1, &k1, &v1})
-    if (t->scalar_type() != kc.scalar_type() || t->device() != kc.device() || !t->is_contiguous() || t->numel() != b * h * d)
-      *t = t->reshape({b, h, d}).to(kc.options()).contiguous();
-  const Tensor y = at::empty({b, h, 1, d}, y_low ? kc.options() : kc.options().dtype(at::kFloat));
-  a.y_dtype = y_low ? a.dtype : SA_F32;
-  a.length = (int32_t)length;
-  a.exempt = (int32_t)exempt;
-  a.q1 = q1.data_ptr(); a.k1 = k1.data_ptr(); a.v1 = v1.data_ptr();
-  a.y = y.data_ptr();
-  a.stream = stream_of(kc);
-  check("sa_decode_step", sa_decode_run(&a));
-  return y;
+  void* const stream = stream_of(kc);
+  const auto selected_at = reinterpret_cast<uint64_t>(selected.data_ptr()), stream_at = reinterpret_cast<uint64_t>(stream);
+  const size_t need = sa_decode_workspace_bytes((int)b, (int)h, (int)groups, (int)(capacity - 1), (int)d);
+  const uint64_t layout = ((uint64_t)(b * h) << 32) + (uint64_t)(b * groups);      // with the capacity: where the tickets are
+  Tensor workspace;
+  if (PyTuple_Check(kept.ptr()) && PyTuple_GET_SIZE(kept.ptr()) == 5) {
+    auto number = [&](int i) { return PyLong_AsUnsignedLongLongMask(PyTuple_GET_ITEM(kept.ptr(), i)); };
+    if (THPVariable_Check(PyTuple_GET_ITEM(kept.ptr(), 0)) && number(1) == selected_at && number(2) == stream_at &&
+        number(3) == layout && number(4) == (uint64_t)capacity) {
+      const Tensor& t = THPVariable_Unpack(PyTuple_GET_ITEM(kept.ptr(), 0));
+      if (t.device() == kc.device() && t.scalar_type() == at::kByte && t.is_contiguous() && (size_t)t.numel() >= need) workspace = t;
+    }
+  }
+  const bool fresh = !workspace.defined();
+  Tensor y;
+  {
+    const pybind11::gil_scoped_release release;
+    for (Tensor* t : {&q1, &k1, &v1})
+      if (t->scalar_type() != kc.scalar_type() || t->device() != kc.device() || !t->is_contiguous() || t->numel() != b * h * d)
+        *t = t->reshape({b, h, d}).to(kc.options()).contiguous();
+    if (fresh) workspace = bytes_on(kc, need);
+    y = at::empty({b, h, 1, d}, y_low ? kc.options() : kc.options().dtype(at::kFloat));
+    sa_decode a{};
+    a.struct_bytes = sizeof(sa_decode);
+    a.dtype = code_of(kc);
+    a.y_dtype = y_low ? a.dtype : SA_F32;
+    a.batch = (int32_t)b; a.heads = (int32_t)h; a.groups = (int32_t)groups; a.capacity = (int32_t)capacity; a.head_dim = (int32_t)d;
+    a.length = (int32_t)length;
+    a.exempt = (int32_t)exempt;
+    a.tickets_zero = fresh ? 2 : 1;
+    a.q1 = q1.data_ptr(); a.k1 = k1.data_ptr(); a.v1 = v1.data_ptr();
+    a.k_cache = kc.data_ptr(); a.v_cache = vc.data_ptr(); a.selected = selected.data_ptr<float>();
+    a.key_norms = norms ? norms->data_ptr<float>() : nullptr;
+    a.y = y.data_ptr();
+    a.workspace = workspace.data_ptr();
+    a.workspace_bytes = workspace.numel();
+    a.stream = stream;
+    check("sa_decode_step", sa_decode_run(&a));
+  }
+  pybind11::object keep = pybind11::none();
+  if (fresh) keep = pybind11::make_tuple(workspace, selected_at, stream_at, layout, capacity);
+  return pybind11::make_tuple(y, keep);
 }
 
 }  // namespace
@@ -325,5 +369,5 @@ PYBIND11_MODULE(_native, m) {
   m.def("attend_packed", &attend_packed, nogil());
   m.def("prefill_rows", &prefill_rows, nogil());
   m.def("store_rows", &store_rows, nogil());
-  m.def("decode", &decode, nogil());
+  m.def("decode", &decode);
 }

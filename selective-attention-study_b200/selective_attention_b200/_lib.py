@@ -47,15 +47,6 @@ class Tensor(ctypes.Structure):
                 ("stride", ctypes.c_int64 * 3)]
 
 
-class Decode(ctypes.Structure):
-    """sa_decode: the arguments of a decode step, kept with its cache."""
-    _fields_ = ([(name, ctypes.c_int32) for name in ("struct_bytes", "dtype", "y_dtype", "batch", "heads", "groups", "length",
-                                                     "capacity", "head_dim", "exempt", "tickets_zero", "reserved")] +
-                [(name, ctypes.c_void_p) for name in ("q1", "k1", "v1", "k_cache", "v_cache", "selected", "key_norms", "y",
-                                                      "workspace")] +
-                [("workspace_bytes", ctypes.c_uint64), ("stream", ctypes.c_void_p)])
-
-
 class LibraryError(RuntimeError):
     def __init__(self, fn: str, status: int, detail: str):
         super().__init__(f"{fn} failed: SA_ERR_{STATUS_NAMES.get(status, status)} ({detail})")

@@ -647,52 +647,14 @@ def decode_step(cache: dict, q1: torch.Tensor, k1: torch.Tensor, v1: torch.Tenso
     return _decode(cache, q1, k1, v1, exempt, torch.float32)
 
 
-class _DecodePlan:
-    """What a decode step finds out about its cache: checked once, kept with the cache for as long as it holds the same
-    tensors.  A step then only fills in its own pointers and position."""
-
-    def __init__(self, cache: dict):
-        kc, vc, selected = self.tensors = (cache["k"], cache["v"], cache["selected"])
-        norms = self.norms = cache.get("key_norms")
-        b, h, cap, d = kc.shape
-        if not (kc.is_cuda and kc.is_contiguous() and vc.is_contiguous() and selected.is_contiguous()):
-            raise ValueError("the cache must be contiguous CUDA tensors")
-        if kc.dtype not in _DTYPE_CODE or vc.dtype != kc.dtype or selected.dtype != torch.float32:
-            raise ValueError("cache dtype must be float16, bfloat16 or float32 with fp32 `selected`")
-        if d not in HEAD_DIMS:
-            raise ValueError(f"head_dim must be one of {HEAD_DIMS}; got {d}")
-        if norms is not None and not (norms.is_cuda and norms.dtype == torch.float32 and norms.is_contiguous()
-                                      and tuple(norms.shape) == (b, h, cap)):
-            raise ValueError("cache['key_norms'] must be a contiguous fp32 CUDA tensor (B, H, capacity)")
-        self.capacity = cap
-        groups = selected.shape[1]
-        # scratch for the longest step that the cache can take
-        need = _lib.load().sa_decode_workspace_bytes(b, h, groups, max(cap - 1, 0), d)
-        self.workspace = torch.zeros(need, device=kc.device, dtype=torch.uint8)
-        a = self.args = _lib.Decode()
-        a.struct_bytes, a.tickets_zero = ctypes.sizeof(_lib.Decode), 1
-        a.dtype, a.batch, a.heads, a.groups, a.capacity, a.head_dim = _DTYPE_CODE[kc.dtype], b, h, groups, cap, d
-        a.k_cache, a.v_cache, a.selected = kc.data_ptr(), vc.data_ptr(), selected.data_ptr()
-        a.key_norms = norms.data_ptr() if norms is not None else None
-        a.workspace, a.workspace_bytes = self.workspace.data_ptr(), need
-        self.address = ctypes.addressof(a)
-
-    def holds(self, cache: dict) -> bool:
-        kc, vc, selected = self.tensors
-        a = self.args
-        return (cache["k"] is kc and cache["v"] is vc and cache["selected"] is selected and cache.get("key_norms") is self.norms
-                and kc.data_ptr() == a.k_cache and vc.data_ptr() == a.v_cache and selected.data_ptr() == a.selected)
-
-
 def _decode(cache: dict, q1: torch.Tensor, k1: torch.Tensor, v1: torch.Tensor, exempt: int, out_dtype: torch.dtype) -> torch.Tensor:
-    """The step with y in fp32 or in the cache's own type."""
+    """The step with y in fp32 or in the cache's own type.  The step's scratch stays in the cache, as ``"_workspace"``: a tensor and
+    what it was made for (see ``decode`` in csrc/torch/sa_torch.cpp)."""
     exempt = _check_exempt(exempt)
-    plan = cache.get("_plan")
-    if plan is None or not plan.holds(cache):
-        plan = cache["_plan"] = _DecodePlan(cache)
     length = int(cache["len"])
-    if length >= plan.capacity:
-        raise ValueError("decode step past the cache capacity (context_length)")
-    y = _lib.native().decode(plan.address, plan.tensors[0], q1, k1, v1, length, exempt, out_dtype != torch.float32)
+    y, workspace = _lib.native().decode(cache["k"], cache["v"], cache["selected"], cache.get("key_norms"), cache.get("_workspace"),
+                                        q1, k1, v1, length, exempt, out_dtype != torch.float32)
+    if workspace is not None:
+        cache["_workspace"] = workspace
     cache["len"] = length + 1
     return y
