@@ -4,6 +4,7 @@
 //
 // A failed library call raises the package's LibraryError, from a backward too.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
@@ -300,7 +301,8 @@ bool store_rows(const Tensor& kc, const Tensor& vc, const Tensor& selected, cons
 // A decode step.  Everything about the cache is looked at in every step.  What stays with it is the step's scratch: (tensor,
 // address of `selected`, stream, tickets), good for steps that have all three alike, since the tickets are at zero only between
 // steps of one order and a copy of a cache, or another stream, must not share them.  Returns y and the scratch to be kept,
-// None where the one that was given is.
+// None where the one that was given is.  A step that is being captured uses scratch of the graph's own: what the graph
+// will write to is not the cache's to replace, and what it is to clear has not been cleared yet.
 pybind11::tuple decode(const Tensor& kc, const Tensor& vc, const Tensor& selected, const std::optional<Tensor>& norms,
                        const pybind11::object& kept, Tensor q1, Tensor k1, Tensor v1, int64_t length, int64_t exempt, bool y_low) {
   TORCH_CHECK_VALUE(kc.dim() == 4 && selected.dim() == 3, "the cache must be (B, H, capacity, D) with (B, G, capacity) `selected`");
@@ -319,10 +321,11 @@ pybind11::tuple decode(const Tensor& kc, const Tensor& vc, const Tensor& selecte
   const c10::cuda::CUDAGuard guard(kc.device());
   void* const stream = stream_of(kc);
   const auto selected_at = reinterpret_cast<uint64_t>(selected.data_ptr()), stream_at = reinterpret_cast<uint64_t>(stream);
-  const size_t need = sa_decode_workspace_bytes((int)b, (int)h, (int)groups, (int)(capacity - 1), (int)d);
+  const bool captured = at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None;
+  const size_t need = sa_decode_workspace_bytes((int)b, (int)h, (int)groups, (int)(captured ? length : capacity - 1), (int)d);
   const uint64_t layout = ((uint64_t)(b * h) << 32) + (uint64_t)(b * groups);      // with the capacity: where the tickets are
   Tensor workspace;
-  if (PyTuple_Check(kept.ptr()) && PyTuple_GET_SIZE(kept.ptr()) == 5) {
+  if (!captured && PyTuple_Check(kept.ptr()) && PyTuple_GET_SIZE(kept.ptr()) == 5) {
     auto number = [&](int i) { return PyLong_AsUnsignedLongLongMask(PyTuple_GET_ITEM(kept.ptr(), i)); };
     if (THPVariable_Check(PyTuple_GET_ITEM(kept.ptr(), 0)) && number(1) == selected_at && number(2) == stream_at &&
         number(3) == layout && number(4) == (uint64_t)capacity) {
@@ -346,7 +349,7 @@ pybind11::tuple decode(const Tensor& kc, const Tensor& vc, const Tensor& selecte
     a.batch = (int32_t)b; a.heads = (int32_t)h; a.groups = (int32_t)groups; a.capacity = (int32_t)capacity; a.head_dim = (int32_t)d;
     a.length = (int32_t)length;
     a.exempt = (int32_t)exempt;
-    a.tickets_zero = fresh ? 2 : 1;
+    a.tickets_zero = captured ? 0 : fresh ? 2 : 1;
     a.q1 = q1.data_ptr(); a.k1 = k1.data_ptr(); a.v1 = v1.data_ptr();
     a.k_cache = kc.data_ptr(); a.v_cache = vc.data_ptr(); a.selected = selected.data_ptr<float>();
     a.key_norms = norms ? norms->data_ptr<float>() : nullptr;
@@ -357,7 +360,7 @@ pybind11::tuple decode(const Tensor& kc, const Tensor& vc, const Tensor& selecte
     check("sa_decode_step", sa_decode_run(&a));
   }
   pybind11::object keep = pybind11::none();
-  if (fresh) keep = pybind11::make_tuple(workspace, selected_at, stream_at, layout, capacity);
+  if (fresh && !captured) keep = pybind11::make_tuple(workspace, selected_at, stream_at, layout, capacity);
   return pybind11::make_tuple(y, keep);
 }
 

@@ -1,5 +1,5 @@
-"""What callers do with a decode cache besides stepping it: copy and save it, give it other tensors or another
-stream.  Every form is compared with a cache that holds nothing but the tensors."""
+"""What callers do with a decode cache besides stepping it: copy and save it, give it other tensors or another stream, capture a
+step.  Every form is compared with a cache that holds nothing but the tensors."""
 
 import copy
 import io
@@ -97,3 +97,30 @@ def test_steps_on_one_stream_and_then_on_another():
         torch.cuda.synchronize()
         assert torch.equal(got, slot.step_cache(*_rows(seed), bare))
 
+
+def test_a_step_captured_first_leaves_nothing_behind():
+    """The first step of a cache is captured in a pool whose memory holds ones; the eager step after it, and the graph's
+    replays, find their scratch as they need it."""
+    slot, cache = _cache()
+    slot.step_cache(*_rows(0), _bare(cache))                 # the library's set-up on this device
+    bare, length = _bare(cache), cache["len"]
+    dirty, graph = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(dirty):
+        torch.ones(250_000, device="cuda")                   # below 1 MiB: where the allocator puts small requests
+    dirty.replay()
+    q, k, v = _rows(7)
+    with torch.cuda.graph(graph, pool=dirty.pool()):
+        y = slot.step_cache(q, k, v, cache)
+    cache["len"] = length
+    dirty.replay()
+    _same(slot, cache, bare, [8])
+    again = _bare(cache)
+    for key in ("k", "v", "selected", "key_norms"):
+        cache[key].copy_(again[key])
+    again["len"] = length                                    # where the graph's step stands
+    for _ in range(2):
+        dirty.replay()
+        graph.replay()
+        assert torch.equal(y, slot.step_cache(q, k, v, again))
+        assert torch.equal(cache["selected"], again["selected"])
+        again["len"] = length
