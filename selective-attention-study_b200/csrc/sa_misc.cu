@@ -708,14 +708,17 @@ int cache_store(int dtype, int batch, int heads, int groups, int seq, int capaci
   if (((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0) return SA_ERR_ALIGNMENT;
   if ((int64_t)batch * heads > 65535) return SA_ERR_UNSUPPORTED;
   const int es = dtype == SA_F32 ? 4 : 2;
-  // A chunk whose rows are dense per head, heads at one pitch, is a plain 2-D copy: no kernel of ours.
-  auto pitched = [&](const RowLayout& r) { return r.st == head_dim && (batch == 1 || r.sb == heads * r.sh); };
-  if (!begin && pitched(k_rows) && pitched(v_rows)) {
-    const size_t row = (size_t)head_dim * es, width = seq * row, dst_pitch = capacity * row, nrows = (size_t)batch * heads;
-    const size_t k_pitch = nrows == 1 ? width : k_rows.sh * (size_t)es, v_pitch = nrows == 1 ? width : v_rows.sh * (size_t)es;
-    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(k_cache) + at * row, dst_pitch, k, k_pitch, width, nrows,
+  // A chunk whose rows are dense per head, heads at one pitch, is a plain 2-D copy: no kernel of ours.  The pitch has to be one
+  // that the copy takes: not less than a row of it (keys broadcast over heads have a pitch of 0), and below 2^31.
+  const size_t row = (size_t)head_dim * es, width = seq * row, dst_pitch = capacity * row, nrows = (size_t)batch * heads;
+  auto pitch = [&](const RowLayout& r) -> size_t { return nrows == 1 ? width : (size_t)(r.sh * es); };
+  auto pitched = [&](const RowLayout& r) {
+    return r.st == head_dim && (batch == 1 || r.sb == heads * r.sh) && r.sh >= 0 && pitch(r) >= width && pitch(r) < (1u << 31);
+  };
+  if (!begin && dst_pitch < (1u << 31) && pitched(k_rows) && pitched(v_rows)) {
+    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(k_cache) + at * row, dst_pitch, k, pitch(k_rows), width, nrows,
                                     cudaMemcpyDeviceToDevice, s));
-    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(v_cache) + at * row, dst_pitch, v, v_pitch, width, nrows,
+    SA_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(v_cache) + at * row, dst_pitch, v, pitch(v_rows), width, nrows,
                                     cudaMemcpyDeviceToDevice, s));
     return SA_OK;
   }

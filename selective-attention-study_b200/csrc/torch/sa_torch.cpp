@@ -282,7 +282,8 @@ Tensor prefill_rows(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, 
 }
 
 // New keys and values into the cache from position `at` on; `begin`: the first ones, with zeros behind them (and in `selected`).
-// False where the rows are not of the cache's type and device with a contiguous last axis: the caller copies.
+// False where the rows are not of the cache's type and device with a contiguous last axis, or are a view of the cache: the
+// caller copies.
 bool store_rows(const Tensor& kc, const Tensor& vc, const Tensor& selected, const Tensor& k, const Tensor& v, int64_t at, bool begin) {
   const int64_t d = kc.size(3);
   if (!kc.is_cuda() || code_of(kc) < 0 || vc.scalar_type() != kc.scalar_type() || k.scalar_type() != kc.scalar_type() ||
@@ -290,6 +291,8 @@ bool store_rows(const Tensor& kc, const Tensor& vc, const Tensor& selected, cons
       v.stride(3) != 1 || !kc.is_contiguous() || !vc.is_contiguous() || !selected.is_contiguous() || kc.size(0) * kc.size(1) > 65535 ||
       (d != 16 && d != 32 && d != 64 && d != 128))
     return false;
+  for (const Tensor* x : {&k, &v})
+    if (x->is_alias_of(kc) || x->is_alias_of(vc)) return false;
   const c10::cuda::CUDAGuard guard(kc.device());
   const sa_tensor kr = rows_of(k), vr = rows_of(v);
   check("sa_cache_store", sa_cache_store(code_of(kc), (int)kc.size(0), (int)kc.size(1), (int)selected.size(1), (int)k.size(2),

@@ -124,3 +124,83 @@ def test_a_step_captured_first_leaves_nothing_behind():
         assert torch.equal(y, slot.step_cache(q, k, v, again))
         assert torch.equal(cache["selected"], again["selected"])
         again["len"] = length
+
+
+def _broadcast(x):
+    return x[:, :1].expand(B, H, -1, -1)
+
+
+def _broadcast_all(x):
+    return x[:1, :1].expand(B, H, -1, -1)
+
+
+def _overlapping(x):                              # every head one token further along the same rows
+    n = x.shape[2]
+    rows = x.reshape(B, H * n, D).contiguous()
+    return rows.as_strided((B, H, n, D), (rows.stride(0), D, D, 1))
+
+
+def _token_major(x):                              # (B, T, H, D) memory
+    return x.transpose(1, 2).contiguous().transpose(1, 2)
+
+
+def _misaligned(x):
+    n = x.numel()
+    flat = torch.empty(n + 3, dtype=x.dtype, device=x.device)
+    flat[3:] = x.reshape(-1)
+    return flat[3:].view(x.shape)
+
+
+def _odd_pitch(x):                                # rows of D + 2 elements
+    wide = torch.zeros(*x.shape[:3], D + 2, dtype=x.dtype, device=x.device)
+    wide[..., :D] = x
+    return wide[..., :D]
+
+
+@pytest.mark.parametrize("form", [_broadcast, _broadcast_all, _overlapping, _token_major, _misaligned, _odd_pitch])
+@pytest.mark.parametrize("n", [1, 20])
+def test_new_rows_of_any_strides(form, n):
+    slot, cache = _cache()
+    bare, length = _bare(cache), cache["len"]
+    q, k, v = _rows(9, n)
+    k, v = form(k), form(v)
+    got = slot.extend_cache(q, k, v, cache)
+    want = slot.extend_cache(q, k.contiguous(), v.contiguous(), bare)
+    assert torch.equal(got, want)
+    for key in ("k", "v", "selected", "key_norms"):
+        assert torch.equal(cache[key], bare[key]), key
+    assert torch.equal(cache["k"][:, :, length:length + n], k) and torch.equal(cache["v"][:, :, length:length + n], v)
+    assert not cache["k"][:, :, length + n:].any() and not cache["v"][:, :, length + n:].any()
+    torch.cuda.synchronize()
+    assert torch.ones(3, device="cuda").sum() == 3           # no error of a refused copy left for the next call
+    # one sequence: the batch stride says nothing about the heads'
+    slot, one = mixers.SelectiveAttentionSlot(n_heads=H, context_length=CAPACITY), {}
+    for key in ("k", "v", "selected"):
+        one[key] = bare[key][:1].contiguous()
+    one["len"] = length
+    two = {key: (x.clone() if torch.is_tensor(x) else x) for key, x in one.items()}
+    assert torch.equal(slot.extend_cache(q[:1], k[:1], v[:1], one), slot.extend_cache(q[:1], k[:1].contiguous(), v[:1].contiguous(), two))
+    assert torch.equal(one["k"], two["k"]) and torch.equal(one["v"], two["v"])
+
+
+def test_new_rows_that_were_written_into_the_cache():
+    slot, cache = _cache()
+    bare, length, n = _bare(cache), cache["len"], 17
+    q, k, v = _rows(10, n)
+    for key, x in (("k", k), ("v", v)):
+        cache[key][:, :, length:length + n] = x
+    rows = [cache[key][:, :, length:length + n] for key in ("k", "v")]
+    assert torch.equal(slot.extend_cache(q, *rows, cache), slot.extend_cache(q, k, v, bare))
+    assert torch.equal(cache["k"], bare["k"]) and torch.equal(cache["v"], bare["v"])
+
+
+@pytest.mark.parametrize("form", [torch.clone, _broadcast, _token_major, _odd_pitch])
+def test_a_new_cache_is_zero_behind_its_prompt(form):
+    for x in [torch.full((B, H, CAPACITY, D), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2)]:
+        del x                                     # memory that the cache may be given
+    q, k, v = _rows(11, 130)
+    slot = mixers.SelectiveAttentionSlot(n_heads=H, context_length=CAPACITY)
+    _, cache = slot.begin_cache(q, form(k), form(v))
+    for key in ("k", "v", "selected"):
+        assert not cache[key][:, :, 130:].any()
+    assert torch.equal(cache["k"][:, :, :130], form(k)) and torch.equal(cache["v"][:, :, :130], form(v))
