@@ -78,7 +78,8 @@ struct PairSmem {
 constexpr uint32_t kDV = 0, kDK = 64, kDQ = 128, kDK0 = 448, kKA = 448, kVA = 480;
 constexpr int DQ0 = DQ + 1;           // completes per tile like DQ
 
-template <bool SELF, bool LIVE>   // LIVE: a table of live tiles is given (sa_tc_skip.cu)
+// LIVE: a table of live tiles is given (sa_tc_skip.cu).  ANY: rows of dk, dv that are not 16-byte aligned.
+template <bool SELF, bool LIVE, bool ANY>
 __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
         uint32_t r0[32];
         tmem_ld32(lane_base + kDK0 + 32 * x, r0);
         tmem_ld_wait();
-        if (j < seq) store_key_grads<false, 32>(nullptr, nullptr, r0, scale, nullptr, nullptr, row + 32 * x, false);
+        if (j < seq) store_key_grads<false, 32, ANY>(nullptr, nullptr, r0, scale, nullptr, nullptr, row + 32 * x, false);
       }
     }
     if (lane == 0) bulk_wait_all();                               // the last reduce-adds must land before the CTA exits
@@ -435,9 +436,9 @@ __global__ void __launch_bounds__(kThreads, 1) backward_kernel(
       tmem_ld_wait();
       if (j < seq) {
         if (c == 0)
-          store_key_grads<SELF, 32>(r, nullptr, nullptr, scale, dv + dv_rows.at(b, h, j) + 32 * x, nullptr, nullptr, false);
+          store_key_grads<SELF, 32, ANY>(r, nullptr, nullptr, scale, dv + dv_rows.at(b, h, j) + 32 * x, nullptr, nullptr, false);
         else
-          store_key_grads<SELF, 32>(nullptr, r, nullptr, scale, nullptr, dk + dk_rows.at(b, h, j) + 32 * x,
+          store_key_grads<SELF, 32, ANY>(nullptr, r, nullptr, scale, nullptr, dk + dk_rows.at(b, h, j) + 32 * x,
                                     dk0 + ((int64_t)b * seq + j) * D + 32 * x, SELF || (h == 0 && dq0_rows != 1));
       }
     }
@@ -489,8 +490,11 @@ int backward(const Problem& p, const float* stats, const float* carry, const voi
         p.dk_rows, p.dv_rows, alive);
     return SA_OK;
   };
-  if (alive != nullptr) st = self ? launch(backward_kernel<true, true>) : launch(backward_kernel<false, true>);
-  else st = self ? launch(backward_kernel<true, false>) : launch(backward_kernel<false, false>);
+  // (the live-tile entry points, like all that take the caller's layout, ask for 16-byte aligned rows)
+  if (alive != nullptr) st = self ? launch(backward_kernel<true, true, false>) : launch(backward_kernel<false, true, false>);
+  else if (((reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15) != 0)
+    st = self ? launch(backward_kernel<true, false, true>) : launch(backward_kernel<false, false, true>);
+  else st = self ? launch(backward_kernel<true, false, false>) : launch(backward_kernel<false, false, false>);
   if (st != SA_OK) return st;
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;

@@ -80,22 +80,35 @@ __device__ __forceinline__ void find_top_tile(const uint8_t* alive, int n, int n
   if (lane == 0) *top = found;
 }
 
+// Eight bf16 of a gradient row.  ANY: the row is at any address of an element (what the plain entry points take).
+template <bool ANY>
+__device__ __forceinline__ void store8(__nv_bfloat16* to, uint4 w) {
+  if constexpr (!ANY) {
+    *reinterpret_cast<uint4*>(to) = w;
+  } else {
+    const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+    uint16_t* out = reinterpret_cast<uint16_t*>(to);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) out[u] = (uint16_t)(x[u >> 1] >> (16 * (u & 1)));
+  }
+}
+
 // N columns of one key row's gradients from the accumulators: dV in bf16, dK and dK0 scaled.  dK0 is added to the selecting
 // head's fp32 rows (every head of the sequence adds its share); `own` says that dK belongs there too (head 0, whose dk is
 // that sum), otherwise dK goes out in bf16.  SELF: dK holds both gradient paths and no one else adds to the row.
-template <bool SELF, int N>
+template <bool SELF, int N, bool ANY>
 __device__ __forceinline__ void store_key_grads(const uint32_t* rv, const uint32_t* rk, const uint32_t* r0, float scale,
                                                 __nv_bfloat16* dv_row, __nv_bfloat16* dk_row, float* dk0_row, bool own) {
 #pragma unroll
   for (int e = 0; e < N; e += 8) {
     auto f = [&](const uint32_t* r, int u) { return __uint_as_float(r[e + u]); };
     if (rv != nullptr)
-      *reinterpret_cast<uint4*>(dv_row + e) = make_uint4(pack_bf16(f(rv, 0), f(rv, 1)), pack_bf16(f(rv, 2), f(rv, 3)),
-                                                         pack_bf16(f(rv, 4), f(rv, 5)), pack_bf16(f(rv, 6), f(rv, 7)));
+      store8<ANY>(dv_row + e, make_uint4(pack_bf16(f(rv, 0), f(rv, 1)), pack_bf16(f(rv, 2), f(rv, 3)),
+                                         pack_bf16(f(rv, 4), f(rv, 5)), pack_bf16(f(rv, 6), f(rv, 7))));
     if (rk != nullptr && !own)
-      *reinterpret_cast<uint4*>(dk_row + e) =
-          make_uint4(pack_bf16(f(rk, 0) * scale, f(rk, 1) * scale), pack_bf16(f(rk, 2) * scale, f(rk, 3) * scale),
-                     pack_bf16(f(rk, 4) * scale, f(rk, 5) * scale), pack_bf16(f(rk, 6) * scale, f(rk, 7) * scale));
+      store8<ANY>(dk_row + e,
+                  make_uint4(pack_bf16(f(rk, 0) * scale, f(rk, 1) * scale), pack_bf16(f(rk, 2) * scale, f(rk, 3) * scale),
+                             pack_bf16(f(rk, 4) * scale, f(rk, 5) * scale), pack_bf16(f(rk, 6) * scale, f(rk, 7) * scale)));
 #pragma unroll
     for (int q = 0; q < 8; q += 4) {
       if (SELF) {

@@ -57,7 +57,8 @@ struct Layout {
 // TMEM columns (W1, W2: sa_tc_bwd_chain.cuh)
 constexpr uint32_t kDV = 0, kDK = 64, kDQT = 128, kDK0 = 448, kVA = 448;
 
-template <bool SELF, bool LIVE>   // LIVE: a table of live tiles is given (sa_tc_skip.cu)
+// LIVE: a table of live tiles is given (sa_tc_skip.cu).  ANY: rows of dk, dv that are not 16-byte aligned.
+template <bool SELF, bool LIVE, bool ANY>
 __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
           uint32_t r0[16];
           tmem_ld16(lane_base + kDK0 + 16 * x, r0);
           tmem_ld_wait();
-          if (j < seq) store_key_grads<false, 16>(nullptr, nullptr, r0, scale, nullptr, nullptr, row + 16 * x, false);
+          if (j < seq) store_key_grads<false, 16, ANY>(nullptr, nullptr, r0, scale, nullptr, nullptr, row + 16 * x, false);
         }
       }
     }
@@ -419,9 +420,9 @@ __global__ void __launch_bounds__(kThreads, 1) backward_wide_kernel(
       if (j < seq) {
         const int col = dh * 64 + 32 * x;
         if (c == 0)
-          store_key_grads<SELF, 32>(r, nullptr, nullptr, scale, dv + dv_rows.at(b, h, j) + col, nullptr, nullptr, false);
+          store_key_grads<SELF, 32, ANY>(r, nullptr, nullptr, scale, dv + dv_rows.at(b, h, j) + col, nullptr, nullptr, false);
         else
-          store_key_grads<SELF, 32>(nullptr, r, nullptr, scale, nullptr, dk + dk_rows.at(b, h, j) + col,
+          store_key_grads<SELF, 32, ANY>(nullptr, r, nullptr, scale, nullptr, dk + dk_rows.at(b, h, j) + col,
                                     dk0 + ((int64_t)b * seq + j) * D + col, SELF || (h == 0 && dq0_rows != 1));
       }
     }
@@ -473,8 +474,11 @@ int backward_wide(const Problem& p, const float* stats, const float* carry, cons
                                         ntiles, p.exempt, p.scale, status, p.dk_rows, p.dv_rows, alive);
     return SA_OK;
   };
-  if (alive != nullptr) st = self ? launch(backward_wide_kernel<true, true>) : launch(backward_wide_kernel<false, true>);
-  else st = self ? launch(backward_wide_kernel<true, false>) : launch(backward_wide_kernel<false, false>);
+  // (the live-tile entry points, like all that take the caller's layout, ask for 16-byte aligned rows)
+  if (alive != nullptr) st = self ? launch(backward_wide_kernel<true, true, false>) : launch(backward_wide_kernel<false, true, false>);
+  else if (((reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15) != 0)
+    st = self ? launch(backward_wide_kernel<true, false, true>) : launch(backward_wide_kernel<false, false, true>);
+  else st = self ? launch(backward_wide_kernel<true, false, false>) : launch(backward_wide_kernel<false, false, false>);
   if (st != SA_OK) return st;
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;
