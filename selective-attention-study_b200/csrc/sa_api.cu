@@ -595,7 +595,20 @@ int sa_prefill_rows(const sa_problem* in, int cached, const void* q, const void*
     if ((reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return SA_ERR_ALIGNMENT;
     p.split_scratch = static_cast<float*>(scratch);
   }
-  return tc_forward(p, nullptr, lse2, carry, selected, static_cast<cudaStream_t>(stream));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (cached == 0) return tc_forward(p, nullptr, lse2, carry, selected, s);
+  // The history moves on last: a call that fails leaves it where the cache's length is.  The totals are the last row of carry.
+  const size_t seq = in->seq, pitch = (size_t)sa_carry_checkpoints(in->engine, in->seq) * seq;
+  st = tc_forward(p, nullptr, lse2, carry, nullptr, s);
+  if (st != SA_OK) return st;
+  const float* totals = carry + pitch - seq;
+  if (pitch * 4 < (1u << 31) && (size_t)selected_stride * 4 < (1u << 31)) {          // (the pitches that a 2-D copy takes)
+    SA_CUDA_CHECK(cudaMemcpy2DAsync(selected, selected_stride * 4, totals, pitch * 4, seq * 4, in->batch, cudaMemcpyDeviceToDevice, s));
+  } else {
+    for (int b = 0; b < in->batch; ++b)
+      SA_CUDA_CHECK(cudaMemcpyAsync(selected + b * selected_stride, totals + b * pitch, seq * 4, cudaMemcpyDeviceToDevice, s));
+  }
+  return SA_OK;
 }
 
 int sa_cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, int begin,

@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, fl
     run += x;
   }
   col[(int64_t)ntiles * seq] = run;
-  total[(int64_t)b * total_stride + j] = run;                    // (a continued prefill: where `init` was)
+  if (total != nullptr) total[(int64_t)b * total_stride + j] = run;
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -5,7 +5,7 @@ import ctypes
 import pytest
 import torch
 
-from selective_attention_b200 import _lib, kernels
+from selective_attention_b200 import _lib, kernels, mixers
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +45,53 @@ def test_backward_writes_gradients_at_any_element(heads, dim):
     for other in got[1:]:
         for a, ref in zip(other, got[0]):
             assert float((a - ref).norm() / ref.norm()) < 2e-3         # the order of the fp32 reductions
+
+
+def _pointer_arguments(driver, node):
+    """The 8-byte arguments of a graph's kernel node."""
+    err, params = driver.cuGraphKernelNodeGetParams(node)
+    assert err == 0
+    values = ctypes.cast(params.kernelParams, ctypes.POINTER(ctypes.c_void_p))
+    found, i = [], 0
+    while True:
+        err, _, size = driver.cuFuncGetParamInfo(params.func, i)
+        if err != 0:
+            return found
+        if size == 8:
+            found.append(ctypes.cast(values[i], ctypes.POINTER(ctypes.c_uint64))[0])
+        i += 1
+
+
+@pytest.mark.parametrize("heads,dim,per_head,skip", [(2, 64, False, False), (2, 64, True, True), (160, 64, False, True), (2, 128, False, False)])
+def test_the_history_of_a_cache_moves_on_last(heads, dim, per_head, skip):
+    """A chunk whose call fails must not leave its selection behind, or trying again would count it twice: nothing but the last
+    launch of the call is given the history to write."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    g = torch.Generator("cpu").manual_seed(3)
+    first, total = 300, 330
+    q, k, v = (torch.randn(1, heads, total, dim, generator=g).bfloat16().cuda() for _ in range(3))
+    slot = mixers.SelectiveAttentionSlot(n_heads=heads, context_length=total, per_head=per_head)
+    _, cache = slot.begin_cache(*(x[:, :, :first] for x in (q, k, v)))
+    new = [x[:, :, first:] for x in (q, k, v)]
+    want = {key: (x.clone() if torch.is_tensor(x) else x) for key, x in cache.items()}
+    slot.extend_cache(*new, want, skip_dead_tiles=skip)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        slot.extend_cache(*new, cache, skip_dead_tiles=skip)
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = {int(n): n for n in driver.cuGraphGetNodes(raw, driver.cuGraphGetNodes(raw)[2])[1]}
+    _, sources, targets, *_ = driver.cuGraphGetEdges(raw, driver.cuGraphGetEdges(raw)[-1])
+    follows = {int(a): int(b) for a, b in zip(sources, targets)}
+    node = next(n for n in nodes if n not in set(follows.values()))
+    order = [node]
+    while node in follows:
+        order.append(node := follows[node])
+    assert len(order) == len(nodes)                             # one stream: a chain
+    kernel, copy = driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL, driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_MEMCPY
+    types = [driver.cuGraphNodeGetType(nodes[n])[1] for n in order]
+    history = cache["selected"].data_ptr()
+    given = sum(_pointer_arguments(driver, nodes[n]).count(history) for n, kind in zip(order, types) if kind == kernel)
+    assert given == 1                                           # the scan reads it
+    assert types[-1] == copy and int(driver.cuGraphMemcpyNodeGetParams(nodes[order[-1]])[1].dstDevice) == history
+    graph.replay()
+    assert torch.equal(cache["selected"], want["selected"])
