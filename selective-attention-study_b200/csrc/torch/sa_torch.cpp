@@ -10,6 +10,8 @@
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+
 #include "../../../include/selective_attention_b200.h"
 
 namespace {
@@ -132,9 +134,11 @@ void run_backward(const sa_problem& p, const Tensor& q, const Tensor& k, const T
   check("sa_backward", st, true);
 }
 
-// The backward is written by hand: a second differentiation through it raises.
-variable_list once_differentiable(variable_list grads) {
+// The backward is written by hand: a second differentiation through it raises.  A cotangent without a graph of its own has none
+// to be differentiated through.
+variable_list once_differentiable(const variable_list& grad_out, variable_list grads) {
   if (!c10::GradMode::is_enabled()) return grads;
+  if (std::none_of(grad_out.begin(), grad_out.end(), [](const Tensor& g) { return g.defined() && g.requires_grad(); })) return grads;
   variable_list fake;
   size_t n = 0;
   for (auto& g : grads)
@@ -197,7 +201,7 @@ struct Attend : public torch::autograd::Function<Attend> {
         grads[i] = all[i]->scalar_type() == want ? *all[i] : all[i]->to(want);
       }
     }
-    return once_differentiable(std::move(grads));
+    return once_differentiable(grad_out, std::move(grads));
   }
 };
 
@@ -241,7 +245,7 @@ struct AttendPacked : public torch::autograd::Function<AttendPacked> {
       run_backward(p, q, k, v, saved[1], at_, saved[2], d_out, part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2));
       grads[0] = d_qkv;
     }
-    return once_differentiable(std::move(grads));
+    return once_differentiable(grad_out, std::move(grads));
   }
 };
 

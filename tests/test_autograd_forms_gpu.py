@@ -26,6 +26,7 @@ def _packed(q, k, v):
     return kernels.selective_attention_packed(torch.stack([x.transpose(1, 2) for x in (q, k, v)], dim=2)).float()
 
 
+@pytest.mark.filterwarnings("ignore")              # what tracing says of shapes and of itself
 @pytest.mark.parametrize("call,dtype,dim", [(_plain, torch.bfloat16, 64), (_plain, torch.float32, 32), (_layer, torch.bfloat16, 64),
                                             (_packed, torch.bfloat16, 64)])
 def test_a_traced_call_follows_its_inputs(call, dtype, dim):
@@ -67,3 +68,17 @@ def test_saved_tensors_may_be_moved():
         out = kernels.selective_attention(*x)
     for a, b in zip(torch.autograd.grad(out.sum(), x), want):
         assert float((a.float() - b.float()).norm() / b.float().norm()) < 2e-3
+
+
+@pytest.mark.parametrize("call", [_plain, _layer, _packed])
+def test_gradients_kept_for_a_graph_are_constants_where_the_cotangent_is_one(call):
+    """create_graph with a cotangent that has no graph: the gradients are plain tensors, and what is built on them can be
+    differentiated with respect to everything else."""
+    x = [t.requires_grad_(True) for t in _inputs(6)]
+    scale = torch.ones((), device="cuda", requires_grad=True)
+    out = call(*x)
+    for create_graph in (False, True):
+        (dq,) = torch.autograd.grad(out, x[:1], torch.ones_like(out), create_graph=create_graph, retain_graph=True)
+        assert not dq.requires_grad
+    (scale * dq.float()).square().sum().backward()
+    assert torch.isfinite(scale.grad) and scale.grad > 0
