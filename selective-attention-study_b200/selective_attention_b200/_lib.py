@@ -57,6 +57,7 @@ _lib = None
 
 
 def available() -> bool:
+    """Whether the Python entry points have what they need: the library, and the extension that calls it."""
     return os.path.exists(LIB_PATH) and os.path.exists(os.path.join(HERE, "_native.so"))
 
 
@@ -77,7 +78,7 @@ def load() -> ctypes.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    if not available():
+    if not os.path.exists(LIB_PATH):
         raise RuntimeError(f"{LIB_PATH} is missing: build it with `python -m selective_attention_b200.build` "
                            "(there is no fallback path)")
     lib = ctypes.CDLL(LIB_PATH)

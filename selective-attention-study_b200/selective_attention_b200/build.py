@@ -1,9 +1,10 @@
-"""Compile the CUDA sources under csrc/ into one shared library for sm_100a, in-tree.
+"""Compile the CUDA sources under csrc/ into one shared library for sm_100a, in-tree, and the torch extension beside it.
 
-    python -m selective_attention_b200.build [--force] [--verbose]
+    python -m selective_attention_b200.build [--library] [--force] [--verbose]
 
 nvcc cross-compiles without a GPU.  The library sits beside this file so that it ships with the
-source tree; nothing is installed into site-packages and nothing is JIT-cached elsewhere.
+source tree; nothing is installed into site-packages and nothing is JIT-cached elsewhere.  ``--library`` builds the C library
+alone, which needs neither torch nor its headers (run this file by its path where torch is not installed).
 """
 
 from __future__ import annotations
@@ -72,8 +73,13 @@ def nvcc_path() -> str:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    path = build_library(force, verbose)
+    build_native(force)
+    return path
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
-        build_native(force)
         return LIB_PATH
     objs = []
     obj_dir = os.path.join(os.path.dirname(HERE), "build")
@@ -100,9 +106,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}")
-    build_native(force)
     return LIB_PATH
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    make = build_library if "--library" in sys.argv else build
+    print(make(force="--force" in sys.argv, verbose="--verbose" in sys.argv))

@@ -156,3 +156,30 @@ def test_selector_and_packed_arguments_are_validated_in_python():
     with pytest.raises(ValueError, match="carry_rows"):
         kernels._carry_rows_request(64)
     assert kernels._carry_rows_request(None) is None and kernels._carry_rows_request(32) == 32
+
+
+def test_the_c_library_needs_no_torch_extension():
+    """A C caller's build and load of the library ask for nothing of torch; the Python entry points say what is missing."""
+    import subprocess
+    import sys
+
+    package = os.path.join(ROOT, "selective-attention-study_b200", "selective_attention_b200")
+    code = f"""
+import importlib.abc, importlib.util, os, sys
+class NoTorch(importlib.abc.MetaPathFinder):
+    def find_spec(self, name, path=None, target=None):
+        if name.split(".")[0] == "torch":
+            raise ImportError("no torch here")
+sys.meta_path.insert(0, NoTorch())
+def load(name):
+    spec = importlib.util.spec_from_file_location(name, os.path.join({package!r}, name + ".py"))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+assert load("build").build_library() == load("_lib").LIB_PATH
+exists = os.path.exists
+os.path.exists = lambda path: not str(path).endswith("_native.so") and exists(path)
+lib = load("_lib")
+assert lib.load().sa_abi_version() == 3 and not lib.available()
+"""
+    subprocess.run([sys.executable, "-c", code], check=True)
