@@ -56,7 +56,9 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   if (!dim_ok(in->head_dim)) return SA_ERR_UNSUPPORTED;
   if (in->damp < SA_DAMP_NONE || in->damp > SA_DAMP_SQRT) return SA_ERR_BAD_ARGUMENT;
   if (in->damp != SA_DAMP_NONE && in->train_len < 1) return SA_ERR_BAD_ARGUMENT;
-  // the CUDA-core kernels put (batch, head) rows on grid.y; the tensor-core kernels use 1-D grids
+  // Both selection passes have the batch on grid.y or grid.z; the other grids are 1-D.  (The CUDA-core engine has never taken
+  // more (batch, head) rows than that either.)
+  if (in->batch > 65535) return SA_ERR_UNSUPPORTED;
   if (in->engine == SA_ENGINE_SIMT && (int64_t)in->batch * in->heads > 65535) return SA_ERR_UNSUPPORTED;
   if ((int64_t)in->batch * in->heads * ((in->seq + 127) / 128) > 0x7fffffffLL) return SA_ERR_UNSUPPORTED;
   if (sel != nullptr && (sel->struct_bytes != (int32_t)sizeof(sa_selector) || !sel->q0 || !sel->k0))

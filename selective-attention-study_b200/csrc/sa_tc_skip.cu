@@ -110,11 +110,12 @@ __global__ void __launch_bounds__(kTile) tile_table_kernel(const float* __restri
 }  // namespace
 
 // Skipping is offered for bf16 operands at head_dim 64 / 128 up to 1024 tiles (the forward keeps a tile's list of live
-// key tiles in shared memory).
+// key tiles in shared memory) and 65535 rows (the norms have them on grid.y).
 size_t tile_table_bytes(const Problem& p) {
   const int64_t ntiles = (p.seq + kTile - 1) / kTile;
   if (p.dtype != SA_BF16 || (p.head_dim != 64 && p.head_dim != 128) || ntiles > 1024 || p.damp != SA_DAMP_NONE) return 0;
   const int64_t nrows = (int64_t)p.batch * p.heads;
+  if (nrows > 65535) return 0;
   const int64_t table = (nrows * ntiles * ntiles + 255) & ~(int64_t)255;
   return (size_t)(table + 2 * nrows * ntiles * 4);
 }

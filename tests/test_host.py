@@ -158,6 +158,20 @@ def test_selector_and_packed_arguments_are_validated_in_python():
     assert kernels._carry_rows_request(None) is None and kernels._carry_rows_request(32) == 32
 
 
+def test_problems_beyond_a_grid_are_refused_before_any_launch():
+    lib = _lib.load()
+    p = _lib.Problem()
+    p.struct_bytes = ctypes.sizeof(_lib.Problem)
+    p.dtype, p.seq, p.head_dim, p.exempt = 1, 130, 64, 1
+    args = (16, 16, 16, 16, 16, 16, 16, None)
+    for p.engine, p.batch, p.heads in ((1, 65536, 1), (0, 65536, 1), (0, 2, 40000)):
+        assert lib.sa_forward(ctypes.byref(p), *args) == 2 and lib.sa_backward_workspace_bytes(ctypes.byref(p)) == 0
+    p.engine, p.batch, p.heads = 1, 1, 65536                     # the rows have a limit of their own where tiles are left out
+    assert lib.sa_backward_workspace_bytes(ctypes.byref(p)) > 0 and lib.sa_tile_table_bytes(ctypes.byref(p)) == 0
+    p.heads = 65535
+    assert lib.sa_tile_table_bytes(ctypes.byref(p)) > 0
+
+
 def test_the_c_library_needs_no_torch_extension():
     """A C caller's build and load of the library ask for nothing of torch; the Python entry points say what is missing."""
     import subprocess
