@@ -150,16 +150,22 @@ __global__ void __launch_bounds__(256) fold_cast_kernel(const float* __restrict_
 // ---- decode -----------------------------------------------------------------------------------------
 constexpr int kDecThreads = 128;
 constexpr int kDecSplitMin = 128;             // keys per CTA: a multiple of 128, at least 128
+constexpr int kDecLiveSplit = 1024;           // with key norms
 constexpr int kDecSplitsMax = 256;            // of a long cache: more would make the merge long
 constexpr int kDecCtasPerSm = 4;              // attend CTAs resident per SM (48 KB of stages each)
 
 // Keys per CTA for `t` cached keys and `rows` = batch * heads query rows: the grid is about one full wave of
 // resident CTAs, so no SM is left with a straggler and the combine pass stays short.  With 512 keys at least, 96 rows of
 // 1,500 keys were 288 CTAs of three ring refills each and took 13.9 us; with 256 they fill the wave.
+static int decode_target_splits(int rows) { return max(1, min(tc::kSms * kDecCtasPerSm / rows, kDecSplitsMax)); }
 static int decode_split_keys(int t, int rows) {
-  const int target_splits = max(1, min(148 * kDecCtasPerSm / rows, kDecSplitsMax));
+  const int target_splits = decode_target_splits(rows);
   const int keys = (t + target_splits - 1) / target_splits;
   return (keys + kDecSplitMin - 1) / kDecSplitMin * kDecSplitMin;
+}
+// The most key ranges that a step over up to `t` keys can have, with key norms or without.
+static int decode_splits_max(int t, int rows) {
+  return max(min(decode_target_splits(rows), (t + kDecSplitMin - 1) / kDecSplitMin), (t + kDecLiveSplit - 1) / kDecLiveSplit);
 }
 
 // 16-byte load of 8 (bf16 / fp16) or two 16-byte loads of 8 fp32 elements, converted to fp32.
@@ -549,11 +555,11 @@ int decode_impl(const DecodeStep& d, cudaStream_t s) {
   const int rows = d.batch * d.heads, t = d.length + 1, D = d.head_dim;
   // With key norms most CTAs find nothing to stream and only the selecting heads stay dense: short key ranges (1024
   // keys; 512 and 2048 measured slower) then spread those heads over the whole GPU.
-  const int split_keys = (d.key_norms != nullptr) ? 1024 : decode_split_keys(t, rows);
+  const int split_keys = (d.key_norms != nullptr) ? kDecLiveSplit : decode_split_keys(t, rows);
   const int splits = (t + split_keys - 1) / split_keys;
   // Tickets first: where they are kept (`tickets_zero`), at a size that does not change from step to step, so that what the last CTAs leave at zero
   // is where the next step looks.
-  const int ticket_splits = d.tickets_zero ? (d.capacity + kDecSplitMin - 1) / kDecSplitMin : splits;
+  const int ticket_splits = d.tickets_zero ? decode_splits_max(d.capacity, rows) : splits;
   unsigned int* row_tickets = reinterpret_cast<unsigned int*>(d.workspace);
   unsigned int* split_tickets = row_tickets + rows;
   const size_t n_tickets = (size_t)rows + (size_t)d.batch * d.groups * ticket_splits;
@@ -735,7 +741,7 @@ int cache_store(int dtype, int batch, int heads, int groups, int seq, int capaci
 
 size_t decode_workspace_floats(int batch, int heads, int groups, int length, int head_dim) {
   const int t = length + 1;
-  const size_t splits = (size_t)(t + kDecSplitMin - 1) / kDecSplitMin;       // upper bound: the smallest split size
+  const size_t splits = decode_splits_max(t, batch * heads);
   return (size_t)batch * heads * splits * (head_dim + 2) + (size_t)batch * groups * t   // partials, new selection
          + (size_t)batch * heads + (size_t)batch * groups * splits;                       // tickets
 }

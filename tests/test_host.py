@@ -172,6 +172,21 @@ def test_problems_beyond_a_grid_are_refused_before_any_launch():
     assert lib.sa_tile_table_bytes(ctypes.byref(p)) > 0
 
 
+@pytest.mark.parametrize("batch,heads,groups,dim", [(1, 16, 1, 64), (8, 16, 16, 128), (1, 1, 1, 64), (40, 16, 4, 16)])
+def test_scratch_of_a_decode_step_covers_the_ranges_that_it_can_have(batch, heads, groups, dim):
+    """A partial sum per row and key range: one wave of CTAs, four an SM, at most 256 ranges of a row and none shorter than 128
+    keys; with key norms, ranges of 1024 keys.  It never shrinks as a cache grows."""
+    size, rows, last = _lib.load().sa_decode_workspace_bytes, batch * heads, 0
+    for length in [*range(0, 3000, 7), 4095, 4096, 30_000, 131_071, 131_072, 500_000]:
+        t = length + 1
+        dense = min(max(1, min(592 // rows, 256)), -(-t // 128))
+        splits = max(dense, -(-t // 1024))
+        need = size(batch, heads, groups, length, dim)
+        assert need == 4 * (rows * splits * (dim + 2) + batch * groups * t + rows + batch * groups * splits)
+        assert need >= last
+        last = need
+
+
 def test_the_c_library_needs_no_torch_extension():
     """A C caller's build and load of the library ask for nothing of torch; the Python entry points say what is missing."""
     import subprocess
