@@ -2,7 +2,8 @@
 device (fp32, TF32 off) because a (T, T) tensor at T = 16384 is 1 GiB.
 
 * whole forward + backward of one sequence at T = 16384, D = 64 and D = 128, bf16: out, dq, dk, dv and the per-key
-  totals, shared selection (three heads) and one head per selector, unit-variance inputs and low-scale q, k;
+  totals, shared selection (three heads) and one head per selector, unit-variance inputs and low-scale q, k: one head a
+  CTA in the forward; and again with two heads of a selector, or two rows that select for themselves, in one CTA;
 * the reference's CPU case exactly (B = 2, H = 4, T = 1024, D = 64, fp32, seed 0) at the fp32 bar;
 * forward rows from a MIDDLE query tile and from the tail, at T = 16384 with all sixteen heads and two
   sequences, and at T = 131072.
@@ -72,6 +73,28 @@ def test_forward_backward_at_16k_against_the_oracle(heads, dim, scale_qk, achiev
     for name, e in errs.items():
         assert e < 2e-2, (name, e)
     assert total_err < 2e-3
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 2), (2, 1)])    # two heads of a selector, two rows each its own
+@pytest.mark.parametrize("scale_qk", [1.0, 0.15, 0.02])
+def test_forward_backward_at_16k_with_two_heads_a_cta(batch, heads, scale_qk, achieved):
+    seq, dim = 16384, 64
+    q, k, v, w = (x.cuda() for x in _inputs((batch, heads, seq, dim), seed=1100 + heads, scale_qk=scale_qk))
+    qq, kk, vv = (t.clone().requires_grad_(True) for t in (q, k, v))
+    out = kernels.selective_attention(qq, kk, vv)
+    grads = torch.autograd.grad(out, (qq, kk, vv), w.float())
+    _, aux = kernels.selective_attention_forward(q, k, v, return_aux=True)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    for b in range(batch):
+        with _ExactMatmul():
+            want = oracle.sequence_fwd_bwd(*(x[b].float() for x in (q, k, v, w)), head_chunk=1)
+        errs = {name: _rel(got[b], ref) for name, got, ref in zip(("out", "dq", "dk", "dv"), (out.detach(), *grads), want)}
+        total_err = float((aux["selected_total"][b] - want[4]).abs().max() / want[4].abs().max().clamp_min(1e-6))
+        achieved(f"fwd+bwd T=16384 B={batch} H={heads} D=64 bf16 scale_qk={scale_qk} sequence {b}", total_max_rel=total_err, **errs)
+        for name, e in errs.items():
+            assert e < 2e-2, (name, e)                       # a NaN fails too
+        assert total_err < 2e-3
 
 
 def test_reference_cpu_case_on_the_gpu_fp32(achieved):

@@ -187,3 +187,45 @@ def test_unsupported_engines_ignore_the_request():
     a = kernels.selective_attention_forward(q, k, v, skip_dead_tiles=True)
     b = kernels.selective_attention_forward(q, k, v)
     assert torch.equal(a, b)
+
+
+# more than 148 (query tile, head) pairs: two heads of a selector, or two rows that select for themselves, in one CTA, which
+# takes the tiles that are live in either
+@pytest.mark.parametrize("batch,heads,seq", [(1, 12, 1700), (2, 6, 2049), (12, 1, 1700), (1, 38, 513)])
+def test_two_heads_a_cta_and_their_live_tiles(batch, heads, seq, achieved):
+    q, k, v, w = _inputs(batch, heads, seq, 64, seed=seq + heads)
+    q.view(batch * heads, seq, 64)[1::2] *= 0.1                # every other row has fewer live tiles than its neighbour
+    with torch.no_grad():
+        full, aux_full = kernels.selective_attention_forward(q.cuda(), k.cuda(), v.cuda(), return_aux=True)
+        lean, aux = kernels.selective_attention_forward(q.cuda(), k.cuda(), v.cuda(), return_aux=True, skip_dead_tiles=True)
+    live = _lower(aux["live_tiles"]) != 0
+    pairs = live.view(-1, 2, live.shape[-1])
+    achieved(f"live tiles T={seq} B={batch} H={heads} two heads a CTA", live_fraction=float(live.float().mean()),
+             in_one_of_two=float((pairs[:, 0] != pairs[:, 1]).float().mean()))
+    if seq > 1000:
+        assert not live.all() and bool((pairs[:, 0] != pairs[:, 1]).any())
+    assert torch.equal(lean, full)
+    assert torch.equal(aux["rmax"], aux_full["rmax"]) and torch.equal(aux["selected_total"], aux_full["selected_total"])
+    got, ref = _run(q, k, v, w, skip=True), _run(q, k, v, w, skip=False)
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[0], full)
+    want = oracle.attention_grads(q.float(), k.float(), v.float(), w.float())
+    for name, a, b, c in zip(("out", "dq", "dk", "dv"), got, ref, want):
+        assert _rel(a, b) < 2e-3, (name, _rel(a, b))           # the order of the fp32 reductions only
+        assert _rel(a.cpu(), c) < 2e-2, (name, _rel(a.cpu(), c))
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("heads,first,total", [(38, 1000, 1500), (76, 1920, 2200)])
+def test_two_heads_a_cta_leave_out_the_dead_part_of_a_cache(heads, first, total, per_head):
+    from selective_attention_b200 import mixers
+    g = torch.Generator("cpu").manual_seed(total)
+    q, k, v = (torch.randn(1, heads, total, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    slot = mixers.SelectiveAttentionSlot(n_heads=heads, context_length=total, per_head=per_head)
+    rows, sels = [], []
+    for skip in (False, True):
+        _, cache = slot.begin_cache(*(x[:, :, :first] for x in (q, k, v)))
+        rows.append(slot.extend_cache(*(x[:, :, first:] for x in (q, k, v)), cache, skip_dead_tiles=skip))
+        sels.append(cache["selected"])
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    assert torch.equal(rows[0], rows[1]) and torch.equal(sels[0], sels[1])
