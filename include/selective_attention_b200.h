@@ -360,7 +360,7 @@ int sa_profile_collect(float* ms_host, int capacity);
 unsigned long long sa_launch_count(void);
 
 /* Bounded device-side waits.  Every wait inside the tensor-core engine and the decode step gives up after a
- * fixed number of clock ticks (~0.2 s), records (site << 8) | 1 in a per-device word, and its kernel returns;
+ * fixed number of clock ticks or of tries (~0.2 s), records (site << 8) | 1 in a per-device word, and its kernel returns;
  * only the launch sequence that gave up is cut short.  The word is also mirrored into mapped host memory (one
  * pinned page per device, created by the first entry-point call on the device), so from then on every
  * sa_forward* / sa_backward* / sa_decode_step call on that device returns SA_ERR_DEVICE_TIMEOUT without
@@ -375,6 +375,10 @@ int sa_device_status(unsigned int* value_host, int clear);
  * limit of limit_kcycles * 1024 clock ticks (1 .. 100000), reports site 900 and returns.  The kernel
  * terminates by itself; nothing faults.  For testing the path above.  No counterpart in the reference. */
 int sa_selftest_wait_timeout(unsigned int limit_kcycles, void* stream);
+
+/* The same with the other form of a bounded wait, which counts tries of a few microseconds each: it gives up after `tries` of
+ * them (1 .. 50000, the kernels' own number), reports site 901, and a second wait of the same thread gives up at once. */
+int sa_selftest_wait_tries(unsigned int tries, void* stream);
 
 /* Known-answer test of the tcgen05 / TMA operand encodings the tensor-core engine uses.
  *   scratch  32 KiB of device memory, 1024-byte aligned

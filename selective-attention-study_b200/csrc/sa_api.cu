@@ -506,6 +506,11 @@ int sa_selftest_wait_timeout(unsigned int limit_kcycles, void* stream) {
   return tc::selftest_wait_timeout(limit_kcycles, static_cast<cudaStream_t>(stream));
 }
 
+int sa_selftest_wait_tries(unsigned int tries, void* stream) {
+  if (tries < 1u || tries > (unsigned int)tc::kWaitTries) return SA_ERR_BAD_ARGUMENT;
+  return tc::selftest_wait_tries(tries, static_cast<cudaStream_t>(stream));
+}
+
 int sa_selftest_tcgen05(void* scratch, float* result, void* stream) {
   if (!scratch || !result) return SA_ERR_BAD_ARGUMENT;
   if ((reinterpret_cast<uintptr_t>(scratch) & 1023) != 0) return SA_ERR_ALIGNMENT;

@@ -40,6 +40,20 @@ __global__ void wait_probe_kernel(WaitCtx ctx) {
   }
 }
 
+__global__ void tries_probe_kernel(WaitCtx ctx, int tries) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    mbar_init_fence();
+    Waiter wait;
+    wait.begin(ctx);
+    wait.left = min(wait.left, tries);
+    wait(smem_u32(&bar), 0, 901);      // nobody arrives: runs out after `tries` tries
+    wait(smem_u32(&bar), 0, 902);      // a single try, and the first site stays
+    wait.end(ctx);
+  }
+}
+
 }  // namespace
 
 NoHostAllocScope::NoHostAllocScope() { ++g_no_host_alloc; }
@@ -107,6 +121,15 @@ int selftest_wait_timeout(unsigned int limit_kcycles, cudaStream_t s) {
   if (rc != SA_OK) return rc;
   ctx.limit_kcycles = limit_kcycles;
   wait_probe_kernel<<<1, 32, 0, s>>>(ctx);
+  SA_CUDA_CHECK(cudaGetLastError());
+  return SA_OK;
+}
+
+int selftest_wait_tries(unsigned int tries, cudaStream_t s) {
+  WaitCtx ctx;
+  int rc = wait_ctx(&ctx);
+  if (rc != SA_OK) return rc;
+  tries_probe_kernel<<<1, 32, 0, s>>>(ctx, (int)tries);
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;
 }

@@ -79,6 +79,10 @@ struct WaitCtx {
   unsigned int limit_kcycles;  // a wait gives up after this many clock64 ticks / 1024
 };
 
+// Tries of a wait that counts them (Waiter): ~0.2 s; a failed try with a suspend-time hint of 1 us takes 4 us (200,000 of them
+// took 0.80 s).
+constexpr int kWaitTries = 50000;
+
 // Context for the next launch sequence on the current device: a fresh epoch and the default limit.  The
 // mapped host flag (one page of pinned host memory per device) is created on first use unless
 // `may_create_host_flag` is false (entry points that must not call an allocating routine), in which case the
@@ -98,6 +102,8 @@ int read_status(unsigned int* host_value, bool clear);
 // Runs one CTA that waits, with the given limit, on an mbarrier nobody arrives on: the wait runs out, reports
 // site 900 and the kernel returns.
 int selftest_wait_timeout(unsigned int limit_kcycles, cudaStream_t s);
+// The same with a wait that counts tries (Waiter), site 901.
+int selftest_wait_tries(unsigned int tries, cudaStream_t s);
 int selftest(void* scratch, float* result, cudaStream_t s);
 
 }  // namespace tc

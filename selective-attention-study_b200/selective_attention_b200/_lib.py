@@ -23,7 +23,7 @@ DAMP_CODES = {"none": 0, "linear": 1, "sqrt": 2}
 EXPORTS = ("sa_abi_version", "sa_status_string", "sa_last_cuda_error", "sa_engine_available", "sa_engine_supports", "sa_carry_rows", "sa_carry_checkpoints", "sa_forward",
            "sa_backward_workspace_bytes", "sa_backward", "sa_decode_workspace_bytes", "sa_decode_step", "sa_device_status", "sa_selftest_tcgen05", "sa_profile_enable",
            "sa_profile_collect", "sa_static_scratch_floats", "sa_forward_static_scratch", "sa_forward_selector",
-           "sa_backward_selector", "sa_forward_fused", "sa_backward_fused", "sa_prefill_extend", "sa_selection_carry", "sa_launch_count", "sa_selftest_wait_timeout",
+           "sa_backward_selector", "sa_forward_fused", "sa_backward_fused", "sa_prefill_extend", "sa_selection_carry", "sa_launch_count", "sa_selftest_wait_timeout", "sa_selftest_wait_tries",
            "sa_tile_table_bytes", "sa_forward_live_tiles", "sa_backward_live_tiles", "sa_prefill_extend_live_tiles", "sa_decode_step_live_keys",
            "sa_decode_run", "sa_prefill_scratch_bytes", "sa_prefill_rows", "sa_cache_store")
 
@@ -123,6 +123,8 @@ def load() -> ctypes.CDLL:
     lib.sa_launch_count.restype = ctypes.c_ulonglong
     lib.sa_selftest_wait_timeout.restype = i32
     lib.sa_selftest_wait_timeout.argtypes = [ctypes.c_uint, vp]
+    lib.sa_selftest_wait_tries.restype = i32
+    lib.sa_selftest_wait_tries.argtypes = [ctypes.c_uint, vp]
     lib.sa_backward_workspace_bytes.restype = sz
     lib.sa_backward_workspace_bytes.argtypes = [pp]
     lib.sa_backward.restype = i32
