@@ -15,6 +15,7 @@
 namespace sa {
 
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kSms = 148;            // streaming multiprocessors of a B200
 constexpr int kSimtCarryRows = 32;   // query rows per carry checkpoint, CUDA-core engine
 constexpr int kTcCarryRows = 128;    // tensor-core engine: one checkpoint per 128-query tile
 

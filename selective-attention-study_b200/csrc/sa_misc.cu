@@ -157,7 +157,7 @@ constexpr int kDecCtasPerSm = 4;              // attend CTAs resident per SM (48
 // Keys per CTA for `t` cached keys and `rows` = batch * heads query rows: the grid is about one full wave of
 // resident CTAs, so no SM is left with a straggler and the combine pass stays short.  With 512 keys at least, 96 rows of
 // 1,500 keys were 288 CTAs of three ring refills each and took 13.9 us; with 256 they fill the wave.
-static int decode_target_splits(int rows) { return max(1, min(tc::kSms * kDecCtasPerSm / rows, kDecSplitsMax)); }
+static int decode_target_splits(int rows) { return max(1, min(kSms * kDecCtasPerSm / rows, kDecSplitsMax)); }
 static int decode_split_keys(int t, int rows) {
   const int target_splits = decode_target_splits(rows);
   const int keys = (t + target_splits - 1) / target_splits;

@@ -770,7 +770,7 @@ int launch_backward(const Problem& p, const float* lse2, const float* carry, con
 // 235 us with one.  With more CTAs than that the SMs that finish early take the rest, and teams without a common barrier are
 // the faster ones: 292 + 540 against 328 + 588 us at (4, 8, 1000, 64), 192 + 345 against 209 + 363 us at (1, 12, 1280, 64).
 inline bool two_teams(const Problem& p) {
-  return (int64_t)p.batch * p.heads * ((p.seq + kQ - 1) / kQ) <= 2 * 148;
+  return (int64_t)p.batch * p.heads * ((p.seq + kQ - 1) / kQ) <= 2 * kSms;
 }
 
 template <typename T, int D>

@@ -31,18 +31,6 @@ __device__ __forceinline__ void init_bars(uint64_t* bars) {
   mbar_init_fence();
 }
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ float load_ahead(const float* p) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-
 // Which (row n = batch x head, key tile nj) a CTA takes.  Dense: one row after the other, key tile 0 (the longest
 // walk) first.  With a table of live tiles most walks are a few tiles long, except those of the key tiles that hold an
 // exempt key, which stay live for every query tile: all rows' key tile 0 go first so that the long walks start together.

@@ -9,20 +9,6 @@ namespace tc {
 
 constexpr int kMaxLiveTiles = 1024;   // key tiles of a sequence when dead tiles are left out (sa_tc_skip.cu)
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// A global load the compiler must issue where it is written (volatile asm keeps its place among the other
-// volatile asm statements), so a value fetched one step ahead is really in flight during that step.
-__device__ __forceinline__ float load_ahead(const float* p) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-
 struct ForwardMaps {                  // boxes of 128 rows x 64 columns
   CUtensorMap q, k, v, q0, k0;
 };

@@ -11,8 +11,6 @@
 namespace sa {
 namespace tc {
 
-constexpr int kSms = 148;             // streaming multiprocessors of a B200
-
 inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void* p = nullptr;
