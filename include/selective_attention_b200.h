@@ -324,9 +324,10 @@ int sa_decode_run(const sa_decode* d);
 
 /* A prompt, or a further chunk of one, for a decode cache (tensor-core engine; replaces mixers.py:105-113 around the
  * kernels).  p->seq counts the cached tokens and the new ones; q holds the queries from position `cached` on, k and v all
- * p->seq keys.  `selected` (batch, >= p->seq at selected_stride) is read where cached > 0 and receives the totals in place, after
- * everything else has been launched: a call that returns an error leaves it unchanged; y receives the new rows in the operand type.  carry, lse2, the table (may be NULL) and `scratch` are scratch; with
- * sa_prefill_scratch_bytes (0: not needed) of the last, a few rows after many keys are spread over the whole GPU (may be NULL). */
+ * p->seq keys.  `selected` (batch, >= p->seq at selected_stride) is read where cached > 0 and receives the totals in place; a
+ * call that returns an error leaves it as it was.  y receives the new rows in the operand type.  carry, lse2, the table (may be
+ * NULL) and `scratch` are scratch; with sa_prefill_scratch_bytes (0: not needed) of the last, a few rows after many keys are
+ * spread over the whole GPU (may be NULL). */
 size_t sa_prefill_scratch_bytes(const sa_problem* p, int cached);
 int sa_prefill_rows(const sa_problem* p, int cached, const void* q, const void* k, const void* v, float* selected,
                     int64_t selected_stride, const sa_tensor* y, float* lse2, float* carry, void* tile_table,

@@ -81,6 +81,7 @@ int to_problem(const sa_problem* in, const void* q, const void* k, const void* v
   p->total_stride = in->seq;
   p->tile_table = nullptr;
   p->split_scratch = nullptr;
+  p->history_moved = nullptr;
   p->out_lowp = nullptr;
   p->out_lowp_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
   p->dv_rows = contiguous_rows(in->heads, in->seq, in->head_dim);
@@ -603,19 +604,17 @@ int sa_prefill_rows(const sa_problem* in, int cached, const void* q, const void*
     p.split_scratch = static_cast<float*>(scratch);
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cached == 0) return tc_forward(p, nullptr, lse2, carry, selected, s);
-  // The history moves on last: a call that fails leaves it where the cache's length is.  The totals are the last row of carry.
-  const size_t seq = in->seq, pitch = (size_t)sa_carry_checkpoints(in->engine, in->seq) * seq;
-  st = tc_forward(p, nullptr, lse2, carry, nullptr, s);
-  if (st != SA_OK) return st;
-  const float* totals = carry + pitch - seq;
-  if (pitch * 4 < (1u << 31) && (size_t)selected_stride * 4 < (1u << 31)) {          // (the pitches that a 2-D copy takes)
-    SA_CUDA_CHECK(cudaMemcpy2DAsync(selected, selected_stride * 4, totals, pitch * 4, seq * 4, in->batch, cudaMemcpyDeviceToDevice, s));
-  } else {
+  // A call that fails leaves the history where the cache's length is: the scan, which writes the totals over what it has read,
+  // keeps that in the last row of carry, and where a launch after it is refused it is put back.
+  bool moved = false;
+  if (cached > 0) p.history_moved = &moved;
+  st = tc_forward(p, nullptr, lse2, carry, selected, s);
+  if (st != SA_OK && moved) {
+    const size_t seq = in->seq, pitch = (size_t)sa_carry_checkpoints(in->engine, in->seq) * seq;
     for (int b = 0; b < in->batch; ++b)
-      SA_CUDA_CHECK(cudaMemcpyAsync(selected + b * selected_stride, totals + b * pitch, seq * 4, cudaMemcpyDeviceToDevice, s));
+      SA_CUDA_CHECK(cudaMemcpyAsync(selected + b * selected_stride, carry + (b + 1) * pitch - seq, seq * 4, cudaMemcpyDeviceToDevice, s));
   }
-  return SA_OK;
+  return st;
 }
 
 int sa_cache_store(int dtype, int batch, int heads, int groups, int seq, int capacity, int head_dim, int at, int begin,

@@ -70,6 +70,7 @@ struct Problem {
   // Tensor-core engine, optional: the table of live (query tile, key tile) pairs (sa_tc_skip.cu).  The forward
   // fills it after its selection pass and leaves out the dead tiles; the backward of the same call reads it.
   void* tile_table;      // null: every causal tile is computed
+  bool* history_moved;   // not null: the last row of carry gets the history as it was read, and this is set once it is overwritten
   float* split_scratch;  // null: a query tile's keys are one walk (else prefill_split_pieces of them)
 };
 

@@ -156,13 +156,14 @@ __global__ void __launch_bounds__(kColsumThreads) colsum_kernel(const __grid_con
 // and total[b][j] receive the sum over all query tiles.  Only rows mi >= j / 128 exist.
 __global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, float* total, int64_t total_stride, int seq,
                                                    int ntiles, int mi_first, const float* init,
-                                                   int64_t init_stride, unsigned int* tickets, int n_tickets) {
+                                                   int64_t init_stride, bool keep_init, unsigned int* tickets, int n_tickets) {
   if (blockIdx.x == 0 && blockIdx.y == 0 && (int)threadIdx.x < n_tickets) tickets[threadIdx.x] = 0u;   // of a split forward
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (j >= seq) return;
   float* col = carry + (int64_t)b * (ntiles + 1) * seq + j;
-  float run = init ? init[(int64_t)b * init_stride + j] : 0.f;   // what the key received before the first query given
+  const float before = init ? init[(int64_t)b * init_stride + j] : 0.f;   // what the key received before the first query given
+  float run = before;
   int mi = max(j / kTile, mi_first);
   for (; mi + 8 <= ntiles; mi += 8) {
     float x[8];
@@ -179,8 +180,8 @@ __global__ void __launch_bounds__(256) scan_kernel(float* __restrict__ carry, fl
     col[(int64_t)mi * seq] = run;
     run += x;
   }
-  col[(int64_t)ntiles * seq] = run;
-  if (total != nullptr) total[(int64_t)b * total_stride + j] = run;
+  col[(int64_t)ntiles * seq] = keep_init ? before : run;
+  total[(int64_t)b * total_stride + j] = run;                    // (a continued prefill: where `init` was)
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -758,9 +759,10 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
     ProfileScope prof(SA_KERNEL_TC_SCAN, s);
     count_launch();
     scan_kernel<<<gs, 256, 0, s>>>(carry, total, p.total_stride, p.seq, ntiles, mi_first, p.carry_init, p.carry_init_stride,
-                                    split.tickets, pieces > 1 ? kSplitTickets : 0);
+                                    p.history_moved != nullptr, split.tickets, pieces > 1 ? kSplitTickets : 0);
   }
   SA_CUDA_CHECK(cudaGetLastError());
+  if (p.history_moved != nullptr) *p.history_moved = true;
 
   const uint8_t* alive = nullptr;
   if (p.tile_table != nullptr && ntiles <= kMaxLiveTiles) {
