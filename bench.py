@@ -647,7 +647,7 @@ def run_decode(args, w, rank, world, device):
             "e2e": {"value": world * b / (results[True] * 1e-3), "unit": "tokens/s", "ms_per_step": results[True],
                     "h2d_bytes_per_step": 3 * b * h * d * 2, "d2h_bytes_per_step": b * h * d * 4},
             "gpu_launches": launches,
-            "roofline": {"bound": "hbm", "kernel": "decode step (append, attend, combine, update)",
+            "roofline": {"bound": "hbm", "kernel": "decode step (one kernel: append, attend, combine, update)",
                          "achieved": None if live else achieved, "peak": hbm_peak, "peak_kind": hbm_kind, "unit": "GB/s",
                          "frac": None if live else achieved / hbm_peak, "traffic": None,
                          **({"note": "no byte count is claimed when dead keys are left out"} if live else {})},

@@ -34,12 +34,14 @@
 // first form of this kernel, with 45 KB of loops, ran at 15.5 k cycles a tile; hence the compact waits (Waiter), rolled MMA
 // loops over halves (the order is the same for both chains), low words of descriptors, 32-bit shared addresses.
 // Measured at B = 4, H = 16, T = 16384: 16.6 ms with sixteen warps in lock step, 12.1 ms with two chains and one MMA warp,
-// 10.3 ms (5.0 k cycles a tile) with three (SELF: 12.3, 8.7, 8.0).
+// 10.3 ms (5.4 k cycles a tile) with three (SELF: 12.3, 8.7, 8.0).
 //
 // SELF variant (one head per selector, i.e. the per-head form reshaped to (B H, 1, T, D)): the selection logits are the
 // head's own logits, so S^T serves as L0^T (read twice), and since Q0 = Q and K0 = K the two gradient paths add before the
 // MMAs: dK += (dz + g)^T Q and dQ = (dz + g) K, with (dz + g)^T in W1.  40 MMAs per query tile instead of 64, no Q0 / K0
 // tiles, and the columns of dK0 hold K and V as bf16 pairs (A of the score products, 64 KB less shared-memory traffic).
+// It moves 240 KB a tile (score operands 32, dV, dK 32, dQ 48, dz + g 32, staged and reduced 64, loads 32), 1.9 k of its 4.2 k
+// cycles; the tensor pipe is busy 32 % of them, the issue slots 60 %.  What bounds it has not been found.
 //
 // The diagonal tile, the only one that needs the causal mask inside the tile, is the LAST tile of a CTA's walk: the loop
 // holds the unmasked form only and the masked form runs once after it.  LIVE: with a table of live tiles (sa_tc_skip.cu)

@@ -16,8 +16,9 @@
 // the statistics (one head per selector: no K0 and Q0, three slots of (Q, dO)).  What a half frees at its dz takes what the
 // chain's next half needs first (Q0, Q), what it frees at g the rest (dO): no load is waited for.
 //
-// What bounds it: shared memory, 560 KB a CTA and 128 x 128 tile = 4.4 k cycles (score operands 288, dQ^T operands 96, loads
-// 96, B operands of the accumulators 48, dz or g written 32); a tile takes ~5.6 k.  Measured at B = 2, H = 8, T = 4097: 817 us
+// What bounds it: shared memory, 688 KB a CTA and 128 x 128 tile = 5.5 k cycles (score operands 288, dQ^T staged and reduced 128,
+// its operands 96, loads 96, B operands of the accumulators 48, dz or g written 32); a tile takes 6.4 k (one head per
+// selector 4.9 k).  Measured at B = 2, H = 8, T = 4097: 817 us
 // with sixteen warps in lock step and reductions from registers, 553 us.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:196-268 (one head), :271-364 (the shared

@@ -16,7 +16,8 @@
 //                   the exponentials.  head_dim 128, and head_dim 64 where two heads a CTA would leave SMs idle; few rows
 //                   after many cached keys: a piece of the walk each, merged by the CTA that finishes last.
 //                   Bound by the chain of a step (L0, selection, running sum, maximum over four warpgroups, exponentials,
-//                   P V): 3.2 k cycles at head_dim 64, 5.3 k at 128, of which the tensor pipe needs 0.8 k and 1.1 k.
+//                   P V): 3.1 k cycles at head_dim 64, 3.7 k at 128 (one head per selector, whose single K tile is waited
+//                   for: 5.0 k), counted over T = 16384; the tensor pipe is busy 57 % of them at 128.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:100-194 (selection, carry, forward).
 #include <float.h>
@@ -772,7 +773,7 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
   }
   const bool self = self_selecting(p);
   // Heads that share a selector go two to a CTA: its selection is made once and the two overlap (1.3x a head-tile).  While
-  // one head a CTA still fits the GPU in one wave, that is faster: a step of it takes 3.2 k cycles, of a pair 4.3 k.
+  // one head a CTA still fits the GPU in one wave, that is faster: a step of it takes 3.1 k cycles, of a pair 4.4 k.
   const int64_t ctas = (int64_t)(ntiles - mi_first) * p.batch * p.heads;
   if (D == 64 && !self && p.heads % 2 == 0 && ctas > kSms) return forward_pair(p, m, carry, out, lse2, status, alive, s);
   if (D == 64 && self && p.batch % 2 == 0 && ctas > kSms) return forward_self(p, m, carry, out, lse2, status, alive, s);

@@ -15,7 +15,7 @@
 // heads (64 each).  Shared memory, 224 KB: Q, Q of the two heads and Q0 48 KB, TRI 32, selection 32, K and V rings of three
 // tiles 48 each (the heads alternate), K0 16.
 //
-// What bounds it: latency around F.  The step of both heads takes 3.9 k cycles: F read by both -> L0 -> selection -> running
+// What bounds it: latency around F.  The step of both heads takes 4.4 k cycles: F read by both -> L0 -> selection -> running
 // sum -> F read by both is a chain of hand-overs, and a head's own chain is as long (S after P V of the step before 1.2 k, read
 // 0.8 k, 128 exponentials a thread 1.5 k).  The exponential unit (16 ex2 a clock and SM) needs 2.0 k of them and is busy 48 % of
 // the time, the tensor pipe 41 %, the issue slots 42 %.  TMEM is full, so neither S nor F can have a second buffer; S in two halves

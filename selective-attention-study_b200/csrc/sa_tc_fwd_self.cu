@@ -15,8 +15,9 @@
 // TMEM, 512 columns: S x 3 (P as bf16 pairs over the first 64 of each) | O of the two rows (64 each).  Shared memory, 224 KB: Q
 // 32, TRI 32, selection 2 x 32, K and V rings of three tiles 48 each.
 //
-// What bounds it: the latency of a tile over three tiles in flight, ~5 k cycles (S 0.4, selection 1.0, running sum 0.7, softmax
-// 2.6, P V 0.5); the exponential unit needs 1.0 k a tile, the tensor pipe 1.0 k.  Measured at 64 rows of T = 16384: 4.21 ms
+// What bounds it: the latency of a tile over three tiles in flight (S 0.4 k cycles, selection 1.0, running sum 0.7, softmax 2.6,
+// P V 0.5, and the waits between them: a tile takes 2.2 k of the CTA's time, so its columns are in use for 6.5 k); the
+// exponential unit needs 1.0 k a tile, the tensor pipe 1.0 k, neither is busy half of the time.  Measured at 64 rows of T = 16384: 4.21 ms
 // (forward_wide_kernel, one row a CTA in lock step: 5.77 ms).
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:140-194; per-head form: mixers.py:76-98.
