@@ -103,6 +103,12 @@ Tensor bytes_on(const Tensor& like, size_t n) {
   return at::empty({(int64_t)std::max<size_t>(n, 1)}, like.options().dtype(at::kByte));
 }
 
+// A saved scratch as it comes back: a hook on saved tensors may have put its bytes anywhere, the kernels read floats.
+Tensor unpacked(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 256 == 0 ? c : c.clone();
+}
+
 Tensor run_forward(const sa_problem& p, const Tensor& q, const Tensor& k, const Tensor& v, const Scratch& at_, const Tensor& scratch,
                    const sa_tensor* low) {
   Tensor out = at::empty({p.batch, p.heads, p.seq, p.head_dim}, q.options().dtype(at::kFloat));
@@ -194,7 +200,7 @@ struct Attend : public torch::autograd::Function<Attend> {
       d_out = d_out.contiguous();
       if (reinterpret_cast<uintptr_t>(d_out.data_ptr()) % 16 != 0) d_out = d_out.clone();
       const Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(q.sizes(), q.options()), dv = at::empty(q.sizes(), q.options());
-      run_backward(p, q, k, v, saved[3], at_, saved[4], d_out, dq, dk, dv);
+      run_backward(p, q, k, v, saved[3], at_, unpacked(saved[4]), d_out, dq, dk, dv);
       const Tensor* all[3] = {&dq, &dk, &dv};
       for (int i = 0; i < 3; ++i) {
         const auto want = (at::ScalarType)args[3 + i];
@@ -242,7 +248,7 @@ struct AttendPacked : public torch::autograd::Function<AttendPacked> {
       if (reinterpret_cast<uintptr_t>(d_out.data_ptr()) % 16 != 0) d_out = d_out.clone();
       d_out = d_out.view({b, t, h, d}).transpose(1, 2);
       const Tensor d_qkv = at::empty(qkv.sizes(), qkv.options());
-      run_backward(p, q, k, v, saved[1], at_, saved[2], d_out, part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2));
+      run_backward(p, q, k, v, saved[1], at_, unpacked(saved[2]), d_out, part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2));
       grads[0] = d_qkv;
     }
     return once_differentiable(grad_out, std::move(grads));

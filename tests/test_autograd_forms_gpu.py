@@ -70,6 +70,28 @@ def test_saved_tensors_may_be_moved():
         assert float((a.float() - b.float()).norm() / b.float().norm()) < 2e-3
 
 
+@pytest.mark.parametrize("call,dtype,dim", [(_plain, torch.bfloat16, 64), (_plain, torch.float32, 32), (_packed, torch.bfloat16, 64)])
+def test_saved_bytes_may_come_back_at_any_address(call, dtype, dim):
+    """A hook that keeps saved bytes one byte into a buffer of its own: the statistics among them are floats."""
+    x = [t.requires_grad_(True) for t in _inputs(7, dim=dim, dtype=dtype)]
+    want = torch.autograd.grad(call(*x).sum(), x)
+
+    def pack(t):
+        if t.dtype != torch.uint8:
+            return t
+        flat = torch.empty(t.numel() + 1, dtype=torch.uint8, device=t.device)
+        flat[1:] = t
+        return flat
+
+    def unpack(t):
+        return t[1:] if t.dtype == torch.uint8 else t
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        out = call(*x)
+    for a, b in zip(torch.autograd.grad(out.sum(), x), want):
+        assert float((a.float() - b.float()).norm() / b.float().norm()) < 2e-3
+
+
 @pytest.mark.parametrize("call", [_plain, _layer, _packed])
 def test_gradients_kept_for_a_graph_are_constants_where_the_cotangent_is_one(call):
     """create_graph with a cotangent that has no graph: the gradients are plain tensors, and what is built on them can be
