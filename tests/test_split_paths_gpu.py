@@ -61,6 +61,33 @@ def test_two_heads_a_cta_in_a_continued_prefill_and_in_bf16(per_head):
         assert _rel(a, b.float().cpu()) < 2e-3
 
 
+@pytest.mark.parametrize("skip", [False, True])
+def test_two_heads_a_cta_with_an_outside_selector_and_in_place_in_a_projection(skip):
+    """More than 148 pairs in every call: two halves of the heads with a replica of the selecting head, and the heads where a
+    fused projection left them, against the plain call."""
+    heads, seq = 80, 600
+    q, k, v, w = (x.cuda() for x in _inputs(1, heads, seq, 64, 1.0, 13))
+    x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    whole = kernels.selective_attention(*x)
+    want = torch.autograd.grad(whole, x, w.float())
+    q0, k0 = (t[:, 0].clone().requires_grad_(True) for t in (q, k))
+    halves = [[t[:, s].clone().requires_grad_(True) for t in (q, k, v)] for s in (slice(0, 40), slice(40, 80))]
+    outs = [kernels.selective_attention(*part, selector=(q0, k0), skip_dead_tiles=skip) for part in halves]
+    assert torch.equal(torch.cat(outs, dim=1), whole)
+    grads = torch.autograd.grad(outs, [*halves[0], *halves[1], q0, k0], [w[:, :40].float(), w[:, 40:].float()])
+    for i in range(3):
+        got = torch.cat([grads[i], grads[3 + i]], dim=1).float()
+        if i < 2:
+            got[:, 0] += grads[6 + i].float()
+        assert _rel(got, want[i].float().cpu()) < 1e-2
+    qkv = torch.stack([t.transpose(1, 2) for t in (q, k, v)], dim=2).requires_grad_(True)
+    y = kernels.selective_attention_packed(qkv, skip_dead_tiles=skip)
+    assert torch.equal(y, whole.detach().bfloat16().transpose(1, 2).reshape(y.shape))
+    (dqkv,) = torch.autograd.grad(y, qkv, w.transpose(1, 2).reshape(y.shape))
+    for i in range(3):
+        assert _rel(dqkv[:, :, i].transpose(1, 2), want[i].float().cpu()) < 2e-3
+
+
 def test_a_second_differentiation_raises():
     q, k, v, _ = (x.cuda().requires_grad_(True) for x in _inputs(1, 2, 70, 64, 1.0, 3))
     out = kernels.selective_attention(q, k, v)
