@@ -17,7 +17,8 @@
 //                   after many cached keys: a piece of the walk each, merged by the CTA that finishes last.
 //                   Bound by the chain of a step (L0, selection, running sum, maximum over four warpgroups, exponentials,
 //                   P V): 3.1 k cycles at head_dim 64, 3.7 k at 128 (one head per selector, whose single K tile is waited
-//                   for: 5.0 k), counted over T = 16384; the tensor pipe is busy 57 % of them at 128.
+//                   for: 5.0 k), counted over T = 16384 with the split walk in the same
+//                   kernel (it is 1 to 5 % shorter without); the tensor pipe is busy 57 % of them at 128.
 //
 // Reference for the arithmetic: src/selective_attention/kernels.py:100-194 (selection, carry, forward).
 #include <float.h>
@@ -240,7 +241,9 @@ struct SplitWalk {
   float *part, *lse;
 };
 
-template <int D, bool SELF, bool LIVE>   // LIVE: a table of live key tiles is given and the dead ones are left out
+// LIVE: a table of live key tiles is given and the dead ones are left out.  SPLIT: more than one piece; walks of one piece have
+// a kernel without the other code, which took 5 % longer with it (15 heads of T = 16384, head_dim 64: 1.41 -> 1.37 ms).
+template <int D, bool SELF, bool LIVE, bool SPLIT>
 __global__ void __launch_bounds__(kWideThreads, 1)
     forward_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q0,
@@ -257,15 +260,16 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   constexpr bool kTmemAB = (D == 64);
   constexpr uint32_t kColTri = 384, kColP = 448;
 
-  const int piece = (int)blockIdx.x % split.pieces, cta = (int)blockIdx.x / split.pieces;
-  const int nrows = gridDim.x / split.pieces / (ntiles - q_offset / kTile);  // batch * heads (the grid covers the query tiles with rows to compute)
+  const int pieces = SPLIT ? split.pieces : 1;
+  const int piece = SPLIT ? (int)blockIdx.x % pieces : 0, cta = SPLIT ? (int)blockIdx.x / pieces : (int)blockIdx.x;
+  const int nrows = gridDim.x / pieces / (ntiles - q_offset / kTile);  // batch * heads (the grid covers the query tiles with rows to compute)
   const int mi = ntiles - 1 - cta / nrows;                    // heaviest query tiles first
   const int n = cta % nrows;
   const int b = n / heads, h = n - b * heads;
   const int i0 = mi * kTile;
   // this piece's key tiles: last, last - 1, .. lowest (the last pieces may have none)
-  const int piece_tiles = (mi + split.pieces) / split.pieces;
-  const int last = mi - piece * piece_tiles, lowest = max(0, last - piece_tiles + 1);
+  const int piece_tiles = SPLIT ? (mi + pieces) / pieces : mi + 1;
+  const int last = mi - piece * piece_tiles, lowest = SPLIT ? max(0, last - piece_tiles + 1) : 0;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -321,27 +325,40 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   auto key_tile = [&](int it) { return LIVE ? (it < steps ? (int)live_s[it] : 0) : last - it; };
   const int q_rows = seq - q_offset;
 
-  if (steps <= 0) {                                            // a piece without keys
+  if (SPLIT && steps <= 0) {                                   // a piece without keys
     if (tid < kTile && i0 + tid < seq && i0 + tid >= q_offset)
       split.lse[((int64_t)piece * nrows + n) * q_rows + i0 + tid - q_offset] = -INFINITY;
   } else if (warp == kWideCompute / 32) {
     // =============================== control warp: TMA loads and MMA issue ===============================
-    // The warp stays converged and one elected lane issues: inside a divergent branch an MMA took about 75 cycles to issue.
+    // The warp stays converged and one elected lane issues: inside a divergent branch an MMA took about 75 cycles to issue.  One
+    // head per selector issues fewer MMAs and waits at as many places: a single lane that polls is the faster there (15 rows of
+    // T = 16384 at head_dim 128 2.20 ms, converged 2.23; 5 rows of 1,000 at 64 22.7 us, converged 23.4).
+    constexpr bool kOneLane = SELF;
     Waiter wait;
-    wait.begin(status);
+    if (!kOneLane) wait.begin(status);
+    auto elected = [&] { return kOneLane || elect_one(); };
+    auto converge = [&] { if (!kOneLane) __syncwarp(); };
+    if (!kOneLane || lane == 0) {
     // A tile of step it lives in stage slot(it); the j-th fill of a stage completes its barrier's phase j.
     auto slot = [](int it) { return ST == 2 ? (it & 1) : 0; };
     auto fill = [](int it) { return (uint32_t)((ST == 2 ? (it >> 1) : it) & 1); };
-    auto await = [&](uint64_t* bar, uint32_t parity, int site) { wait.left = wait_call(smem_u32(bar), parity, site, wait.left); };
+    auto await = [&](uint64_t* bar, uint32_t parity, int site) {
+      if (kOneLane) {
+        mbar_wait(bar, parity, status, site);
+        tc_fence_after_sync();
+      } else {
+        wait.left = wait_call(smem_u32(bar), parity, site, wait.left);
+      }
+    };
     auto load_tile = [&](int off, const CUtensorMap* map, uint64_t* bars, int it, int head) {
       const int j0 = key_tile(it) * kTile;
-      if (elect_one()) {
+      if (elected()) {
         uint64_t* bar = &bars[slot(it)];
         mbar_expect_tx(bar, L::kTileBytes);
         for (int s2 = 0; s2 < DK; ++s2)
           tma_load_4d(smem + off + slot(it) * L::kTileBytes + s2 * kRowTile, map, bar, s2 * 64, j0, head, b);
       }
-      __syncwarp();
+      converge();
     };
     auto load_k = [&](int it) { load_tile(L::k, &map_k, bar_k, it, h); };
     auto load_k0 = [&](int it) { if (!SELF) load_tile(L::k0, &map_k0, bar_k0, it, 0); };   // SELF: K0 is K
@@ -355,18 +372,18 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     auto kstep = [](int ks) { return (uint32_t)((ks >> 2) * kRowTile + (ks & 3) * 32); };
     auto issue_l0 = [&](int it) {                              // L0 = Q0 K0^T
       await(SELF ? &bar_k[slot(it)] : &bar_k0[slot(it)], fill(it), 311);
-      if (elect_one()) {
+      if (elected()) {
         const uint32_t tile = at(kBase, (SELF ? L::k : L::k0) + slot(it) * L::kTileBytes);
 #pragma unroll
         for (int ks = 0; ks < 4 * DK; ++ks)
           mma_ts_low(tmem + kColL, tmem + (SELF ? kColQ : kColQ0) + ks * 8, at(tile, kstep(ks)), idesc_s, ks > 0);
         mma_commit(&bar_l0);
       }
-      __syncwarp();
+      converge();
     };
     auto issue_s_tri = [&](int it) {                           // S = Q K^T, then S -= TRI x selection
       await(&bar_k[slot(it)], fill(it), 312);
-      if (elect_one()) {
+      if (elected()) {
         const uint32_t tile = at(kBase, L::k + slot(it) * L::kTileBytes);
 #pragma unroll
         for (int ks = 0; ks < 4 * DK; ++ks) mma_ts_low(tmem + kColS, tmem + kColQ + ks * 8, at(tile, kstep(ks)), idesc_s, ks > 0);
@@ -377,11 +394,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         }
         mma_commit(&bar_tri);
       }
-      __syncwarp();
+      converge();
     };
     auto issue_pv = [&](int it, uint64_t* bar) {               // O += P V
       await(&bar_v[slot(it)], fill(it), 315);
-      if (elect_one()) {
+      if (elected()) {
         const uint32_t v = at(mBase, L::v + slot(it) * L::kTileBytes);
         const uint32_t more = it > 0 ? 1u : 0u;
 #pragma unroll
@@ -393,17 +410,17 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         }
         mma_commit(bar);
       }
-      __syncwarp();
+      converge();
     };
 
-    if (elect_one()) {
+    if (elected()) {
       mbar_expect_tx(&bar_q, (SELF ? 1 : 2) * DK * kRowTile);
       for (int s2 = 0; s2 < DK; ++s2) {
         tma_load_4d(smem + L::q + s2 * kRowTile, &map_q, &bar_q, s2 * 64, i0 - q_offset, h, b);
         if (!SELF) tma_load_4d(smem + L::q0_landing + s2 * kRowTile, &map_q0, &bar_q, s2 * 64, i0 - q_offset, 0, b);
       }
     }
-    __syncwarp();
+    converge();
     load_k0(0);
     load_k(0);
     load_v(0);
@@ -439,7 +456,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     }
     await(&bar_p, (steps - 1) & 1, 322);
     issue_pv(steps - 1, &bar_fin);
-    if (lane == 0) wait.end(status);
+    if (!kOneLane && lane == 0) wait.end(status);
+    }
+    __syncwarp();
   } else {
     // ======================================= arithmetic warps ============================================
     const int row = tid & 127, wg = tid >> 7;
@@ -647,7 +666,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     tmem_ld_wait();
     if (i < seq && i >= q_offset) {                            // rows before q_offset belong to an earlier call
       const int iq = i - q_offset;                             // row inside the query tensor
-      const bool whole = split.pieces == 1;
+      constexpr bool whole = !SPLIT;
       const int64_t nr = ((int64_t)piece * nrows + n) * q_rows + iq;
       float* rows_to = whole ? out : split.part;
       if (rows_to != nullptr) {
@@ -669,13 +688,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       }
     }
   }
-  if (split.pieces > 1) __threadfence();
+  if (SPLIT) __threadfence();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
-  if (split.pieces == 1) return;
+  if constexpr (!SPLIT) return;
   // The CTA that finishes last merges the pieces of its 128 rows, D / 8 threads a row.
-  if (tid == 0) last_s = atomicAdd(split.tickets + cta, 1u) == (unsigned)split.pieces - 1;
+  if (tid == 0) last_s = atomicAdd(split.tickets + cta, 1u) == (unsigned)pieces - 1;
   __syncthreads();
   if (!last_s || tid >= kWideCompute) return;
   __threadfence();
@@ -686,9 +705,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     if (iq < 0 || iq >= q_rows) continue;
     const int64_t at = (int64_t)n * q_rows + iq;
     float top = -INFINITY;
-    for (int s2 = 0; s2 < split.pieces; ++s2) top = fmaxf(top, __ldcg(split.lse + s2 * stride + at));
+    for (int s2 = 0; s2 < pieces; ++s2) top = fmaxf(top, __ldcg(split.lse + s2 * stride + at));
     float acc[8] = {}, den = 0.f;
-    for (int s2 = 0; s2 < split.pieces; ++s2) {
+    for (int s2 = 0; s2 < pieces; ++s2) {
       const float l = __ldcg(split.lse + s2 * stride + at);
       if (l == -INFINITY) continue;                            // no keys, and no rows written
       const float w = ex2(l - top);
@@ -789,8 +808,14 @@ int forward_impl(const Problem& p, float* out, float* lse2, float* carry, float*
                                                  p.q_offset, alive, split);
     return SA_OK;
   };
-  if (alive != nullptr) st = self ? launch(forward_wide_kernel<D, true, true>) : launch(forward_wide_kernel<D, false, true>);
-  else st = self ? launch(forward_wide_kernel<D, true, false>) : launch(forward_wide_kernel<D, false, false>);
+  auto by_split = [&](auto self_tag, auto live_tag) {
+    constexpr bool kSelf = decltype(self_tag)::value, kLive = decltype(live_tag)::value;
+    return pieces > 1 ? launch(forward_wide_kernel<D, kSelf, kLive, true>) : launch(forward_wide_kernel<D, kSelf, kLive, false>);
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  if (alive != nullptr) st = self ? by_split(yes, yes) : by_split(no, yes);
+  else st = self ? by_split(yes, no) : by_split(no, no);
   if (st != SA_OK) return st;
   SA_CUDA_CHECK(cudaGetLastError());
   return SA_OK;
